@@ -237,7 +237,7 @@ struct glu_handle_s {
     DevBuf d_src_lu, d_src_scale, d_a0_rptr, d_a0_cidx, d_a0_vmap, d_a0_cptr, d_a0_ridx, d_a0_ident, d_ax0;
     bool ax0_loaded = false;
     // work buffers
-    DevBuf d_status, d_pert, d_colmax, d_diag_scratch, d_counters, d_ticket, d_flags, d_y, d_io32, d_b64,
+    DevBuf d_status, d_pert, d_colmax, d_diag_scratch, d_counters, d_ticket, d_dense_tickets, d_y, d_io32, d_b64,
         d_x64, d_r64, d_norms;
     uint32_t *h_status = nullptr;  // pinned
     double *h_norms = nullptr;     // pinned
@@ -1084,6 +1084,7 @@ Status create_handle(int device, SymbolicData &&s, uint32_t batch, glu_handle_t 
     GLU_CUDA(h->d_diag_scratch.alloc(sizeof(float) * kDenseNB * kDenseNB * batch), "allocate");
     GLU_CUDA(h->d_counters.alloc(sizeof(uint32_t) * (size_t(h->n) + 64)), "allocate");
     GLU_CUDA(h->d_ticket.alloc(256), "allocate");
+    GLU_CUDA(h->d_dense_tickets.alloc(sizeof(uint32_t) * 2), "allocate");
     GLU_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h->h_status), 256), "allocate pinned");
     GLU_CUDA(cudaEventCreate(&h->ev0), "event");
     GLU_CUDA(cudaEventCreate(&h->ev1), "event");
@@ -1204,14 +1205,21 @@ SolvePlanDev solve_plan(glu_handle_s *h) {
     return S;
 }
 
+// The buffer of finished unknowns of a solve over nvec vectors, and what the
+// solve's input transform writes for the dense tail sweeps.
+Status solve_buffers(glu_handle_s *h, size_t nvec, SolveInit *init) {
+    GLU_CUDA(h->d_xo.ensure(sizeof(float) * size_t(h->n) * nvec), "allocate solve buffer");
+    *init = h->m ? SolveInit{h->d_xo.as<float>(), h->t, h->d_dense_tickets.as<uint32_t>()} : SolveInit{};
+    return GLU_OK;
+}
+
 // One FP32 solve of y in place (nrhs vectors of n per value set), in the
-// permuted system, with the factors of value sets [z, z + count).
+// permuted system, with the factors of value sets [z, z + count); after the
+// input transform with solve_buffers' SolveInit.
 Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint32_t nrhs, bool trans,
                      cudaStream_t st) {
-    const uint32_t nb = (h->m + 63) / 64 + 1;
-    GLU_CUDA(h->d_flags.ensure(sizeof(uint32_t) * size_t(nb) * count), "allocate solve flags");
-    GLU_CUDA(h->d_ticket.ensure(sizeof(uint32_t) * std::max<size_t>(count, 64)), "allocate solve flags");
-    uint32_t *cnt = h->d_flags.as<uint32_t>();
+    GLU_CUDA(h->d_ticket.ensure(sizeof(uint32_t) * std::max<size_t>(count, 64)), "allocate solve tickets");
+    uint32_t *cnt = h->d_dense_tickets.as<uint32_t>();
     uint32_t *tk = h->d_ticket.as<uint32_t>();
     uint32_t *status = h->d_status.as<uint32_t>();
     const float *val = h->d_val.as<float>() + size_t(z) * h->nnz;
@@ -1226,7 +1234,6 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
         GLU_CUDA(h->d_sweep_done.ensure(sizeof(uint32_t) * ns * count + 4), "allocate sweep counters");
         B.sweep_done = h->d_sweep_done.as<uint32_t>();
     }
-    GLU_CUDA(h->d_xo.ensure(sizeof(float) * size_t(h->n) * nrhs * count), "allocate solve buffer");
     float *xo = h->d_xo.as<float>();
     const SolvePlanDev S = solve_plan(h);
     h->stats.solve_launches += solve_kernel_count(h, trans);
@@ -1262,13 +1269,16 @@ Status solve_f32(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const float *b, 
     GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
     const TransformDev &T = h->T;
     h->stats.solve_launches = 2;  // the two transforms; solve_inplace adds the sweeps
+    SolveInit init;
+    Status s = solve_buffers(h, nrhs, &init);
+    if (s != GLU_OK) return s;
     GLU_CUDA(launch_transform_f32(trans ? T.tin_idx : T.in_idx, trans ? T.tin_scale : T.in_scale, bin, y,
-                                  h->n, nrhs, st), "transform");
-    Status s = solve_inplace(h, inst, 1, y, nrhs, trans, st);
+                                  h->n, nrhs, init, st), "transform");
+    s = solve_inplace(h, inst, 1, y, nrhs, trans, st);
     if (s != GLU_OK) return s;
     float *xout = (where == GLU_HOST) ? io : x;
     GLU_CUDA(launch_transform_f32(trans ? T.tout_idx : T.out_idx, trans ? T.tout_scale : T.out_scale, y,
-                                  xout, h->n, nrhs, st), "transform");
+                                  xout, h->n, nrhs, SolveInit{}, st), "transform");
     if (where == GLU_HOST)
         GLU_CUDA(cudaMemcpyAsync(x, io, sizeof(float) * len, cudaMemcpyDeviceToHost, st), "copy x");
     uint32_t flags = 0;
@@ -1300,7 +1310,8 @@ Status solve_f32_scratch(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const fl
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
     const TransformDev &T = h->T;
-    GLU_CUDA(launch_transform_f32(T.in_idx, T.in_scale, b, y, h->n, nrhs, st), "transform");
+    const SolveInit init = h->m ? SolveInit{xo, h->t, flags} : SolveInit{};
+    GLU_CUDA(launch_transform_f32(T.in_idx, T.in_scale, b, y, h->n, nrhs, init, st), "transform");
     const float *val = h->d_val.as<float>() + size_t(inst) * h->nnz;
     const float *dval = h->dense_buffer ? h->d_dense.as<float>() + size_t(inst) * h->m * h->m : val;
     uint32_t *status = h->d_status.as<uint32_t>();
@@ -1309,7 +1320,7 @@ Status solve_f32_scratch(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const fl
     one.dinv = h->m ? h->d_dinv.as<float>() + size_t(inst) * dinv_per_set(h) : nullptr;
     GLU_CUDA(solve_lower_unit(h->P, S, val, dval, y, xo, nrhs, flags, ticket, status, one, st), "lower solve");
     GLU_CUDA(solve_upper(h->P, S, val, dval, y, xo, nrhs, flags, ticket, status, one, st), "upper solve");
-    GLU_CUDA(launch_transform_f32(T.out_idx, T.out_scale, y, x, h->n, nrhs, st), "transform");
+    GLU_CUDA(launch_transform_f32(T.out_idx, T.out_scale, y, x, h->n, nrhs, SolveInit{}, st), "transform");
     uint32_t fl = 0;
     Status s = read_status(h, st, &fl);
     if (s != GLU_OK) return s;
@@ -2008,10 +2019,13 @@ Status refine_solve(RefineJob &j, const double *src, int accumulate) {
     const TransformDev &T = h->T;
     float *y = h->d_y.as<float>();
     h->stats.solve_launches += 2;  // the two transforms
+    SolveInit init;
+    Status s = solve_buffers(h, j.nvec, &init);
+    if (s != GLU_OK) return s;
     GLU_CUDA(launch_transform_f64_to_f32(j.tr ? T.tin_idx : T.in_idx, j.tr ? T.tin_scale : T.in_scale, src, y, h->n,
-                                         j.nvec, j.st),
+                                         j.nvec, init, j.st),
              "transform");
-    Status s = solve_inplace(h, j.first, j.count, y, j.nrhs, j.tr, j.st);
+    s = solve_inplace(h, j.first, j.count, y, j.nrhs, j.tr, j.st);
     if (s != GLU_OK) return s;
     GLU_CUDA(launch_transform_f32_to_f64_add(j.tr ? T.tout_idx : T.out_idx, j.tr ? T.tout_scale : T.out_scale, y,
                                              j.xz, h->n, j.nvec, accumulate, j.st),

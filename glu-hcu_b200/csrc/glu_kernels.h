@@ -272,7 +272,7 @@ struct SolvePlanDev {
     uint32_t cluster;               // CTAs of the thin-level cluster kernel
     uint32_t spin_limit;            // polls of a device-side wait before it gives up
     uint32_t ticket_base;           // first block ticket of the dense sweeps (0; 1 leaves the first
-                                    // block's flag unset: a diagnostic of the bounded waits)
+                                    // block unsolved: a diagnostic of the bounded waits)
 };
 
 // Supernodal sweep over the columns [0, t) (forward L, or backward U), then
@@ -296,30 +296,41 @@ struct TransformDev {
 };
 
 constexpr uint32_t kSolveChainThreads = 512;
+// An entry of the dense tail that its sweep has not solved yet.
+constexpr uint32_t kUnsolved = 0xFFFFFFFFu;
+// Written by the input transform of a solve for the dense tail sweeps: entries
+// [t, n) of every vector of xo as kUnsolved, the two block tickets zero.
+struct SolveInit {
+    float *xo = nullptr;  // null: nothing (a solve's output transform)
+    uint32_t t = 0;
+    uint32_t *tickets = nullptr;
+};
 // FP32 triangular solves on y (nrhs vectors of n per value set, one after
 // another, B.count value sets), in place.  val: CSC factor values; dval: base
 // of the dense tail view.  xo: scratch of y's size (finished values of the
-// dividing sweeps); counters / ticket: scratch of the dense tail sweeps
-// (B.count * (m / 64 + 1) flags, B.count tickets).
+// dividing sweeps, the forward sweep's dense tail); tickets: the dense tail
+// sweeps' two block tickets; both as SolveInit leaves them.  ticket: scratch
+// of the fused supernodal sweeps (B.count values).
 cudaError_t solve_lower_unit(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                             const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                             const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                              uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st);
 cudaError_t solve_upper(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                        const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                        const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                         uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st);
 // Transposed: U^T z = y (forward), then L^T w = z (backward).
 cudaError_t solve_upper_trans(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                              const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                              const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                               uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st);
 cudaError_t solve_lower_unit_trans(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                                   const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                                   const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                                    uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st);
 
 // Permute/scale kernels of the solve transforms.
 cudaError_t launch_transform_f32(const uint32_t *idx, const double *scale, const float *in,
-                                 float *out, uint32_t n, uint32_t nrhs, cudaStream_t st);
+                                 float *out, uint32_t n, uint32_t nrhs, const SolveInit &init, cudaStream_t st);
 cudaError_t launch_transform_f64_to_f32(const uint32_t *idx, const double *scale, const double *in,
-                                        float *out, uint32_t n, uint32_t nrhs, cudaStream_t st);
+                                        float *out, uint32_t n, uint32_t nrhs, const SolveInit &init,
+                                        cudaStream_t st);
 cudaError_t launch_transform_f32_to_f64_add(const uint32_t *idx, const double *scale,
                                             const float *in, double *x, uint32_t n, uint32_t nrhs,
                                             int accumulate, cudaStream_t st);

@@ -16,9 +16,9 @@
 // GLU_NOALLOC_BLOCK_LIMIT, read once, can lower the second bound (to check
 // the rejection path on small matrices); it cannot raise it.
 //
-// The array keeps the last call's contents.  The sweeps reset the block flags
-// and the ticket they wait on at the start of every call; y and xo are fully
-// written before they are read.
+// The array keeps the last call's contents.  Every call's input transform
+// resets the block tickets and the entries the dense sweeps wait on; y and xo
+// are fully written before they are read.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -33,8 +33,8 @@ constexpr uint32_t kNoAllocMaxBlocks = 4096;             // 64-row blocks of the
 constexpr size_t kNoAllocFloats = 2 * kNoAllocMaxValues + kNoAllocMaxBlocks + 64;
 
 // Working vectors of glu_solve_noalloc: y (permuted right-hand sides), xo
-// (finished values of the dividing sweeps), the dense-tail block flags and
-// the ticket.  About 8 MiB per GPU.
+// (finished values of the sweeps), the dense tail sweeps' block tickets (in
+// the place of one flag per 64-row block) and the fused sweeps' ticket.  About 8 MiB per GPU.
 static __device__ __align__(256) float g_noalloc_scratch[kNoAllocFloats];
 
 constexpr int kMaxDevices = 64;

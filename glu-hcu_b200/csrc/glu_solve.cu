@@ -13,9 +13,9 @@
 //    L and U sweeps scatter (x_i -= L(i,j) x_j with atomics), the transposed
 //    sweeps gather (dot products, no atomics);
 //  * the dense trailing block is solved by row blocks of 64: a block adds the
-//    contribution of every finished earlier block (one 64 x 64 tile each,
-//    staged in shared memory) and then solves its diagonal tile; blocks are
-//    claimed in order through a ticket and wait (bounded) on per-block flags;
+//    contribution of every finished earlier block (one 64 x 64 tile each, in
+//    registers) and then solves its diagonal tile; blocks are claimed in order
+//    through a ticket and wait (bounded) for the entries they read;
 //  * the coupling between the two (U entries of tail columns in sparse rows)
 //    is one parallel scatter or gather over the tail columns.
 #include <cooperative_groups.h>
@@ -200,218 +200,498 @@ static cudaError_t run_sweep(const DevPattern &P, const SolvePlanDev &S, const f
 }
 
 // --------------------------------------------------------- dense tail sweeps --
-// Solve T x = y on the dense block (rows [t, t+m) of y), where
+// Solve T x = r on the dense block (entries [t, t + m) of the vectors), where
 //   kMode 0: T = L   (unit lower,      T(i,c) = val[doff[c] + i])
 //   kMode 1: T = U   (upper,           T(i,c) = val[doff[c] + i])
 //   kMode 2: T = U^T (lower,           T(i,c) = val[doff[i] + c])
 //   kMode 3: T = L^T (unit upper,      T(i,c) = val[doff[i] + c])
-// Row blocks of 64 are claimed in solve order (ascending for lower, descending
-// for upper), interleaved over the value sets; flags[b] = 1 once block b of
-// a set is solved.  The diagonal block's
-// solve is a product with its inverse (dinv, computed once per factorization
-// by k_dense_diag_inv), so the step between two blocks of the chain is a
-// parallel 64 x 64 mat-vec instead of 64 dependent substitution steps.
+// A block of threads owns 64 rows of up to R right-hand sides of one value
+// set; these items are claimed in solve order (ascending for lower, descending
+// for upper) through a ticket, interleaved over the value sets and the groups
+// of right-hand sides, so every chain advances at once and an item waits only
+// on items of smaller tickets, which are running or done.
+//
+// What bounds it: the chain of m / 64 blocks, each of which needs the one
+// before.  Hence
+//  * a solved entry is its own flag: the output starts as kUnsolved (a NaN
+//    pattern no solution holds) and a reader polls the value it needs, which
+//    saves the fence, the flag and the second trip to L2 on every link;
+//  * a warp polls, stages and multiplies its own columns: no barrier of the
+//    block while the finished blocks' tiles stream by (the next tile and its x
+//    are in flight meanwhile);
+//  * the diagonal block's solve is a product with its inverse (dinv, computed
+//    once per factorization by k_dense_diag_inv), a parallel mat-vec instead
+//    of 64 dependent steps; two block barriers per link remain.
+// Measured (B200): a link takes 0.87 us at order 1,920 with one right-hand side
+// (26 us a sweep; 87 us with a flag per block and three barriers per tile), and
+// 32 right-hand sides take 43 us (8.5 ms as groups of four one after another
+// inside the block); transposed, order 3,776, 62-74 us (193 us).
+// The forward sweep reads y and writes xo, the backward sweep reads xo and
+// writes y: the forward one leaves kUnsolved in the rows of y it has read, and
+// the transform in front of the solve leaves it in xo (SolveInit).
 constexpr int kRB = 64;
 constexpr int kRHSChunk = 4;
 
+__device__ __forceinline__ float ld_poll(const float *p) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool unsolved(float v) { return __float_as_uint(v) == kUnsolved; }
+__device__ __forceinline__ void publish(float *p, float v) {
+    // (arithmetic gives the canonical NaN, never this pattern; an input may)
+    if (unsolved(v)) v = __uint_as_float(0x7FFFFFFFu);
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+// Polls the warp's N values per lane (v[k] at at(k); entries that are not
+// needed hold 0) until all are solved; bounded, a wait that sees another's
+// timeout gives up early.
+template <int N, class At>
+__device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, uint32_t *status, uint32_t limit) {
+    for (uint32_t spins = 0;; ++spins) {
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < N; ++k) open |= unsolved(v[k]);
+        if (!__any_sync(0xffffffffu, open)) return;
+        if (spins >= limit) {
+            if ((threadIdx.x & 31) == 0) atomicOr(status, DEV_TIMEOUT);
+            return;
+        }
+        if ((spins & 1023u) == 1023u && (ld_acquire_gpu(status) & DEV_TIMEOUT)) return;
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (unsolved(v[k])) v[k] = ld_poll(at(k));
+    }
+}
+
 // Inverses of the 64 x 64 diagonal blocks of the dense tail: blockIdx.y = 0
-// the unit lower L_bb, 1 the upper U_bb; dinv[z][b][which] row-major.  Thread
-// j computes column j by substitution (rows past the tail's end are the
-// identity).  blockIdx.z selects the value set.
-__global__ void __launch_bounds__(kRB) k_dense_diag_inv(const float *__restrict__ val, uint64_t dstride,
+// the unit lower L_bb, 1 the upper U_bb; dinv[z][b][which] row-major (rows
+// past the tail's end are the identity).  U_bb is taken as its transpose, so
+// both are the inverse of a lower triangular M: the four 16 x 16 diagonal
+// blocks by substitution (a column per thread, in registers), then twice the
+// off-diagonal block of a pair, X21 = -X22 M21 X11, as products over all
+// threads -- 16 dependent steps instead of 64 (8.3 us at order 128, 28 us
+// with 64 threads of serial substitution).  blockIdx.z selects the value set.
+__global__ void __launch_bounds__(256) k_dense_diag_inv(const float *__restrict__ val, uint64_t dstride,
                                                          const uint32_t *__restrict__ doff, uint32_t m,
                                                          float *__restrict__ dinv) {
-    __shared__ float T[kRB][kRB + 1];
-    __shared__ float X[kRB][kRB + 1];
-    const uint32_t b = blockIdx.x, which = blockIdx.y, j = threadIdx.x;
+    constexpr int LD = kRB + 1;
+    __shared__ float M[kRB][LD];
+    __shared__ float X[kRB][LD];
+    __shared__ float W[kRB / 2][kRB / 2 + 1];
+    const uint32_t b = blockIdx.x, which = blockIdx.y, tid = threadIdx.x;
     const uint32_t nb = (m + kRB - 1) / kRB;
     val += blockIdx.z * dstride;
     const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
-    for (uint32_t e = j; e < uint32_t(kRB * kRB); e += kRB) {
+#pragma unroll 4
+    for (uint32_t e = tid; e < uint32_t(kRB * kRB); e += 256) {
         const uint32_t c = e / kRB, i = e % kRB;
-        T[i][c] = (i < rows && c < rows) ? val[doff[rb0 + c] + rb0 + i] : (i == c ? 1.0f : 0.0f);
+        float v = i == c ? 1.0f : 0.0f;
+        if (i < rows && c < rows && (which == 0 ? i > c : i <= c)) v = val[doff[rb0 + c] + rb0 + i];
+        if (which == 0)
+            M[i][c] = v;
+        else
+            M[c][i] = v;
+        X[i][c] = 0.0f;
     }
     __syncthreads();
-    if (which == 0) {  // unit lower: X(:, j) = L^-1 e_j
-        for (uint32_t i = 0; i < uint32_t(kRB); ++i) X[i][j] = i == j ? 1.0f : 0.0f;
-        for (uint32_t i = j + 1; i < uint32_t(kRB); ++i) {
+    if (tid < uint32_t(kRB)) {  // column j of the 16 x 16 block at g
+        const uint32_t g = tid & ~15u, j = tid & 15u;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
             float acc = 0.0f;
-            for (uint32_t k = j; k < i; ++k) acc = fmaf(T[i][k], X[k][j], acc);
-            X[i][j] = -acc;
+#pragma unroll
+            for (int k = 0; k < i; ++k) acc = fmaf(M[g + i][g + k], x[k], acc);
+            // zero above the diagonal: x[k] = 0 for k < j
+            x[i] = (uint32_t(i) == j ? 1.0f : uint32_t(i) > j ? -acc : 0.0f) / M[g + i][g + i];
         }
-    } else {  // upper: X(:, j) = U^-1 e_j
-        for (uint32_t i = 0; i < uint32_t(kRB); ++i) X[i][j] = 0.0f;
-        X[j][j] = 1.0f / T[j][j];
-        for (uint32_t i = j; i-- > 0;) {
-            float acc = 0.0f;
-            for (uint32_t k = i + 1; k <= j; ++k) acc = fmaf(T[i][k], X[k][j], acc);
-            X[i][j] = -acc / T[i][i];
-        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) X[g + i][g + j] = x[i];
     }
+    __syncthreads();
+    // pairs of 16-blocks: 2 x 256 outputs; W = M21 X11, X21 = -X22 W
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const uint32_t g = u * 32, i = tid / 16, j = tid % 16;
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc = fmaf(M[g + 16 + i][g + k], X[g + k][g + j], acc);
+        W[u * 16 + i][j] = acc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const uint32_t g = u * 32, i = tid / 16, j = tid % 16;
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc = fmaf(X[g + 16 + i][g + 16 + k], W[u * 16 + k][j], acc);
+        X[g + 16 + i][g + j] = -acc;
+    }
+    __syncthreads();
+    // the pair of 32-blocks
+    const uint32_t j = tid % 32, i0 = tid / 32;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+        const float xv = X[k][j];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fmaf(M[32 + i0 + 8 * u][k], xv, acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        W[i0 + 8 * u][j] = acc[u];
+        acc[u] = 0.0f;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+        const float wv = W[k][j];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fmaf(X[32 + i0 + 8 * u][32 + k], wv, acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) X[32 + i0 + 8 * u][j] = -acc[u];
+    __syncthreads();
     float *out = dinv + ((size_t(blockIdx.z) * nb + b) * 2 + which) * kRB * kRB;
-    for (uint32_t i = 0; i < uint32_t(kRB); ++i) out[i * kRB + j] = X[i][j];
+#pragma unroll 4
+    for (uint32_t e = tid; e < uint32_t(kRB * kRB); e += 256)
+        out[e] = which == 0 ? X[e / kRB][e % kRB] : X[e % kRB][e / kRB];
 }
 
-template <int kMode>
-__global__ void __launch_bounds__(256, 4) k_dense_trsv(const float *__restrict__ val, const uint32_t *__restrict__ doff,
-                                                    uint32_t t, uint32_t m, float *y, uint32_t n, uint32_t nrhs,
-                                                    uint32_t *flags, uint32_t *ticket, uint32_t *status,
-                                                    uint32_t spin_limit, uint32_t ticket_base, uint64_t dstride,
-                                                    uint64_t ystride, const float *__restrict__ dinv) {
-    constexpr bool kLower = (kMode == 0 || kMode == 2);
-    constexpr bool kTrans = (kMode >= 2);
-    constexpr int kWhich = (kMode == 0 || kMode == 3) ? 0 : 1;  // inverse of L or of U
-    __shared__ float tile[kRB][kRB + 1];
-    __shared__ float xs[kRB][kRHSChunk];
-    __shared__ float part[4][kRB][kRHSChunk];
-    __shared__ uint32_t s_blk;
-    const uint32_t tid = threadIdx.x;
+// One item: its value set, first right-hand side and block (in solve order).
+struct TrsvItem {
+    uint32_t z, v0, tk;
+};
+__device__ __forceinline__ TrsvItem trsv_item(uint32_t tg, uint32_t count, uint32_t chunks, uint32_t R) {
+    const uint32_t per = count * chunks, rem = tg % per;
+    return TrsvItem{rem / chunks, (rem % chunks) * R, tg / per};
+}
+
+// T = L (kMode 0) or U (kMode 1): T(i, c) down the columns.  Warp w: rows
+// 32 (w & 1) + lane, columns 16 (w >> 1) .. + 15 of every tile, in registers;
+// the 16 x R values of x go through a stretch of shared memory of the warp's
+// own, read back as broadcasts.
+template <int kMode, int R>
+__global__ void __launch_bounds__(256, R == 1 ? 4 : 3)
+    k_dense_trsv(const float *__restrict__ val, const uint32_t *__restrict__ doff, uint32_t t, uint32_t m, float *rin,
+                 float *out, uint32_t n, uint32_t nrhs, uint32_t chunks, uint32_t count, uint32_t *ticket,
+                 uint32_t *status, uint32_t spin_limit, uint32_t ticket_base, uint64_t dstride, uint64_t ystride,
+                 const float *__restrict__ dinv) {
+    constexpr bool kLower = kMode == 0;
+    constexpr int kW = 16;               // columns per warp and tile
+    constexpr int kX = R == 1 ? 1 : R / 2;  // x values a lane polls: kW * R of them on 32 lanes
+    __shared__ __align__(16) float xs[8][2][kW * R];
+    __shared__ float part[2][4][kRB][R];
+    __shared__ uint32_t s_item;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nb = (m + kRB - 1) / kRB;
-    // One ticket counter for the launch, handed out block-row-major over the
-    // value sets (ticket = block * count + set): every set's chain advances
-    // at once, and a block waits only on blocks of smaller tickets, which
-    // are running or done.
-    if (tid == 0) s_blk = atomicAdd(ticket, 1u) + ticket_base;
+    if (tid == 0) s_item = atomicAdd(ticket, 1u) + ticket_base;
     __syncthreads();
-    const uint32_t count = gridDim.z, tg = s_blk;
-    if (tg >= nb * count) return;
-    const uint32_t z = tg % count, tk = tg / count;
-    val += z * dstride;
-    y += z * ystride;
-    flags += size_t(z) * nb;
+    if (s_item >= nb * count * chunks) return;
+    const TrsvItem it = trsv_item(s_item, count, chunks, R);
+    const uint32_t tk = it.tk, nr = min(uint32_t(R), nrhs - it.v0);
+    val += it.z * dstride;
+    rin += it.z * ystride + size_t(it.v0) * n + t;
+    out += it.z * ystride + size_t(it.v0) * n + t;
     const uint32_t b = kLower ? tk : nb - 1 - tk;
-    const uint32_t rb0 = b * kRB, rb1 = min(rb0 + kRB, m);
-    const uint32_t rows = rb1 - rb0;
-    auto T = [&](uint32_t i, uint32_t c) -> float {
-        return kTrans ? val[doff[i] + c] : val[doff[c] + i];
-    };
-    constexpr int kTilePer = kRB * kRB / 256;
-    const float *inv = dinv + ((size_t(z) * nb + b) * 2 + kWhich) * kRB * kRB;  // row-major
-    // tile T(rb0.., block s in solve order): independent of x
-    auto load_tile = [&](uint32_t s, float (&tv)[kTilePer]) {
-        const uint32_t c = kLower ? s : nb - 1 - s;
-        const uint32_t cb0 = c * kRB, cb1 = min(cb0 + kRB, m);
+    const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
+    const uint32_t row = tid & (kRB - 1), q = tid / kRB, col0 = q * kW;
+    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kMode) * kRB * kRB + row * kRB + col0;
+    // lane's x values: column lane % 16, right-hand sides lane / 16 + 2 k
+    const uint32_t xc = lane & 15, xr = lane >> 4;
+    const bool rowok = row < rows;
+    auto load_tile = [&](uint32_t s, float (&tv)[kW]) {
+        const uint32_t cb = (kLower ? s : nb - 1 - s) * kRB + col0;
+        const uint32_t off = cb + xc < m ? __ldg(doff + cb + xc) : 0u;
 #pragma unroll
-        for (int qq = 0; qq < kTilePer; ++qq) {
-            const uint32_t e = tid + qq * 256, a = e / kRB, bb = e % kRB;  // coalesced along bb
-            const uint32_t i = kTrans ? a : bb, cc = kTrans ? bb : a;
-            tv[qq] = (rb0 + i < rb1 && cb0 + cc < cb1) ? T(rb0 + i, cb0 + cc) : 0.0f;
+        for (int k = 0; k < kW; ++k) {
+            const uint32_t o = __shfl_sync(0xffffffffu, off, k);
+            tv[k] = (rowok && cb + k < m) ? __ldg(val + o + rb0 + row) : 0.0f;
         }
     };
-    for (uint32_t rc0 = 0; rc0 < nrhs; rc0 += kRHSChunk) {
-        const uint32_t nr = min(uint32_t(kRHSChunk), nrhs - rc0);
-        const uint32_t row = tid & (kRB - 1), q = tid / kRB;  // 4 quarters of 16 columns
-        float acc[kRHSChunk] = {0.f, 0.f, 0.f, 0.f};
-        // contributions of the finished blocks, in solve order; the next
-        // block's tile is in flight while this one waits and computes
-        float tv[kTilePer], tn[kTilePer];
-        if (tk > 0) load_tile(0, tv);
-        for (uint32_t s = 0; s < tk; ++s) {
-            const uint32_t c = kLower ? s : nb - 1 - s;
-            const uint32_t cb0 = c * kRB, cb1 = min(cb0 + kRB, m);
-            if (s + 1 < tk) load_tile(s + 1, tn);
-            if (kTrans) {  // transposed: through shared memory, loads coalesced along the rows
+    auto x_at = [&](uint32_t s, int k) -> const float * {
+        const uint32_t c = (kLower ? s : nb - 1 - s) * kRB + col0 + xc;
+        return out + size_t(R == 1 ? 0u : xr + 2 * k) * n + c;
+    };
+    auto load_x = [&](uint32_t s, float (&v)[kX]) {
+        const uint32_t c = (kLower ? s : nb - 1 - s) * kRB + col0 + xc;
 #pragma unroll
-                for (int qq = 0; qq < kTilePer; ++qq) {
-                    const uint32_t e = tid + qq * 256, a = e / kRB, bb = e % kRB;
-                    tile[a][bb] = tv[qq];
+        for (int k = 0; k < kX; ++k) v[k] = (c < m && (R == 1 ? 0u : xr + 2 * k) < nr) ? ld_poll(x_at(s, k)) : 0.0f;
+    };
+    auto stage = [&](float *dst, const float (&v)[kX]) {
+#pragma unroll
+        for (int k = 0; k < kX; ++k)
+            if (R > 1 || xr == 0) dst[xc * R + (R == 1 ? 0u : xr + 2 * k)] = v[k];
+        __syncwarp();
+    };
+    auto multiply = [&](float (&acc)[R], const float (&tv)[kW], const float *src) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(src);
+        if (R == 1) {
+#pragma unroll
+            for (int k = 0; k < kW; k += 4) {
+                const float4 v = s4[k / 4];
+                acc[0] = fmaf(tv[k], v.x, acc[0]);
+                acc[0] = fmaf(tv[k + 1], v.y, acc[0]);
+                acc[0] = fmaf(tv[k + 2], v.z, acc[0]);
+                acc[0] = fmaf(tv[k + 3], v.w, acc[0]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kW; ++k)
+#pragma unroll
+                for (int r = 0; r < R; r += 4) {
+                    const float4 v = s4[(k * R + r) / 4];
+                    acc[r % R] = fmaf(tv[k], v.x, acc[r % R]);
+                    acc[(r + 1) % R] = fmaf(tv[k], v.y, acc[(r + 1) % R]);
+                    acc[(r + 2) % R] = fmaf(tv[k], v.z, acc[(r + 2) % R]);
+                    acc[(r + 3) % R] = fmaf(tv[k], v.w, acc[(r + 3) % R]);
                 }
-            }
-            if (tid == 0) wait_count(flags + c, 1u, status, spin_limit);
-            __syncthreads();
-            for (uint32_t e = tid; e < kRB * kRHSChunk; e += 256) {
-                uint32_t cc = e / kRHSChunk, r = e % kRHSChunk;
-                float v = 0.0f;
-                if (cb0 + cc < cb1 && r < nr) v = __ldcg(y + size_t(rc0 + r) * n + t + cb0 + cc);
-                xs[cc][r] = v;
-            }
-            __syncthreads();
-            if (kTrans) {
-#pragma unroll 4
-                for (uint32_t cc = q * 16; cc < q * 16 + 16; ++cc) {
-                    float tv2 = tile[row][cc];
-#pragma unroll
-                    for (int r = 0; r < kRHSChunk; ++r) acc[r] = fmaf(tv2, xs[cc][r], acc[r]);
-                }
-            } else {  // thread (row, q) holds T(row, q + 4 j), j < 16: multiplied in registers
-#pragma unroll
-                for (int qq = 0; qq < kTilePer; ++qq) {
-                    const uint32_t cc = q + 4 * qq;
-#pragma unroll
-                    for (int r = 0; r < kRHSChunk; ++r) acc[r] = fmaf(tv[qq], xs[cc][r], acc[r]);
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int qq = 0; qq < kTilePer; ++qq) tv[qq] = tn[qq];
         }
+    };
+    // the right-hand sides of the columns this warp takes in the diagonal product
+    float rv[kX];
 #pragma unroll
-        for (int r = 0; r < kRHSChunk; ++r) part[q][row][r] = acc[r];
-        // r = y - (contributions) for the block's rows, then x = T_bb^-1 r
-#pragma unroll
-        for (int qq = 0; qq < kTilePer; ++qq) {
-            const uint32_t e = tid + qq * 256, a = e / kRB, bb = e % kRB;  // inverse element (a, bb)
-            const float dv = __ldg(inv + e);
-            if (kTrans)
-                tile[bb][a] = dv;
-            else
-                tile[a][bb] = dv;
-        }
-        __syncthreads();
-        if (tid < kRB * kRHSChunk) {
-            const uint32_t i = tid % kRB, r = tid / kRB;
-            float v = 0.0f;
-            if (i < rows && r < nr)
-                v = __ldcg(y + size_t(rc0 + r) * n + t + rb0 + i) -
-                    (part[0][i][r] + part[1][i][r] + part[2][i][r] + part[3][i][r]);
-            xs[i][r] = v;
-        }
-        __syncthreads();
-        {
-            float acc2[kRHSChunk] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (uint32_t cc = q * 16; cc < q * 16 + 16; ++cc) {
-                const float tv = tile[row][cc];
-#pragma unroll
-                for (int r = 0; r < kRHSChunk; ++r) acc2[r] = fmaf(tv, xs[cc][r], acc2[r]);
-            }
-#pragma unroll
-            for (int r = 0; r < kRHSChunk; ++r) part[q][row][r] = acc2[r];
-        }
-        __syncthreads();
-        if (tid < kRB * kRHSChunk) {
-            const uint32_t i = tid % kRB, r = tid / kRB;
-            if (i < rows && r < nr)
-                __stcg(y + size_t(rc0 + r) * n + t + rb0 + i,
-                       (part[0][i][r] + part[1][i][r]) + (part[2][i][r] + part[3][i][r]));
-        }
-        __syncthreads();
+    for (int k = 0; k < kX; ++k) {
+        const uint32_t r = R == 1 ? 0u : xr + 2 * k;
+        rv[k] = (col0 + xc < rows && r < nr) ? __ldcg(rin + size_t(r) * n + rb0 + col0 + xc) : 0.0f;
     }
-    if (tid == 0) {
-        __threadfence();
-        st_release_gpu(flags + b, 1u);
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+    float tv[kW], xv[kX];
+    if (tk > 0) {
+        load_tile(0, tv);
+        load_x(0, xv);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kW; k += 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + k));
+            tv[k] = v.x, tv[k + 1] = v.y, tv[k + 2] = v.z, tv[k + 3] = v.w;
+        }
+    }
+    for (uint32_t s = 0; s < tk; ++s) {
+        float tn[kW], xn[kX];
+        if (s + 1 < tk) {  // the next tile and a first look at its x, else the diagonal's inverse
+            load_tile(s + 1, tn);
+            load_x(s + 1, xn);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kW; k += 4) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + k));
+                tn[k] = v.x, tn[k + 1] = v.y, tn[k + 2] = v.z, tn[k + 3] = v.w;
+            }
+#pragma unroll
+            for (int k = 0; k < kX; ++k) xn[k] = 0.0f;
+        }
+        wait_solved(xv, [&](int k) { return x_at(s, k); }, status, spin_limit);
+        float *buf = xs[warp][s & 1];
+        stage(buf, xv);
+        multiply(acc, tv, buf);
+#pragma unroll
+        for (int k = 0; k < kW; ++k) tv[k] = tn[k];
+#pragma unroll
+        for (int k = 0; k < kX; ++k) xv[k] = xn[k];
+    }
+    // r = b - (contributions) for the block's rows, then x = T_bb^-1 r
+#pragma unroll
+    for (int r = 0; r < R; ++r) part[0][q][row][r] = acc[r];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kX; ++k) {
+        const uint32_t c = col0 + xc, r = R == 1 ? 0u : xr + 2 * k;
+        xv[k] = rv[k] - ((part[0][0][c][r] + part[0][1][c][r]) + (part[0][2][c][r] + part[0][3][c][r]));
+    }
+    float *buf = xs[warp][tk & 1];
+    stage(buf, xv);
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+    multiply(acc, tv, buf);
+#pragma unroll
+    for (int r = 0; r < R; ++r) part[1][q][row][r] = acc[r];
+    __syncthreads();
+    for (uint32_t e = tid; e < uint32_t(kRB * R); e += 256) {
+        const uint32_t i = e % kRB, r = e / kRB;
+        if (i < rows && r < nr) {
+            publish(out + size_t(r) * n + rb0 + i,
+                    (part[1][0][i][r] + part[1][1][i][r]) + (part[1][2][i][r] + part[1][3][i][r]));
+            if (kLower) rin[size_t(r) * n + rb0 + i] = __uint_as_float(kUnsolved);  // read by all warps: output of the backward sweep
+        }
+    }
+}
+
+// Sums of N values per lane over the warp: lane L returns with the sum of
+// value L % N (N = 8 or 32, the sums repeat every N lanes).  Each halving
+// step keeps one half of the values and adds the partner's.
+template <int N>
+__device__ __forceinline__ float warp_transpose_sum(float (&v)[N], uint32_t lane) {
+#pragma unroll
+    for (int h = N / 2; h > 0; h >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float keep = up ? v[k + h] : v[k], give = up ? v[k] : v[k + h];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    }
+    float s = v[0];
+#pragma unroll
+    for (int h = N; h < 32; h <<= 1) s += __shfl_xor_sync(0xffffffffu, s, h);
+    return s;
+}
+
+// T = U^T (kMode 2) or L^T (kMode 3): T(i, c) along c.  Warp w: rows 8 w ..
+// 8 w + 7, lane: columns lane and lane + 32 of every tile; a lane polls the x
+// of its own two columns and the row sums are reduced once, after the last
+// tile.
+template <int kMode, int R>
+__global__ void __launch_bounds__(256, R == 1 ? 3 : 2)
+    k_dense_trsv_trans(const float *__restrict__ val, const uint32_t *__restrict__ doff, uint32_t t, uint32_t m,
+                       float *rin, float *out, uint32_t n, uint32_t nrhs, uint32_t chunks, uint32_t count,
+                       uint32_t *ticket, uint32_t *status, uint32_t spin_limit, uint32_t ticket_base,
+                       uint64_t dstride, uint64_t ystride, const float *__restrict__ dinv) {
+    constexpr bool kLower = kMode == 2;
+    constexpr int kRows = 8;
+    constexpr int kWhich = kMode == 3 ? 0 : 1;  // inverse of L or of U
+    __shared__ float rs[kRB][R];
+    __shared__ uint32_t s_item;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t nb = (m + kRB - 1) / kRB;
+    if (tid == 0) s_item = atomicAdd(ticket, 1u) + ticket_base;
+    __syncthreads();
+    if (s_item >= nb * count * chunks) return;
+    const TrsvItem it = trsv_item(s_item, count, chunks, R);
+    const uint32_t tk = it.tk, nr = min(uint32_t(R), nrhs - it.v0);
+    val += it.z * dstride;
+    rin += it.z * ystride + size_t(it.v0) * n + t;
+    out += it.z * ystride + size_t(it.v0) * n + t;
+    const uint32_t b = kLower ? tk : nb - 1 - tk;
+    const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
+    const uint32_t i0 = warp * kRows;
+    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kWhich) * kRB * kRB;  // row-major
+    uint32_t base[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) base[i] = i0 + i < rows ? __ldg(doff + rb0 + i0 + i) : 0u;
+    auto load_tile = [&](uint32_t s, float (&tv)[2 * kRows]) {
+        const uint32_t c = (kLower ? s : nb - 1 - s) * kRB + lane;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            tv[2 * i] = (i0 + i < rows && c < m) ? __ldg(val + base[i] + c) : 0.0f;
+            tv[2 * i + 1] = (i0 + i < rows && c + 32 < m) ? __ldg(val + base[i] + c + 32) : 0.0f;
+        }
+    };
+    // row i of T_bb^-1 is column i of the stored inverse
+    auto load_inv = [&](float (&tv)[2 * kRows]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < kRows; i += 4) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + (lane + 32 * h) * kRB + i0 + i));
+                tv[2 * i + h] = v.x, tv[2 * i + 2 + h] = v.y, tv[2 * i + 4 + h] = v.z, tv[2 * i + 6 + h] = v.w;
+            }
+    };
+    auto x_at = [&](uint32_t s, int k) -> const float * {
+        return out + size_t(k >> 1) * n + (kLower ? s : nb - 1 - s) * kRB + lane + 32 * (k & 1);
+    };
+    auto load_x = [&](uint32_t s, float (&v)[2 * R]) {
+        const uint32_t c = (kLower ? s : nb - 1 - s) * kRB + lane;
+#pragma unroll
+        for (int k = 0; k < 2 * R; ++k)
+            v[k] = (c + 32 * (k & 1) < m && uint32_t(k >> 1) < nr) ? ld_poll(x_at(s, k)) : 0.0f;
+    };
+    float acc[kRows * R];
+    auto multiply = [&](const float (&tv)[2 * kRows], const float (&xv)[2 * R]) {
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                acc[i * R + r] = fmaf(tv[2 * i + 1], xv[2 * r + 1], fmaf(tv[2 * i], xv[2 * r], acc[i * R + r]));
+    };
+    // after the reduction lane L holds row i0 + (L % (8 R)) / R, right-hand side L % R
+    const uint32_t li = (lane % (kRows * R)) / R, lr = lane % R;
+    const bool mine = lane < uint32_t(kRows * R) && i0 + li < rows && lr < nr;
+    const float rv = mine ? __ldcg(rin + size_t(lr) * n + rb0 + i0 + li) : 0.0f;
+#pragma unroll
+    for (int e = 0; e < kRows * R; ++e) acc[e] = 0.0f;
+    float tv[2 * kRows], xv[2 * R];
+    if (tk > 0) {
+        load_tile(0, tv);
+        load_x(0, xv);
+    } else {
+        load_inv(tv);
+    }
+    for (uint32_t s = 0; s < tk; ++s) {
+        float tn[2 * kRows], xn[2 * R];
+        if (s + 1 < tk) {
+            load_tile(s + 1, tn);
+            load_x(s + 1, xn);
+        } else {
+            load_inv(tn);
+#pragma unroll
+            for (int k = 0; k < 2 * R; ++k) xn[k] = 0.0f;
+        }
+        wait_solved(xv, [&](int k) { return x_at(s, k); }, status, spin_limit);
+        multiply(tv, xv);
+#pragma unroll
+        for (int k = 0; k < 2 * kRows; ++k) tv[k] = tn[k];
+#pragma unroll
+        for (int k = 0; k < 2 * R; ++k) xv[k] = xn[k];
+    }
+    const float r0 = rv - warp_transpose_sum(acc, lane);
+    if (lane < uint32_t(kRows * R)) rs[i0 + li][lr] = r0;  // zero for rows and right-hand sides that are not there
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        xv[2 * r] = rs[lane][r];
+        xv[2 * r + 1] = rs[lane + 32][r];
+    }
+#pragma unroll
+    for (int e = 0; e < kRows * R; ++e) acc[e] = 0.0f;
+    multiply(tv, xv);
+    const float x = warp_transpose_sum(acc, lane);
+    if (mine) {
+        publish(out + size_t(lr) * n + rb0 + i0 + li, x);
+        if (kLower) rin[size_t(lr) * n + rb0 + i0 + li] = __uint_as_float(kUnsolved);
     }
 }
 
 cudaError_t launch_dense_diag_inv(const float *dval, uint64_t dstride, uint32_t count, const uint32_t *doff,
                                   uint32_t m, float *dinv, cudaStream_t st) {
     if (m == 0) return cudaSuccess;
-    k_dense_diag_inv<<<dim3((m + kRB - 1) / kRB, 2, count), kRB, 0, st>>>(dval, dstride, doff, m, dinv);
+    k_dense_diag_inv<<<dim3((m + kRB - 1) / kRB, 2, count), 256, 0, st>>>(dval, dstride, doff, m, dinv);
     return cudaGetLastError();
 }
 
+// The forward sweeps (modes 0, 2) read y and write xo with ticket 0, the
+// backward ones (1, 3) read xo and write y with ticket 1.  Right-hand sides in
+// groups of one, or of kRHSChunk when there are several.
 template <int kMode>
-static cudaError_t dense_sweep(const SolvePlanDev &S, const float *dval, float *y, uint32_t n,
-                               uint32_t nrhs, uint32_t *flags, uint32_t *ticket, uint32_t *status,
-                               const SolveBatch &B, cudaStream_t st) {
+static cudaError_t dense_sweep(const SolvePlanDev &S, const float *dval, float *y, float *xo, uint32_t n,
+                               uint32_t nrhs, uint32_t *tickets, uint32_t *status, const SolveBatch &B,
+                               cudaStream_t st) {
     if (S.m == 0) return cudaSuccess;
-    uint32_t nb = (S.m + kRB - 1) / kRB;
-    cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(uint32_t) * nb * B.count, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t) * B.count, st);
-    if (e != cudaSuccess) return e;
-    k_dense_trsv<kMode><<<dim3(nb, 1, B.count), 256, 0, st>>>(dval, S.doff, S.t, S.m, y, n, nrhs, flags, ticket,
-                                                              status, S.spin_limit, S.ticket_base, B.dstride,
-                                                              uint64_t(nrhs) * n, B.dinv);
+    constexpr bool kForward = kMode == 0 || kMode == 2;
+    const uint32_t nb = (S.m + kRB - 1) / kRB;
+    const uint32_t chunks = nrhs == 1 ? 1u : (nrhs + kRHSChunk - 1) / kRHSChunk;
+    const uint64_t items = uint64_t(nb) * chunks * B.count;
+    if (items > 0x7FFFFFFFu) return cudaErrorInvalidValue;
+    auto go = [&](auto kern) {
+        kern<<<uint32_t(items), 256, 0, st>>>(dval, S.doff, S.t, S.m, kForward ? y : xo, kForward ? xo : y, n, nrhs,
+                                              chunks, B.count, tickets + (kForward ? 0 : 1), status, S.spin_limit,
+                                              S.ticket_base, B.dstride, uint64_t(nrhs) * n, B.dinv);
+    };
+    if constexpr (kMode >= 2) {
+        if (nrhs == 1)
+            go(k_dense_trsv_trans<kMode, 1>);
+        else
+            go(k_dense_trsv_trans<kMode, kRHSChunk>);
+    } else {
+        if (nrhs == 1)
+            go(k_dense_trsv<kMode, 1>);
+        else
+            go(k_dense_trsv<kMode, kRHSChunk>);
+    }
     return cudaGetLastError();
 }
 
@@ -428,19 +708,19 @@ static cudaError_t tail_coupling(const DevPattern &P, const SolvePlanDev &S, con
 }
 
 cudaError_t solve_lower_unit(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                             const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                             const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                              uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st) {
     cudaError_t e = S.sn[0].nlev ? run_sn_sweep(P, S.sn[0], false, S.t, val, y, xo, nrhs, B, B.sweep_done, ticket,
                                                 status, S.spin_limit, st)
                                  : run_sweep<SWEEP_L>(P, S, val, y, xo, nrhs, B, st);
     if (e != cudaSuccess) return e;
-    return dense_sweep<0>(S, dval, y, P.n, nrhs, counters, ticket, status, B, st);
+    return dense_sweep<0>(S, dval, y, xo, P.n, nrhs, tickets, status, B, st);
 }
 
 cudaError_t solve_upper(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                        const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                        const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                         uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st) {
-    cudaError_t e = dense_sweep<1>(S, dval, y, P.n, nrhs, counters, ticket, status, B, st);
+    cudaError_t e = dense_sweep<1>(S, dval, y, xo, P.n, nrhs, tickets, status, B, st);
     if (e == cudaSuccess) e = tail_coupling(P, S, val, y, nrhs, false, B, st);
     if (e == cudaSuccess)
         e = S.sn[1].nlev ? run_sn_sweep(P, S.sn[1], true, S.t, val, y, xo, nrhs, B, B.sweep_done, ticket, status,
@@ -450,27 +730,35 @@ cudaError_t solve_upper(const DevPattern &P, const SolvePlanDev &S, const float 
 }
 
 cudaError_t solve_upper_trans(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                              const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                              const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                               uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st) {
     cudaError_t e = run_sweep<SWEEP_UT>(P, S, val, y, xo, nrhs, B, st);
-    if (e == cudaSuccess) e = dense_sweep<2>(S, dval, y, P.n, nrhs, counters, ticket, status, B, st);
+    if (e == cudaSuccess) e = dense_sweep<2>(S, dval, y, xo, P.n, nrhs, tickets, status, B, st);
     return e;
 }
 
 cudaError_t solve_lower_unit_trans(const DevPattern &P, const SolvePlanDev &S, const float *val,
-                                   const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *counters,
+                                   const float *dval, float *y, float *xo, uint32_t nrhs, uint32_t *tickets,
                                    uint32_t *ticket, uint32_t *status, const SolveBatch &B, cudaStream_t st) {
-    cudaError_t e = dense_sweep<3>(S, dval, y, P.n, nrhs, counters, ticket, status, B, st);
+    cudaError_t e = dense_sweep<3>(S, dval, y, xo, P.n, nrhs, tickets, status, B, st);
     if (e == cudaSuccess) e = tail_coupling(P, S, val, y, nrhs, true, B, st);
     if (e == cudaSuccess) e = run_sweep<SWEEP_LT>(P, S, val, y, xo, nrhs, B, st);
     return e;
 }
 
 // --------------------------------------------------------------- transforms --
+// What the dense tail sweeps find at their start (SolveInit), written along
+// with entry j of vector blockIdx.y of a solve's input transform.
+__device__ __forceinline__ void solve_init(const SolveInit &I, size_t off, uint32_t j) {
+    if (I.xo && j >= I.t) I.xo[off + j] = __uint_as_float(kUnsolved);
+    if (I.tickets && j == 0 && blockIdx.y == 0) I.tickets[0] = I.tickets[1] = 0u;
+}
+
 __global__ void k_transform_f32(const uint32_t *__restrict__ idx, const double *__restrict__ scale,
-                                const float *__restrict__ in, float *__restrict__ out, uint32_t n) {
+                                const float *__restrict__ in, float *__restrict__ out, uint32_t n, SolveInit I) {
     const size_t off = size_t(blockIdx.y) * n;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        solve_init(I, off, j);
         float v = in[off + idx[j]];
         // float * double evaluated in double, stored as float (symbolic.cc:219,244)
         out[off + j] = scale ? static_cast<float>(static_cast<double>(v) * scale[j]) : v;
@@ -478,9 +766,11 @@ __global__ void k_transform_f32(const uint32_t *__restrict__ idx, const double *
 }
 
 __global__ void k_transform_f64_to_f32(const uint32_t *__restrict__ idx, const double *__restrict__ scale,
-                                       const double *__restrict__ in, float *__restrict__ out, uint32_t n) {
+                                       const double *__restrict__ in, float *__restrict__ out, uint32_t n,
+                                       SolveInit I) {
     const size_t off = size_t(blockIdx.y) * n;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        solve_init(I, off, j);
         double v = in[off + idx[j]];
         out[off + j] = static_cast<float>(scale ? v * scale[j] : v);
     }
@@ -504,13 +794,14 @@ static inline dim3 tgrid(uint32_t n, uint32_t nrhs) {
 }
 
 cudaError_t launch_transform_f32(const uint32_t *idx, const double *scale, const float *in,
-                                 float *out, uint32_t n, uint32_t nrhs, cudaStream_t st) {
-    k_transform_f32<<<tgrid(n, nrhs), 256, 0, st>>>(idx, scale, in, out, n);
+                                 float *out, uint32_t n, uint32_t nrhs, const SolveInit &init, cudaStream_t st) {
+    k_transform_f32<<<tgrid(n, nrhs), 256, 0, st>>>(idx, scale, in, out, n, init);
     return cudaGetLastError();
 }
 cudaError_t launch_transform_f64_to_f32(const uint32_t *idx, const double *scale, const double *in,
-                                        float *out, uint32_t n, uint32_t nrhs, cudaStream_t st) {
-    k_transform_f64_to_f32<<<tgrid(n, nrhs), 256, 0, st>>>(idx, scale, in, out, n);
+                                        float *out, uint32_t n, uint32_t nrhs, const SolveInit &init,
+                                        cudaStream_t st) {
+    k_transform_f64_to_f32<<<tgrid(n, nrhs), 256, 0, st>>>(idx, scale, in, out, n, init);
     return cudaGetLastError();
 }
 cudaError_t launch_transform_f32_to_f64_add(const uint32_t *idx, const double *scale,
