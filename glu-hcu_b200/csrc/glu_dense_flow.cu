@@ -1,0 +1,359 @@
+// The whole dense trailing block factored by one launch: a dataflow of 64 x 64
+// tiles.
+//
+// The blocked algorithm of glu_factor_dense.cu takes a panel kernel, an
+// operand pack and an update kernel (three with look-ahead) per 64 columns.
+// On trailing blocks of a few thousand columns those are bound by their own
+// latency, not by their work: the panel's serial 64-pivot LU repeated in every
+// block, C read and written once per panel, a launch and a drain each.  Here a
+// block of threads owns one tile (i, j) for good:
+//   for s < min(i, j): C -= L(i, s) U(s, j), as the two tiles become ready
+//   i == j: C = L11 U11;  i > j: L = C U11^-1;  i < j: U = L11^-1 C
+// (left-looking per tile), so C is read and written once, tiles of later
+// columns are updated while the diagonal chain advances, and a column step
+// costs the chain diagonal LU -> one triangular solve -> one tile product
+// instead of three kernels.
+//
+// Tiles are claimed in the order of min(i, j), the diagonal tile first,
+// interleaved over the value sets (a ticket); a tile needs only tiles claimed
+// before it, so every wait is for a running or finished block.  Besides its
+// place in the factor a finished tile is written to a workspace, K-major and
+// contiguous (16 KB; the diagonal tile as both operand layouts of the solves),
+// and its ready flag released; a producer warp waits (bounded) for the flags
+// and brings the operands in by bulk copies, two stages ahead of the products.
+// The workspace is the block's size again; the rule that chooses this kernel
+// is in glu_engine.cpp (dense_flow).
+//
+// What a column step of the chain takes (order 1,920, one block per SM): LU
+// 7.0 us, publishing it 1.5, flag and copy 1.1, triangular solve 2.6, publishing
+// 0.8, flag and copy 1.2, product 1.9 -- 16.5 us, against 50 us for panel, pack
+// and update kernels.  The whole block: 0.49 ms (1.51 ms).
+//
+// FP32 fused multiply-add throughout; the 64 products of a step are summed by
+// themselves and subtracted from the entry once (relative error against 64 bits of random
+// filled blocks, order 1,920: 1.8e-7; one at a time 7.9e-7, panels and updates
+// 4.5e-7).
+//
+// The reference's counterpart is the per-column work of RL_onecol_factorizeCurrentCol
+// and RL_onecol_updateSubmat (src/numeric.cu:205-319).
+#include "glu_common.cuh"
+#include "glu_kernels.h"
+#include "glu_tri.cuh"
+
+namespace glu {
+namespace {
+
+constexpr int kT = kFlowTile;                        // 64
+constexpr int kStages = 2;
+constexpr uint32_t kTileBytes = kT * kT * 4;         // 16 KB
+constexpr uint32_t kDiagBytes = kT * kTriML * 4;     // 17 KB: rows of 64 and the pivot's reciprocal, padded
+constexpr uint32_t kStageBytes = 2 * kTileBytes;
+constexpr int kLdW = kT + 1;                         // solve tile, [k][vector]
+constexpr size_t kWorkBytes = sizeof(float) * kT * kLuLD;  // LU tile, or solve tile
+constexpr size_t kSmem = kStages * kStageBytes + kWorkBytes;
+constexpr size_t kSmemAlone = 120 * 1024;  // keeps a second block off the SM
+constexpr int kThreads = kTriThreads + 32;           // eight computing warps and the producer
+static_assert(kFlowTile == kTriMax && kFlowDiagFloats == kT * kTriML, "layouts");
+static_assert(kDiagBytes <= kStageBytes && kLdW <= kLuLD, "the diagonal tile fits a stage");
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void bar_init(uint64_t *bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+// Between the acquire of a tile's flag and its bulk copy: the tile was written
+// by ordinary stores, the copy reads through the asynchronous proxy.
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Bounded wait for a tile's ready flag (one thread).
+__device__ __forceinline__ void wait_tile(const uint32_t *flag, uint32_t *status, uint32_t limit) {
+    for (uint32_t spins = 0; !ld_acquire_gpu(flag); ++spins) {
+        if (spins >= limit) {
+            atomicOr(status, DEV_TIMEOUT);
+            return;
+        }
+        if ((spins & 255u) == 255u && (ld_acquire_gpu(status) & DEV_TIMEOUT)) return;
+    }
+}
+
+// x M = a for the 64 vectors of W ([k][vector], leading dimension kLdW) by 256
+// threads: chunks of 16, each solved a vector per thread (64 threads), then
+// applied to the columns behind it by all.  M row-major, leading dimension
+// kTriML (kDiv: with the pivots' reciprocals in the padding).
+template <bool kDiv>
+__device__ __forceinline__ void solve_tile(float *W, const float *M, uint32_t tid) {
+    const uint32_t v = tid & 63, q = tid >> 6;
+#pragma unroll 1
+    for (uint32_t cb = 0; cb < 4; ++cb) {
+        if (tid < 64) {
+            float x[kTriChunk];
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) x[k] = W[(cb * kTriChunk + k) * kLdW + v];
+            tri_chunk_solve<kDiv>(x, M, cb, kT);
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) W[(cb * kTriChunk + k) * kLdW + v] = x[k];
+        }
+        tri_sync();
+        // columns 16 (cb + 1) .. 63: four groups of 4 (3 - cb)
+        for (uint32_t g = 0; g < 3 - cb; ++g) {
+            const uint32_t j0 = (cb + 1) * kTriChunk + q * 4 * (3 - cb) + 4 * g;
+            float y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = W[(j0 + e) * kLdW + v];
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) {
+                const float x = W[(cb * kTriChunk + k) * kLdW + v];
+                const float4 t = *reinterpret_cast<const float4 *>(M + (cb * kTriChunk + k) * kTriML + j0);
+                y[0] = fmaf(-x, t.x, y[0]);
+                y[1] = fmaf(-x, t.y, y[1]);
+                y[2] = fmaf(-x, t.z, y[2]);
+                y[3] = fmaf(-x, t.w, y[3]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) W[(j0 + e) * kLdW + v] = y[e];
+        }
+        tri_sync();
+    }
+}
+
+struct FlowTile {
+    uint32_t i, j, k;  // tile row and column, k = min
+};
+// Tile number idx of nt x nt in the order of the tickets.
+__device__ __forceinline__ FlowTile flow_tile(uint32_t idx, uint32_t nt) {
+    const uint32_t left = nt * nt - idx;  // tiles from here on: (nt - k)^2 at the start of step k
+    uint32_t s = uint32_t(sqrtf(float(left)));
+    while (s * s < left) ++s;
+    while (s > 1 && (s - 1) * (s - 1) >= left) --s;
+    const uint32_t k = nt - s, o = s * s - left;  // o-th tile of step k
+    FlowTile t{k, k, k};
+    if (o & 1)
+        t.i = k + (o + 1) / 2;
+    else
+        t.j = k + o / 2;
+    return t;
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_dense_flow(float *val_base, uint64_t stride, const uint32_t *__restrict__ doff, uint32_t m, uint32_t nt,
+                 uint32_t count, const float *pert_z, float *work, uint64_t work_stride, uint32_t *ctl,
+                 uint32_t *status, uint32_t spin_limit) {
+    extern __shared__ __align__(128) unsigned char flow_smem[];
+    __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
+    __shared__ uint32_t s_item;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        s_item = atomicAdd(ctl, 1u);
+        for (int s = 0; s < kStages; ++s) {
+            bar_init(&full[s], 1);
+            bar_init(&empty[s], kTriThreads / 32);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const uint32_t item = s_item;
+    if (item >= nt * nt * count) return;
+    const uint32_t z = item % count;
+    const FlowTile t = flow_tile(item / count, nt);
+    uint32_t *ready = ctl + 4 + size_t(z) * nt * nt;
+    float *tiles = work + z * work_stride;                       // [i][j][k][v]
+    float *diags = tiles + size_t(nt) * nt * kT * kT;            // [k][0: U rows, 1: L columns]
+    if (warp == kTriThreads / 32) {
+        if (lane == 0) {
+            const uint32_t steps = t.k + (t.i != t.j ? 1u : 0u);
+            for (uint32_t s = 0; s < steps; ++s) {
+                const uint32_t st = s % kStages;
+                unsigned char *dst = flow_smem + st * kStageBytes;
+                if (s >= uint32_t(kStages) && !bar_wait(&empty[st], (s / kStages - 1) & 1, spin_limit))
+                    atomicOr(status, DEV_TIMEOUT);
+                if (s < t.k) {
+                    wait_tile(ready + size_t(t.i) * nt + s, status, spin_limit);
+                    wait_tile(ready + size_t(s) * nt + t.j, status, spin_limit);
+                    proxy_fence();
+                    bar_expect(&full[st], 2 * kTileBytes);
+                    bulk_load(dst, tiles + (size_t(t.i) * nt + s) * kT * kT, kTileBytes, &full[st]);
+                    bulk_load(dst + kTileBytes, tiles + (size_t(s) * nt + t.j) * kT * kT, kTileBytes, &full[st]);
+                } else {
+                    wait_tile(ready + size_t(t.k) * nt + t.k, status, spin_limit);
+                    proxy_fence();
+                    bar_expect(&full[st], kDiagBytes);
+                    bulk_load(dst, diags + (size_t(t.k) * 2 + (t.i > t.j ? 0 : 1)) * kFlowDiagFloats, kDiagBytes,
+                              &full[st]);
+                }
+            }
+            // the block must not end with copies in flight
+            for (uint32_t s = steps > uint32_t(kStages) ? steps - kStages : 0; s < steps; ++s)
+                bar_wait(&full[s % kStages], (s / kStages) & 1, spin_limit);
+        }
+        return;
+    }
+    float *val = val_base + z * stride;
+    const uint32_t tr = tid & 15, tc = tid >> 4;
+    const uint32_t r0 = t.i * kT, c0 = t.j * kT;
+    const uint32_t rows = min(uint32_t(kT), m - r0), cols = min(uint32_t(kT), m - c0);
+    // C: rows 4 tr .. + 3, columns 4 tc .. + 3 (the identity past the block's end)
+    float acc[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const uint32_t c = tc * 4 + b;
+        const float *src = c < cols ? val + doff[c0 + c] + r0 + tr * 4 : nullptr;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const uint32_t r = tr * 4 + a;
+            acc[a][b] = (src && r < rows) ? ld_cg(src + a) : (t.i == t.j && r == c ? 1.0f : 0.0f);
+        }
+    }
+    for (uint32_t s = 0; s < t.k; ++s) {
+        const uint32_t st = s % kStages;
+        if (!bar_wait(&full[st], (s / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+        const float *sL = reinterpret_cast<const float *>(flow_smem + st * kStageBytes) + tr * 4;
+        const float *sU = reinterpret_cast<const float *>(flow_smem + st * kStageBytes + kTileBytes) + tc * 4;
+        // the 64 products in a sum of their own, subtracted once: its roundings
+        // are relative to the sum, not to C
+        float sum[4][4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) sum[a][b] = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < kT; ++k) {
+            const float4 av = *reinterpret_cast<const float4 *>(sL + k * kT);
+            const float4 bv = *reinterpret_cast<const float4 *>(sU + k * kT);
+            const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) sum[a][b] = fmaf(ar[a], br[b], sum[a][b]);
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(&empty[st]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] -= sum[a][b];
+    }
+    float *W = reinterpret_cast<float *>(flow_smem + kStages * kStageBytes);
+    if (t.i == t.j) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            *reinterpret_cast<float4 *>(W + (tc * 4 + b) * kLuLD + tr * 4) =
+                make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
+        tri_sync();
+        tri_lu_smem(W, rows, t.k + 1 < nt, pert_z ? pert_z[z] : 0.0f);
+        if (t.k + 1 < nt) {
+            float *du = diags + size_t(t.k) * 2 * kFlowDiagFloats, *dl = du + kFlowDiagFloats;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t a = tid & 63, b = (tid >> 6) * 4 + 16 * u;  // row a of U, columns b .. b + 3
+                *reinterpret_cast<float4 *>(du + a * kTriML + b) =
+                    make_float4(W[b * kLuLD + a], W[(b + 1) * kLuLD + a], W[(b + 2) * kLuLD + a], W[(b + 3) * kLuLD + a]);
+                const uint32_t c = (tid >> 4) + 16 * u, r = (tid & 15) * 4;  // column c of L, rows r .. r + 3
+                *reinterpret_cast<float4 *>(dl + c * kTriML + r) = *reinterpret_cast<const float4 *>(W + c * kLuLD + r);
+            }
+            if (tid < uint32_t(kT)) du[tid * kTriML + kT] = 1.0f / W[tid * kLuLD + tid];
+            tri_sync();
+            if (tid == 0) st_release_gpu(ready + size_t(t.k) * nt + t.k, 1u);
+        }
+#pragma unroll 4
+        for (uint32_t e = tid; e < uint32_t(kT * kT); e += kTriThreads) {
+            const uint32_t c = e >> 6, r = e & 63;
+            if (c < cols && r < rows) st_cg(val + doff[c0 + c] + r0 + r, W[c * kLuLD + r]);
+        }
+        return;
+    }
+    // solve: [k][vector]; L: k = column, vector = row; U: k = row, vector = column
+    const bool lower = t.i > t.j;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t k = (lower ? tc * 4 + b : tr * 4 + a), v = (lower ? tr * 4 + a : tc * 4 + b);
+            W[k * kLdW + v] = acc[a][b];
+        }
+    const uint32_t st = t.k % kStages;
+    if (!bar_wait(&full[st], (t.k / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+    tri_sync();
+    const float *M = reinterpret_cast<const float *>(flow_smem + st * kStageBytes);
+    if (lower)
+        solve_tile<true>(W, M, tid);
+    else
+        solve_tile<false>(W, M, tid);
+    float *out = tiles + (size_t(t.i) * nt + t.j) * kT * kT;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint32_t k = (tid >> 4) + 16 * u, v = (tid & 15) * 4;
+        const float *w = W + k * kLdW + v;
+        *reinterpret_cast<float4 *>(out + k * kT + v) = make_float4(w[0], w[1], w[2], w[3]);
+    }
+    tri_sync();
+    if (tid == 0) st_release_gpu(ready + size_t(t.i) * nt + t.j, 1u);
+#pragma unroll 4
+    for (uint32_t e = tid; e < uint32_t(kT * kT); e += kTriThreads) {
+        const uint32_t c = e >> 6, r = e & 63;  // down the columns
+        if (c < cols && r < rows)
+            st_cg(val + doff[c0 + c] + r0 + r, lower ? W[c * kLdW + r] : W[r * kLdW + c]);
+    }
+}
+
+size_t dense_flow_floats(uint32_t m) {
+    const size_t nt = (m + kT - 1) / kT;
+    return nt * nt * kT * kT + nt * 2 * kFlowDiagFloats;
+}
+size_t dense_flow_ctl_words(uint32_t m, uint32_t count) {
+    const size_t nt = (m + kT - 1) / kT;
+    return 4 + nt * nt * count;
+}
+
+cudaError_t launch_dense_flow(float *val, uint64_t stride, uint32_t count, const uint32_t *doff, uint32_t m,
+                              const float *pert_z, float *work, uint32_t *ctl, uint32_t *status, uint32_t spin_limit,
+                              cudaStream_t st) {
+    static PerDeviceOnce attr;
+    cudaError_t e = attr.run([] {
+        return cudaFuncSetAttribute(k_dense_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlone));
+    });
+    if (e != cudaSuccess) return e;
+    const uint32_t nt = (m + kT - 1) / kT;
+    e = cudaMemsetAsync(ctl, 0, sizeof(uint32_t) * dense_flow_ctl_words(m, count), st);
+    if (e != cudaSuccess) return e;
+    // One block per SM while the diagonal chain is what takes the time (a
+    // second block's products slow its LU down), two when the tiles' products
+    // do.  Measured, one against two: order 1,920 0.49 / 0.57 ms, order 3,000
+    // 0.90 / 1.02, four of order 1,920 0.81 / 0.75, 96 of order 576 0.73 / 0.59;
+    // equal at order 3,968 and sixteen of 641.
+    const size_t smem = uint64_t(nt) * nt * count <= 3000 ? kSmemAlone : kSmem;
+    k_dense_flow<<<nt * nt * count, kThreads, smem, st>>>(val, stride, doff, m, nt, count, pert_z, work,
+                                                           dense_flow_floats(m), ctl, status, spin_limit);
+    return cudaGetLastError();
+}
+
+}  // namespace glu

@@ -237,7 +237,7 @@ struct glu_handle_s {
     DevBuf d_src_lu, d_src_scale, d_a0_rptr, d_a0_cidx, d_a0_vmap, d_a0_cptr, d_a0_ridx, d_a0_ident, d_ax0;
     bool ax0_loaded = false;
     // work buffers
-    DevBuf d_status, d_pert, d_colmax, d_diag_scratch, d_counters, d_ticket, d_dense_tickets, d_y, d_io32, d_b64,
+    DevBuf d_status, d_pert, d_colmax, d_diag_scratch, d_ticket, d_y, d_io32, d_b64,
         d_x64, d_r64, d_norms;
     uint32_t *h_status = nullptr;  // pinned
     double *h_norms = nullptr;     // pinned
@@ -250,6 +250,10 @@ struct glu_handle_s {
     // tensor-core dense update: BF16 three-part operand packs and their TMA maps
     // (allocated on the first factorization that uses them)
     DevBuf d_packA, d_packB, d_tc_counter;
+    // dataflow factorization of the dense tail: finished tiles of every value
+    // set, then ticket and ready flags (allocated on the first factorization
+    // that uses them)
+    DevBuf d_flow_work;
     // inverses of the dense tail's 64 x 64 diagonal blocks (L and U) per value
     // set, for the dense triangular solves
     DevBuf d_dinv;
@@ -342,6 +346,27 @@ constexpr uint32_t kDenseTcMin = 1024;
 // block.
 constexpr double kCoupleGroupCost = 0.25;
 constexpr double kSparseRate = 0.2e12, kLevelLatency = 8e-6;
+
+// Whether the trailing blocks of order m of `count` value sets are factored by
+// the dataflow kernel (glu_dense_flow.cu) or by panels and updates.  With
+// widths set for look-ahead or tensor-core updates, the blocks below them.
+// With the default widths, whichever a model of both takes less time for:
+//   dataflow  16.8 us per 64 columns (the diagonal chain) against the products
+//             at 36 TFLOP/s, the longer and three tenths of the shorter;
+//   panels    55 us per 64 columns plus the products at 130 TFLOP/s on the
+//             tensor cores.
+// Measured, dataflow / panels: order 1,920 0.49 / 1.51 ms, eight of them 1.22 /
+// 2.18, order 3,968 1.48 / 4.73, three of them 3.39 / 5.75, order 5,000 2.52 /
+// 6.27, 96 of order 576 0.59 / 0.99; twelve of order 9,360 take the panels
+// about 58 ms, the dataflow would take 180.
+bool dense_flow(const glu_tuning &tu, uint32_t m, uint32_t count) {
+    if (m == 0) return false;
+    if (tu.dense_lookahead != kLookaheadMin || tu.dense_tc_min != kDenseTcMin)
+        return (tu.dense_lookahead == 0 || m < tu.dense_lookahead) && (tu.dense_tc_min == 0 || m < tu.dense_tc_min);
+    const double steps = std::ceil(double(m) / kFlowTile), work = double(count) * (2.0 / 3.0) * m * m * m;
+    const double chain = steps * 16.8e-6, products = work / 36e12;
+    return std::max(chain, products) + 0.3 * std::min(chain, products) <= steps * 55e-6 + work / 130e12;
+}
 
 uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_ptr,
                       const std::vector<int32_t> &level_idx, uint32_t max_m, const glu_tuning &tu) {
@@ -1082,9 +1107,7 @@ Status create_handle(int device, SymbolicData &&s, uint32_t batch, glu_handle_t 
     GLU_CUDA(h->d_pert.alloc(sizeof(float) * batch), "allocate");
     GLU_CUDA(h->d_colmax.alloc(sizeof(float) * batch), "allocate");
     GLU_CUDA(h->d_diag_scratch.alloc(sizeof(float) * kDenseNB * kDenseNB * batch), "allocate");
-    GLU_CUDA(h->d_counters.alloc(sizeof(uint32_t) * (size_t(h->n) + 64)), "allocate");
     GLU_CUDA(h->d_ticket.alloc(256), "allocate");
-    GLU_CUDA(h->d_dense_tickets.alloc(sizeof(uint32_t) * 2), "allocate");
     GLU_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h->h_status), 256), "allocate pinned");
     GLU_CUDA(cudaEventCreate(&h->ev0), "event");
     GLU_CUDA(cudaEventCreate(&h->ev1), "event");
@@ -1205,11 +1228,14 @@ SolvePlanDev solve_plan(glu_handle_s *h) {
     return S;
 }
 
+// The dense tail sweeps' two block tickets: behind the status word, in its buffer.
+uint32_t *dense_tickets(const glu_handle_s *h) { return h->d_status.as<uint32_t>() + 16; }
+
 // The buffer of finished unknowns of a solve over nvec vectors, and what the
 // solve's input transform writes for the dense tail sweeps.
 Status solve_buffers(glu_handle_s *h, size_t nvec, SolveInit *init) {
     GLU_CUDA(h->d_xo.ensure(sizeof(float) * size_t(h->n) * nvec), "allocate solve buffer");
-    *init = h->m ? SolveInit{h->d_xo.as<float>(), h->t, h->d_dense_tickets.as<uint32_t>()} : SolveInit{};
+    *init = h->m ? SolveInit{h->d_xo.as<float>(), h->t, dense_tickets(h)} : SolveInit{};
     return GLU_OK;
 }
 
@@ -1219,7 +1245,7 @@ Status solve_buffers(glu_handle_s *h, size_t nvec, SolveInit *init) {
 Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint32_t nrhs, bool trans,
                      cudaStream_t st) {
     GLU_CUDA(h->d_ticket.ensure(sizeof(uint32_t) * std::max<size_t>(count, 64)), "allocate solve tickets");
-    uint32_t *cnt = h->d_dense_tickets.as<uint32_t>();
+    uint32_t *cnt = dense_tickets(h);
     uint32_t *tk = h->d_ticket.as<uint32_t>();
     uint32_t *status = h->d_status.as<uint32_t>();
     const float *val = h->d_val.as<float>() + size_t(z) * h->nnz;
@@ -1683,16 +1709,29 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
     // high-priority internal stream, the rest of the group's update on st,
     // concurrently with the next group's first panel, which it does not touch;
     // the next strips wait for it (the same entries, updated in column order).
-    const bool lookahead = h->aux && h->tune.dense_lookahead && h->m >= h->tune.dense_lookahead && h->m > kDenseNB;
+    bool lookahead = h->aux && h->tune.dense_lookahead && h->m >= h->tune.dense_lookahead && h->m > kDenseNB;
     const uint32_t *doff = h->d_doff.as<uint32_t>();
     float *dscr = h->d_diag_scratch.as<float>();
-    cudaStream_t ps = lookahead ? h->aux : st;  // panels and strips
     bool rest_pending = false;
     const uint32_t nb = kDenseNB;
+    // the whole block by one dataflow launch, where its workspace fits in half
+    // of the free memory
+    bool flow = dense_flow(h->tune, h->m, count);
+    const size_t flow_floats = flow ? dense_flow_floats(h->m) * count : 0;
+    if (flow) {
+        const size_t bytes = sizeof(float) * flow_floats + sizeof(uint32_t) * dense_flow_ctl_words(h->m, count);
+        size_t free_b = 0, total_b = 0;
+        if (bytes > h->d_flow_work.bytes && bytes > (size_t(256) << 20))  // (the query is slow)
+            flow = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= free_b / 2;
+        flow = flow && h->d_flow_work.ensure(bytes) == cudaSuccess;
+        if (!flow) cudaGetLastError();
+    }
+    lookahead = lookahead && !flow;
+    cudaStream_t ps = lookahead ? h->aux : st;  // panels and strips
     // tensor-core updates for wide trailing blocks; their operand packs are
     // allocated once per handle
     const bool tc = h->m && h->tune.dense_tc_min && h->m >= h->tune.dense_tc_min;
-    if (tc && h->pack_m != h->m) {
+    if (tc && (!flow || !h->couple_groups.empty()) && h->pack_m != h->m) {
         const size_t pack_bytes = sizeof(uint16_t) * kDensePackRow * size_t(h->m) * h->batch;
         GLU_CUDA(h->d_packA.alloc(pack_bytes), "allocate tensor-core operand packs");
         GLU_CUDA(h->d_packB.alloc(pack_bytes), "allocate tensor-core operand packs");
@@ -1723,6 +1762,16 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
             upd_bytes += double(count) * (8.0 * mm * mm + 8.0 * nc * mm);
             upd_flops += double(count) * 2.0 * nc * mm * mm;
         }
+    }
+    if (flow) {
+        GLU_LAUNCH(KK_UPDATE,
+                   launch_dense_flow(dbase, dstride, count, doff, h->m, pert, h->d_flow_work.as<float>(),
+                                     reinterpret_cast<uint32_t *>(h->d_flow_work.as<float>() + flow_floats), dstatus,
+                                     h->spin_limit, st),
+                   "factor (dense block)");
+        const double mm = h->m;
+        upd_bytes += double(count) * 8.0 * mm * mm;
+        upd_flops += double(count) * (2.0 / 3.0) * mm * mm * mm;
     }
     if (lookahead) {
         GLU_CUDA(cudaEventRecord(h->ev_fork, st), "event");
@@ -1781,7 +1830,7 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
     const uint32_t group = lookahead ? std::min<uint32_t>(std::max<uint32_t>(h->tune.dense_group, 2u),
                                                           kDenseGroupMax)
                                      : 1u;
-    for (uint32_t k0 = 0; k0 < h->m;) {
+    for (uint32_t k0 = flow ? h->m : 0u; k0 < h->m;) {
         const uint32_t kb0 = std::min<uint32_t>(nb, h->m - k0);
         const uint32_t rest0 = h->m - (k0 + kb0);
         GLU_CUDA(panel(k0, kb0), "factor (dense panel)");

@@ -23,7 +23,7 @@
 namespace glu {
 
 // Panel step (kb <= kDenseNB columns at k0).  Every block factors the
-// diagonal block itself (tri_diag_lu, 256 threads); block 0 stores it to
+// diagonal block itself (tri_lu_smem, 256 threads); block 0 stores it to
 // diag_scratch (the update kernel writes it back, so no block here overwrites
 // an entry another block may still read); blocks [1, 1 + nL) then solve 128
 // rows of L21 (x U11 = a), the rest 128 columns of U12 (L11 x = a), one per
@@ -36,7 +36,9 @@ namespace glu {
 // factorizations would outweigh the row solves.
 constexpr int kPW = kPanelRows + 1;  // leading dimension of the panel work tile
 constexpr size_t kPanelSmem =
-    sizeof(float) * (size_t(kDenseNB) * kPW + size_t(kDenseNB) * kTriML + 2 * kTriMax) + sizeof(uint32_t) * kDenseNB;
+    sizeof(float) * (size_t(kDenseNB) * kPW + size_t(kDenseNB) * kTriML + size_t(kDenseNB) * kLuLD) +
+    sizeof(uint32_t) * kDenseNB;
+static_assert((kDenseNB * kPW) % 4 == 0, "16-byte aligned operand tiles");
 static_assert(kDenseNB == kTriMax, "panel width is the triangular block width");
 static_assert(2 * kPanelRows == kTriThreads, "128 rows per panel block");
 
@@ -48,8 +50,8 @@ __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, ui
     extern __shared__ float4 psm4[];
     float *sW = reinterpret_cast<float *>(psm4);  // [k][thread]: rows of L21 or columns of U12
     float *sM = sW + kDenseNB * kPW;               // U11 (row-major, pivot reciprocals in the padding) or L11^T
-    float(*urow)[kTriMax] = reinterpret_cast<float(*)[kTriMax]>(sM + kDenseNB * kTriML);
-    uint32_t *sCol = reinterpret_cast<uint32_t *>(sM + kDenseNB * kTriML + 2 * kTriMax);
+    float *sS = sM + kDenseNB * kTriML;            // the diagonal block, column-major (tri_lu_smem)
+    uint32_t *sCol = reinterpret_cast<uint32_t *>(sS + kDenseNB * kLuLD);
     float *val = val_base + blockIdx.z * stride;
     const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
     const uint32_t tid = threadIdx.x, b = blockIdx.x + from_scratch;
@@ -72,43 +74,33 @@ __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, ui
     }
     tri_async_commit();
     __syncthreads();
-    // the diagonal block
-    const uint32_t row = tid >> 2, q = tid & 3;
-    float a[kTriChunk];
-    if (from_scratch) {
-        const float *ds = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
-#pragma unroll
-        for (int jj = 0; jj < kTriChunk; ++jj) {
-            const uint32_t cc = q * kTriChunk + jj;
-            a[jj] = (row < kb && cc < kb) ? ld_cg(ds + cc * kDenseNB + row) : 0.0f;
-        }
-    } else {
-#pragma unroll
-        for (int jj = 0; jj < kTriChunk; ++jj) {
-            const uint32_t cc = q * kTriChunk + jj;
-            a[jj] = (row < kb && cc < kb) ? ld_cg(val + sCol[cc] + row) : 0.0f;
-        }
-        // a pivot is perturbed only when its column has an L part
-        tri_diag_lu(a, kb, (r0 < m) || last_has_l, pert, urow);
+    // the diagonal block (the identity past its end)
+    const float *ds = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
+#pragma unroll 16
+    for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kTriThreads) {
+        const uint32_t c = e / kDenseNB, r = e % kDenseNB;
+        float v = r == c ? 1.0f : 0.0f;
+        if (r < kb && c < kb) v = from_scratch ? ld_cg(ds + e) : ld_cg(val + sCol[c] + r);
+        sS[c * kLuLD + r] = v;
     }
+    __syncthreads();
+    // a pivot is perturbed only when its column has an L part
+    if (!from_scratch) tri_lu_smem(sS, kb, (r0 < m) || last_has_l, pert);
     if (b == 0) {
-        float *ds = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
-#pragma unroll
-        for (int jj = 0; jj < kTriChunk; ++jj) {
-            const uint32_t cc = q * kTriChunk + jj;
-            if (row < kb && cc < kb) ds[cc * kDenseNB + row] = a[jj];
-        }
+        float *out = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
+        for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kTriThreads)
+            out[e] = sS[(e / kDenseNB) * kLuLD + e % kDenseNB];
         tri_async_wait();
         return;
     }
     const bool lrows = b <= nL;
-#pragma unroll
-    for (int jj = 0; jj < kTriChunk; ++jj) {
-        const uint32_t cc = q * kTriChunk + jj;
+#pragma unroll 4
+    for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kTriThreads) {
+        const uint32_t i = e / kDenseNB, j = e % kDenseNB;
         if (lrows)
-            sM[row * kTriML + cc] = a[jj];  // M = U11 (row-major)
+            sM[j * kTriML + i] = sS[i * kLuLD + j];  // M = U11 (row-major)
         else
-            sM[cc * kTriML + row] = a[jj];  // M = L11^T
+            sM[i * kTriML + j] = sS[i * kLuLD + j];  // M = L11^T
     }
     if (lrows) {
         __syncthreads();

@@ -100,7 +100,7 @@ constexpr uint32_t kFull = 0xffffffffu;
 
 // Diagonal block of one narrow supernode (2 <= w <= kSnSmallWidth) by one
 // warp: lane r holds row r; step c broadcasts row c by shuffles.  Same
-// operations as tri_diag_lu: pivot c perturbed (GESP) when its column has an
+// operations as tri_lu_smem: pivot c perturbed (GESP) when its column has an
 // L part (c < w - 1, or m > 0); L(r,c) = A(r,c) / U(c,c), then A(r,j) -=
 // L(r,c) U(c,j) for j > c.
 __device__ __forceinline__ void sn_diag_small(const DevPattern &P, const SnPlanDev &S, float *__restrict__ val,
@@ -274,15 +274,15 @@ __device__ __forceinline__ void sn_update_small(const DevPattern &P, const SnPla
 }  // namespace
 
 // Diagonal-block launch of one level: blocks [b0, b0 + gridDim.x) of the
-// diagonal map, each one supernode wider than kSnSmallWidth (tri_diag_lu) or
+// diagonal map, each one supernode wider than kSnSmallWidth (tri_lu_smem) or
 // up to eight narrower ones (a warp each).  The diagonal block is factored in
 // place: pivot c is perturbed (GESP, numeric.cu:139-140) when its column has
 // an L part (c < w - 1, or m > 0); step c: L(i,c) = A(i,c) / U(c,c), then
 // A(i,j) -= L(i,c) U(c,j) for j > c, as in the column algorithm.  blockIdx.z
 // selects the value set.
-__global__ void __launch_bounds__(kTriThreads, 1) k_sn_diag(DevPattern P, SnPlanDev S, float *val_base, uint64_t stride,
+__global__ void __launch_bounds__(kTriThreads, 2) k_sn_diag(DevPattern P, SnPlanDev S, float *val_base, uint64_t stride,
                                                             const float *pert_z, uint32_t b0) {
-    __shared__ __align__(16) float urow[2][kTriMax];
+    __shared__ __align__(16) float sS[kSnMaxWidth * kLuLD];
     __shared__ uint32_t sBase[kSnMaxWidth];
     pdl_release();
     pdl_wait();  // the previous level's updates
@@ -298,18 +298,18 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_sn_diag(DevPattern P, SnPlan
     const uint32_t tid = threadIdx.x, w = d.w;
     if (tid < w) sBase[tid] = P.diag[d.s + tid] - tid;  // position of row s in column s + tid
     __syncthreads();
-    const uint32_t row = tid >> 2, q = tid & 3;
-    float a[kTriChunk];
-#pragma unroll
-    for (int jj = 0; jj < kTriChunk; ++jj) {
-        const uint32_t cc = q * kTriChunk + jj;
-        a[jj] = (row < w && cc < w) ? ld_cg(val + sBase[cc] + row) : 0.0f;
+    const uint32_t end = (w + kLuChunk - 1) / kLuChunk * kLuChunk;  // (the identity past the block's end)
+#pragma unroll 8
+    for (uint32_t e = tid; e < end * kSnMaxWidth; e += kTriThreads) {
+        const uint32_t c = e / kSnMaxWidth, r = e % kSnMaxWidth;
+        sS[c * kLuLD + r] = (r < w && c < w) ? ld_cg(val + sBase[c] + r) : (r == c ? 1.0f : 0.0f);
     }
-    tri_diag_lu(a, w, d.m > 0, pert, urow);
-#pragma unroll
-    for (int jj = 0; jj < kTriChunk; ++jj) {
-        const uint32_t cc = q * kTriChunk + jj;
-        if (row < w && cc < w) st_cg(val + sBase[cc] + row, a[jj]);
+    __syncthreads();
+    tri_lu_smem(sS, w, d.m > 0, pert);
+#pragma unroll 4
+    for (uint32_t e = tid; e < w * kSnMaxWidth; e += kTriThreads) {
+        const uint32_t c = e / kSnMaxWidth, r = e % kSnMaxWidth;
+        if (r < w) st_cg(val + sBase[c] + r, sS[c * kLuLD + r]);
     }
 }
 

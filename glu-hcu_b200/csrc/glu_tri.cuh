@@ -23,58 +23,248 @@ constexpr int kTriML = kTriMax + 4;  // leading dimension of the operand matrix 
 
 #ifdef __CUDACC__
 
-// LU of the w x w block (w <= 64) in registers.  256 threads: thread
-// (row = tid / 4, quarter q = tid % 4) holds a[jj] = A(row, 16 q + jj); rows
-// and columns >= w hold zeros.  Step c: the four threads of row c publish the
-// row (pivot perturbed by GESP, numeric.cu:139-140, when its column has an L
-// part: c < w - 1, or c = w - 1 and last_l), one barrier, then every row
-// below computes L(row, c) = A(row, c) / U(c, c) and A(row, j) -= L(row, c)
-// U(c, j) for j > c.  On return a holds L (strictly lower) and U.  urow:
-// 2 x 64 floats of shared memory, 16-byte aligned.
-__device__ __forceinline__ void tri_diag_lu(float (&a)[kTriChunk], uint32_t w, bool last_l, float pert,
-                                            float (*urow)[kTriMax]) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31;
-    const uint32_t row = tid >> 2, q = tid & 3;
-    const uint32_t warp_last_row = (tid >> 5) * 8 + 7;
-    const uint32_t nq = (w + kTriChunk - 1) / kTriChunk;
-    for (uint32_t cq = 0; cq < nq; ++cq) {
+// Barrier of the first 256 threads of a block (a block may hold further warps
+// with other work).
+__device__ __forceinline__ void tri_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// Leading dimension of the block in shared memory: 16-byte columns, two
+// neighbours' float4 at four rows apart on different banks.
+constexpr int kLuLD = kTriMax + 16;
+
+constexpr int kLuChunk = 8;         // columns per step of the block LU
+
+// a / p from r, p's reciprocal to about one unit in the last place: the
+// quotient's estimate corrected by its remainder (Markstein, IBM J. Res. Dev.
+// 34, 1990).
+__device__ __forceinline__ float lu_quotient(float a, float p, float r) {
+    const float q = a * r;
+    return fmaf(fmaf(-q, p, a), r, q);
+}
+__device__ __forceinline__ float lu_reciprocal(float p) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p));
+    return r;
+}
+
+// Columns [base, base + 8) of the 64 x 64 block S (column-major, leading
+// dimension kLuLD) factored by one warp.  Every lane keeps the 8 x 8 diagonal
+// block in registers and factors it for itself, so the chain of pivots holds
+// no shuffle and no trip through shared memory, only reciprocal, quotient and
+// multiply-add; each lane carries two of the rows below along.
+// kDivide: quotients by division; otherwise by lu_quotient, and nothing is
+// stored and false returned when a pivot is too large or too small for it.
+template <bool kDivide>
+__device__ __forceinline__ bool lu_panel_try(float *S, uint32_t base, uint32_t w, bool last_l, float pert,
+                                             uint32_t lane) {
+    constexpr int N = kLuChunk;
+    float d[N][N], a0[N], a1[N];  // d[row][column]
+    const uint32_t r0 = base + N + lane, r1 = r0 + 32;
+    // (rows past the block: the last row once more, not stored)
+    float *p0 = S + base * kLuLD + min(r0, uint32_t(kTriMax) - 1), *p1 = S + base * kLuLD + min(r1, uint32_t(kTriMax) - 1);
 #pragma unroll
-        for (int jc = 0; jc < kTriChunk; ++jc) {
-            const uint32_t c = cq * kTriChunk + jc;
-            if (c >= w) break;
-            float *u = urow[c & 1];
-            if (row == c) {
-                if (q == cq) {
-                    const bool has_l = c + 1 < w || last_l;
-                    float p = a[jc];
-                    if (has_l && pert > 0.0f && fabsf(p) < pert) p = pert;
-                    a[jc] = p;
-                }
-                float4 *u4 = reinterpret_cast<float4 *>(u + q * kTriChunk);
+    for (int c = 0; c < N; ++c) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(S + (base + c) * kLuLD + base);
 #pragma unroll
-                for (int v = 0; v < kTriChunk / 4; ++v)
-                    u4[v] = make_float4(a[4 * v], a[4 * v + 1], a[4 * v + 2], a[4 * v + 3]);
-            }
-            __syncthreads();
-            if (warp_last_row > c) {  // the warp has rows below the pivot
-                const float lsrc = __shfl_sync(0xffffffffu, a[jc], (lane & ~3u) | cq);
-                if (row > c && row < w) {
-                    const float l = lsrc / u[c];
-                    if (q == cq) a[jc] = l;
-                    const float4 *u4 = reinterpret_cast<const float4 *>(u + q * kTriChunk);
-#pragma unroll
-                    for (int v = 0; v < kTriChunk / 4; ++v) {
-                        const float4 uv = u4[v];
-                        const float us[4] = {uv.x, uv.y, uv.z, uv.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t j = q * kTriChunk + 4 * v + e;
-                            if (j > c) a[4 * v + e] = fmaf(-l, us[e], a[4 * v + e]);
-                        }
-                    }
-                }
-            }
+        for (int v = 0; v < N / 4; ++v) {
+            const float4 t = s4[v];
+            d[4 * v][c] = t.x, d[4 * v + 1][c] = t.y, d[4 * v + 2][c] = t.z, d[4 * v + 3][c] = t.w;
         }
+        a0[c] = p0[c * kLuLD];
+        a1[c] = p1[c * kLuLD];
+    }
+    bool ok = true;  // the same in all lanes, as the diagonal block is
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        const uint32_t next = base + c + 1;
+        if (pert > 0.0f && (next < w || (next == w && last_l)) && fabsf(d[c][c]) < pert) d[c][c] = pert;
+        const float p = d[c][c], mag = fabsf(p);
+        ok = ok && mag > 1e-30f && mag < 1e30f;
+        const float r = kDivide ? 0.0f : lu_reciprocal(p);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i > c) d[i][c] = kDivide ? d[i][c] / p : lu_quotient(d[i][c], p, r);
+        a0[c] = kDivide ? a0[c] / p : lu_quotient(a0[c], p, r);
+        a1[c] = kDivide ? a1[c] / p : lu_quotient(a1[c], p, r);
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (j <= c) continue;
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (i > c) d[i][j] = fmaf(-d[i][c], d[c][j], d[i][j]);
+            a0[j] = fmaf(-a0[c], d[c][j], a0[j]);
+            a1[j] = fmaf(-a1[c], d[c][j], a1[j]);
+        }
+    }
+    if (!kDivide && !ok) return false;
+    __syncwarp();  // every lane has read the panel
+    if (r0 < uint32_t(kTriMax)) {
+#pragma unroll
+        for (int c = 0; c < N; ++c) p0[c * kLuLD] = a0[c];
+    }
+    if (r1 < uint32_t(kTriMax)) {
+#pragma unroll
+        for (int c = 0; c < N; ++c) p1[c * kLuLD] = a1[c];
+    }
+    // lane 2 c + v stores rows 4 v .. 4 v + 3 of column c, chosen by selects (a
+    // branch per value, or one lane storing all of them, takes longer)
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        float t[N];
+#pragma unroll
+        for (int c = 0; c < N; ++c) t[c] = (lane & 1) ? d[4 + e][c] : d[e][c];
+#pragma unroll
+        for (int c = 0; c < N / 2; ++c) t[c] = (lane & 2) ? t[2 * c + 1] : t[2 * c];
+#pragma unroll
+        for (int c = 0; c < N / 4; ++c) t[c] = (lane & 4) ? t[2 * c + 1] : t[2 * c];
+        o[e] = (lane & 8) ? t[1] : t[0];
+    }
+    if (lane < 2 * N)
+        *reinterpret_cast<float4 *>(S + (base + (lane >> 1)) * kLuLD + base + 4 * (lane & 1)) =
+            make_float4(o[0], o[1], o[2], o[3]);
+    return true;
+}
+// (out of line: its divisions would take the common path's registers)
+static __device__ __noinline__ void lu_panel_divide(float *S, uint32_t base, uint32_t w, bool last_l, float pert,
+                                                    uint32_t lane) {
+    lu_panel_try<true>(S, base, w, last_l, pert, lane);
+}
+__device__ __forceinline__ void lu_panel(float *S, uint32_t base, uint32_t w, bool last_l, float pert, uint32_t lane) {
+    if (!lu_panel_try<false>(S, base, w, last_l, pert, lane)) lu_panel_divide(S, base, w, last_l, pert, lane);
+}
+
+// Columns j and j + 1 of the block behind columns [base, base + 8), by eight
+// threads: each solves the columns' 8 entries of U (L11 x = a, the same values
+// in all eight) and updates the rows base + 8 + 4 q + 32 g .. + 3 with them.
+// (Shared-memory loads bound it: an entry of L serves two columns.)
+__device__ __forceinline__ void lu_columns(float *S, uint32_t base, uint32_t j, uint32_t q) {
+    constexpr int N = kLuChunk;
+    float *col[2] = {S + j * kLuLD + base, S + (j + 1) * kLuLD + base};
+    // rows of this thread, relative to base (past the block: the last four, not stored)
+    const uint32_t last = uint32_t(kTriMax) - 4 - base, r0 = N + 4 * q, r1 = r0 + 32;
+    const uint32_t o0 = min(r0, last), o1 = min(r1, last);
+    float x[2][N];
+    float4 c[2][2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const float4 u = *reinterpret_cast<const float4 *>(col[b]), v = *reinterpret_cast<const float4 *>(col[b] + 4);
+        x[b][0] = u.x, x[b][1] = u.y, x[b][2] = u.z, x[b][3] = u.w;
+        x[b][4] = v.x, x[b][5] = v.y, x[b][6] = v.z, x[b][7] = v.w;
+        c[b][0] = *reinterpret_cast<const float4 *>(col[b] + o0);
+        c[b][1] = *reinterpret_cast<const float4 *>(col[b] + o1);
+    }
+    const float *lp = S + base * kLuLD + base;
+#pragma unroll
+    for (int k = 0; k + 1 < N; ++k) {
+        const float4 u = *reinterpret_cast<const float4 *>(lp + k * kLuLD);
+        const float4 v = *reinterpret_cast<const float4 *>(lp + k * kLuLD + 4);
+        const float l[N] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int r = 0; r < N; ++r)
+            if (r > k) {
+                x[0][r] = fmaf(-l[r], x[0][k], x[0][r]);
+                x[1][r] = fmaf(-l[r], x[1][k], x[1][r]);
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float4 l0 = *reinterpret_cast<const float4 *>(lp + k * kLuLD + o0);
+        const float4 l1 = *reinterpret_cast<const float4 *>(lp + k * kLuLD + o1);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            c[b][0].x = fmaf(-l0.x, x[b][k], c[b][0].x);
+            c[b][0].y = fmaf(-l0.y, x[b][k], c[b][0].y);
+            c[b][0].z = fmaf(-l0.z, x[b][k], c[b][0].z);
+            c[b][0].w = fmaf(-l0.w, x[b][k], c[b][0].w);
+            c[b][1].x = fmaf(-l1.x, x[b][k], c[b][1].x);
+            c[b][1].y = fmaf(-l1.y, x[b][k], c[b][1].y);
+            c[b][1].z = fmaf(-l1.z, x[b][k], c[b][1].z);
+            c[b][1].w = fmaf(-l1.w, x[b][k], c[b][1].w);
+        }
+    }
+    __syncwarp();  // the eight threads of the columns have read them
+    if (r0 <= last) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) *reinterpret_cast<float4 *>(col[b] + r0) = c[b][0];
+    }
+    if (r1 <= last) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) *reinterpret_cast<float4 *>(col[b] + r1) = c[b][1];
+    }
+    if (q == 0) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            *reinterpret_cast<float4 *>(col[b]) = make_float4(x[b][0], x[b][1], x[b][2], x[b][3]);
+            *reinterpret_cast<float4 *>(col[b] + 4) = make_float4(x[b][4], x[b][5], x[b][6], x[b][7]);
+        }
+    }
+}
+
+// Column j of the block behind columns [base, base + 8), by one warp: every lane
+// solves the column's 8 entries of U and updates rows base + 8 + lane and
+// base + 40 + lane with them.
+__device__ __forceinline__ void lu_one_column(float *S, uint32_t base, uint32_t j, uint32_t lane) {
+    constexpr int N = kLuChunk;
+    float *col = S + j * kLuLD + base;
+    const float *lp = S + base * kLuLD + base;
+    // (rows past the block: the last one once more, not stored)
+    const uint32_t last = uint32_t(kTriMax) - 1 - base, r0 = N + lane, r1 = r0 + 32;
+    const uint32_t o0 = min(r0, last), o1 = min(r1, last);
+    const float4 u = *reinterpret_cast<const float4 *>(col), v = *reinterpret_cast<const float4 *>(col + 4);
+    float x[N] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    float c0 = col[o0], c1 = col[o1], l0[N], l1[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        l0[k] = lp[k * kLuLD + o0];
+        l1[k] = lp[k * kLuLD + o1];
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float4 lu = *reinterpret_cast<const float4 *>(lp + k * kLuLD);
+        const float4 lv = *reinterpret_cast<const float4 *>(lp + k * kLuLD + 4);
+        const float l[N] = {lu.x, lu.y, lu.z, lu.w, lv.x, lv.y, lv.z, lv.w};
+#pragma unroll
+        for (int r = 0; r < N; ++r)
+            if (r > k) x[r] = fmaf(-l[r], x[k], x[r]);
+        c0 = fmaf(-l0[k], x[k], c0);
+        c1 = fmaf(-l1[k], x[k], c1);
+    }
+    __syncwarp();  // every lane has read the column
+    if (r0 <= last) col[r0] = c0;
+    if (r1 <= last) col[r1] = c1;
+    if (lane == 0) {
+        *reinterpret_cast<float4 *>(col) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4 *>(col + 4) = make_float4(x[4], x[5], x[6], x[7]);
+    }
+}
+
+// LU of the w x w block (w <= 64) in shared memory, S column-major with leading
+// dimension kLuLD, 256 threads; rows and columns >= w must hold the identity.
+// Right-looking by chunks of 8 columns.  Behind a chunk, each warp first takes
+// one column of the next chunk (lu_one_column); then warp 0 factors that chunk
+// (lu_panel) while the others update the columns further right (lu_columns).
+// Every entry receives its updates in increasing column order, then (L
+// entries) its division by the pivot, GESP as numeric.cu:139-140 (a pivot
+// whose column has an L part: c < w - 1, or c = w - 1 and last_l).
+// A 64-wide block takes 12,100 cycles on its own; 30,700 with a row per four
+// threads, a barrier and a division per pivot (the division's slow path is
+// taken for every zero of a sparse or padded row).
+// The caller has a barrier between its writes of S and the call; on return the
+// block is complete for all 256 threads.
+__device__ __forceinline__ void tri_lu_smem(float *S, uint32_t w, bool last_l, float pert) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t end = (w + kLuChunk - 1) / kLuChunk * kLuChunk;  // columns to factor
+    if (warp == 0) lu_panel(S, 0, w, last_l, pert, lane);
+    tri_sync();
+#pragma unroll 1
+    for (uint32_t base = 0; base + kLuChunk < end; base += kLuChunk) {
+        lu_one_column(S, base, base + kLuChunk + warp, lane);
+        tri_sync();
+        if (warp == 0)
+            lu_panel(S, base + kLuChunk, w, last_l, pert, lane);
+        else if (base + kLuChunk * (warp + 1) < end)
+            lu_columns(S, base, base + kLuChunk * (warp + 1) + 2 * (lane >> 3), lane & 7);
+        tri_sync();
     }
 }
 

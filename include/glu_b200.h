@@ -290,7 +290,11 @@ typedef struct {
                                   per warp, grouped into blocks; 0: a block each */
     uint32_t dense_lookahead;  /* dense trailing blocks at least this wide factor
                                   the next panel during the current update
-                                  (0: never)                                     */
+                                  (0: never).  A block below this width and
+                                  below dense_tc_min is factored by one dataflow
+                                  launch over its tiles (profiled as
+                                  k_dense_update); with both at their defaults
+                                  a cost model chooses                          */
     uint32_t dense_tc_min;     /* dense trailing blocks at least this wide update
                                   on the tensor cores (tcgen05, FP32 accuracy by
                                   a three-part BF16 split), each update region
