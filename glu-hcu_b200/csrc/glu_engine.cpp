@@ -221,6 +221,11 @@ struct glu_handle_s {
     uint32_t couple_cols = 0;
     DevBuf d_ss_map[2], d_ss_meta[2], d_ss_small[2];  // supernodal L and U sweeps
     DevBuf d_ss_woff[2], d_ss_widx[2], d_ss_roff[2], d_ss_ridx[2], d_ss_indeg[2];  // their fused form
+    // wide supernodes {first column, width}, their number in each sweep's order,
+    // and per value set the inverses of their diagonal blocks (empty: the
+    // sweeps solve those blocks column by column)
+    DevBuf d_wide, d_ss_wide[2], d_sn_inv;
+    uint32_t nwide = 0;
     DevBuf d_sweep_done;  // per value set and supernode: releases received (fused sweeps)
     std::vector<SnSweepLevel> ss_levels[2];
     // solve plan
@@ -732,6 +737,22 @@ Status build_sn_plan(glu_handle_s *h) {
         upd_bytes += 4.0 * double(entries);
     }
     cudaGetLastError();
+    // Wide supernodes, whose diagonal blocks the sweeps multiply by their
+    // inverses.  Those take 32 KB each and value set: kept while they are at
+    // most half of the values themselves, or 64 MB.
+    std::vector<uint2> wide;
+    std::vector<uint32_t> wide_no(ns, UINT32_MAX);
+    for (uint32_t q = 0; q < ns; ++q)
+        if (first[q + 1] - first[q] > kSnSmallWidth) {
+            wide_no[q] = uint32_t(wide.size());
+            wide.push_back(make_uint2(first[q], first[q + 1] - first[q]));
+        }
+    if (sizeof(float) * kSnInvFloats * double(wide.size()) * h->batch >
+        std::max(0.5 * sizeof(float) * double(h->nnz) * h->batch, 64e6))
+        wide.clear();
+    h->nwide = uint32_t(wide.size());
+    h->d_sn_inv.release();
+    GLU_CUDA(upload(h->d_wide, wide), "upload solve plan");
     // supernodal solve sweeps: L forward (waits for the supernodes whose L21
     // rows fall in it), U backward (waits for the supernodes holding its targets)
     for (int u = 0; u < 2; ++u) {
@@ -765,6 +786,8 @@ Status build_sn_plan(glu_handle_s *h) {
             for (uint32_t q = 0; q < ns; ++q) ord[cur[sl[q]]++] = q;
         }
         std::vector<uint4> smeta(ns);
+        std::vector<uint32_t> swide(ns);
+        for (uint32_t i = 0; i < ns; ++i) swide[i] = wide_no[ord[i]];
         std::vector<uint2> smap;
         std::vector<uint32_t> ssmall;
         h->ss_levels[u].clear();
@@ -857,6 +880,7 @@ Status build_sn_plan(glu_handle_s *h) {
         GLU_CUDA(upload(h->d_ss_roff[u], roff), "upload solve plan");
         GLU_CUDA(upload(h->d_ss_ridx[u], ridx), "upload solve plan");
         GLU_CUDA(upload(h->d_ss_indeg[u], indeg), "upload solve plan");
+        GLU_CUDA(upload(h->d_ss_wide[u], swide), "upload solve plan");
         GLU_CUDA(upload(h->d_ss_small[u], ssmall), "upload solve plan");
         GLU_CUDA(upload(h->d_ss_map[u], smap), "upload solve plan");
         GLU_CUDA(upload(h->d_ss_meta[u], smeta), "upload solve plan");
@@ -864,6 +888,7 @@ Status build_sn_plan(glu_handle_s *h) {
         pl.map = h->d_ss_map[u].as<uint2>();
         pl.meta = h->d_ss_meta[u].as<uint4>();
         pl.small = h->d_ss_small[u].as<uint32_t>();
+        pl.wide = h->d_ss_wide[u].as<uint32_t>();
         pl.levels = h->ss_levels[u].data();
         pl.nlev = uint32_t(h->ss_levels[u].size());
         pl.fused = h->tune.sn_sweep_fused;
@@ -1217,6 +1242,13 @@ uint64_t solve_kernel_count(const glu_handle_s *h, bool trans) {
 // Floats of the dense tail's diagonal-block inverses of one value set.
 size_t dinv_per_set(const glu_handle_s *h) { return size_t((h->m + 63) / 64) * 2 * 64 * 64; }
 
+// The wide supernodes' inverses of value set z (none: null).
+void set_sn_inv(const glu_handle_s *h, uint32_t z, SolveBatch &B) {
+    if (!h->use_sn || !h->nwide || !h->d_sn_inv.p) return;
+    B.sn_inv_stride = uint64_t(h->nwide) * kSnInvFloats;
+    B.sn_inv = h->d_sn_inv.as<float>() + z * B.sn_inv_stride;
+}
+
 // The solve plan of the next solve: the handle's, with a pending
 // GLU_INJECT_UNSET_SOLVE_FLAG applied (and consumed).
 SolvePlanDev solve_plan(glu_handle_s *h) {
@@ -1255,6 +1287,7 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
     B.vstride = h->nnz;
     B.dstride = h->dense_buffer ? uint64_t(h->m) * h->m : h->nnz;
     B.dinv = h->m ? h->d_dinv.as<float>() + size_t(z) * dinv_per_set(h) : nullptr;
+    set_sn_inv(h, z, B);
     if (h->tune.sn_sweep_fused && h->use_sn) {
         const size_t ns = std::max(h->S.sn[0].ns, h->S.sn[1].ns);
         GLU_CUDA(h->d_sweep_done.ensure(sizeof(uint32_t) * ns * count + 4), "allocate sweep counters");
@@ -1263,16 +1296,19 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
     float *xo = h->d_xo.as<float>();
     const SolvePlanDev S = solve_plan(h);
     h->stats.solve_launches += solve_kernel_count(h, trans);
-    if (!trans) {
-        GLU_CUDA(solve_lower_unit(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, st), "lower solve");
-        GLU_CUDA(solve_upper(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, st), "upper solve");
-    } else {
-        GLU_CUDA(solve_upper_trans(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, st),
-                 "transposed upper solve");
-        GLU_CUDA(solve_lower_unit_trans(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, st),
-                 "transposed lower solve");
-    }
-    return GLU_OK;
+    auto enqueue = [&](cudaStream_t s) -> Status {
+        if (!trans) {
+            GLU_CUDA(solve_lower_unit(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s), "lower solve");
+            GLU_CUDA(solve_upper(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s), "upper solve");
+        } else {
+            GLU_CUDA(solve_upper_trans(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s),
+                     "transposed upper solve");
+            GLU_CUDA(solve_lower_unit_trans(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s),
+                     "transposed lower solve");
+        }
+        return GLU_OK;
+    };
+    return enqueue(st);
 }
 
 Status solve_f32(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const float *b, float *x,
@@ -1344,6 +1380,7 @@ Status solve_f32_scratch(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const fl
     const SolvePlanDev S = solve_plan(h);
     SolveBatch one;
     one.dinv = h->m ? h->d_dinv.as<float>() + size_t(inst) * dinv_per_set(h) : nullptr;
+    set_sn_inv(h, inst, one);
     GLU_CUDA(solve_lower_unit(h->P, S, val, dval, y, xo, nrhs, flags, ticket, status, one, st), "lower solve");
     GLU_CUDA(solve_upper(h->P, S, val, dval, y, xo, nrhs, flags, ticket, status, one, st), "upper solve");
     GLU_CUDA(launch_transform_f32(T.out_idx, T.out_scale, y, x, h->n, nrhs, SolveInit{}, st), "transform");
@@ -1896,6 +1933,16 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
                    launch_dense_diag_inv(dbase, dstride, count, doff, h->m,
                                          h->d_dinv.as<float>() + size_t(first) * dinv_per_set(h), st),
                    "factor (diagonal-block inverses)");
+    }
+    if (h->use_sn && h->nwide) {
+        const uint64_t per = uint64_t(h->nwide) * kSnInvFloats;
+        if (h->d_sn_inv.ensure(sizeof(float) * per * h->batch) == cudaSuccess)
+            GLU_LAUNCH(KK_DIAG_INV,
+                       launch_sn_diag_inv(h->P, h->d_wide.as<uint2>(), h->nwide, val, stride, count,
+                                          h->d_sn_inv.as<float>() + first * per, per, st),
+                       "factor (supernode inverses)");
+        else
+            cudaGetLastError();
     }
     GLU_LAUNCH(KK_CHECK, launch_check_pivots(h->P, val, stride, count, h->d_status.as<uint32_t>(), st), "pivot check");
 #undef GLU_LAUNCH

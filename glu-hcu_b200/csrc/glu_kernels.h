@@ -242,6 +242,7 @@ struct SnSweepPlan {
     const uint2 *map = nullptr;     // {supernode, part} or {first of small[], kSnSmallFlag | count}
     const uint4 *meta = nullptr;
     const uint32_t *small = nullptr;  // small supernodes, grouped eight to a block
+    const uint32_t *wide = nullptr;   // per supernode its number among the wide ones (UINT32_MAX: not wide)
     const SnSweepLevel *levels = nullptr;  // host array
     uint32_t nlev = 0;
     // One launch for the whole sweep (fused != 0): blocks take tickets in map
@@ -265,12 +266,22 @@ struct SolveBatch {
     uint64_t vstride = 0;
     uint64_t dstride = 0;
     const float *dinv = nullptr;  // inverses of the dense tail's diagonal blocks of the first set
+    // inverses of the wide supernodes' diagonal blocks of the first set (null:
+    // none), the next set's sn_inv_stride further
+    const float *sn_inv = nullptr;
+    uint64_t sn_inv_stride = 0;
     uint32_t *sweep_done = nullptr;  // count x (supernodes) counters of the fused sweeps (null: per level)
 };
 // Inverses of the 64 x 64 diagonal blocks of the dense tail's L and U, per
 // value set: dinv[z][b][0: L, 1: U][64 x 64] (row-major), from the factors.
 cudaError_t launch_dense_diag_inv(const float *dval, uint64_t dstride, uint32_t count, const uint32_t *doff,
                                   uint32_t m, float *dinv, cudaStream_t st);
+
+constexpr uint32_t kSnInvFloats = 2 * kSnMaxWidth * kSnMaxWidth;  // of one wide supernode
+// Inverses of the diagonal blocks of `nwide` supernodes {first column, width},
+// width > kSnSmallWidth: invs[z][k][0: L, 1: U][64 x 64] (row-major).
+cudaError_t launch_sn_diag_inv(const DevPattern &P, const uint2 *wide, uint32_t nwide, const float *val,
+                               uint64_t vstride, uint32_t count, float *invs, uint64_t inv_stride, cudaStream_t st);
 
 struct SolvePlanDev {
     uint32_t t;                     // first column of the dense tail (n if none)

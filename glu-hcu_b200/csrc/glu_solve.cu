@@ -24,6 +24,7 @@
 
 #include "glu_common.cuh"
 #include "glu_kernels.h"
+#include "glu_tri.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -267,97 +268,17 @@ __device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, uint32_t *st
 
 // Inverses of the 64 x 64 diagonal blocks of the dense tail: blockIdx.y = 0
 // the unit lower L_bb, 1 the upper U_bb; dinv[z][b][which] row-major (rows
-// past the tail's end are the identity).  U_bb is taken as its transpose, so
-// both are the inverse of a lower triangular M: the four 16 x 16 diagonal
-// blocks by substitution (a column per thread, in registers), then twice the
-// off-diagonal block of a pair, X21 = -X22 M21 X11, as products over all
-// threads -- 16 dependent steps instead of 64 (8.3 us at order 128, 28 us
-// with 64 threads of serial substitution).  blockIdx.z selects the value set.
+// past the tail's end are the identity).  blockIdx.z selects the value set.
 __global__ void __launch_bounds__(256) k_dense_diag_inv(const float *__restrict__ val, uint64_t dstride,
                                                          const uint32_t *__restrict__ doff, uint32_t m,
                                                          float *__restrict__ dinv) {
-    constexpr int LD = kRB + 1;
-    __shared__ float M[kRB][LD];
-    __shared__ float X[kRB][LD];
-    __shared__ float W[kRB / 2][kRB / 2 + 1];
-    const uint32_t b = blockIdx.x, which = blockIdx.y, tid = threadIdx.x;
+    __shared__ TriInverse T;
+    const uint32_t b = blockIdx.x, which = blockIdx.y;
     const uint32_t nb = (m + kRB - 1) / kRB;
     val += blockIdx.z * dstride;
     const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
-#pragma unroll 4
-    for (uint32_t e = tid; e < uint32_t(kRB * kRB); e += 256) {
-        const uint32_t c = e / kRB, i = e % kRB;
-        float v = i == c ? 1.0f : 0.0f;
-        if (i < rows && c < rows && (which == 0 ? i > c : i <= c)) v = val[doff[rb0 + c] + rb0 + i];
-        if (which == 0)
-            M[i][c] = v;
-        else
-            M[c][i] = v;
-        X[i][c] = 0.0f;
-    }
-    __syncthreads();
-    if (tid < uint32_t(kRB)) {  // column j of the 16 x 16 block at g
-        const uint32_t g = tid & ~15u, j = tid & 15u;
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int k = 0; k < i; ++k) acc = fmaf(M[g + i][g + k], x[k], acc);
-            // zero above the diagonal: x[k] = 0 for k < j
-            x[i] = (uint32_t(i) == j ? 1.0f : uint32_t(i) > j ? -acc : 0.0f) / M[g + i][g + i];
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) X[g + i][g + j] = x[i];
-    }
-    __syncthreads();
-    // pairs of 16-blocks: 2 x 256 outputs; W = M21 X11, X21 = -X22 W
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const uint32_t g = u * 32, i = tid / 16, j = tid % 16;
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) acc = fmaf(M[g + 16 + i][g + k], X[g + k][g + j], acc);
-        W[u * 16 + i][j] = acc;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const uint32_t g = u * 32, i = tid / 16, j = tid % 16;
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) acc = fmaf(X[g + 16 + i][g + 16 + k], W[u * 16 + k][j], acc);
-        X[g + 16 + i][g + j] = -acc;
-    }
-    __syncthreads();
-    // the pair of 32-blocks
-    const uint32_t j = tid % 32, i0 = tid / 32;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-        const float xv = X[k][j];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = fmaf(M[32 + i0 + 8 * u][k], xv, acc[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        W[i0 + 8 * u][j] = acc[u];
-        acc[u] = 0.0f;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-        const float wv = W[k][j];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = fmaf(X[32 + i0 + 8 * u][32 + k], wv, acc[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) X[32 + i0 + 8 * u][j] = -acc[u];
-    __syncthreads();
-    float *out = dinv + ((size_t(blockIdx.z) * nb + b) * 2 + which) * kRB * kRB;
-#pragma unroll 4
-    for (uint32_t e = tid; e < uint32_t(kRB * kRB); e += 256)
-        out[e] = which == 0 ? X[e / kRB][e % kRB] : X[e % kRB][e / kRB];
+    tri_invert(T, which, rows, dinv + ((size_t(blockIdx.z) * nb + b) * 2 + which) * kRB * kRB,
+               [&](uint32_t i, uint32_t c) { return val[doff[rb0 + c] + rb0 + i]; });
 }
 
 // One item: its value set, first right-hand side and block (in solve order).

@@ -4,8 +4,10 @@
 // src/symbolic.cc:226-239).  With the factor's supernodes (runs of columns
 // [s, s+w) with a dense diagonal block and a common lower pattern) a sweep
 // step is a whole supernode: its w unknowns are solved against the dense
-// diagonal block (one warp, the block staged in shared memory) and their
-// off-diagonal entries are then scattered into the unknowns they feed:
+// diagonal block (wide ones: a product with the block's inverse, computed once
+// per factorization by k_sn_diag_inv; else a chain over the columns by one
+// warp) and their off-diagonal entries are then scattered into the unknowns
+// they feed:
 //   L (forward, unit):  x_S = L11^-1 y_S;  y_r -= L21(r,:) x_S for the m rows
 //                       below the block (one thread per row, dot over w);
 //   U (backward):       x_S = U11^-1 y_S;  y_i -= U(i,c) x_c for the entries
@@ -17,8 +19,21 @@
 // Every block finds its supernode and part through a precomputed map; small
 // supernodes (width <= kSnSmallWidth with at most 32 off-diagonal rows or
 // entries) go eight to a block, one warp each.
+//
+// What bounds the sweeps is the chain of levels, each a launch chained to the
+// one before, so the time from a level's last scatter to the next one's counts:
+// a block reads everything that does not depend on the unknowns (plan,
+// pattern, factors, inverse) before it waits for the previous level, and
+// between that wait and its own scatter there is one read of y, the solve
+// against the diagonal block and the products.  Several right-hand sides are
+// spread over the grid's second dimension.  (FP32 solve of a 251 x 251 grid, 70
+// levels: 656 -> 399 us against waiting first and solving the block by a chain
+// with divisions; 32 right-hand sides at n = 4,960: 576 -> 286 us.)
+#include <algorithm>
+
 #include "glu_common.cuh"
 #include "glu_kernels.h"
+#include "glu_tri.cuh"
 
 namespace glu {
 
@@ -26,11 +41,20 @@ namespace {
 constexpr int kLD = kSnMaxWidth + 1;
 constexpr uint32_t kFull = 0xffffffffu;
 
+// Right-hand sides [q0, q1) of a block: blockIdx.y's share of nrhs.
+struct Rhs {
+    uint32_t q0, q1;
+};
+__device__ __forceinline__ Rhs rhs_share(uint32_t nrhs) {
+    const uint32_t per = (nrhs + gridDim.y - 1) / gridDim.y, q0 = blockIdx.y * per;
+    return Rhs{q0, min(q0 + per, nrhs)};
+}
+
 // L sweep of one small supernode (w <= kSnSmallWidth, m <= 32) by one warp:
 // lane k holds unknown s+k and L21 row k; the entries it needs are loaded
 // before the dependency chain starts.
 __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSweepPlan &W,
-                                                 const float *__restrict__ val, float *y, float *xo, uint32_t nrhs,
+                                                 const float *__restrict__ val, float *y, float *xo, Rhs Q,
                                                  uint32_t i, uint32_t lane) {
     constexpr int SW = int(kSnSmallWidth);
     const uint4 md = W.meta[i];
@@ -44,7 +68,8 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
         l21[c] = (lane < m && uint32_t(c) < w) ? __ldg(val + dc + (l + 1 - (s + c)) + lane) : 0.0f;
     }
     const uint32_t target = lane < m ? __ldg(P.ridx + lbase + lane) : 0u;
-    for (uint32_t q = 0; q < nrhs; ++q) {
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
         float v = lane < w ? __ldcg(yq + s + lane) : 0.0f;
 #pragma unroll
@@ -67,7 +92,7 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
 // U sweep of one small supernode (w <= kSnSmallWidth, at most 32 entries above
 // the block) by one warp: lane k holds unknown s+k and above-block entry k.
 __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSweepPlan &W,
-                                                 const float *__restrict__ val, float *y, float *xo, uint32_t nrhs,
+                                                 const float *__restrict__ val, float *y, float *xo, Rhs Q,
                                                  uint32_t i, uint32_t lane) {
     constexpr int SW = int(kSnSmallWidth);
     const uint4 md = W.meta[i];
@@ -99,13 +124,19 @@ __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSw
         urow[cc] = (lane < uint32_t(cc) && uint32_t(cc) < w) ? __ldg(val + dcc - (cc - lane)) : 0.0f;
     }
     const float piv = lane < w ? __ldg(val + dl) : 1.0f;
-    for (uint32_t q = 0; q < nrhs; ++q) {
+    // reciprocals before the chain, unless a pivot is too large or too small
+    const float mag = fabsf(piv), rec = lu_reciprocal(piv);
+    const bool quick = __all_sync(kFull, mag > 1e-30f && mag < 1e30f);
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
         float v = lane < w ? __ldcg(yq + s + lane) : 0.0f;
 #pragma unroll
         for (int cc = SW - 1; cc >= 0; --cc) {
             if (uint32_t(cc) >= w) continue;
-            const float xc = __shfl_sync(kFull, v, cc) / __shfl_sync(kFull, piv, cc);
+            // every lane divides its own value, so that the step is one shuffle long
+            const float d = quick ? lu_quotient(v, piv, rec) : v / piv;
+            const float xc = __shfl_sync(kFull, d, cc);
             if (lane == uint32_t(cc)) v = xc;
             if (lane < uint32_t(cc)) v = __fsub_rn(v, __fmul_rn(urow[cc], xc));
         }
@@ -154,12 +185,42 @@ __device__ __forceinline__ void sweep_release(const SnSweepPlan &W, uint32_t blk
 }
 }  // namespace
 
+// x = T^-1 v of a wide supernode by all 256 threads: thread (row, quarter) holds
+// the inverse's 16 entries iv of its row and quarter; v (w values, zero beyond)
+// in shared memory before the call, x in xs after it (two barriers inside).
+__device__ __forceinline__ void wide_solve(const float (&iv)[16], const float *vs, float (*part)[kSnMaxWidth], float *xs,
+                                           uint32_t tid) {
+    const uint32_t row = tid & 63, q = tid >> 6;
+    const float4 *v4 = reinterpret_cast<const float4 *>(vs + q * 16);
+    float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+        const float4 v = v4[k / 4];
+        a0 = fmaf(iv[k], v.x, a0);
+        a1 = fmaf(iv[k + 1], v.y, a1);
+        a0 = fmaf(iv[k + 2], v.z, a0);
+        a1 = fmaf(iv[k + 3], v.w, a1);
+    }
+    part[q][row] = a0 + a1;
+    __syncthreads();
+    if (tid < kSnMaxWidth) xs[tid] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+    __syncthreads();
+}
+__device__ __forceinline__ void load_inverse(float (&iv)[16], const float *__restrict__ inv, uint32_t tid) {
+    const float4 *p = reinterpret_cast<const float4 *>(inv + (tid & 63) * kSnMaxWidth + (tid >> 6) * 16);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 v = __ldg(p + k);
+        iv[4 * k] = v.x, iv[4 * k + 1] = v.y, iv[4 * k + 2] = v.z, iv[4 * k + 3] = v.w;
+    }
+}
+
 __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
-                                                    uint64_t vstride, uint64_t ystride, uint32_t *done,
+                                                    uint64_t vstride, uint64_t ystride,
+                                                    const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
                                                     uint32_t *ticket, uint32_t *status, uint32_t spin_limit) {
     pdl_release();
-    pdl_wait();  // the previous level's x (per-level launches are chained)
     const uint2 bz = sweep_block(W, b0, done, ticket, status, spin_limit);
     const uint32_t blk = bz.x;
     val += bz.y * vstride;  // value set bz.y, its right-hand sides
@@ -167,12 +228,14 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     xo += bz.y * ystride;
     if (done) done += size_t(bz.y) * W.ns;
     if (blk == UINT32_MAX) return;
+    const Rhs Q = rhs_share(nrhs);
     __shared__ float sT[kSnMaxWidth * kLD];
-    __shared__ float xs[kSnMaxWidth];
+    __shared__ __align__(16) float xs[kSnMaxWidth], vs[kSnMaxWidth];
+    float(*part)[kSnMaxWidth] = reinterpret_cast<float(*)[kSnMaxWidth]>(sT);
     const uint2 bi = W.map[blk];
     if (bi.y & kSnSmallFlag) {  // a group of small supernodes, one per warp
         const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_l_small(P, W, val, y, xo, nrhs, W.small[bi.x + wi], threadIdx.x & 31);
+        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_l_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
         sweep_release(W, blk, done);
         return;
     }
@@ -180,6 +243,7 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     const uint32_t s = md.x, w = md.y, lbase = md.z, m = md.w, t = bi.y;
     const uint32_t l = s + w - 1;
     const uint32_t tid = threadIdx.x, n = P.n;
+    const uint32_t wide = (invs && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
     __shared__ uint32_t sB[kSnMaxWidth];
     if (tid < w) sB[tid] = P.diag[s + tid];
     __syncthreads();
@@ -188,64 +252,83 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     const uint32_t r = t * blockDim.x + tid;  // L21 row of this thread
     float lr[kSnMaxWidth];
     uint32_t target = 0;
-    if (r < m) {
-        target = __ldg(P.ridx + lbase + r);
 #pragma unroll
-        for (int c = 0; c < int(kSnMaxWidth); ++c)
-            lr[c] = uint32_t(c) < w ? __ldg(val + sB[c] + (l + 1 - (s + c)) + r) : 0.0f;
-    }
-    // L11, strictly lower: L(s+k, s+c) at diag[s+c] + (k - c); eight loads in flight per thread
-    for (uint32_t e0 = 0; e0 < w * kSnMaxWidth; e0 += 8 * 256) {
-        float v[8];
+    for (int c = 0; c < int(kSnMaxWidth); ++c)
+        lr[c] = (r < m && uint32_t(c) < w) ? __ldg(val + sB[c] + (l + 1 - (s + c)) + r) : 0.0f;
+    if (r < m) target = __ldg(P.ridx + lbase + r);
+    float iv[16];
+    if (wide != UINT32_MAX) {
+        load_inverse(iv, invs + bz.y * inv_stride + (size_t(wide) * 2) * kSnMaxWidth * kSnMaxWidth, tid);
+    } else {
+        // L11, strictly lower: L(s+k, s+c) at diag[s+c] + (k - c); eight loads in flight per thread
+        for (uint32_t e0 = 0; e0 < w * kSnMaxWidth; e0 += 8 * 256) {
+            float v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
-            v[u] = (c < w && k < w && k > c) ? __ldg(val + sB[c] + (k - c)) : 0.0f;
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
+                v[u] = (c < w && k < w && k > c) ? __ldg(val + sB[c] + (k - c)) : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
+                if (c < w && k < w && k > c) sT[c * kLD + k] = v[u];
+            }
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
-            if (c < w && k < w && k > c) sT[c * kLD + k] = v[u];
-        }
+        if (tid < kSnMaxWidth) xs[tid] = 0.0f;
+        __syncthreads();
     }
-    __syncthreads();
-    for (uint32_t q = 0; q < nrhs; ++q) {
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
-        if (tid < 32) {
-            const uint32_t k0 = tid, k1 = tid + 32;
-            float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
-            float v1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
-            for (uint32_t c = 0; c + 1 < w; ++c) {
-                const float xc = __shfl_sync(0xffffffffu, c < 32 ? v0 : v1, c & 31);
-                if (k0 > c && k0 < w) v0 = __fsub_rn(v0, __fmul_rn(sT[c * kLD + k0], xc));
-                if (k1 > c && k1 < w) v1 = __fsub_rn(v1, __fmul_rn(sT[c * kLD + k1], xc));
+        if (wide != UINT32_MAX) {
+            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
+            __syncthreads();
+            wide_solve(iv, vs, part, xs, tid);
+            if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
+        } else {
+            if (tid < 32) {
+                const uint32_t k0 = tid, k1 = tid + 32;
+                float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
+                float v1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
+                for (uint32_t c = 0; c + 1 < w; ++c) {
+                    const float xc = __shfl_sync(0xffffffffu, c < 32 ? v0 : v1, c & 31);
+                    if (k0 > c && k0 < w) v0 = __fsub_rn(v0, __fmul_rn(sT[c * kLD + k0], xc));
+                    if (k1 > c && k1 < w) v1 = __fsub_rn(v1, __fmul_rn(sT[c * kLD + k1], xc));
+                }
+                if (k0 < w) xs[k0] = v0;
+                if (k1 < w) xs[k1] = v1;
+                if (t == 0) {
+                    if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
+                    if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
+                }
             }
-            if (k0 < w) xs[k0] = v0;
-            if (k1 < w) xs[k1] = v1;
-            if (t == 0) {
-                if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
-                if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
-            }
+            __syncthreads();
         }
-        __syncthreads();
-        if (r < m) {
-            float acc = 0.0f;
+        // four sums: one chain of 64 multiply-adds would take as long as the solve
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const float4 *x4 = reinterpret_cast<const float4 *>(xs);
 #pragma unroll
-            for (int c = 0; c < int(kSnMaxWidth); ++c)
-                if (uint32_t(c) < w) acc = fmaf(lr[c], xs[c], acc);
-            if (acc != 0.0f) atomicAdd(yq + target, -acc);
+        for (int c = 0; c < int(kSnMaxWidth); c += 4) {
+            if (uint32_t(c) >= w) break;
+            const float4 x = x4[c / 4];
+            acc[0] = fmaf(lr[c], x.x, acc[0]);
+            acc[1] = fmaf(lr[c + 1], x.y, acc[1]);
+            acc[2] = fmaf(lr[c + 2], x.z, acc[2]);
+            acc[3] = fmaf(lr[c + 3], x.w, acc[3]);
         }
-        __syncthreads();
+        const float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        if (r < m && sum != 0.0f) atomicAdd(yq + target, -sum);
+        if (q + 1 < Q.q1) __syncthreads();
     }
     sweep_release(W, blk, done);
 }
 
 __global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
-                                                    uint64_t vstride, uint64_t ystride, uint32_t *done,
+                                                    uint64_t vstride, uint64_t ystride,
+                                                    const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
                                                     uint32_t *ticket, uint32_t *status, uint32_t spin_limit) {
     pdl_release();
-    pdl_wait();  // the previous level's x (per-level launches are chained)
     const uint2 bz = sweep_block(W, b0, done, ticket, status, spin_limit);
     const uint32_t blk = bz.x;
     val += bz.y * vstride;  // value set bz.y, its right-hand sides
@@ -253,18 +336,21 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan
     xo += bz.y * ystride;
     if (done) done += size_t(bz.y) * W.ns;
     if (blk == UINT32_MAX) return;
+    const Rhs Q = rhs_share(nrhs);
     __shared__ float sT[kSnMaxWidth * kLD];
-    __shared__ float xs[kSnMaxWidth];
+    __shared__ __align__(16) float xs[kSnMaxWidth], vs[kSnMaxWidth];
     __shared__ uint32_t pre[kSnMaxWidth + 1];
+    float(*part)[kSnMaxWidth] = reinterpret_cast<float(*)[kSnMaxWidth]>(sT);
     const uint2 bi = W.map[blk];
     if (bi.y & kSnSmallFlag) {  // a group of small supernodes, one per warp
         const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_u_small(P, W, val, y, xo, nrhs, W.small[bi.x + wi], threadIdx.x & 31);
+        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_u_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
         sweep_release(W, blk, done);
         return;
     }
     const uint32_t s = W.meta[bi.x].x, w = W.meta[bi.x].y, t = bi.y;
     const uint32_t tid = threadIdx.x, n = P.n;
+    const uint32_t wide = (invs && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
     __shared__ uint32_t sB[kSnMaxWidth], sC[kSnMaxWidth];
     if (tid < 32) {
         // entries of column s+c above the block: positions cptr[s+c] .. diag[s+c]-c-1
@@ -296,21 +382,26 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan
         if (c1 == w - 1) pre[w] = tot0 + a1;
     }
     __syncthreads();
-    // U11 with its diagonal: U(s+k, s+c), k <= c, at diag[s+c] - (c - k); eight loads in flight
-    for (uint32_t e0 = 0; e0 < w * kSnMaxWidth; e0 += 8 * 256) {
-        float v[8];
+    float iv[16];
+    if (wide != UINT32_MAX) {
+        load_inverse(iv, invs + bz.y * inv_stride + (size_t(wide) * 2 + 1) * kSnMaxWidth * kSnMaxWidth, tid);
+    } else {
+        // U11 with its diagonal: U(s+k, s+c), k <= c, at diag[s+c] - (c - k); eight loads in flight
+        for (uint32_t e0 = 0; e0 < w * kSnMaxWidth; e0 += 8 * 256) {
+            float v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
-            v[u] = (c < w && k <= c) ? __ldg(val + sB[c] - (c - k)) : 0.0f;
-        }
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
+                v[u] = (c < w && k <= c) ? __ldg(val + sB[c] - (c - k)) : 0.0f;
+            }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
-            if (c < w && k <= c) sT[c * kLD + k] = v[u];
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t e = e0 + u * 256 + tid, c = e >> 6, k = e & 63;
+                if (c < w && k <= c) sT[c * kLD + k] = v[u];
+            }
         }
+        __syncthreads();
     }
-    __syncthreads();
     const uint32_t e0 = t * kSnSweepAbove, e1 = min(e0 + kSnSweepAbove, pre[w]);
     // kSnSweepAbove / 256 entries above the block per thread: column, target
     // and value do not depend on x, so they are loaded before the chain
@@ -338,34 +429,53 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan
             eval[u] = __ldg(val + p);
         }
     }
-    for (uint32_t q = 0; q < nrhs; ++q) {
+    // the chain's lanes: pivots and reciprocals of columns tid and tid + 32
+    float pv0 = 1.0f, pv1 = 1.0f;
+    if (wide == UINT32_MAX && tid < 32) {
+        if (tid < w) pv0 = sT[tid * kLD + tid];
+        if (tid + 32 < w) pv1 = sT[(tid + 32) * kLD + tid + 32];
+    }
+    const float rc0 = lu_reciprocal(pv0), rc1 = lu_reciprocal(pv1);
+    const float g0 = fabsf(pv0), g1 = fabsf(pv1);
+    const bool quick = __all_sync(kFull, g0 > 1e-30f && g0 < 1e30f && g1 > 1e-30f && g1 < 1e30f);
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
-        if (tid < 32) {
-            const uint32_t k0 = tid, k1 = tid + 32;
-            float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
-            float v1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
-            for (uint32_t cc = w; cc-- > 0;) {
-                const float xc = __shfl_sync(0xffffffffu, cc < 32 ? v0 : v1, cc & 31) / sT[cc * kLD + cc];
-                if (k0 == cc) v0 = xc;
-                if (k1 == cc) v1 = xc;
-                if (k0 < cc) v0 = __fsub_rn(v0, __fmul_rn(sT[cc * kLD + k0], xc));
-                if (k1 < cc) v1 = __fsub_rn(v1, __fmul_rn(sT[cc * kLD + k1], xc));
+        if (wide != UINT32_MAX) {
+            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
+            __syncthreads();
+            wide_solve(iv, vs, part, xs, tid);
+            if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
+        } else {
+            if (tid < 32) {
+                const uint32_t k0 = tid, k1 = tid + 32;
+                float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
+                float v1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
+                for (uint32_t cc = w; cc-- > 0;) {
+                    // every lane divides its own value, so that the step is one shuffle long
+                    const float v = cc < 32 ? v0 : v1, p = cc < 32 ? pv0 : pv1, rc = cc < 32 ? rc0 : rc1;
+                    const float xc = __shfl_sync(0xffffffffu, quick ? lu_quotient(v, p, rc) : v / p, cc & 31);
+                    if (k0 == cc) v0 = xc;
+                    if (k1 == cc) v1 = xc;
+                    if (k0 < cc) v0 = __fsub_rn(v0, __fmul_rn(sT[cc * kLD + k0], xc));
+                    if (k1 < cc) v1 = __fsub_rn(v1, __fmul_rn(sT[cc * kLD + k1], xc));
+                }
+                if (k0 < w) xs[k0] = v0;
+                if (k1 < w) xs[k1] = v1;
+                if (t == 0) {
+                    if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
+                    if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
+                }
             }
-            if (k0 < w) xs[k0] = v0;
-            if (k1 < w) xs[k1] = v1;
-            if (t == 0) {
-                if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
-                if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
-            }
+            __syncthreads();
         }
-        __syncthreads();
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
             if (ecol[u] >= kSnMaxWidth) continue;
             const float xc = xs[ecol[u]];
             if (xc != 0.0f) atomicAdd(yq + etg[u], -__fmul_rn(eval[u], xc));
         }
-        __syncthreads();
+        if (q + 1 < Q.q1) __syncthreads();
     }
     sweep_release(W, blk, done);
 }
@@ -382,24 +492,44 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_l_small(DevPattern P, SnSwe
                                                           float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                           uint64_t vstride, uint64_t ystride) {
     pdl_release();
-    pdl_wait();  // the previous level's x
     const uint2 bi = W.map[b0 + blockIdx.x];
     const uint32_t wi = threadIdx.x >> 5;
     if (!(bi.y & kSnSmallFlag) || wi >= (bi.y & ~kSnSmallFlag)) return;
-    sn_sweep_l_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride, nrhs,
-                     W.small[bi.x + wi], threadIdx.x & 31);
+    sn_sweep_l_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
+                     rhs_share(nrhs), W.small[bi.x + wi], threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(256, 5) k_sn_sweep_u_small(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                           float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                           uint64_t vstride, uint64_t ystride) {
     pdl_release();
-    pdl_wait();  // the previous level's x
     const uint2 bi = W.map[b0 + blockIdx.x];
     const uint32_t wi = threadIdx.x >> 5;
     if (!(bi.y & kSnSmallFlag) || wi >= (bi.y & ~kSnSmallFlag)) return;
-    sn_sweep_u_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride, nrhs,
-                     W.small[bi.x + wi], threadIdx.x & 31);
+    sn_sweep_u_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
+                     rhs_share(nrhs), W.small[bi.x + wi], threadIdx.x & 31);
+}
+
+// Inverses of the diagonal blocks of the wide supernodes (blockIdx.x; first
+// column and width): blockIdx.y = 0 L, 1 U, blockIdx.z the value set.
+__global__ void __launch_bounds__(256) k_sn_diag_inv(DevPattern P, const uint2 *__restrict__ wide,
+                                                      const float *__restrict__ val, uint64_t vstride,
+                                                      float *__restrict__ invs, uint64_t inv_stride) {
+    __shared__ TriInverse T;
+    __shared__ uint32_t sB[kSnMaxWidth];
+    const uint2 d = wide[blockIdx.x];
+    val += blockIdx.z * vstride;
+    if (threadIdx.x < d.y) sB[threadIdx.x] = P.diag[d.x + threadIdx.x];
+    __syncthreads();
+    tri_invert(T, blockIdx.y, d.y,
+               invs + blockIdx.z * inv_stride + (size_t(blockIdx.x) * 2 + blockIdx.y) * kSnMaxWidth * kSnMaxWidth,
+               [&](uint32_t i, uint32_t c) { return val[sB[c] + i - c]; });
+}
+
+cudaError_t launch_sn_diag_inv(const DevPattern &P, const uint2 *wide, uint32_t nwide, const float *val,
+                               uint64_t vstride, uint32_t count, float *invs, uint64_t inv_stride, cudaStream_t st) {
+    k_sn_diag_inv<<<dim3(nwide, 2, count), 256, 0, st>>>(P, wide, val, vstride, invs, inv_stride);
+    return cudaGetLastError();
 }
 
 __global__ void k_sn_copy(const float *__restrict__ xo, float *y, uint32_t t, uint32_t n) {
@@ -411,6 +541,12 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
                          float *y, float *xo, uint32_t nrhs, const SolveBatch &B, uint32_t *done, uint32_t *ticket,
                          uint32_t *status, uint32_t spin_limit, cudaStream_t st) {
     const uint64_t ystride = uint64_t(nrhs) * P.n;
+    // blocks per level and value set over which the right-hand sides are
+    // spread: as many as leave about four blocks per SM in all
+    auto shares = [&](uint32_t blocks) {
+        const uint64_t have = std::max<uint64_t>(uint64_t(blocks) * B.count, 1);
+        return uint32_t(std::min<uint64_t>(nrhs, std::max<uint64_t>(1, 4 * 148 / have)));
+    };
     if (W.fused && done && W.nblocks) {
         // one launch: blocks in map order by ticket, supernodes wait for their releases
         cudaError_t e = cudaMemsetAsync(done, 0, sizeof(uint32_t) * size_t(W.ns) * B.count, st);
@@ -418,11 +554,11 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
         if (e != cudaSuccess) return e;
         const dim3 grid(W.nblocks, 1, B.count);
         if (upper)
-            k_sn_sweep_u<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, done, ticket, status,
-                                               spin_limit);
+            k_sn_sweep_u<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv,
+                                               B.sn_inv_stride, done, ticket, status, spin_limit);
         else
-            k_sn_sweep_l<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, done, ticket, status,
-                                               spin_limit);
+            k_sn_sweep_l<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv,
+                                               B.sn_inv_stride, done, ticket, status, spin_limit);
     } else {
         // one launch per level (two where its small-supernode groups get
         // their own), each chained to the one before (its blocks start while
@@ -434,17 +570,20 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
             const uint2 k2 = sn_sweep_level_launches(lv, upper);
             cudaError_t e = cudaSuccess;
             if (k2.x) {  // the full kernel: the parts, and the groups unless they launch apart
-                const dim3 grid(k2.y ? lv.big : lv.blocks, 1, B.count);
+                const uint32_t nblk = k2.y ? lv.big : lv.blocks;
+                const dim3 grid(nblk, shares(nblk), B.count);
                 if (upper)
                     e = launch_chained(k_sn_sweep_u, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride,
-                                       ystride, (uint32_t *)nullptr, (uint32_t *)nullptr, status, spin_limit);
+                                       ystride, B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr,
+                                       status, spin_limit);
                 else
                     e = launch_chained(k_sn_sweep_l, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride,
-                                       ystride, (uint32_t *)nullptr, (uint32_t *)nullptr, status, spin_limit);
+                                       ystride, B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr,
+                                       status, spin_limit);
                 if (e != cudaSuccess) return e;
             }
             if (k2.y) {  // the small-supernode groups
-                const dim3 grid(lv.blocks - lv.big, 1, B.count);
+                const dim3 grid(lv.blocks - lv.big, shares(lv.blocks - lv.big), B.count);
                 if (upper)
                     e = launch_chained(k_sn_sweep_u_small, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs,
                                        lv.b0 + lv.big, B.vstride, ystride);
