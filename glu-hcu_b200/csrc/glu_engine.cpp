@@ -703,7 +703,7 @@ Status build_sn_plan(glu_handle_s *h) {
     std::vector<uint32_t> psmall, usmall, dsmall, tgt(size_t(ns) + 1, 0);
     std::vector<uint2> dmap;
     std::vector<uint64_t> pos_off(size_t(ns) + 1, 0);
-    const uint32_t PT = kSnPanelThreads, UT = 64, TW = kSnPanelThreads / 32;
+    const uint32_t UT = 64;
     double upd_flops = 0, upd_bytes = 0, pan_bytes = 0;
     for (int32_t l = 0; l < nlev; ++l) {
         uint32_t updating = 0, panel_w = 0;
@@ -715,7 +715,8 @@ Status build_sn_plan(glu_handle_s *h) {
             const uint64_t m = nl(last), nt = nu(last);
             meta[i] = make_uint4(first[q], w, uint32_t(m), uint32_t(nt));
             const uint64_t tiles = ((m + UT - 1) / UT) * ((nt + UT - 1) / UT);
-            const uint64_t pb = (m + PT - 1) / PT + (w >= 2 ? (nt + TW - 1) / TW : 0);
+            const uint32_t PT = w > kSnSmallWidth ? kSnPanelWideRows : kSnPanelThreads;
+            const uint64_t pb = (m + PT - 1) / PT + (w >= 2 ? (nt + PT - 1) / PT : 0);
             if (tiles) ++updating;
             // diagonal blocks: a warp each up to kSnSmallWidth (eight to a block), else a block
             if (w > kSnSmallWidth)

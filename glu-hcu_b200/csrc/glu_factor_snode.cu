@@ -15,7 +15,7 @@
 // (symbolic.cc:106-151) contracted to supernodes.  Per level three launches:
 //   diag:   A11 = L11 U11 in place (GESP pivots, numeric.cu:139-140);
 //   panel:  L21 = A21 U11^-1 (a row per thread), U12(:, j) = L11^-1 A12(:, j)
-//           for every target j (a column per warp);
+//           for every target j (a column per thread);
 //   update: A(rows of L21, j) -= L21 U12(:, j) for every target j, as 64 x 64
 //           output tiles (FP32 FMA, K = w), scattered to the CSC positions of
 //           column j (a position table built once per pattern, or a search in
@@ -35,7 +35,7 @@ namespace glu {
 namespace {
 
 constexpr int kLD = kSnMaxWidth + 1;  // leading dimension of the diagonal block in shared memory
-constexpr int kSnPW = kSnPanelThreads + 1;  // leading dimension of the L21 rows in shared memory
+constexpr int kSnPW = kSnPanelWideRows + 1;  // leading dimension of the rows in shared memory
 // panel shared memory: the diagonal block (either layout), plus the rows of
 // L21 in launches with a supernode wider than one chunk
 constexpr size_t kSnPanelSmem = sizeof(float) * kSnMaxWidth * kTriML;
@@ -75,27 +75,6 @@ __device__ __forceinline__ uint32_t seg_len(const DevPattern &P, uint32_t j, uin
     return lo;
 }
 
-// Target column j of U12 by one warp: L11 x = a over the supernode's rows
-// present in column j (a suffix from row z; the rows above it are structural
-// zeros and stay untouched).  Lane k holds rows k and k + 32.
-__device__ __forceinline__ void sn_u12_warp(float *__restrict__ val, const Sn &d, uint4 g, const float *sF,
-                                            uint32_t lane) {
-    const uint32_t pl = g.x;
-    const uint32_t w = d.w;
-    const uint32_t z = w - g.y;
-    const uint32_t k0 = lane, k1 = lane + 32;
-    const bool p0 = k0 < w && k0 >= z, p1 = k1 < w && k1 >= z;
-    float a0 = p0 ? ld_cg(val + pl - (w - 1 - k0)) : 0.0f;
-    float a1 = p1 ? ld_cg(val + pl - (w - 1 - k1)) : 0.0f;
-    for (uint32_t r = z; r < w; ++r) {
-        const float u = __shfl_sync(0xffffffffu, r < 32 ? a0 : a1, r & 31);
-        if (k0 > r && k0 < w) a0 = fmaf(-sF[r * kLD + k0], u, a0);
-        if (k1 > r && k1 < w) a1 = fmaf(-sF[r * kLD + k1], u, a1);
-    }
-    if (p0) st_cg(val + pl - (w - 1 - k0), a0);
-    if (p1) st_cg(val + pl - (w - 1 - k1), a1);
-}
-
 constexpr uint32_t kFull = 0xffffffffu;
 
 // Diagonal block of one narrow supernode (2 <= w <= kSnSmallWidth) by one
@@ -104,12 +83,14 @@ constexpr uint32_t kFull = 0xffffffffu;
 // L part (c < w - 1, or m > 0); L(r,c) = A(r,c) / U(c,c), then A(r,j) -=
 // L(r,c) U(c,j) for j > c.
 __device__ __forceinline__ void sn_diag_small(const DevPattern &P, const SnPlanDev &S, float *__restrict__ val,
-                                              uint32_t i, float pert, uint32_t lane) {
+                                              uint32_t i, const float *pert_z, uint32_t lane) {
     constexpr int SW = int(kSnSmallWidth);
     const Sn d = sn_load(S, i);
     const uint32_t w = d.w;
     const bool rv = lane < w;
     const uint32_t bc = rv ? P.diag[d.s + lane] - lane : 0u;  // position of row s in column s + lane
+    pdl_wait();  // the previous level's updates
+    const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
     float a[SW];
 #pragma unroll
     for (int c = 0; c < SW; ++c) {
@@ -158,13 +139,15 @@ __device__ __forceinline__ void sn_l21_chunk(float *__restrict__ val, const uint
 // warp: lane r solves L21 row r, lane j solves target column j of U12, with
 // the factored diagonal block read in place (broadcast loads).
 __device__ __forceinline__ void sn_panel_small(const DevPattern &P, const SnPlanDev &S, float *__restrict__ val,
-                                               uint32_t i, float pert, uint32_t lane) {
+                                               uint32_t i, const float *pert_z, uint32_t lane) {
     constexpr int SW = int(kSnSmallWidth);
     const Sn d = sn_load(S, i);
     const uint32_t w = d.w;
     if (w == 1) {
         // numeric.cu:133-143: pivot (perturbed when the column has an L part), L /= pivot
         const uint32_t dk = P.diag[d.s];
+        pdl_wait();  // this level's diagonal blocks
+        const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
         const float p = ld_cg(val + dk);
         const float de = (pert > 0.0f && fabsf(p) < pert) ? pert : p;  // m > 0 here
         if (lane < d.m) st_cg(val + dk + 1 + lane, ld_cg(val + dk + 1 + lane) / de);
@@ -172,6 +155,9 @@ __device__ __forceinline__ void sn_panel_small(const DevPattern &P, const SnPlan
         return;
     }
     const uint32_t dl = lane < w ? P.diag[d.s + lane] : 0u;  // position of the diagonal of column s+lane
+    uint4 g = make_uint4(0u, 0u, 0u, 0u);
+    if (lane < d.nt) g = S.tgt[S.tgt_off[i] + lane];
+    pdl_wait();  // this level's diagonal blocks
     // row `lane` of L21: x U11 = a
     {
         const bool rv = lane < d.m;
@@ -200,8 +186,6 @@ __device__ __forceinline__ void sn_panel_small(const DevPattern &P, const SnPlan
     }
     // target column `lane` of U12: L11 x = a over the rows present
     {
-        uint4 g = make_uint4(0u, 0u, 0u, 0u);
-        if (lane < d.nt) g = S.tgt[S.tgt_off[i] + lane];
         const uint32_t z = w - g.y;  // g.y == 0: no target (z = w, nothing loaded or stored)
         float a[SW];
 #pragma unroll
@@ -285,24 +269,31 @@ __global__ void __launch_bounds__(kTriThreads, 2) k_sn_diag(DevPattern P, SnPlan
     __shared__ __align__(16) float sS[kSnMaxWidth * kLuLD];
     __shared__ uint32_t sBase[kSnMaxWidth];
     pdl_release();
-    pdl_wait();  // the previous level's updates
     float *val = val_base + blockIdx.z * stride;
-    const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
     const uint2 bi = S.dmap[b0 + blockIdx.x];
     if (bi.y & kSnSmallFlag) {
         const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_diag_small(P, S, val, S.dsmall[bi.x + wi], pert, threadIdx.x & 31);
+        if (wi < (bi.y & ~kSnSmallFlag)) sn_diag_small(P, S, val, S.dsmall[bi.x + wi], pert_z, threadIdx.x & 31);
         return;
     }
     const Sn d = sn_load(S, bi.x);
     const uint32_t tid = threadIdx.x, w = d.w;
     if (tid < w) sBase[tid] = P.diag[d.s + tid] - tid;  // position of row s in column s + tid
     __syncthreads();
-    const uint32_t end = (w + kLuChunk - 1) / kLuChunk * kLuChunk;  // (the identity past the block's end)
-#pragma unroll 8
-    for (uint32_t e = tid; e < end * kSnMaxWidth; e += kTriThreads) {
-        const uint32_t c = e / kSnMaxWidth, r = e % kSnMaxWidth;
-        sS[c * kLuLD + r] = (r < w && c < w) ? ld_cg(val + sBase[c] + r) : (r == c ? 1.0f : 0.0f);
+    pdl_wait();  // the previous level's updates
+    const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
+    {   // (the identity past the block's end); all loads in flight together
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t e = tid + u * kTriThreads, c = e / kSnMaxWidth, r = e % kSnMaxWidth;
+            v[u] = (r < w && c < w) ? ld_cg(val + sBase[c] + r) : (r == c ? 1.0f : 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t e = tid + u * kTriThreads;
+            sS[(e / kSnMaxWidth) * kLuLD + e % kSnMaxWidth] = v[u];
+        }
     }
     __syncthreads();
     tri_lu_smem(sS, w, d.m > 0, pert);
@@ -314,24 +305,25 @@ __global__ void __launch_bounds__(kTriThreads, 2) k_sn_diag(DevPattern P, SnPlan
 }
 
 // Panel launch of one level (after its diagonal blocks): blocks [b0, b0 +
-// gridDim.x) of the panel map.  Per supernode: ceil(m / 128) blocks of L21 rows (one row per
-// thread), then, for width >= 2, ceil(nt / 4) blocks of U12 target columns
-// (one column per warp).  Width 1: the blocks scale the column by its pivot
+// gridDim.x) of the panel map.  Per supernode its rows of L21, then, for width
+// >= 2, its target columns of U12: up to 16 columns wide, 128 to a block, a
+// thread each in registers; wider, 64 to a block, two threads each (tri_rows_
+// solve_halves; the broadcast loads of M bound it, so fewer rows per block are
+// quicker).  Width 1: the blocks scale the column by its pivot
 // (numeric.cu:133-143).  blockIdx.z selects the value set.
-__global__ void __launch_bounds__(kSnPanelThreads, 4) k_sn_panel(DevPattern P, SnPlanDev S, float *val_base,
+__global__ void __launch_bounds__(kSnPanelThreads, 6) k_sn_panel(DevPattern P, SnPlanDev S, float *val_base,
                                                               uint64_t stride, const float *pert_z, uint32_t b0) {
     extern __shared__ float4 snp_sm4[];
-    float *sF = reinterpret_cast<float *>(snp_sm4);  // L11 column-major (U12 blocks) or U11 row-major (L21 blocks)
-    float *sW = sF + kSnMaxWidth * kTriML;           // rows of L21 when w > kTriChunk
+    float *sF = reinterpret_cast<float *>(snp_sm4);  // L11 column-major (U12 blocks) or U11 row-major (L21 blocks), ld kTriML
+    float *sW = sF + kSnMaxWidth * kTriML;           // rows of L21 or columns of U12 when w > kTriChunk
     __shared__ uint32_t sOff[kSnMaxWidth];
+    __shared__ uint32_t sPl[kSnPanelThreads], sLen[kSnPanelThreads];  // target columns
     pdl_release();
-    pdl_wait();  // this level's diagonal blocks
     float *val = val_base + blockIdx.z * stride;
-    const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
     const uint2 bi = S.pmap[b0 + blockIdx.x];
     if (bi.y & kSnSmallFlag) {  // small supernodes, one per warp
         const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_panel_small(P, S, val, S.psmall[bi.x + wi], pert, threadIdx.x & 31);
+        if (wi < (bi.y & ~kSnSmallFlag)) sn_panel_small(P, S, val, S.psmall[bi.x + wi], pert_z, threadIdx.x & 31);
         return;
     }
     const uint32_t i = bi.x, t = bi.y;
@@ -340,6 +332,8 @@ __global__ void __launch_bounds__(kSnPanelThreads, 4) k_sn_panel(DevPattern P, S
     if (d.w == 1) {
         const uint32_t dk = P.diag[d.s];
         const uint32_t r = t * kSnPanelThreads + tid;
+        pdl_wait();  // this level's diagonal blocks
+        const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
         const float p = ld_cg(val + dk);
         const float de = (pert > 0.0f && fabsf(p) < pert) ? pert : p;  // m > 0 here
         if (r < d.m) st_cg(val + dk + 1 + r, ld_cg(val + dk + 1 + r) / de);
@@ -348,69 +342,117 @@ __global__ void __launch_bounds__(kSnPanelThreads, 4) k_sn_panel(DevPattern P, S
         return;
     }
     const uint32_t w = d.w;
-    const uint32_t nLb = (d.m + kSnPanelThreads - 1) / kSnPanelThreads;
+    const bool narrow = w <= uint32_t(kTriChunk);
+    // rows or columns per block: a thread each, or two threads each
+    const uint32_t per = narrow ? kSnPanelThreads : kSnPanelWideRows;
+    const uint32_t nLb = (d.m + per - 1) / per;
     const bool lrows = t < nLb;
     if (tid < w) sOff[tid] = P.diag[d.s + tid];
-    __syncthreads();
-    // This thread's row of A21 (w <= kTriChunk) does not depend on the
-    // diagonal block: its loads are issued first.
-    const uint32_t rr = t * kSnPanelThreads + tid;
-    float xr[kTriChunk];
-    if (lrows && w <= uint32_t(kTriChunk) && rr < d.m) {
-#pragma unroll
-        for (int c = 0; c < kTriChunk; ++c)
-            xr[c] = uint32_t(c) < w ? ld_cg(val + sOff[c] + (d.l + 1 - (d.s + c)) + rr) : 0.0f;
+    if (!lrows && tid < per) {  // this block's target columns: position of row l, rows present
+        const uint32_t jt = (t - nLb) * per + tid;
+        const uint4 g = jt < d.nt ? S.tgt[S.tgt_off[i] + jt] : make_uint4(0u, 0u, 0u, 0u);
+        sPl[tid] = g.x;
+        sLen[tid] = g.y;
     }
-    // the factored diagonal block, eight independent loads in flight per thread:
-    // L21 blocks keep U11 row-major (leading dimension kTriML), U12 blocks L11
-    // column-major (leading dimension kLD)
-    for (uint32_t e0 = 0; e0 < kSnMaxWidth * kSnMaxWidth; e0 += 8 * kSnPanelThreads) {
-        float v[8];
+    __syncthreads();
+    pdl_wait();  // this level's diagonal blocks
+    // Narrow: this thread's row of A21 or column of A12, in registers; it does
+    // not depend on the diagonal block and its loads are issued first.
+    // Wide: half of the entries of 64 rows or columns, through shared memory.
+    const uint32_t v = narrow ? tid : tid & (kSnPanelWideRows - 1), half = narrow ? 0u : tid / kSnPanelWideRows;
+    const uint32_t rr = t * per + v;
+    float xr[kTriChunk];
+    if (narrow) {
+        const uint32_t z = lrows ? 0u : w - sLen[tid];  // the rows above it are structural zeros and stay untouched
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const uint32_t e = e0 + q * kSnPanelThreads + tid, cc = e >> 6, r = e & 63;
-            v[q] = (cc < w && r < w) ? ld_cg(val + sOff[cc] + r - cc) : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const uint32_t e = e0 + q * kSnPanelThreads + tid, cc = e >> 6, r = e & 63;
-            if (cc < w && r < w) {
-                if (lrows)
-                    sF[r * kTriML + cc] = v[q];
-                else
-                    sF[cc * kLD + r] = v[q];
+        for (int c = 0; c < kTriChunk; ++c) {
+            xr[c] = 0.0f;
+            if (uint32_t(c) >= w) continue;
+            if (lrows) {
+                if (rr < d.m) xr[c] = ld_cg(val + sOff[c] + (d.l + 1 - (d.s + c)) + rr);
+            } else if (uint32_t(c) >= z) {
+                xr[c] = ld_cg(val + sPl[tid] - (w - 1 - c));
             }
         }
-        if (e0 + 8 * kSnPanelThreads >= w * kSnMaxWidth) break;
-    }
-    __syncthreads();
-    if (tid < w) {
-        sOff[tid] += d.l + 1 - (d.s + tid);
-        if (lrows) sF[tid * kTriML + kTriMax] = 1.0f / sF[tid * kTriML + tid];  // pivot reciprocals
-    }
-    __syncthreads();
-    if (lrows) {
-        // row r of L21: x U11 = a (a = row r of A21)
-        const uint32_t r = t * kSnPanelThreads + tid;
-        if (r >= d.m) return;
-        if (w <= 2) {
-            sn_l21_chunk<2>(val, sOff, w, r, sF, xr);
-        } else if (w <= 4) {
-            sn_l21_chunk<4>(val, sOff, w, r, sF, xr);
-        } else if (w <= 8) {
-            sn_l21_chunk<8>(val, sOff, w, r, sF, xr);
-        } else if (w <= uint32_t(kTriChunk)) {
-            sn_l21_chunk<kTriChunk>(val, sOff, w, r, sF, xr);
-        } else {
-            for (uint32_t c = 0; c < w; ++c) sW[c * kSnPW + tid] = ld_cg(val + sOff[c] + r);
-            tri_rows_solve<true>(sW, kSnPW, tid, sF, w);
-            for (uint32_t c = 0; c < w; ++c) st_cg(val + sOff[c] + r, sW[c * kSnPW + tid]);
+    } else if (lrows) {
+#pragma unroll 1
+        for (uint32_t c0 = half * 32; c0 < half * 32 + 32 && c0 < w; c0 += kTriChunk) {
+#pragma unroll
+            for (int c = 0; c < kTriChunk; ++c)
+                xr[c] = (rr < d.m && c0 + c < w) ? ld_cg(val + sOff[c0 + c] + (d.l + 1 - (d.s + c0 + c)) + rr) : 0.0f;
+#pragma unroll
+            for (int c = 0; c < kTriChunk; ++c) sW[(c0 + c) * kSnPW + v] = xr[c];
         }
+    } else {  // lanes along k, contiguous in a target column
+#pragma unroll 1
+        for (uint32_t e0 = 0; e0 < kSnMaxWidth * kSnPanelWideRows; e0 += kTriChunk * kSnPanelThreads) {
+#pragma unroll
+            for (int q = 0; q < kTriChunk; ++q) {
+                const uint32_t e = e0 + q * kSnPanelThreads + tid, k = e & 63, j = e >> 6;
+                xr[q] = (k < w && k + sLen[j] >= w) ? ld_cg(val + sPl[j] - (w - 1 - k)) : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < kTriChunk; ++q) {
+                const uint32_t e = e0 + q * kSnPanelThreads + tid;
+                sW[(e & 63) * kSnPW + (e >> 6)] = xr[q];
+            }
+        }
+    }
+    // the factored diagonal block, sixteen independent loads in flight per
+    // thread, as the matrix M of the row solves: L21 blocks U11 row-major, U12
+    // blocks L11 column-major
+#pragma unroll 1
+    for (uint32_t e0 = 0; e0 < w * kSnMaxWidth; e0 += 16 * kSnPanelThreads) {
+        float m[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const uint32_t e = e0 + q * kSnPanelThreads + tid, cc = e >> 6, r = e & 63;
+            m[q] = (cc < w && r < w) ? ld_cg(val + sOff[cc] + r - cc) : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const uint32_t e = e0 + q * kSnPanelThreads + tid, cc = e >> 6, r = e & 63;
+            if (cc < w && r < w) sF[lrows ? r * kTriML + cc : cc * kTriML + r] = m[q];
+        }
+    }
+    __syncthreads();
+    if (lrows && tid < w) {
+        sOff[tid] += d.l + 1 - (d.s + tid);
+        sF[tid * kTriML + kTriMax] = 1.0f / sF[tid * kTriML + tid];  // pivot reciprocals
+    }
+    __syncthreads();
+    if (narrow && lrows) {
+        // row r of L21: x U11 = a (a = row r of A21)
+        if (rr >= d.m) return;
+        if (w <= 2) {
+            sn_l21_chunk<2>(val, sOff, w, rr, sF, xr);
+        } else if (w <= 4) {
+            sn_l21_chunk<4>(val, sOff, w, rr, sF, xr);
+        } else if (w <= 8) {
+            sn_l21_chunk<8>(val, sOff, w, rr, sF, xr);
+        } else {
+            sn_l21_chunk<kTriChunk>(val, sOff, w, rr, sF, xr);
+        }
+    } else if (narrow) {
+        // column of U12: L11 x = a
+        tri_chunk_solve<false>(xr, sF, 0, w);
+        const uint32_t z = w - sLen[tid];
+#pragma unroll
+        for (int k = 0; k < kTriChunk; ++k)
+            if (uint32_t(k) < w && uint32_t(k) >= z) st_cg(val + sPl[tid] - (w - 1 - k), xr[k]);
+    } else if (lrows) {
+        tri_rows_solve_halves<true>(sW, kSnPW, v, half, sF, w);
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t c = half; c < w; c += 2)
+            if (rr < d.m) st_cg(val + sOff[c] + rr, sW[c * kSnPW + v]);
     } else {
-        const uint32_t jt = (t - nLb) * (kSnPanelThreads / 32) + tid / 32;
-        if (jt < d.nt) {
-            const uint4 g = S.tgt[S.tgt_off[i] + jt];
-            if (g.y != 0) sn_u12_warp(val, d, g, sF, tid & 31);
+        tri_rows_solve_halves<false>(sW, kSnPW, v, half, sF, w);
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t e = tid; e < kSnMaxWidth * kSnPanelWideRows; e += kSnPanelThreads) {
+            const uint32_t k = e & 63, j = e >> 6;
+            if (k < w && k + sLen[j] >= w) st_cg(val + sPl[j] - (w - 1 - k), sW[k * kSnPW + j]);
         }
     }
 }
@@ -449,20 +491,23 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
     const uint32_t w = d.w;
     const uint32_t nrt = (d.m + kTile - 1) / kTile;
     const uint32_t r0 = (t % nrt) * kTile, c0 = (t / nrt) * kTile;
+    // rows tr + 16 a: sixteen lanes on neighbouring rows, whose positions in a
+    // target column are mostly neighbours too (sectors of the table's loads and
+    // of the atomics are shared)
     const uint32_t tr = tid & 15, tc = tid >> 4;
     // Target positions from the table depend only on the tile: issued first,
     // in flight while the metadata and the operands are staged (a target that
     // cannot hold the rows has 0xffffffff in the table).
     uint32_t pos[4][4];
     if (S.pos) {
-        const uint32_t *tab = S.pos + S.pos_off[i] + r0 + tr * 4;
+        const uint32_t *tab = S.pos + S.pos_off[i] + r0 + tr;
 #pragma unroll
         for (int bb = 0; bb < 4; ++bb) {
             const uint32_t jt = tc * 4 + bb;
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const uint32_t r = r0 + tr * 4 + a;
-                pos[a][bb] = (c0 + jt < d.nt && r < d.m) ? __ldg(tab + uint64_t(c0 + jt) * d.m + a) : 0xffffffffu;
+                const uint32_t r = r0 + tr + 16 * a;
+                pos[a][bb] = (c0 + jt < d.nt && r < d.m) ? __ldg(tab + uint64_t(c0 + jt) * d.m + 16 * a) : 0xffffffffu;
             }
         }
     }
@@ -488,7 +533,7 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
         const uint32_t lbase = P.diag[d.l] + 1;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const uint32_t r = r0 + tr * 4 + a;
+            const uint32_t r = r0 + tr + 16 * a;
             rowid[a] = r < d.m ? __ldg(P.ridx + lbase + r) : 0u;
         }
 #pragma unroll
@@ -501,7 +546,7 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
             const uint32_t ts = tcol ? __ldg(S.tail_start + (tj - S.t)) : 0u;
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const uint32_t r = r0 + tr * 4 + a;
+                const uint32_t r = r0 + tr + 16 * a;
                 uint32_t q = 0xffffffffu;
                 if (tv && r < d.m) {
                     if (tcol && rowid[a] >= S.t) {
@@ -521,21 +566,34 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int bb = 0; bb < 4; ++bb)
-                if (r0 + tr * 4 + a >= cu.x && c0 + tc * 4 + bb >= cu.y) pos[a][bb] = 0xffffffffu;
+                if (r0 + tr + 16 * a >= cu.x && c0 + tc * 4 + bb >= cu.y) pos[a][bb] = 0xffffffffu;
     }
+    const uint32_t lg = w > 1 ? 32 - __clz(w - 1) : 0;
     // the metadata and positions above are plan data, read while this
     // level's panels finish; the values only after them
     pdl_wait();
     for (uint32_t z = z0; z < z1; ++z) {
     float *val = val_base + z * stride;
     if (z > z0) __syncthreads();  // the previous value set's operands are read
-    for (uint32_t e = tid; e < w * kTile; e += blockDim.x) {
-        const uint32_t k = e / kTile, r = e - k * kTile;
-        sL[k][r] = (r0 + r < d.m) ? ld_cg(val + sOff[k] + r) : 0.0f;
-    }
-    for (uint32_t e = tid; e < w * kTile; e += blockDim.x) {
-        const uint32_t jt = e / w, k = e - jt * w;
-        sU[k][jt] = (k + sLen[jt] >= w) ? ld_cg(val + sPl[jt] - (w - 1 - k)) : 0.0f;
+    // operands, eight loads of each in flight per thread: L21 with the lanes
+    // down the rows, U12 with them along k (contiguous in a target column; 2^lg
+    // >= w of them)
+    for (uint32_t e0 = 0; e0 < w * kTile || e0 < (uint32_t(kTile) << lg); e0 += 8 * 256) {
+        float v[8], u[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t e = e0 + q * 256 + tid, k = e / kTile, r = e % kTile;
+            v[q] = (k < w && r0 + r < d.m) ? ld_cg(val + sOff[k] + r) : 0.0f;
+            const uint32_t ku = e & ((1u << lg) - 1), jt = e >> lg;
+            u[q] = (jt < uint32_t(kTile) && ku < w && ku + sLen[jt] >= w) ? ld_cg(val + sPl[jt] - (w - 1 - ku)) : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t e = e0 + q * 256 + tid, k = e / kTile, r = e % kTile;
+            if (k < w) sL[k][r] = v[q];
+            const uint32_t ku = e & ((1u << lg) - 1), jt = e >> lg;
+            if (jt < uint32_t(kTile) && ku < w) sU[ku][jt] = u[q];
+        }
     }
     float acc[4][4];
 #pragma unroll
@@ -545,9 +603,9 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
     __syncthreads();
     if (atomic) {
         for (uint32_t k = 0; k < w; ++k) {
-            const float4 av = *reinterpret_cast<const float4 *>(&sL[k][tr * 4]);
             const float4 bv = *reinterpret_cast<const float4 *>(&sU[k][tc * 4]);
-            const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+            const float ar[4] = {sL[k][tr], sL[k][tr + 16], sL[k][tr + 32], sL[k][tr + 48]};
+            const float br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -560,9 +618,9 @@ __global__ void __launch_bounds__(256, 5) k_sn_update(DevPattern P, SnPlanDev S,
                 if (pos[a][bb] != 0xffffffffu) atomicAdd(val + pos[a][bb], -acc[a][bb]);
     } else {
         for (uint32_t k = 0; k < w; ++k) {
-            const float4 av = *reinterpret_cast<const float4 *>(&sL[k][tr * 4]);
             const float4 bv = *reinterpret_cast<const float4 *>(&sU[k][tc * 4]);
-            const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+            const float ar[4] = {sL[k][tr], sL[k][tr + 16], sL[k][tr + 32], sL[k][tr + 48]};
+            const float br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll

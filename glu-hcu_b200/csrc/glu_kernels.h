@@ -41,7 +41,8 @@ cudaError_t launch_factor_chain(const DevPattern &P, const FactorPlanDev &F, flo
 
 // ------------------------------------------------------- supernodal factor --
 constexpr uint32_t kSnMaxWidth = 64;       // widest supernode
-constexpr uint32_t kSnPanelThreads = 128;  // threads of a panel block (rows or targets per block)
+constexpr uint32_t kSnPanelThreads = 128;  // threads of a panel block: rows or targets of a narrow supernode per block
+constexpr uint32_t kSnPanelWideRows = 64;  // and of one wider than kSnSmallWidth
 
 constexpr uint32_t kSnSmallWidth = 16;         // small supernode: width <= this, few off-diagonal rows/entries
 constexpr uint32_t kSnSmallFlag = 0x80000000u;  // block-map entry of a group of small supernodes

@@ -342,6 +342,40 @@ __device__ __forceinline__ void tri_rows_solve(float *sW, uint32_t ldw, uint32_t
     }
 }
 
+// The same with two threads per row (half 0 or 1; all 2 x rows threads of the
+// block take part): chunk cj belongs to half cj % 2, which applies the earlier
+// chunks to it and solves it, so the two halves share the updates and only a
+// solved chunk is waited for (a block barrier each).  The caller has a barrier
+// between its writes and the call and before it reads the result.
+template <bool kDiv>
+__device__ __forceinline__ void tri_rows_solve_halves(float *sW, uint32_t ldw, uint32_t t, uint32_t half, const float *sM,
+                                                      uint32_t w) {
+    const uint32_t nch = (w + kTriChunk - 1) / kTriChunk;
+    for (uint32_t cb = 0; cb < nch; ++cb) {
+        if (half == (cb & 1)) {
+            float x[kTriChunk];
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) x[k] = sW[(cb * kTriChunk + k) * ldw + t];
+            tri_chunk_solve<kDiv>(x, sM, cb, w);
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) sW[(cb * kTriChunk + k) * ldw + t] = x[k];
+        }
+        if (cb + 1 == nch) break;
+        __syncthreads();
+        float x[kTriChunk];
+#pragma unroll
+        for (int k = 0; k < kTriChunk; ++k) x[k] = sW[(cb * kTriChunk + k) * ldw + t];
+        for (uint32_t cj = cb + 1 + ((cb + 1 + half) & 1); cj < nch; cj += 2) {
+            float y[kTriChunk];
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) y[k] = sW[(cj * kTriChunk + k) * ldw + t];
+            tri_chunk_update(y, x, sM, cb, cj, w);
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) sW[(cj * kTriChunk + k) * ldw + t] = y[k];
+        }
+    }
+}
+
 // Working arrays of tri_invert.
 struct TriInverse {
     float M[kTriMax][kTriMax + 1], X[kTriMax][kTriMax + 1], W[kTriMax / 2][kTriMax / 2 + 1];
