@@ -16,6 +16,8 @@
 // correctly rounded reciprocal instead of divided by the pivot).  GESP
 // perturbation (numeric.cu:139-140) is applied to every pivot whose column
 // has an L part.
+#include <algorithm>
+
 #include "glu_common.cuh"
 #include "glu_kernels.h"
 #include "glu_tri.cuh"
@@ -315,54 +317,66 @@ cudaError_t launch_dense_update(float *val, uint64_t stride, uint32_t count, con
 }
 
 // ------------------------------------------------ dense buffer gather/scatter --
-// One warp per tail column; blockIdx.z selects the value set.
-__global__ void __launch_bounds__(256) k_dense_gather(DevPattern P, const float *__restrict__ val_base,
+// A block per tail column (a warp per column leaves a chain of one load per 32
+// entries: 36 us at order 1,920, now 9); the gather first clears its column.
+// blockIdx.z selects the value set.
+__global__ void __launch_bounds__(128) k_dense_gather(DevPattern P, const float *__restrict__ val_base,
                                                       uint64_t stride, uint32_t t, uint32_t m,
                                                       const uint32_t *__restrict__ tail_start, float *dbuf) {
     const float *val = val_base + blockIdx.z * stride;
-    float *D = dbuf + size_t(blockIdx.z) * m * m;
-    const uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (j >= m) return;
-    float *col = D + size_t(j) * m;
-    for (uint32_t p = tail_start[j] + lane; p < P.cptr[t + j + 1]; p += 32) col[P.ridx[p] - t] = val[p];
+    const uint32_t j = blockIdx.x;
+    float *col = dbuf + size_t(blockIdx.z) * m * m + size_t(j) * m;
+    const uint32_t p0 = tail_start[j], p1 = P.cptr[t + j + 1];
+    if (p1 - p0 < m) {
+        for (uint32_t i = threadIdx.x; i < m; i += 128) col[i] = 0.0f;
+        __syncthreads();
+    }
+#pragma unroll 8
+    for (uint32_t p = p0 + threadIdx.x; p < p1; p += 128) col[__ldg(P.ridx + p) - t] = __ldg(val + p);
 }
 
-__global__ void __launch_bounds__(256) k_dense_scatter(DevPattern P, float *val_base, uint64_t stride,
+__global__ void __launch_bounds__(128) k_dense_scatter(DevPattern P, float *val_base, uint64_t stride,
                                                        uint32_t t, uint32_t m,
                                                        const uint32_t *__restrict__ tail_start,
                                                        const float *__restrict__ dbuf) {
     float *val = val_base + blockIdx.z * stride;
-    const float *D = dbuf + size_t(blockIdx.z) * m * m;
-    const uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (j >= m) return;
-    const float *col = D + size_t(j) * m;
-    for (uint32_t p = tail_start[j] + lane; p < P.cptr[t + j + 1]; p += 32) val[p] = col[P.ridx[p] - t];
+    const uint32_t j = blockIdx.x;
+    const float *col = dbuf + size_t(blockIdx.z) * m * m + size_t(j) * m;
+    const uint32_t p1 = P.cptr[t + j + 1];
+#pragma unroll 8
+    for (uint32_t p = tail_start[j] + threadIdx.x; p < p1; p += 128) val[p] = __ldg(col + (__ldg(P.ridx + p) - t));
 }
 
 cudaError_t launch_dense_gather(const DevPattern &P, const float *val, uint64_t stride, uint32_t count,
                                 uint32_t t, uint32_t m, const uint32_t *tail_start, float *dbuf,
                                 cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(dbuf, 0, sizeof(float) * size_t(m) * m * count, st);
-    if (e != cudaSuccess) return e;
-    k_dense_gather<<<dim3((m + 7) / 8, 1, count), 256, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
+    k_dense_gather<<<dim3(m, 1, count), 128, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dense_scatter(const DevPattern &P, float *val, uint64_t stride, uint32_t count,
                                  uint32_t t, uint32_t m, const uint32_t *tail_start, const float *dbuf,
                                  cudaStream_t st) {
-    k_dense_scatter<<<dim3((m + 7) / 8, 1, count), 256, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
+    k_dense_scatter<<<dim3(m, 1, count), 128, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
     return cudaGetLastError();
 }
 
 // --------------------------------------------------------------- utilities --
-__global__ void k_colsum(DevPattern P, const float *val_base, uint64_t stride, float *colmax) {
+__global__ void __launch_bounds__(32) k_colsum(DevPattern P, const float *val_base, uint64_t stride, float *colmax) {
     const float *val = val_base + blockIdx.z * stride;
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     float tmp = 0.0f;
     if (c < P.n) {
-        // same order and precision as the reference's host loop (numeric.cu:495-502)
-        for (uint32_t p = P.cptr[c]; p < P.cptr[c + 1]; ++p) tmp += fabsf(val[p]);
+        // same order and precision as the reference's host loop (numeric.cu:495-502);
+        // 32 loads in flight, or the sum waits for each (n = 2,777: 56 -> 24 us)
+        const uint32_t p1 = P.cptr[c + 1];
+        for (uint32_t p = P.cptr[c]; p < p1; p += 32) {
+            float v[32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = p + k < p1 ? __ldg(val + p + k) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) tmp += fabsf(v[k]);
+        }
     }
     // block max, then one atomic (non-negative floats compare as integers)
     for (int o = 16; o > 0; o >>= 1) tmp = fmaxf(tmp, __shfl_xor_sync(0xffffffffu, tmp, o));
@@ -378,7 +392,7 @@ cudaError_t launch_pert(const DevPattern &P, const float *val, uint64_t stride, 
                         float *colsum_scratch, float *pert_z, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(colsum_scratch, 0, sizeof(float) * count, st);
     if (e != cudaSuccess) return e;
-    k_colsum<<<dim3((P.n + 255) / 256, 1, count), 256, 0, st>>>(P, val, stride, colsum_scratch);
+    k_colsum<<<dim3((P.n + 31) / 32, 1, count), 32, 0, st>>>(P, val, stride, colsum_scratch);
     k_pert_finish<<<(count + 255) / 256, 256, 0, st>>>(colsum_scratch, pert_z, count);
     return cudaGetLastError();
 }
@@ -402,30 +416,42 @@ cudaError_t launch_check_pivots(const DevPattern &P, const float *val, uint64_t 
     return cudaGetLastError();
 }
 
-__global__ void k_gather_values(const int64_t *__restrict__ lu_src, const double *__restrict__ ax_base,
+__global__ void k_gather_values(const uint32_t *__restrict__ lu_src, const double *__restrict__ ax_base,
                                 uint64_t ax_stride, const double *__restrict__ scale, uint32_t nnz,
                                 float *val_base, uint64_t stride) {
     const double *ax = ax_base + blockIdx.z * ax_stride;
     float *val = val_base + blockIdx.z * stride;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += gridDim.x * blockDim.x) {
-        int64_t q = __ldg(lu_src + p);
+        const uint32_t q = __ldg(lu_src + p);
         float v = 0.0f;
-        if (q >= 0) {
-            double a = ax[q];
-            if (scale) a = a * __ldg(scale + q);
-            v = static_cast<float>(a);
-        }
+        if (q != UINT32_MAX) v = static_cast<float>(ax[q] * __ldg(scale + q));
         val[p] = v;
     }
 }
 
-cudaError_t launch_gather_values(const int64_t *lu_src, const double *ax, uint64_t ax_stride,
-                                 const double *scale, uint32_t nnz, float *val, uint64_t stride,
-                                 uint32_t count, cudaStream_t st) {
-    uint32_t blocks = (nnz + 255) / 256;
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    if (blocks == 0) blocks = 1;
-    k_gather_values<<<dim3(blocks, 1, count), 256, 0, st>>>(lu_src, ax, ax_stride, scale, nnz, val, stride);
+// Source entry q to its LU position (UINT32_MAX: an earlier entry has it).
+__global__ void k_scatter_values(const uint32_t *__restrict__ slot, const double *__restrict__ ax_base,
+                                 uint64_t ax_stride, const double *__restrict__ scale, uint32_t nnz_src,
+                                 float *val_base, uint64_t stride) {
+    const double *ax = ax_base + blockIdx.z * ax_stride;
+    float *val = val_base + blockIdx.z * stride;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nnz_src; q += gridDim.x * blockDim.x) {
+        const uint32_t p = __ldg(slot + q);
+        if (p != UINT32_MAX) val[p] = static_cast<float>(ax[q] * __ldg(scale + q));
+    }
+}
+
+cudaError_t launch_place_values(const uint32_t *map, bool by_source, const double *ax, uint32_t nnz_src,
+                                const double *scale, uint32_t nnz, float *val, uint32_t count, cudaStream_t st) {
+    const uint32_t len = by_source ? nnz_src : nnz;
+    const uint32_t blocks = std::max<uint32_t>(std::min<uint32_t>((len + 255) / 256, 148 * 32), 1);
+    if (by_source) {
+        cudaError_t e = cudaMemsetAsync(val, 0, sizeof(float) * size_t(nnz) * count, st);
+        if (e != cudaSuccess) return e;
+        k_scatter_values<<<dim3(blocks, 1, count), 256, 0, st>>>(map, ax, nnz_src, scale, nnz_src, val, nnz);
+    } else {
+        k_gather_values<<<dim3(blocks, 1, count), 256, 0, st>>>(map, ax, nnz_src, scale, nnz, val, nnz);
+    }
     return cudaGetLastError();
 }
 

@@ -180,10 +180,13 @@ cudaError_t launch_pert(const DevPattern &P, const float *val, uint64_t stride, 
 // ORs DEV_ZERO_PIVOT / DEV_NONFINITE_PIVOT into *status for bad pivots.
 cudaError_t launch_check_pivots(const DevPattern &P, const float *val, uint64_t stride,
                                 uint32_t count, uint32_t *status, cudaStream_t st);
-// LU values from source values: val[p] = src[p] < 0 ? 0 : (float)(ax[src[p]] * scale[src[p]]).
-cudaError_t launch_gather_values(const int64_t *lu_src, const double *ax, uint64_t ax_stride,
-                                 const double *scale, uint32_t nnz, float *val, uint64_t stride,
-                                 uint32_t count, cudaStream_t st);
+// LU values of `count` value sets from source values (nnz_src per set): 0, or
+// (float)(ax[q] * scale[q]) at the LU position of source entry q.  by_source:
+// map[q] is that position (UINT32_MAX: none) and the values are cleared and
+// then scattered; else map[p] is the source entry of LU position p (UINT32_MAX:
+// none) and every position is written once.
+cudaError_t launch_place_values(const uint32_t *map, bool by_source, const double *ax, uint32_t nnz_src,
+                                const double *scale, uint32_t nnz, float *val, uint32_t count, cudaStream_t st);
 
 // ------------------------------------------------------------------ levels --
 // Level sets (symbolic.cc:106-151) built on the device; scratch must hold

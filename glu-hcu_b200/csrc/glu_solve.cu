@@ -734,32 +734,62 @@ cudaError_t launch_transform_f32_to_f64_add(const uint32_t *idx, const double *s
 
 // ---------------------------------------------------------- FP64 residuals --
 // r = b - A0 x with A0 in CSR form (a_rptr/a_cidx; a_vmap gives the CSC
-// position of each CSR entry in ax0), one warp per row, deterministic order.
-// norms[2v] += sum r^2, norms[2v+1] = max |r| for right-hand side v.
-__global__ void __launch_bounds__(256) k_residual(const uint32_t *__restrict__ rptr, const uint32_t *__restrict__ cidx,
-                                                  const uint32_t *__restrict__ vmap, const double *__restrict__ ax0,
-                                                  uint32_t n, const double *__restrict__ b,
-                                                  const double *__restrict__ x, double *__restrict__ r,
-                                                  double *norms, uint32_t nrhs_per_set, uint64_t ax0_stride) {
-    const uint32_t lane = threadIdx.x & 31;
+// position of each CSR entry in ax0), kLanes lanes per row (circuit and grid
+// rows hold five to ten entries: with a warp per row most lanes had none and
+// the rows' loads waited for each other), deterministic order within a row.
+// norms[2v] += sum r^2, norms[2v+1] = max |r| for right-hand side v, one
+// atomic each per block (one per warp of a large launch queued at the one
+// address).  Measured, n = 490,000: 120 us with a warp per row and an atomic per
+// warp, 20 us now.
+constexpr int kResidualThreads = 256;
+template <int kLanes>
+__global__ void __launch_bounds__(kResidualThreads) k_residual(const uint32_t *__restrict__ rptr,
+                                                               const uint32_t *__restrict__ cidx,
+                                                               const uint32_t *__restrict__ vmap,
+                                                               const double *__restrict__ ax0, uint32_t n,
+                                                               const double *__restrict__ b,
+                                                               const double *__restrict__ x, double *__restrict__ r,
+                                                               double *norms, uint32_t nrhs_per_set,
+                                                               uint64_t ax0_stride) {
+    __shared__ double s_ss[kResidualThreads / 32], s_mx[kResidualThreads / 32];
+    const uint32_t sub = threadIdx.x % kLanes;
     const uint32_t v = blockIdx.y;
     const size_t off = size_t(v) * n;
     ax0 += (v / nrhs_per_set) * ax0_stride;  // the value set of vector v
     double ss = 0.0, mx = 0.0;
-    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / 32; row < n;
-         row += gridDim.x * blockDim.x / 32) {
+    const uint32_t step = gridDim.x * (kResidualThreads / kLanes);
+    // (every lane of a warp makes the same number of rounds, for the shuffles)
+    for (uint32_t row0 = blockIdx.x * (kResidualThreads / kLanes) + (threadIdx.x & ~31u) / kLanes; row0 < n; row0 += step) {
+        const uint32_t row = row0 + (threadIdx.x & 31) / kLanes;
+        const bool in = row < n;
         double acc = 0.0;
-        for (uint32_t e = rptr[row] + lane; e < rptr[row + 1]; e += 32)
-            acc = fma(ax0[vmap[e]], x[off + cidx[e]], acc);
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        double rv = b[off + row] - acc;
-        if (lane == 0) {
+        if (in)
+            for (uint32_t e = rptr[row] + sub; e < rptr[row + 1]; e += kLanes)
+                acc = fma(ax0[vmap[e]], x[off + cidx[e]], acc);
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (in && sub == 0) {
+            const double rv = b[off + row] - acc;
             r[off + row] = rv;
             ss += rv * rv;
             mx = fmax(mx, fabs(rv));
         }
     }
-    if (lane == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_ss[threadIdx.x / 32] = ss;
+        s_mx[threadIdx.x / 32] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kResidualThreads / 32; ++w) {
+            ss += s_ss[w];
+            mx = fmax(mx, s_mx[w]);
+        }
         atomicAdd(norms + 2 * v, ss);
         // non-negative doubles order like their bit patterns
         atomicMax(reinterpret_cast<unsigned long long *>(norms + 2 * v + 1),
@@ -773,12 +803,24 @@ cudaError_t launch_residual(const uint32_t *a_rptr, const uint32_t *a_cidx, cons
                             double *norms, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(double) * 2 * nvec, st);
     if (e != cudaSuccess) return e;
-    uint32_t blocks = (n + 7) / 8;
+    // lanes per row by the mean row length (ax0_stride entries in n rows)
+    const double mean = double(ax0_stride) / std::max<uint32_t>(n, 1);
+    const uint32_t lanes = mean <= 6 ? 4 : mean <= 14 ? 8 : 32;
+    const uint32_t rows = kResidualThreads / lanes;
+    uint32_t blocks = (n + rows - 1) / rows;
     // about eight blocks per SM in all
     const uint32_t cap = std::max<uint32_t>(1u, (148u * 8u + nvec - 1) / nvec);
     if (blocks > cap) blocks = cap;
-    k_residual<<<dim3(blocks, nvec, 1), 256, 0, st>>>(a_rptr, a_cidx, a_vmap, ax0, n, b, x, r, norms,
-                                                      std::max<uint32_t>(nrhs_per_set, 1u), ax0_stride);
+    auto go = [&](auto kern) {
+        kern<<<dim3(blocks, nvec, 1), kResidualThreads, 0, st>>>(a_rptr, a_cidx, a_vmap, ax0, n, b, x, r, norms,
+                                                                 std::max<uint32_t>(nrhs_per_set, 1u), ax0_stride);
+    };
+    if (lanes == 4)
+        go(k_residual<4>);
+    else if (lanes == 8)
+        go(k_residual<8>);
+    else
+        go(k_residual<32>);
     return cudaGetLastError();
 }
 
