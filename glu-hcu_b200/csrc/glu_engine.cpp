@@ -17,6 +17,7 @@
 #include <memory>
 #include <numeric>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -863,7 +864,8 @@ Status build_sn_plan(glu_handle_s *h) {
         h->ss_levels[u].clear();
         for (int32_t l = 0; l < snl; ++l) {
             const uint32_t b0 = uint32_t(smap.size());
-            const size_t small0 = ssmall.size();
+            std::vector<uint2> narrow;
+            std::vector<uint32_t> tiny, small;
             for (uint32_t i = lc[l]; i < lc[l + 1]; ++i) {
                 const uint32_t q = ord[i];
                 const uint32_t s0 = first[q], w = first[q + 1] - s0, last = first[q + 1] - 1;
@@ -875,21 +877,30 @@ Status build_sn_plan(glu_handle_s *h) {
                 } else {
                     off = 0;
                     for (uint32_t c = s0; c <= last; ++c) off += (s.l_col_ptr[c] - (c - s0)) - s.sym_c_ptr[c];
-                    smeta[i] = make_uint4(s0, w, 0u, 0u);
+                    smeta[i] = make_uint4(s0, w, s.sym_c_ptr[s0], s.l_col_ptr[s0]);
                     work = (off + kSnSweepAbove - 1) / kSnSweepAbove;
                 }
                 if (h->tune.sn_small && w <= kSnSmallWidth && off <= 32) {
-                    ssmall.push_back(i);
+                    (w == 1 && off <= kSnTinyEntries ? tiny : small).push_back(i);
                     continue;
                 }
                 work = std::max<uint64_t>(work, 1);
-                if (smap.size() + work > UINT32_MAX) return set_error(GLU_ERR_UNSUPPORTED, "solve schedule too large");
-                for (uint64_t bb = 0; bb < work; ++bb) smap.push_back(make_uint2(i, uint32_t(bb)));
+                if (smap.size() + narrow.size() + work > UINT32_MAX)
+                    return set_error(GLU_ERR_UNSUPPORTED, "solve schedule too large");
+                std::vector<uint2> &to = w > kSnSmallWidth ? smap : narrow;
+                for (uint64_t bb = 0; bb < work; ++bb) to.push_back(make_uint2(i, uint32_t(bb)));
             }
+            const uint32_t nwide = uint32_t(smap.size()) - b0;
+            smap.insert(smap.end(), narrow.begin(), narrow.end());
             const uint32_t big = uint32_t(smap.size()) - b0;
-            for (size_t g = small0; g < ssmall.size(); g += 8)
-                smap.push_back(make_uint2(uint32_t(g), kSnSmallFlag | uint32_t(std::min<size_t>(8, ssmall.size() - g))));
-            h->ss_levels[u].push_back(SnSweepLevel{b0, uint32_t(smap.size()) - b0, big});
+            for (const auto &[list, flags, per] : {std::tuple(&tiny, kSnSmallFlag | kSnTinyFlag, size_t(32)),
+                                                   std::tuple(&small, kSnSmallFlag, size_t(8))})
+                for (size_t g = 0; g < list->size(); g += per) {
+                    const size_t cnt = std::min(per, list->size() - g);
+                    smap.push_back(make_uint2(uint32_t(ssmall.size()), flags | uint32_t(cnt)));
+                    ssmall.insert(ssmall.end(), list->begin() + g, list->begin() + g + cnt);
+                }
+            h->ss_levels[u].push_back(SnSweepLevel{b0, uint32_t(smap.size()) - b0, nwide, big});
         }
         // fused form: per block the supernodes it solves (waits for) and the
         // supernodes whose unknowns its scatter updates (releases)
@@ -914,7 +925,7 @@ Status build_sn_plan(glu_handle_s *h) {
             const uint2 bi = smap[blk];
             std::vector<uint32_t> mine;
             if (bi.y & kSnSmallFlag) {
-                for (uint32_t g = 0; g < (bi.y & ~kSnSmallFlag); ++g) mine.push_back(ssmall[bi.x + g]);
+                for (uint32_t g = 0; g < (bi.y & kSnGroupCount); ++g) mine.push_back(ssmall[bi.x + g]);
             } else {
                 mine.push_back(bi.x);
             }
@@ -1296,8 +1307,8 @@ uint64_t solve_kernel_count(const glu_handle_s *h, bool trans) {
         if (sn) {
             uint32_t lev = 0;
             for (uint32_t l = 0; l < S.sn[u].nlev; ++l) {
-                const uint2 k2 = sn_sweep_level_launches(S.sn[u].levels[l], u == 1);
-                lev += k2.x + k2.y;
+                const uint3 k3 = sn_sweep_level_launches(S.sn[u].levels[l], u == 1);
+                lev += k3.x + k3.y + k3.z;
             }
             k += (S.sn[u].fused && h->use_sn ? 1 : lev) + (S.t > 0 ? 1 : 0);
         } else {

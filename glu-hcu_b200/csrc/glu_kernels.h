@@ -46,6 +46,9 @@ constexpr uint32_t kSnPanelWideRows = 64;  // and of one wider than kSnSmallWidt
 
 constexpr uint32_t kSnSmallWidth = 16;         // small supernode: width <= this, few off-diagonal rows/entries
 constexpr uint32_t kSnSmallFlag = 0x80000000u;  // block-map entry of a group of small supernodes
+constexpr uint32_t kSnTinyFlag = 0x40000000u;   // of the sweeps' maps: a group of single columns with few entries, 32 to a block
+constexpr uint32_t kSnTinyEntries = 8;          // most off-diagonal entries of one
+constexpr uint32_t kSnGroupCount = 0xFFFFu;     // the group's size in its map entry
 constexpr uint32_t kSnDiagSmallPerBlock = 8;    // narrow diagonal blocks per block of the diagonal launches (a warp each)
 
 // Supernodes in level order: their records, the block maps of the panel and
@@ -221,26 +224,33 @@ constexpr uint32_t kSweepChunk = 128;
 // Supernodal L or U sweep (used when the factor is supernodal): per block of
 // the sweep (levels one after another) its supernode and part, per supernode
 // (sweep order) its record {first column, width, L: first L21 position,
-// L: L21 rows}; the host-side levels.  A level's blocks are its supernodes'
-// parts first, then its groups of small supernodes.
+// L: L21 rows; U: first position and diagonal of the first column}; the
+// host-side levels.  A level's blocks are its wide supernodes' parts first,
+// then its narrow ones' (width <= kSnSmallWidth, more than 32 rows or entries),
+// then its groups of small supernodes (the tiny ones' first).
 struct SnSweepLevel {
     uint32_t b0, blocks;  // first block, blocks
-    uint32_t big;         // blocks [b0, b0 + big) are supernode parts, the rest small groups
+    uint32_t wide;        // blocks [b0, b0 + wide) are parts of wide supernodes,
+    uint32_t big;         // [b0 + wide, b0 + big) parts of narrow ones, the rest groups
 };
-// Blocks of small-supernode groups from which a per-level sweep gives them a
-// launch of their own: a warp-per-supernode kernel that keeps four (L) or
-// five (U) blocks per SM resident, against the full kernel's two (L) or four
-// (U).  The thresholds are where the waves saved on 148 SMs outweigh one more
-// chained launch; below them the level stays one launch.
+// Launches of one level of a per-level sweep: {full kernel, narrow kernel,
+// small-group kernel}.  The full kernel runs any block but keeps only two (L)
+// or three (U) of them on an SM; narrow and small kernels keep four or five.
+// Blocks of small groups, and in the L sweep of narrow parts, get a launch of
+// their own from the numbers on where the waves saved on 148 SMs outweigh one
+// more chained launch.
 constexpr uint32_t kSnSweepSplitL = 592;
 constexpr uint32_t kSnSweepSplitU = 2048;
-// Launches of one level of a per-level sweep: {full kernel, small-group kernel}.
-inline uint2 sn_sweep_level_launches(const SnSweepLevel &lv, bool upper) {
-    const uint32_t small = lv.blocks - lv.big;
-    if (lv.blocks == 0) return {0u, 0u};
-    if (lv.big == 0) return {0u, 1u};
-    if (small >= (upper ? kSnSweepSplitU : kSnSweepSplitL)) return {1u, 1u};
-    return {1u, 0u};
+inline uint3 sn_sweep_level_launches(const SnSweepLevel &lv, bool upper) {
+    const uint32_t small = lv.blocks - lv.big, narrow = lv.big - lv.wide;
+    if (lv.blocks == 0) return {0u, 0u, 0u};
+    if (lv.big == 0) return {0u, 0u, 1u};
+    const uint32_t s = small >= (upper ? kSnSweepSplitU : kSnSweepSplitL) ? 1u : 0u;
+    if (upper) return {1u, 0u, s};
+    // L: the narrow parts apart, together with small groups too few for a launch
+    const uint32_t rest = narrow + (s ? 0u : small);
+    if (lv.wide == 0) return {0u, 1u, s};
+    return {1u, rest >= kSnSweepSplitL / 2 ? 1u : 0u, s};
 }
 struct SnSweepPlan {
     const uint2 *map = nullptr;     // {supernode, part} or {first of small[], kSnSmallFlag | count}
@@ -260,7 +270,7 @@ struct SnSweepPlan {
     const uint32_t *indeg = nullptr;
 };
 constexpr uint32_t kSnSweepRows = 256;    // L21 rows per block of the L sweep
-constexpr uint32_t kSnSweepAbove = 1024;  // U entries per block of the U sweep
+constexpr uint32_t kSnSweepAbove = 2048;  // U entries per block of the U sweep
 
 // Value sets solved together: set z uses the factors at val + z * vstride
 // (dense tail at dval + z * dstride) and the right-hand sides

@@ -59,6 +59,20 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
     constexpr int SW = int(kSnSmallWidth);
     const uint4 md = W.meta[i];
     const uint32_t s = md.x, w = md.y, lbase = md.z, m = md.w, l = s + w - 1, n = P.n;
+    if (w == 1) {
+        const bool in = lane < m;
+        const float lv = in ? __ldg(val + lbase + lane) : 0.0f;
+        const uint32_t target = in ? __ldg(P.ridx + lbase + lane) : 0u;
+        pdl_wait();  // the previous level's x
+        for (uint32_t q = Q.q0; q < Q.q1; ++q) {
+            float *yq = y + size_t(q) * n;
+            const float x = __ldcg(yq + s);
+            if (lane == 0) xo[size_t(q) * n + s] = x;
+            const float u = __fmul_rn(lv, x);
+            if (in && u != 0.0f) atomicAdd(yq + target, -u);
+        }
+        return;
+    }
     const uint32_t dl = lane < w ? P.diag[s + lane] : 0u;
     float lrow[SW], l21[SW];
 #pragma unroll
@@ -89,6 +103,46 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
     }
 }
 
+// Groups of tiny supernodes (one column, at most eight off-diagonal entries):
+// eight lanes each, 32 to a block.  They are most of a grid's leaves, and a
+// warp each left most lanes without an entry.
+__device__ __forceinline__ void sn_sweep_l_tiny(const DevPattern &P, const SnSweepPlan &W,
+                                                const float *__restrict__ val, float *y, float *xo, Rhs Q, uint2 bi) {
+    const uint32_t g = threadIdx.x >> 3, sub = threadIdx.x & 7;
+    if (g >= (bi.y & kSnGroupCount)) return;
+    const uint4 md = W.meta[W.small[bi.x + g]];
+    const uint32_t s = md.x, lbase = md.z, m = md.w;
+    const bool in = sub < m;
+    const float l21 = in ? __ldg(val + lbase + sub) : 0.0f;
+    const uint32_t target = in ? __ldg(P.ridx + lbase + sub) : 0u;
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
+        float *yq = y + size_t(q) * P.n;
+        const float x = __ldcg(yq + s);
+        if (sub == 0) xo[size_t(q) * P.n + s] = x;
+        const float u = __fmul_rn(l21, x);
+        if (in && u != 0.0f) atomicAdd(yq + target, -u);
+    }
+}
+__device__ __forceinline__ void sn_sweep_u_tiny(const DevPattern &P, const SnSweepPlan &W,
+                                                const float *__restrict__ val, float *y, float *xo, Rhs Q, uint2 bi) {
+    const uint32_t g = threadIdx.x >> 3, sub = threadIdx.x & 7;
+    if (g >= (bi.y & kSnGroupCount)) return;
+    const uint4 md = W.meta[W.small[bi.x + g]];
+    const uint32_t s = md.x, cp = md.z, dk = md.w;
+    const bool in = cp + sub < dk;
+    const float u = in ? __ldg(val + cp + sub) : 0.0f;
+    const uint32_t target = in ? __ldg(P.ridx + cp + sub) : 0u;
+    const float piv = __ldg(val + dk);
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
+        float *yq = y + size_t(q) * P.n;
+        const float x = __ldcg(yq + s) / piv;
+        if (sub == 0) xo[size_t(q) * P.n + s] = x;
+        if (in && x != 0.0f) atomicAdd(yq + target, -__fmul_rn(u, x));
+    }
+}
+
 // U sweep of one small supernode (w <= kSnSmallWidth, at most 32 entries above
 // the block) by one warp: lane k holds unknown s+k and above-block entry k.
 __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSweepPlan &W,
@@ -97,6 +151,20 @@ __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSw
     constexpr int SW = int(kSnSmallWidth);
     const uint4 md = W.meta[i];
     const uint32_t s = md.x, w = md.y, n = P.n;
+    if (w == 1) {
+        const bool in = md.z + lane < md.w;
+        const float uv = in ? __ldg(val + md.z + lane) : 0.0f;
+        const uint32_t target = in ? __ldg(P.ridx + md.z + lane) : 0u;
+        const float piv = __ldg(val + md.w);
+        pdl_wait();  // the previous level's x
+        for (uint32_t q = Q.q0; q < Q.q1; ++q) {
+            float *yq = y + size_t(q) * n;
+            const float x = __ldcg(yq + s) / piv;
+            if (lane == 0) xo[size_t(q) * n + s] = x;
+            if (in && x != 0.0f) atomicAdd(yq + target, -__fmul_rn(uv, x));
+        }
+        return;
+    }
     const uint32_t dl = lane < w ? P.diag[s + lane] : 0u;
     const uint32_t cp = lane < w ? P.cptr[s + lane] : 0u;
     const uint32_t cnt = lane < w ? (dl - lane) - cp : 0u;  // entries of column s+lane above the block
@@ -145,6 +213,24 @@ __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSw
         if (ev && xe != 0.0f) atomicAdd(yq + tg, -__fmul_rn(ue, xe));
     }
 }
+// A group of small supernodes: tiny ones, or one per warp.
+__device__ __forceinline__ void sn_sweep_l_group(const DevPattern &P, const SnSweepPlan &W,
+                                                 const float *__restrict__ val, float *y, float *xo, Rhs Q, uint2 bi) {
+    const uint32_t wi = threadIdx.x >> 5;
+    if (bi.y & kSnTinyFlag)
+        sn_sweep_l_tiny(P, W, val, y, xo, Q, bi);
+    else if (wi < (bi.y & kSnGroupCount))
+        sn_sweep_l_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
+}
+__device__ __forceinline__ void sn_sweep_u_group(const DevPattern &P, const SnSweepPlan &W,
+                                                 const float *__restrict__ val, float *y, float *xo, Rhs Q, uint2 bi) {
+    const uint32_t wi = threadIdx.x >> 5;
+    if (bi.y & kSnTinyFlag)
+        sn_sweep_u_tiny(P, W, val, y, xo, Q, bi);
+    else if (wi < (bi.y & kSnGroupCount))
+        sn_sweep_u_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
+}
+
 // Fused sweeps: the block's item and value set from one ticket counter of the
 // launch, handed out item-major over the value sets (ticket = item * count +
 // set, so every set's sweep advances at once), and a wait (thread 0, bounded)
@@ -234,8 +320,7 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     float(*part)[kSnMaxWidth] = reinterpret_cast<float(*)[kSnMaxWidth]>(sT);
     const uint2 bi = W.map[blk];
     if (bi.y & kSnSmallFlag) {  // a group of small supernodes, one per warp
-        const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_l_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
+        sn_sweep_l_group(P, W, val, y, xo, Q, bi);
         sweep_release(W, blk, done);
         return;
     }
@@ -323,7 +408,72 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     sweep_release(W, blk, done);
 }
 
-__global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
+// The L sweep's parts of narrow supernodes (w <= kSnSmallWidth, 256 rows of L21
+// each, a row per thread in 16 registers) and groups of small ones.
+__global__ void __launch_bounds__(256, 4) k_sn_sweep_l_narrow(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
+                                                           float *y, float *xo, uint32_t nrhs, uint32_t b0,
+                                                           uint64_t vstride, uint64_t ystride) {
+    constexpr int SW = int(kSnSmallWidth);
+    __shared__ uint32_t sB[SW];
+    __shared__ __align__(16) float sT[SW * (SW + 1)], xs[SW];
+    pdl_release();
+    val += blockIdx.z * vstride;
+    y += blockIdx.z * ystride;
+    xo += blockIdx.z * ystride;
+    const Rhs Q = rhs_share(nrhs);
+    const uint2 bi = W.map[b0 + blockIdx.x];
+    if (bi.y & kSnSmallFlag) {
+        sn_sweep_l_group(P, W, val, y, xo, Q, bi);
+        return;
+    }
+    const uint4 md = W.meta[bi.x];
+    const uint32_t s = md.x, w = md.y, lbase = md.z, m = md.w, t = bi.y;
+    const uint32_t l = s + w - 1;
+    const uint32_t tid = threadIdx.x, n = P.n;
+    if (tid < w) sB[tid] = P.diag[s + tid];
+    __syncthreads();
+    const uint32_t r = t * blockDim.x + tid;  // L21 row of this thread
+    float lr[SW];
+#pragma unroll
+    for (int c = 0; c < SW; ++c)
+        lr[c] = (r < m && uint32_t(c) < w) ? __ldg(val + sB[c] + (l + 1 - (s + c)) + r) : 0.0f;
+    const uint32_t target = r < m ? __ldg(P.ridx + lbase + r) : 0u;
+    {   // L11, strictly lower: L(s+k, s+c) at diag[s+c] + (k - c)
+        const uint32_t c = tid / SW, k = tid % SW;
+        sT[c * (SW + 1) + k] = (c < w && k < w && k > c) ? __ldg(val + sB[c] + (k - c)) : 0.0f;
+    }
+    if (tid < SW) xs[tid] = 0.0f;
+    __syncthreads();
+    pdl_wait();  // the previous level's x
+    for (uint32_t q = Q.q0; q < Q.q1; ++q) {
+        float *yq = y + size_t(q) * n;
+        if (tid < 32) {
+            float v = tid < w ? __ldcg(yq + s + tid) : 0.0f;
+            for (uint32_t c = 0; c + 1 < w; ++c) {
+                const float xc = __shfl_sync(kFull, v, c);
+                if (tid > c && tid < w) v = __fsub_rn(v, __fmul_rn(sT[c * (SW + 1) + tid], xc));
+            }
+            if (tid < w) xs[tid] = v;
+            if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = v;
+        }
+        __syncthreads();
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const float4 *x4 = reinterpret_cast<const float4 *>(xs);
+#pragma unroll
+        for (int c = 0; c < SW; c += 4) {
+            const float4 x = x4[c / 4];
+            acc[0] = fmaf(lr[c], x.x, acc[0]);
+            acc[1] = fmaf(lr[c + 1], x.y, acc[1]);
+            acc[2] = fmaf(lr[c + 2], x.z, acc[2]);
+            acc[3] = fmaf(lr[c + 3], x.w, acc[3]);
+        }
+        const float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        if (r < m && sum != 0.0f) atomicAdd(yq + target, -sum);
+        if (q + 1 < Q.q1) __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                     uint64_t vstride, uint64_t ystride,
                                                     const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
@@ -343,8 +493,7 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_u(DevPattern P, SnSweepPlan
     float(*part)[kSnMaxWidth] = reinterpret_cast<float(*)[kSnMaxWidth]>(sT);
     const uint2 bi = W.map[blk];
     if (bi.y & kSnSmallFlag) {  // a group of small supernodes, one per warp
-        const uint32_t wi = threadIdx.x >> 5;
-        if (wi < (bi.y & ~kSnSmallFlag)) sn_sweep_u_small(P, W, val, y, xo, Q, W.small[bi.x + wi], threadIdx.x & 31);
+        sn_sweep_u_group(P, W, val, y, xo, Q, bi);
         sweep_release(W, blk, done);
         return;
     }
@@ -492,22 +641,16 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_l_small(DevPattern P, SnSwe
                                                           float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                           uint64_t vstride, uint64_t ystride) {
     pdl_release();
-    const uint2 bi = W.map[b0 + blockIdx.x];
-    const uint32_t wi = threadIdx.x >> 5;
-    if (!(bi.y & kSnSmallFlag) || wi >= (bi.y & ~kSnSmallFlag)) return;
-    sn_sweep_l_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
-                     rhs_share(nrhs), W.small[bi.x + wi], threadIdx.x & 31);
+    sn_sweep_l_group(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
+                     rhs_share(nrhs), W.map[b0 + blockIdx.x]);
 }
 
 __global__ void __launch_bounds__(256, 5) k_sn_sweep_u_small(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                           float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                           uint64_t vstride, uint64_t ystride) {
     pdl_release();
-    const uint2 bi = W.map[b0 + blockIdx.x];
-    const uint32_t wi = threadIdx.x >> 5;
-    if (!(bi.y & kSnSmallFlag) || wi >= (bi.y & ~kSnSmallFlag)) return;
-    sn_sweep_u_small(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
-                     rhs_share(nrhs), W.small[bi.x + wi], threadIdx.x & 31);
+    sn_sweep_u_group(P, W, val + blockIdx.z * vstride, y + blockIdx.z * ystride, xo + blockIdx.z * ystride,
+                     rhs_share(nrhs), W.map[b0 + blockIdx.x]);
 }
 
 // Inverses of the diagonal blocks of the wide supernodes (blockIdx.x; first
@@ -567,10 +710,11 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
         // either order
         for (uint32_t l = 0; l < W.nlev; ++l) {
             const SnSweepLevel &lv = W.levels[l];
-            const uint2 k2 = sn_sweep_level_launches(lv, upper);
+            const uint3 k3 = sn_sweep_level_launches(lv, upper);
             cudaError_t e = cudaSuccess;
-            if (k2.x) {  // the full kernel: the parts, and the groups unless they launch apart
-                const uint32_t nblk = k2.y ? lv.big : lv.blocks;
+            const uint32_t rest = k3.z ? lv.big : lv.blocks;  // blocks not in the small-group launch
+            if (k3.x) {  // the full kernel: every block that no other launch takes
+                const uint32_t nblk = k3.y ? lv.wide : rest;
                 const dim3 grid(nblk, shares(nblk), B.count);
                 if (upper)
                     e = launch_chained(k_sn_sweep_u, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride,
@@ -582,7 +726,14 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
                                        status, spin_limit);
                 if (e != cudaSuccess) return e;
             }
-            if (k2.y) {  // the small-supernode groups
+            if (k3.y) {  // L: the narrow parts (and the groups, unless they launch apart)
+                const uint32_t nblk = rest - lv.wide;
+                const dim3 grid(nblk, shares(nblk), B.count);
+                e = launch_chained(k_sn_sweep_l_narrow, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0 + lv.wide,
+                                   B.vstride, ystride);
+                if (e != cudaSuccess) return e;
+            }
+            if (k3.z) {  // the small-supernode groups
                 const dim3 grid(lv.blocks - lv.big, shares(lv.blocks - lv.big), B.count);
                 if (upper)
                     e = launch_chained(k_sn_sweep_u_small, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs,
