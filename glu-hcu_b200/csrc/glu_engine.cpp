@@ -190,6 +190,9 @@ struct LaunchGraph {
     std::array<uint64_t, 12> key{};
     cudaGraphExec_t exec = nullptr;
     bool failed = false;  // could not be captured: launched one by one
+    // what the sequence's launches add to a factorization's statistics
+    uint64_t launches = 0;
+    double upd_bytes = 0, upd_flops = 0;
 };
 constexpr size_t kMaxGraphs = 8;  // per handle
 
@@ -382,9 +385,13 @@ constexpr double kSparseRate = 0.2e12, kLevelLatency = 8e-6;
 // (measured: FP32 solve of a 251 x 251 grid, 77 launches, 399 -> 369 us;
 // transposed refined solve at n = 9,973 1,035 -> 931 us).  Waiting for the
 // second call keeps a handle's first solve as quick as it was.
+// enqueue(stream, slot) makes the launches and notes their statistics in the
+// slot, which `slot` (nullable) returns.
 template <class Enqueue>
-Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStream_t st, Enqueue &&enqueue) {
+Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStream_t st, Enqueue &&enqueue,
+                   LaunchGraph *slot = nullptr) {
     LaunchGraph *g = nullptr;
+    Status s = GLU_OK;
     for (LaunchGraph &c : h->graphs)
         if (c.key == key) g = &c;
     if (!g) {
@@ -397,14 +404,16 @@ Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStr
             *g = LaunchGraph{};
         }
         g->key = key;
-        return enqueue(st);
+        s = enqueue(st, *g);
+        if (slot) *slot = *g;
+        return s;
     }
     if (!g->exec && !g->failed) {
         g->failed = true;
         if (!h->capture && cudaStreamCreateWithFlags(&h->capture, cudaStreamNonBlocking) != cudaSuccess)
             h->capture = nullptr;
         if (h->capture && cudaStreamBeginCapture(h->capture, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            const Status s = enqueue(h->capture);
+            s = enqueue(h->capture, *g);
             cudaGraph_t graph = nullptr;
             const cudaError_t e = cudaStreamEndCapture(h->capture, &graph);
             if (s == GLU_OK && e == cudaSuccess && graph &&
@@ -416,9 +425,13 @@ Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStr
         }
         cudaGetLastError();
     }
-    if (!g->exec) return enqueue(st);
-    GLU_CUDA(cudaGraphLaunch(g->exec, st), "launch graph");
-    return GLU_OK;
+    s = GLU_OK;
+    if (!g->exec)
+        s = enqueue(st, *g);
+    else
+        GLU_CUDA(cudaGraphLaunch(g->exec, st), "launch graph");
+    if (slot) *slot = *g;
+    return s;
 }
 uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 
@@ -1377,7 +1390,8 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
     float *xo = h->d_xo.as<float>();
     const SolvePlanDev S = solve_plan(h);
     h->stats.solve_launches += solve_kernel_count(h, trans);
-    auto enqueue = [&](cudaStream_t s) -> Status {
+    LaunchGraph none;
+    auto enqueue = [&](cudaStream_t s, LaunchGraph &) -> Status {
         if (!trans) {
             GLU_CUDA(solve_lower_unit(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s), "lower solve");
             GLU_CUDA(solve_upper(h->P, S, val, dval, y, xo, nrhs, cnt, tk, status, B, s), "upper solve");
@@ -1389,7 +1403,7 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
         }
         return GLU_OK;
     };
-    if (S.ticket_base) return enqueue(st);  // an injected failure, for this solve only
+    if (S.ticket_base) return enqueue(st, none);  // an injected failure, for this solve only
     return run_graphed(h, {trans ? 2u : 1u, z, count, nrhs, key_of(val), key_of(dval), key_of(y), key_of(xo),
                            key_of(B.dinv), key_of(B.sn_inv), key_of(B.sweep_done) ^ key_of(tk), S.spin_limit},
                        st, enqueue);
@@ -1770,18 +1784,52 @@ glu_status glu_load_source_values(glu_handle_t h, uint32_t first, uint32_t count
 
 namespace {
 
-// Everything of a factorization up to its last launch, on st; the status word
-// (and the perturbation of value set `first`) are copied to pinned memory
-// asynchronously.  factor_finish reads them once st has completed.
-Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, cudaStream_t st) {
+// Buffers of a factorization of `count` value sets: the dataflow's workspace
+// (and whether the dense block takes it), the tensor-core operand packs, the
+// diagonal blocks' inverses.
+Status factor_buffers(glu_handle_s *h, uint32_t count, bool *use_flow) {
+    // the whole block by one dataflow launch, where its workspace fits in half
+    // of the free memory
+    bool flow = dense_flow(h->tune, h->m, count);
+    if (flow) {
+        const size_t bytes = sizeof(float) * dense_flow_floats(h->m) * count +
+                             sizeof(uint32_t) * dense_flow_ctl_words(h->m, count);
+        size_t free_b = 0, total_b = 0;
+        if (bytes > h->d_flow_work.bytes && bytes > (size_t(256) << 20))  // (the query is slow)
+            flow = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= free_b / 2;
+        flow = flow && h->d_flow_work.ensure(bytes) == cudaSuccess;
+        if (!flow) cudaGetLastError();
+    }
+    *use_flow = flow;
+    // tensor-core updates for wide trailing blocks; their operand packs are
+    // allocated once per handle
+    const bool tc = h->m && h->tune.dense_tc_min && h->m >= h->tune.dense_tc_min;
+    if (tc && (!flow || !h->couple_groups.empty()) && h->pack_m != h->m) {
+        const size_t pack_bytes = sizeof(uint16_t) * kDensePackRow * size_t(h->m) * h->batch;
+        GLU_CUDA(h->d_packA.alloc(pack_bytes), "allocate tensor-core operand packs");
+        GLU_CUDA(h->d_packB.alloc(pack_bytes), "allocate tensor-core operand packs");
+        GLU_CUDA(dense_tc_tensor_map(h->d_packA.as<uint16_t>(), h->m, h->batch, &h->map_packA), "tensor map");
+        GLU_CUDA(dense_tc_tensor_map(h->d_packB.as<uint16_t>(), h->m, h->batch, &h->map_packB), "tensor map");
+        GLU_CUDA(h->d_tc_counter.alloc(sizeof(uint32_t) * 2), "allocate tile counters");
+        h->pack_m = h->m;
+    }
+    if (h->m)
+        GLU_CUDA(h->d_dinv.ensure(sizeof(float) * dinv_per_set(h) * h->batch), "allocate diagonal-block inverses");
+    if (h->use_sn && h->nwide &&
+        h->d_sn_inv.ensure(sizeof(float) * uint64_t(h->nwide) * kSnInvFloats * h->batch) != cudaSuccess)
+        cudaGetLastError();  // (the sweeps then solve those blocks column by column)
+    return GLU_OK;
+}
+
+// The kernels of a factorization, on st; their number and the dense update's
+// statistics go to `note`.
+Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, bool flow, cudaStream_t st,
+                       LaunchGraph &note) {
     Status s = GLU_OK;
     float *val = h->d_val.as<float>() + size_t(first) * h->nnz;
     const uint64_t stride = h->nnz;
     const float *pert = nullptr;
-    GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
-    GLU_CUDA(cudaEventRecord(h->ev0, st), "event");
     KernelProfiler &pf = h->prof;
-    pf.used = 0;
     uint64_t nlaunch = 0;  // kernel launches of this call
 #define GLU_LAUNCH(kind, call, what)                    \
     do {                                                \
@@ -1850,32 +1898,10 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
     float *dscr = h->d_diag_scratch.as<float>();
     bool rest_pending = false;
     const uint32_t nb = kDenseNB;
-    // the whole block by one dataflow launch, where its workspace fits in half
-    // of the free memory
-    bool flow = dense_flow(h->tune, h->m, count);
     const size_t flow_floats = flow ? dense_flow_floats(h->m) * count : 0;
-    if (flow) {
-        const size_t bytes = sizeof(float) * flow_floats + sizeof(uint32_t) * dense_flow_ctl_words(h->m, count);
-        size_t free_b = 0, total_b = 0;
-        if (bytes > h->d_flow_work.bytes && bytes > (size_t(256) << 20))  // (the query is slow)
-            flow = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= free_b / 2;
-        flow = flow && h->d_flow_work.ensure(bytes) == cudaSuccess;
-        if (!flow) cudaGetLastError();
-    }
     lookahead = lookahead && !flow;
     cudaStream_t ps = lookahead ? h->aux : st;  // panels and strips
-    // tensor-core updates for wide trailing blocks; their operand packs are
-    // allocated once per handle
-    const bool tc = h->m && h->tune.dense_tc_min && h->m >= h->tune.dense_tc_min;
-    if (tc && (!flow || !h->couple_groups.empty()) && h->pack_m != h->m) {
-        const size_t pack_bytes = sizeof(uint16_t) * kDensePackRow * size_t(h->m) * h->batch;
-        GLU_CUDA(h->d_packA.alloc(pack_bytes), "allocate tensor-core operand packs");
-        GLU_CUDA(h->d_packB.alloc(pack_bytes), "allocate tensor-core operand packs");
-        GLU_CUDA(dense_tc_tensor_map(h->d_packA.as<uint16_t>(), h->m, h->batch, &h->map_packA), "tensor map");
-        GLU_CUDA(dense_tc_tensor_map(h->d_packB.as<uint16_t>(), h->m, h->batch, &h->map_packB), "tensor map");
-        GLU_CUDA(h->d_tc_counter.alloc(sizeof(uint32_t) * 2), "allocate tile counters");
-        h->pack_m = h->m;
-    }
+    const bool tc = h->m && h->tune.dense_tc_min && h->m >= h->tune.dense_tc_min;  // tensor-core updates
     uint32_t *dstatus = h->d_status.as<uint32_t>();
     double upd_bytes = 0, upd_flops = 0;
     // The sparse columns' deferred updates of the block (the plan has them
@@ -2027,24 +2053,48 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
                    launch_dense_scatter(h->P, val, stride, count, h->t, h->m, h->d_tail_start.as<uint32_t>(), dbase, st),
                    "factor (dense scatter)");
     if (h->m) {
-        GLU_CUDA(h->d_dinv.ensure(sizeof(float) * dinv_per_set(h) * h->batch), "allocate diagonal-block inverses");
         GLU_LAUNCH(KK_DIAG_INV,
                    launch_dense_diag_inv(dbase, dstride, count, doff, h->m,
                                          h->d_dinv.as<float>() + size_t(first) * dinv_per_set(h), st),
                    "factor (diagonal-block inverses)");
     }
-    if (h->use_sn && h->nwide) {
+    if (h->use_sn && h->nwide && h->d_sn_inv.p) {
         const uint64_t per = uint64_t(h->nwide) * kSnInvFloats;
-        if (h->d_sn_inv.ensure(sizeof(float) * per * h->batch) == cudaSuccess)
-            GLU_LAUNCH(KK_DIAG_INV,
-                       launch_sn_diag_inv(h->P, h->d_wide.as<uint2>(), h->nwide, val, stride, count,
-                                          h->d_sn_inv.as<float>() + first * per, per, st),
-                       "factor (supernode inverses)");
-        else
-            cudaGetLastError();
+        GLU_LAUNCH(KK_DIAG_INV,
+                   launch_sn_diag_inv(h->P, h->d_wide.as<uint2>(), h->nwide, val, stride, count,
+                                      h->d_sn_inv.as<float>() + first * per, per, st),
+                   "factor (supernode inverses)");
     }
     GLU_LAUNCH(KK_CHECK, launch_check_pivots(h->P, val, stride, count, h->d_status.as<uint32_t>(), st), "pivot check");
 #undef GLU_LAUNCH
+    note.launches = nlaunch;
+    note.upd_bytes = upd_bytes;
+    note.upd_flops = upd_flops;
+    return s;
+}
+
+// Everything of a factorization up to its last launch, on st; the status word
+// (and the perturbation of value set `first`) are copied to pinned memory
+// asynchronously.  factor_finish reads them once st has completed.
+Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, cudaStream_t st) {
+    bool flow = false;
+    Status s = factor_buffers(h, count, &flow);
+    if (s != GLU_OK) return s;
+    GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
+    GLU_CUDA(cudaEventRecord(h->ev0, st), "event");
+    h->prof.used = 0;
+    LaunchGraph note;
+    auto enqueue = [&](cudaStream_t to, LaunchGraph &n) { return factor_launches(h, first, count, perturb, flow, to, n); };
+    // (the profiler's events are per launch; with look-ahead the launches of
+    // two streams are long enough to hide their cost)
+    const bool lookahead = !flow && h->tune.dense_lookahead && h->m >= h->tune.dense_lookahead;
+    if (h->prof.on || lookahead)
+        s = enqueue(st, note);
+    else
+        s = run_graphed(h, {3u, first, count, perturb != 0, flow, key_of(h->d_flow_work.p), key_of(h->d_dinv.p),
+                            key_of(h->d_sn_inv.p), key_of(h->d_packA.p), key_of(h->d_dense.p), h->spin_limit, 0u},
+                        st, enqueue, &note);
+    if (s != GLU_OK) return s;
     GLU_CUDA(cudaEventRecord(h->ev1, st), "event");
     GLU_CUDA(cudaMemcpyAsync(h->h_status, h->d_status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
              "read status");
@@ -2052,10 +2102,10 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
         GLU_CUDA(cudaMemcpyAsync(h->h_status + 1, h->d_pert.as<float>() + first, sizeof(float),
                                  cudaMemcpyDeviceToHost, st),
                  "read perturbation");
-    h->pending_launches = nlaunch;
-    h->pending_upd_bytes = upd_bytes;
-    h->pending_upd_flops = upd_flops;
-    return s;
+    h->pending_launches = note.launches;
+    h->pending_upd_bytes = note.upd_bytes;
+    h->pending_upd_flops = note.upd_flops;
+    return GLU_OK;
 }
 
 // The host half of a factorization whose stream has completed: status,
