@@ -18,16 +18,22 @@
 // interleaved over the value sets (a ticket); a tile needs only tiles claimed
 // before it, so every wait is for a running or finished block.  Besides its
 // place in the factor a finished tile is written to a workspace, K-major and
-// contiguous (16 KB; the diagonal tile as both operand layouts of the solves),
-// and its ready flag released; a producer warp waits (bounded) for the flags
-// and brings the operands in by bulk copies, two stages ahead of the products.
-// The workspace is the block's size again; the rule that chooses this kernel
-// is in glu_engine.cpp (dense_flow).
+// contiguous (16 KB; the diagonal tile as both operand layouts of the solves).
+// What is on the chain is handed on in quarters: 16 columns of the diagonal
+// tile's LU while the next 16 are factored (by warps that have no columns
+// left), 16 columns of a solved tile while it solves the next; the solve and
+// the last product in front of a diagonal tile start on them.  A publisher warp
+// releases the pieces (their count is the tile's flag), so no computing warp
+// waits for its stores; a producer warp waits (bounded) for the flags and
+// brings the operands in by bulk copies, two stages ahead of the products.  The
+// workspace is the block's size again; the rule that chooses this kernel is
+// in glu_engine.cpp (dense_flow).
 //
-// What a column step of the chain takes (order 1,920, one block per SM): LU
-// 7.0 us, publishing it 1.5, flag and copy 1.1, triangular solve 2.6, publishing
-// 0.8, flag and copy 1.2, product 1.9 -- 16.5 us, against 50 us for panel, pack
-// and update kernels.  The whole block: 0.49 ms (1.51 ms).
+// A column step of the chain takes 12.5 us (order 1,920, one block per SM), 7 of
+// them the LU; 16.5 us with whole tiles handed on (LU 7.0, publishing it 1.5,
+// flag and copy 1.1, triangular solve 2.6, publishing 0.8, flag and copy 1.2,
+// product 1.9), 50 us in panel, pack and update kernels.  The whole block: 0.40
+// ms, 0.49 ms and 1.51 ms.
 //
 // FP32 fused multiply-add throughout; the 64 products of a step are summed by
 // themselves and subtracted from the entry once (relative error against 64 bits of random
@@ -52,7 +58,9 @@ constexpr int kLdW = kT + 1;                         // solve tile, [k][vector]
 constexpr size_t kWorkBytes = sizeof(float) * kT * kLuLD;  // LU tile, or solve tile
 constexpr size_t kSmem = kStages * kStageBytes + kWorkBytes;
 constexpr size_t kSmemAlone = 120 * 1024;  // keeps a second block off the SM
-constexpr int kThreads = kTriThreads + 32;           // eight computing warps and the producer
+constexpr int kThreads = kTriThreads + 64;           // eight computing warps, the producer and the publisher
+constexpr int kPieces = 4;                           // of a tile: 16 of its 64 k each, ready one after another
+constexpr uint32_t kPieceBytes = kTileBytes / kPieces, kDiagPieceBytes = kDiagBytes / kPieces;
 static_assert(kFlowTile == kTriMax && kFlowDiagFloats == kT * kTriML, "layouts");
 static_assert(kDiagBytes <= kStageBytes && kLdW <= kLuLD, "the diagonal tile fits a stage");
 
@@ -93,9 +101,9 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
 // by ordinary stores, the copy reads through the asynchronous proxy.
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-// Bounded wait for a tile's ready flag (one thread).
-__device__ __forceinline__ void wait_tile(const uint32_t *flag, uint32_t *status, uint32_t limit) {
-    for (uint32_t spins = 0; !ld_acquire_gpu(flag); ++spins) {
+// Bounded wait until `pieces` pieces of a tile are ready (one thread).
+__device__ __forceinline__ void wait_tile(const uint32_t *flag, uint32_t pieces, uint32_t *status, uint32_t limit) {
+    for (uint32_t spins = 0; ld_acquire_gpu(flag) < pieces; ++spins) {
         if (spins >= limit) {
             atomicOr(status, DEV_TIMEOUT);
             return;
@@ -107,12 +115,15 @@ __device__ __forceinline__ void wait_tile(const uint32_t *flag, uint32_t *status
 // x M = a for the 64 vectors of W ([k][vector], leading dimension kLdW) by 256
 // threads: chunks of 16, each solved a vector per thread (64 threads), then
 // applied to the columns behind it by all.  M row-major, leading dimension
-// kTriML (kDiv: with the pivots' reciprocals in the padding).
-template <bool kDiv>
-__device__ __forceinline__ void solve_tile(float *W, const float *M, uint32_t tid) {
+// kTriML (kDiv: with the pivots' reciprocals in the padding).  before(cb) waits
+// for rows 16 cb .. + 15 of M; after(cb) is called by all threads once chunk cb
+// of the result stands in W.
+template <bool kDiv, class Before, class After>
+__device__ __forceinline__ void solve_tile(float *W, const float *M, uint32_t tid, Before &&before, After &&after) {
     const uint32_t v = tid & 63, q = tid >> 6;
 #pragma unroll 1
     for (uint32_t cb = 0; cb < 4; ++cb) {
+        before(cb);
         if (tid < 64) {
             float x[kTriChunk];
 #pragma unroll
@@ -122,6 +133,7 @@ __device__ __forceinline__ void solve_tile(float *W, const float *M, uint32_t ti
             for (int k = 0; k < kTriChunk; ++k) W[(cb * kTriChunk + k) * kLdW + v] = x[k];
         }
         tri_sync();
+        after(cb);
         // columns 16 (cb + 1) .. 63: four groups of 4 (3 - cb)
         for (uint32_t g = 0; g < 3 - cb; ++g) {
             const uint32_t j0 = (cb + 1) * kTriChunk + q * 4 * (3 - cb) + 4 * g;
@@ -169,14 +181,22 @@ __global__ void __launch_bounds__(kThreads, 2)
                  uint32_t count, const float *pert_z, float *work, uint64_t work_stride, uint32_t *ctl,
                  uint32_t *status, uint32_t spin_limit) {
     extern __shared__ __align__(128) unsigned char flow_smem[];
-    __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
+    __shared__ __align__(8) uint64_t full[kStages], empty[kStages], last_full[kPieces], diag_full[kPieces];
+    __shared__ __align__(8) uint64_t written[kPieces];  // one phase each: a piece may be written before the last is released
     __shared__ uint32_t s_item;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         s_item = atomicAdd(ctl, 1u);
+        const uint32_t item = s_item;
+        const FlowTile t0 = item < nt * nt * count ? flow_tile(item / count, nt) : FlowTile{0, 0, 0};
         for (int s = 0; s < kStages; ++s) {
             bar_init(&full[s], 1);
             bar_init(&empty[s], kTriThreads / 32);
+        }
+        for (int p = 0; p < kPieces; ++p) {
+            bar_init(&last_full[p], 1);
+            bar_init(&diag_full[p], 1);
+            bar_init(&written[p], t0.i == t0.j ? 3 : kTriThreads / 32);  // the warps that write a piece
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -185,36 +205,66 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (item >= nt * nt * count) return;
     const uint32_t z = item % count;
     const FlowTile t = flow_tile(item / count, nt);
-    uint32_t *ready = ctl + 4 + size_t(z) * nt * nt;
+    uint32_t *ready = ctl + 4 + size_t(z) * nt * nt;             // pieces of each tile that are ready
     float *tiles = work + z * work_stride;                       // [i][j][k][v]
     float *diags = tiles + size_t(nt) * nt * kT * kT;            // [k][0: U rows, 1: L columns]
-    if (warp == kTriThreads / 32) {
+    if (warp == kTriThreads / 32) {  // producer: operands as they become ready
         if (lane == 0) {
-            const uint32_t steps = t.k + (t.i != t.j ? 1u : 0u);
-            for (uint32_t s = 0; s < steps; ++s) {
+            for (uint32_t s = 0; s < t.k; ++s) {
                 const uint32_t st = s % kStages;
                 unsigned char *dst = flow_smem + st * kStageBytes;
+                const float *srcL = tiles + (size_t(t.i) * nt + s) * kT * kT, *srcU = tiles + (size_t(s) * nt + t.j) * kT * kT;
+                const uint32_t *fL = ready + size_t(t.i) * nt + s, *fU = ready + size_t(s) * nt + t.j;
                 if (s >= uint32_t(kStages) && !bar_wait(&empty[st], (s / kStages - 1) & 1, spin_limit))
                     atomicOr(status, DEV_TIMEOUT);
-                if (s < t.k) {
-                    wait_tile(ready + size_t(t.i) * nt + s, status, spin_limit);
-                    wait_tile(ready + size_t(s) * nt + t.j, status, spin_limit);
+                if (s + 1 < t.k) {
+                    wait_tile(fL, kPieces, status, spin_limit);
+                    wait_tile(fU, kPieces, status, spin_limit);
                     proxy_fence();
                     bar_expect(&full[st], 2 * kTileBytes);
-                    bulk_load(dst, tiles + (size_t(t.i) * nt + s) * kT * kT, kTileBytes, &full[st]);
-                    bulk_load(dst + kTileBytes, tiles + (size_t(s) * nt + t.j) * kT * kT, kTileBytes, &full[st]);
-                } else {
-                    wait_tile(ready + size_t(t.k) * nt + t.k, status, spin_limit);
+                    bulk_load(dst, srcL, kTileBytes, &full[st]);
+                    bulk_load(dst + kTileBytes, srcU, kTileBytes, &full[st]);
+                } else {  // the last step's operands may be in the making: piece by piece
+                    for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
+                        wait_tile(fL, p + 1, status, spin_limit);
+                        wait_tile(fU, p + 1, status, spin_limit);
+                        proxy_fence();
+                        bar_expect(&last_full[p], 2 * kPieceBytes);
+                        bulk_load(dst + p * kPieceBytes, srcL + p * (kPieceBytes / 4), kPieceBytes, &last_full[p]);
+                        bulk_load(dst + kTileBytes + p * kPieceBytes, srcU + p * (kPieceBytes / 4), kPieceBytes,
+                                  &last_full[p]);
+                    }
+                }
+            }
+            if (t.i != t.j) {
+                const uint32_t st = t.k % kStages;
+                if (t.k >= uint32_t(kStages) && !bar_wait(&empty[st], (t.k / kStages - 1) & 1, spin_limit))
+                    atomicOr(status, DEV_TIMEOUT);
+                const float *src = diags + (size_t(t.k) * 2 + (t.i > t.j ? 0 : 1)) * kFlowDiagFloats;
+                for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
+                    wait_tile(ready + size_t(t.k) * nt + t.k, p + 1, status, spin_limit);
                     proxy_fence();
-                    bar_expect(&full[st], kDiagBytes);
-                    bulk_load(dst, diags + (size_t(t.k) * 2 + (t.i > t.j ? 0 : 1)) * kFlowDiagFloats, kDiagBytes,
-                              &full[st]);
+                    bar_expect(&diag_full[p], kDiagPieceBytes);
+                    bulk_load(flow_smem + st * kStageBytes + p * kDiagPieceBytes, src + p * (kDiagPieceBytes / 4),
+                              kDiagPieceBytes, &diag_full[p]);
                 }
             }
             // the block must not end with copies in flight
-            for (uint32_t s = steps > uint32_t(kStages) ? steps - kStages : 0; s < steps; ++s)
+            for (uint32_t s = t.k > uint32_t(kStages) + 1 ? t.k - 1 - kStages : 0; s + 1 < t.k; ++s)
                 bar_wait(&full[s % kStages], (s / kStages) & 1, spin_limit);
+            for (int p = 0; p < kPieces; ++p) {
+                if (t.k) bar_wait(&last_full[p], 0, spin_limit);
+                if (t.i != t.j) bar_wait(&diag_full[p], 0, spin_limit);
+            }
         }
+        return;
+    }
+    if (warp == kTriThreads / 32 + 1) {  // publisher: releases each piece once it is written
+        if (lane == 0 && (t.i != t.j || t.k + 1 < nt))
+            for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
+                if (!bar_wait(&written[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+                st_release_gpu(ready + size_t(t.i) * nt + t.j, p + 1);
+            }
         return;
     }
     float *val = val_base + z * stride;
@@ -235,7 +285,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     for (uint32_t s = 0; s < t.k; ++s) {
         const uint32_t st = s % kStages;
-        if (!bar_wait(&full[st], (s / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+        const bool last = s + 1 == t.k;
+        if (!last && !bar_wait(&full[st], (s / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
         const float *sL = reinterpret_cast<const float *>(flow_smem + st * kStageBytes) + tr * 4;
         const float *sU = reinterpret_cast<const float *>(flow_smem + st * kStageBytes + kTileBytes) + tc * 4;
         // the 64 products in a sum of their own, subtracted once: its roundings
@@ -245,15 +296,20 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int b = 0; b < 4; ++b) sum[a][b] = 0.0f;
-#pragma unroll 8
-        for (int k = 0; k < kT; ++k) {
-            const float4 av = *reinterpret_cast<const float4 *>(sL + k * kT);
-            const float4 bv = *reinterpret_cast<const float4 *>(sU + k * kT);
-            const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll 1
+        for (int p = 0; p < kPieces; ++p) {
+            if (last && !bar_wait(&last_full[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int kk = 0; kk < kT / kPieces; ++kk) {
+                const int k = p * (kT / kPieces) + kk;
+                const float4 av = *reinterpret_cast<const float4 *>(sL + k * kT);
+                const float4 bv = *reinterpret_cast<const float4 *>(sU + k * kT);
+                const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-                for (int b = 0; b < 4; ++b) sum[a][b] = fmaf(ar[a], br[b], sum[a][b]);
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) sum[a][b] = fmaf(ar[a], br[b], sum[a][b]);
+            }
         }
         __syncwarp();
         if (lane == 0) bar_arrive(&empty[st]);
@@ -269,21 +325,23 @@ __global__ void __launch_bounds__(kThreads, 2)
             *reinterpret_cast<float4 *>(W + (tc * 4 + b) * kLuLD + tr * 4) =
                 make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
         tri_sync();
-        tri_lu_smem(W, rows, t.k + 1 < nt, pert_z ? pert_z[z] : 0.0f);
-        if (t.k + 1 < nt) {
-            float *du = diags + size_t(t.k) * 2 * kFlowDiagFloats, *dl = du + kFlowDiagFloats;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t a = tid & 63, b = (tid >> 6) * 4 + 16 * u;  // row a of U, columns b .. b + 3
+        // piece p by warps 5 .. 7: rows 16 p .. + 15 of U with the pivots'
+        // reciprocals, columns 16 p .. + 15 of L
+        float *du = diags + size_t(t.k) * 2 * kFlowDiagFloats, *dl = du + kFlowDiagFloats;
+        auto publish = [&](uint32_t p) {
+            if (t.k + 1 == nt) return;
+            for (uint32_t e = tid - 5 * 32; e < 256u; e += 96) {
+                const uint32_t a = 16 * p + (e & 15), b = (e >> 4) * 4;  // row a of U, columns b .. b + 3
                 *reinterpret_cast<float4 *>(du + a * kTriML + b) =
                     make_float4(W[b * kLuLD + a], W[(b + 1) * kLuLD + a], W[(b + 2) * kLuLD + a], W[(b + 3) * kLuLD + a]);
-                const uint32_t c = (tid >> 4) + 16 * u, r = (tid & 15) * 4;  // column c of L, rows r .. r + 3
+                const uint32_t c = 16 * p + (e >> 4), r = (e & 15) * 4;  // column c of L, rows r .. r + 3
                 *reinterpret_cast<float4 *>(dl + c * kTriML + r) = *reinterpret_cast<const float4 *>(W + c * kLuLD + r);
+                if (e < 16u) du[a * kTriML + kT] = 1.0f / W[a * kLuLD + a];
             }
-            if (tid < uint32_t(kT)) du[tid * kTriML + kT] = 1.0f / W[tid * kLuLD + tid];
-            tri_sync();
-            if (tid == 0) st_release_gpu(ready + size_t(t.k) * nt + t.k, 1u);
-        }
+            __syncwarp();
+            if (lane == 0) bar_arrive(&written[p]);
+        };
+        tri_lu_smem(W, rows, t.k + 1 < nt, pert_z ? pert_z[z] : 0.0f, publish);
 #pragma unroll 4
         for (uint32_t e = tid; e < uint32_t(kT * kT); e += kTriThreads) {
             const uint32_t c = e >> 6, r = e & 63;
@@ -300,23 +358,23 @@ __global__ void __launch_bounds__(kThreads, 2)
             const uint32_t k = (lower ? tc * 4 + b : tr * 4 + a), v = (lower ? tr * 4 + a : tc * 4 + b);
             W[k * kLdW + v] = acc[a][b];
         }
-    const uint32_t st = t.k % kStages;
-    if (!bar_wait(&full[st], (t.k / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
     tri_sync();
-    const float *M = reinterpret_cast<const float *>(flow_smem + st * kStageBytes);
-    if (lower)
-        solve_tile<true>(W, M, tid);
-    else
-        solve_tile<false>(W, M, tid);
+    const float *M = reinterpret_cast<const float *>(flow_smem + (t.k % kStages) * kStageBytes);
     float *out = tiles + (size_t(t.i) * nt + t.j) * kT * kT;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const uint32_t k = (tid >> 4) + 16 * u, v = (tid & 15) * 4;
+    auto before = [&](uint32_t p) {
+        if (!bar_wait(&diag_full[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+    };
+    auto after = [&](uint32_t p) {  // piece p of the tile
+        const uint32_t k = 16 * p + (tid >> 4), v = (tid & 15) * 4;
         const float *w = W + k * kLdW + v;
         *reinterpret_cast<float4 *>(out + k * kT + v) = make_float4(w[0], w[1], w[2], w[3]);
-    }
-    tri_sync();
-    if (tid == 0) st_release_gpu(ready + size_t(t.i) * nt + t.j, 1u);
+        __syncwarp();
+        if (lane == 0) bar_arrive(&written[p]);
+    };
+    if (lower)
+        solve_tile<true>(W, M, tid, before, after);
+    else
+        solve_tile<false>(W, M, tid, before, after);
 #pragma unroll 4
     for (uint32_t e = tid; e < uint32_t(kT * kT); e += kTriThreads) {
         const uint32_t c = e >> 6, r = e & 63;  // down the columns
@@ -347,9 +405,9 @@ cudaError_t launch_dense_flow(float *val, uint64_t stride, uint32_t count, const
     if (e != cudaSuccess) return e;
     // One block per SM while the diagonal chain is what takes the time (a
     // second block's products slow its LU down), two when the tiles' products
-    // do.  Measured, one against two: order 1,920 0.49 / 0.57 ms, order 3,000
-    // 0.90 / 1.02, four of order 1,920 0.81 / 0.75, 96 of order 576 0.73 / 0.59;
-    // equal at order 3,968 and sixteen of 641.
+    // do.  Measured with whole tiles handed on, one against two: order 1,920 0.49
+    // / 0.57 ms, order 3,000 0.90 / 1.02, four of order 1,920 0.81 / 0.75, 96 of
+    // order 576 0.73 / 0.59; equal at order 3,968 and sixteen of 641.
     const size_t smem = uint64_t(nt) * nt * count <= 3000 ? kSmemAlone : kSmem;
     k_dense_flow<<<nt * nt * count, kThreads, smem, st>>>(val, stride, doff, m, nt, count, pert_z, work,
                                                            dense_flow_floats(m), ctl, status, spin_limit);

@@ -439,20 +439,20 @@ uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 // the dataflow kernel (glu_dense_flow.cu) or by panels and updates.  With
 // widths set for look-ahead or tensor-core updates, the blocks below them.
 // With the default widths, whichever a model of both takes less time for:
-//   dataflow  16.8 us per 64 columns (the diagonal chain) against the products
+//   dataflow  12.7 us per 64 columns (the diagonal chain) against the products
 //             at 36 TFLOP/s, the longer and three tenths of the shorter;
 //   panels    55 us per 64 columns plus the products at 130 TFLOP/s on the
 //             tensor cores.
-// Measured, dataflow / panels: order 1,920 0.49 / 1.51 ms, eight of them 1.22 /
-// 2.18, order 3,968 1.48 / 4.73, three of them 3.39 / 5.75, order 5,000 2.52 /
-// 6.27, 96 of order 576 0.59 / 0.99; twelve of order 9,360 take the panels
+// Measured, dataflow / panels: order 1,920 0.40 / 1.51 ms, eight of them 1.18 /
+// 2.18, order 3,968 1.32 / 4.73, three of them 3.32 / 5.75, order 5,000 2.35 /
+// 6.27, 96 of order 576 0.60 / 0.99; twelve of order 9,360 take the panels
 // about 58 ms, the dataflow would take 180.
 bool dense_flow(const glu_tuning &tu, uint32_t m, uint32_t count) {
     if (m == 0) return false;
     if (tu.dense_lookahead != kLookaheadMin || tu.dense_tc_min != kDenseTcMin)
         return (tu.dense_lookahead == 0 || m < tu.dense_lookahead) && (tu.dense_tc_min == 0 || m < tu.dense_tc_min);
     const double steps = std::ceil(double(m) / kFlowTile), work = double(count) * (2.0 / 3.0) * m * m * m;
-    const double chain = steps * 16.8e-6, products = work / 36e12;
+    const double chain = steps * 12.7e-6, products = work / 36e12;
     return std::max(chain, products) + 0.3 * std::min(chain, products) <= steps * 55e-6 + work / 130e12;
 }
 

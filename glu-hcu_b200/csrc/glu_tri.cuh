@@ -250,8 +250,14 @@ __device__ __forceinline__ void lu_one_column(float *S, uint32_t base, uint32_t 
 // threads, a barrier and a division per pivot (the division's slow path is
 // taken for every zero of a sparse or padded row).
 // The caller has a barrier between its writes of S and the call; on return the
-// block is complete for all 256 threads.
-__device__ __forceinline__ void tri_lu_smem(float *S, uint32_t w, bool last_l, float pert) {
+// block is complete for all 256 threads.  done(p) is called by warps 5, 6 and 7,
+// which have no columns left by then, as soon as columns 16 p .. 16 p + 15 of L
+// and rows 16 p .. 16 p + 15 of U are final (p = 0 .. 3, for w = 64 only).
+struct TriNothing {
+    __device__ __forceinline__ void operator()(uint32_t) const {}
+};
+template <class Done = TriNothing>
+__device__ __forceinline__ void tri_lu_smem(float *S, uint32_t w, bool last_l, float pert, Done &&done = Done()) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t end = (w + kLuChunk - 1) / kLuChunk * kLuChunk;  // columns to factor
     if (warp == 0) lu_panel(S, 0, w, last_l, pert, lane);
@@ -264,8 +270,11 @@ __device__ __forceinline__ void tri_lu_smem(float *S, uint32_t w, bool last_l, f
             lu_panel(S, base + kLuChunk, w, last_l, pert, lane);
         else if (base + kLuChunk * (warp + 1) < end)
             lu_columns(S, base, base + kLuChunk * (warp + 1) + 2 * (lane >> 3), lane & 7);
+        else if (warp >= 5 && w == uint32_t(kTriMax) && base >= 16 && (base & 15) == 0)
+            done(base / 16 - 1);
         tri_sync();
     }
+    if (warp >= 5 && w == uint32_t(kTriMax)) done(3);
 }
 
 // Solve within chunk cb of one row: x = the chunk's N <= 16 entries after the
