@@ -287,13 +287,13 @@ struct SolveBatch {
     uint32_t *sweep_done = nullptr;  // count x (supernodes) counters of the fused sweeps (null: per level)
 };
 // Inverses of the 64 x 64 diagonal blocks of the dense tail's L and U, per
-// value set: dinv[z][b][0: L, 1: U][64 x 64] (row-major), from the factors.
+// value set: dinv[z][b][0: L, 1: U][64 x 64] (column-major), from the factors.
 cudaError_t launch_dense_diag_inv(const float *dval, uint64_t dstride, uint32_t count, const uint32_t *doff,
                                   uint32_t m, float *dinv, cudaStream_t st);
 
 constexpr uint32_t kSnInvFloats = 2 * kSnMaxWidth * kSnMaxWidth;  // of one wide supernode
 // Inverses of the diagonal blocks of `nwide` supernodes {first column, width},
-// width > kSnSmallWidth: invs[z][k][0: L, 1: U][64 x 64] (row-major).
+// width > kSnSmallWidth: invs[z][k][0: L, 1: U][64 x 64] (column-major).
 cudaError_t launch_sn_diag_inv(const DevPattern &P, const uint2 *wide, uint32_t nwide, const float *val,
                                uint64_t vstride, uint32_t count, float *invs, uint64_t inv_stride, cudaStream_t st);
 

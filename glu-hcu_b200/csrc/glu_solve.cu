@@ -222,11 +222,15 @@ static cudaError_t run_sweep(const DevPattern &P, const SolvePlanDev &S, const f
 //    are in flight meanwhile);
 //  * the diagonal block's solve is a product with its inverse (dinv, computed
 //    once per factorization by k_dense_diag_inv), a parallel mat-vec instead
-//    of 64 dependent steps; two block barriers per link remain.
-// Measured (B200): a link takes 0.87 us at order 1,920 with one right-hand side
-// (26 us a sweep; 87 us with a flag per block and three barriers per tile), and
-// 32 right-hand sides take 43 us (8.5 ms as groups of four one after another
-// inside the block); transposed, order 3,776, 62-74 us (193 us).
+//    of 64 dependent steps; two block barriers per link remain.  It stands
+//    column-major, so a warp's load of it is one line (row-major its 32 lines
+//    per load took as long as a link).
+// Measured (B200): a link takes 0.82 us at order 1,920 with one right-hand side
+// (24.7 us a sweep; 26.5 us with row-major inverses, 87 us with a flag per block
+// and three barriers per tile), and 32 right-hand sides take 36 us (8.5 ms as
+// groups of four one after another inside the block); transposed, order 3,776,
+// 54 us (193 us).  Blocks of 128 rows take 22, 34 and 39 us, but their inverses
+// cost 10 us more per factorization than these, which a step pays every time.
 // The forward sweep reads y and writes xo, the backward sweep reads xo and
 // writes y: the forward one leaves kUnsolved in the rows of y it has read, and
 // the transform in front of the solve leaves it in xo (SolveInit).
@@ -247,9 +251,11 @@ __device__ __forceinline__ void publish(float *p, float v) {
 
 // Polls the warp's N values per lane (v[k] at at(k); entries that are not
 // needed hold 0) until all are solved; bounded, a wait that sees another's
-// timeout gives up early.
+// timeout gives up early.  Only the block whose turn is next polls without a
+// pause: the others' polls go to the same L2 slice as its own (transposed,
+// order 3,776: 54 us, 59 without the pause).
 template <int N, class At>
-__device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, uint32_t *status, uint32_t limit) {
+__device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, bool next, uint32_t *status, uint32_t limit) {
     for (uint32_t spins = 0;; ++spins) {
         bool open = false;
 #pragma unroll
@@ -259,6 +265,7 @@ __device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, uint32_t *st
             if ((threadIdx.x & 31) == 0) atomicOr(status, DEV_TIMEOUT);
             return;
         }
+        if (!next) __nanosleep(60);
         if ((spins & 1023u) == 1023u && (ld_acquire_gpu(status) & DEV_TIMEOUT)) return;
 #pragma unroll
         for (int k = 0; k < N; ++k)
@@ -267,7 +274,7 @@ __device__ __forceinline__ void wait_solved(float (&v)[N], At &&at, uint32_t *st
 }
 
 // Inverses of the 64 x 64 diagonal blocks of the dense tail: blockIdx.y = 0
-// the unit lower L_bb, 1 the upper U_bb; dinv[z][b][which] row-major (rows
+// the unit lower L_bb, 1 the upper U_bb; dinv[z][b][which] column-major (rows
 // past the tail's end are the identity).  blockIdx.z selects the value set.
 __global__ void __launch_bounds__(256) k_dense_diag_inv(const float *__restrict__ val, uint64_t dstride,
                                                          const uint32_t *__restrict__ doff, uint32_t m,
@@ -319,7 +326,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3)
     const uint32_t b = kLower ? tk : nb - 1 - tk;
     const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
     const uint32_t row = tid & (kRB - 1), q = tid / kRB, col0 = q * kW;
-    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kMode) * kRB * kRB + row * kRB + col0;
+    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kMode) * kRB * kRB + col0 * kRB + row;
     // lane's x values: column lane % 16, right-hand sides lane / 16 + 2 k
     const uint32_t xc = lane & 15, xr = lane >> 4;
     const bool rowok = row < rows;
@@ -387,10 +394,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3)
         load_x(0, xv);
     } else {
 #pragma unroll
-        for (int k = 0; k < kW; k += 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + k));
-            tv[k] = v.x, tv[k + 1] = v.y, tv[k + 2] = v.z, tv[k + 3] = v.w;
-        }
+        for (int k = 0; k < kW; ++k) tv[k] = __ldg(inv + k * kRB);
     }
     for (uint32_t s = 0; s < tk; ++s) {
         float tn[kW], xn[kX];
@@ -399,14 +403,11 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3)
             load_x(s + 1, xn);
         } else {
 #pragma unroll
-            for (int k = 0; k < kW; k += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + k));
-                tn[k] = v.x, tn[k + 1] = v.y, tn[k + 2] = v.z, tn[k + 3] = v.w;
-            }
+            for (int k = 0; k < kW; ++k) tn[k] = __ldg(inv + k * kRB);
 #pragma unroll
             for (int k = 0; k < kX; ++k) xn[k] = 0.0f;
         }
-        wait_solved(xv, [&](int k) { return x_at(s, k); }, status, spin_limit);
+        wait_solved(xv, [&](int k) { return x_at(s, k); }, s + 1 == tk, status, spin_limit);
         float *buf = xs[warp][s & 1];
         stage(buf, xv);
         multiply(acc, tv, buf);
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 3 : 2)
     const uint32_t b = kLower ? tk : nb - 1 - tk;
     const uint32_t rb0 = b * kRB, rows = min(uint32_t(kRB), m - rb0);
     const uint32_t i0 = warp * kRows;
-    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kWhich) * kRB * kRB;  // row-major
+    const float *inv = dinv + ((size_t(it.z) * nb + b) * 2 + kWhich) * kRB * kRB;
     uint32_t base[kRows];
 #pragma unroll
     for (int i = 0; i < kRows; ++i) base[i] = i0 + i < rows ? __ldg(doff + rb0 + i0 + i) : 0u;
@@ -507,10 +508,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 3 : 2)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < kRows; i += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(inv + (lane + 32 * h) * kRB + i0 + i));
-                tv[2 * i + h] = v.x, tv[2 * i + 2 + h] = v.y, tv[2 * i + 4 + h] = v.z, tv[2 * i + 6 + h] = v.w;
-            }
+            for (int i = 0; i < kRows; ++i) tv[2 * i + h] = __ldg(inv + (i0 + i) * kRB + lane + 32 * h);
     };
     auto x_at = [&](uint32_t s, int k) -> const float * {
         return out + size_t(k >> 1) * n + (kLower ? s : nb - 1 - s) * kRB + lane + 32 * (k & 1);
@@ -552,7 +550,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 3 : 2)
 #pragma unroll
             for (int k = 0; k < 2 * R; ++k) xn[k] = 0.0f;
         }
-        wait_solved(xv, [&](int k) { return x_at(s, k); }, status, spin_limit);
+        wait_solved(xv, [&](int k) { return x_at(s, k); }, s + 1 == tk, status, spin_limit);
         multiply(tv, xv);
 #pragma unroll
         for (int k = 0; k < 2 * kRows; ++k) tv[k] = tn[k];

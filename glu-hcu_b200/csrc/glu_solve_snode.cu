@@ -293,12 +293,9 @@ __device__ __forceinline__ void wide_solve(const float (&iv)[16], const float *v
     __syncthreads();
 }
 __device__ __forceinline__ void load_inverse(float (&iv)[16], const float *__restrict__ inv, uint32_t tid) {
-    const float4 *p = reinterpret_cast<const float4 *>(inv + (tid & 63) * kSnMaxWidth + (tid >> 6) * 16);
+    inv += (tid >> 6) * 16 * kSnMaxWidth + (tid & 63);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 v = __ldg(p + k);
-        iv[4 * k] = v.x, iv[4 * k + 1] = v.y, iv[4 * k + 2] = v.z, iv[4 * k + 3] = v.w;
-    }
+    for (int k = 0; k < 16; ++k) iv[k] = __ldg(inv + k * kSnMaxWidth);
 }
 
 __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,

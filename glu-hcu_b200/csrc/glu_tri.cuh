@@ -391,7 +391,7 @@ struct TriInverse {
 };
 
 // The inverse of a factored diagonal block of w <= 64 columns by 256 threads,
-// row-major 64 x 64 at out (the identity past w): which = 0 the unit lower L,
+// column-major 64 x 64 at out (the identity past w): which = 0 the unit lower L,
 // 1 the upper U; at(i, c) reads the block's entry.  U is taken as its
 // transpose, so both are the inverse of a lower triangular M: the four 16 x 16
 // diagonal blocks by substitution (a column per thread, in registers), then
@@ -476,7 +476,7 @@ __device__ __forceinline__ void tri_invert(TriInverse &T, uint32_t which, uint32
     __syncthreads();
 #pragma unroll 4
     for (uint32_t e = tid; e < uint32_t(kTriMax * kTriMax); e += 256)
-        out[e] = which == 0 ? X[e / kTriMax][e % kTriMax] : X[e % kTriMax][e / kTriMax];
+        out[e] = which == 0 ? X[e % kTriMax][e / kTriMax] : X[e / kTriMax][e % kTriMax];
 }
 
 // Four-byte asynchronous copy global -> shared (completes at tri_async_wait).
