@@ -243,7 +243,7 @@ struct glu_handle_s {
     DevBuf d_sweep_done;  // per value set and supernode: releases received (fused sweeps)
     std::vector<SnSweepLevel> ss_levels[2];
     // solve plan
-    DevBuf d_sw_cols[4], d_sw_lptr[4], d_sw_ioff[4], d_tail_row_start, d_xo;
+    DevBuf d_sw_items[4], d_sw_info[4], d_sw_off[4], d_tail_row_start, d_xo;
     std::vector<SweepStep> sw_steps[4];
     SolvePlanDev S{};
     // transforms (forward in/out, transposed in/out)
@@ -507,8 +507,8 @@ uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_p
 // Work items of pivot j: its entries in chunks of kSweepChunk (at least one,
 // the dividing sweeps store x_j).  Levels with more than `thin` items get
 // their own launch; runs of thinner levels go to the cluster kernel.
-void build_sweep(const SymbolicData &s, uint32_t t, int mode, uint32_t thin, std::vector<uint32_t> &cols,
-                 std::vector<uint32_t> &lptr, std::vector<uint32_t> &item_off, std::vector<SweepStep> &steps) {
+void build_sweep(const SymbolicData &s, uint32_t t, int mode, uint32_t thin, std::vector<uint2> &items,
+                 std::vector<uint16_t> &info, std::vector<uint32_t> &level_off, std::vector<SweepStep> &steps) {
     std::vector<int32_t> lev(t, 0);
     int32_t nlev = 0;
     const bool forward = (mode == SWEEP_L || mode == SWEEP_UT);
@@ -533,41 +533,40 @@ void build_sweep(const SymbolicData &s, uint32_t t, int mode, uint32_t thin, std
         lev[j] = mx + 1;
         nlev = std::max(nlev, mx + 2);
     }
-    lptr.assign(size_t(nlev) + 1, 0);
-    for (uint32_t j = 0; j < t; ++j) lptr[lev[j] + 1]++;
-    for (int32_t l = 0; l < nlev; ++l) lptr[l + 1] += lptr[l];
-    cols.assign(t, 0);
+    // pivot j's entries [first, first + second)
+    auto entries = [&](uint32_t j) -> std::pair<uint32_t, uint32_t> {
+        if (mode == SWEEP_L) return {s.l_col_ptr[j] + 1, s.sym_c_ptr[j + 1] - s.l_col_ptr[j] - 1};
+        if (mode == SWEEP_U) return {s.sym_c_ptr[j], s.l_col_ptr[j] - s.sym_c_ptr[j]};
+        if (mode == SWEEP_UT) return {s.csr_diag_ptr[j] + 1, s.csr_r_ptr[j + 1] - s.csr_diag_ptr[j] - 1};
+        return {s.csr_r_ptr[j], s.csr_diag_ptr[j] - s.csr_r_ptr[j]};
+    };
+    auto chunks = [&](uint32_t j) { return std::max<uint32_t>(1, (entries(j).second + kSweepChunk - 1) / kSweepChunk); };
+    level_off.assign(size_t(nlev) + 1, 0);
+    for (uint32_t j = 0; j < t; ++j) level_off[lev[j] + 1] += chunks(j);
+    for (int32_t l = 0; l < nlev; ++l) level_off[l + 1] += level_off[l];
+    items.resize(level_off[nlev]);
+    info.resize(level_off[nlev]);
     {
-        std::vector<uint32_t> cur(lptr.begin(), lptr.end() - 1);
-        for (uint32_t j = 0; j < t; ++j) cols[cur[lev[j]]++] = j;
+        std::vector<uint32_t> cur(level_off.begin(), level_off.end() - 1);
+        for (uint32_t j = 0; j < t; ++j) {
+            const auto [p0, len] = entries(j);
+            for (uint32_t c = 0, nc = chunks(j); c < nc; ++c) {
+                const uint32_t i = cur[lev[j]]++, e = c * kSweepChunk;
+                items[i] = make_uint2(j, p0 + e);
+                info[i] = uint16_t(std::min(kSweepChunk, len - e) | (c == 0 ? kSweepFirst : 0u));
+            }
+        }
     }
-    item_off.assign(size_t(t) + 1, 0);
-    for (uint32_t q = 0; q < t; ++q) {
-        const uint32_t j = cols[q];
-        uint32_t len;
-        if (mode == SWEEP_L)
-            len = s.sym_c_ptr[j + 1] - s.l_col_ptr[j] - 1;
-        else if (mode == SWEEP_U)
-            len = s.l_col_ptr[j] - s.sym_c_ptr[j];
-        else if (mode == SWEEP_UT)
-            len = s.csr_r_ptr[j + 1] - s.csr_diag_ptr[j] - 1;
-        else
-            len = s.csr_diag_ptr[j] - s.csr_r_ptr[j];
-        item_off[q + 1] = item_off[q] + std::max<uint32_t>(1, (len + kSweepChunk - 1) / kSweepChunk);
-    }
-    auto items = [&](int32_t l) { return item_off[lptr[l + 1]] - item_off[lptr[l]]; };
+    auto count = [&](int32_t l) { return level_off[l + 1] - level_off[l]; };
     steps.clear();
     int32_t l = 0;
     while (l < nlev) {
-        if (items(l) > thin) {
-            steps.push_back(SweepStep{0, uint32_t(l), uint32_t(l + 1), lptr[l], lptr[l + 1]});
-            ++l;
-        } else {
-            int32_t e = l;
-            while (e < nlev && items(e) <= thin) ++e;
-            steps.push_back(SweepStep{1, uint32_t(l), uint32_t(e), lptr[l], lptr[e]});
-            l = e;
-        }
+        int32_t e = l + 1;
+        const bool wide = count(l) > thin;
+        if (!wide)
+            while (e < nlev && count(e) <= thin) ++e;
+        steps.push_back(SweepStep{wide ? 0u : 1u, uint32_t(l), uint32_t(e), level_off[l], level_off[e]});
+        l = e;
     }
 }
 
@@ -1139,18 +1138,20 @@ Status build_plan(glu_handle_s *h) {
         h->S.tail_row_start = h->d_tail_row_start.as<uint32_t>();
     }
     for (int mode = 0; mode < 4; ++mode) {
-        std::vector<uint32_t> cols, lptr, ioff;
-        build_sweep(s, t, mode, h->tune.solve_thin, cols, lptr, ioff, h->sw_steps[mode]);
-        GLU_CUDA(upload(h->d_sw_cols[mode], cols), "upload solve plan");
-        GLU_CUDA(upload(h->d_sw_lptr[mode], lptr), "upload solve plan");
-        GLU_CUDA(upload(h->d_sw_ioff[mode], ioff), "upload solve plan");
+        std::vector<uint2> items;
+        std::vector<uint16_t> info;
+        std::vector<uint32_t> level_off;
+        build_sweep(s, t, mode, h->tune.solve_thin, items, info, level_off, h->sw_steps[mode]);
+        GLU_CUDA(upload(h->d_sw_items[mode], items), "upload solve plan");
+        GLU_CUDA(upload(h->d_sw_info[mode], info), "upload solve plan");
+        GLU_CUDA(upload(h->d_sw_off[mode], level_off), "upload solve plan");
         SweepPlan &sp = h->S.sweep[mode];
-        sp.cols = h->d_sw_cols[mode].as<uint32_t>();
-        sp.lptr = h->d_sw_lptr[mode].as<uint32_t>();
-        sp.item_off = h->d_sw_ioff[mode].as<uint32_t>();
+        sp.items = h->d_sw_items[mode].as<uint2>();
+        sp.info = h->d_sw_info[mode].as<uint16_t>();
+        sp.level_off = h->d_sw_off[mode].as<uint32_t>();
         sp.steps = h->sw_steps[mode].data();
         sp.nsteps = uint32_t(h->sw_steps[mode].size());
-        sp.nlev = uint32_t(lptr.size() - 1);
+        sp.nlev = uint32_t(level_off.size() - 1);
     }
 
     Status sn = build_sn_plan(h);

@@ -200,26 +200,28 @@ cudaError_t build_levels(const DevPattern &P, void *scratch, int32_t *level_of, 
                          cudaStream_t st);
 
 // ------------------------------------------------------------------ solves --
-// Level schedule of one sparse sweep over the columns [0, t): the columns
-// level by level (cols, lptr on the device) and the launches that run them.
-// A step is one level with its own launch (kind 0, columns [c0, c1) of cols)
-// or a run of thin levels [l0, l1) inside one thread-block cluster (kind 1).
+// Level schedule of one sparse sweep over the columns [0, t): their work items
+// level by level and the launches that run them.  A step is one level with its
+// own launch (kind 0) or a run of thin levels [l0, l1) inside one thread-block cluster (kind 1).
 // Every sweep is in scatter form: once x_j is final, its column (L, U: CSC)
 // or row (U^T, L^T: CSR) is subtracted from the other unknowns.  Work items
-// are (j, chunk of kSweepChunk entries); item_off is their prefix over cols.
+// are chunks of kSweepChunk entries of j, level by level: items[i] = {j, first
+// entry}, info[i] = entries | kSweepFirst on j's first item; level l has the
+// items [level_off[l], level_off[l + 1]).
 struct SweepStep {
-    uint32_t kind, l0, l1, s0, s1;  // levels [l0, l1), columns cols[s0, s1)
+    uint32_t kind, l0, l1, i0, i1;  // levels [l0, l1), items [i0, i1)
 };
 struct SweepPlan {
-    const uint32_t *cols = nullptr;
-    const uint32_t *lptr = nullptr;
-    const uint32_t *item_off = nullptr;
+    const uint2 *items = nullptr;
+    const uint16_t *info = nullptr;
+    const uint32_t *level_off = nullptr;
     const SweepStep *steps = nullptr;  // host array
     uint32_t nsteps = 0;
     uint32_t nlev = 0;
 };
 enum SweepMode : int { SWEEP_L = 0, SWEEP_U = 1, SWEEP_UT = 2, SWEEP_LT = 3 };
 constexpr uint32_t kSweepChunk = 128;
+constexpr uint16_t kSweepFirst = 1u << 15;
 
 // Supernodal L or U sweep (used when the factor is supernodal): per block of
 // the sweep (levels one after another) its supernode and part, per supernode
