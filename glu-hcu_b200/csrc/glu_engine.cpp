@@ -1981,10 +1981,15 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
         ++nlaunch;
         return e;
     };
-    auto panel = [&](uint32_t k0, uint32_t kb) -> cudaError_t {
+    // whether the panel's second launch writes its packs (else `pack` does)
+    auto panel_packs = [&](uint32_t k0, uint32_t kb) {
+        return dense_panel_launches(count, h->m, k0, kb, h->num_sms) == 2;
+    };
+    auto panel = [&](uint32_t k0, uint32_t kb, uint32_t slot0, bool packed) -> cudaError_t {
         cudaError_t e = pf.begin(ps);
         if (e == cudaSuccess)
-            e = launch_dense_panel(dbase, dstride, count, doff, h->m, k0, kb, pert, dscr, 0, h->num_sms, ps);
+            e = launch_dense_panel(dbase, dstride, count, doff, h->m, k0, kb, pert, dscr, 0, h->num_sms, slot0,
+                                   packed ? h->d_packA.as<uint16_t>() : nullptr, h->d_packB.as<uint16_t>(), ps);
         if (e == cudaSuccess) e = pf.end(KK_PANEL, ps);
         nlaunch += dense_panel_launches(count, h->m, k0, kb, h->num_sms);
         return e;
@@ -1996,18 +2001,22 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
     for (uint32_t k0 = flow ? h->m : 0u; k0 < h->m;) {
         const uint32_t kb0 = std::min<uint32_t>(nb, h->m - k0);
         const uint32_t rest0 = h->m - (k0 + kb0);
-        GLU_CUDA(panel(k0, kb0), "factor (dense panel)");
+        // panels of this group: all but the last are full width
+        const uint32_t g = std::min<uint32_t>(group, (h->m - k0 + nb - 1) / nb);
+        // packs are written when any update of this group may read them: every
+        // region of the group lies in the trailing block from k0 on; they wait
+        // for the previous group's update, which reads the packs
+        const bool packed = tc_region(h->m - k0, h->m - k0);
+        const bool fused = packed && panel_packs(k0, kb0);
+        if (!fused) GLU_CUDA(panel(k0, kb0, 0, false), "factor (dense panel)");
         if (rest_pending) {
             GLU_CUDA(cudaStreamWaitEvent(ps, h->ev_rest, 0), "stream wait");
             rest_pending = false;
         }
-        // panels of this group: all but the last are full width
-        const uint32_t g = std::min<uint32_t>(group, (h->m - k0 + nb - 1) / nb);
-        // packs are written when any update of this group may read them: every
-        // region of the group lies in the trailing block from k0 on
-        const bool packed = tc_region(h->m - k0, h->m - k0);
-        // after the previous group's update, which reads the packs
-        GLU_CUDA(pack(k0, kb0, 0, packed), "factor (dense pack)");
+        if (fused)
+            GLU_CUDA(panel(k0, kb0, 0, true), "factor (dense panel)");
+        else
+            GLU_CUDA(pack(k0, kb0, 0, packed), "factor (dense pack)");
         if (g == 1) {  // small trailing blocks, last panels: plain steps
             GLU_CUDA(update(k0, kb0, DenseRegion{0, rest0, 0, rest0, 1, k0}, ps), "factor (dense update)");
             k0 += kb0;
@@ -2022,8 +2031,8 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
             const uint32_t hj = std::min<uint32_t>(nb, tj);
             GLU_CUDA(update(k0, kk, DenseRegion{0, hj, 0, tj, 1, kj - nb}, ps), "factor (dense update)");
             if (tj > hj) GLU_CUDA(update(k0, kk, DenseRegion{hj, tj, 0, hj, 0, kj - nb}, ps), "factor (dense update)");
-            GLU_CUDA(panel(kj, kbj), "factor (dense panel)");
-            GLU_CUDA(pack(kj, kbj, kDenseNB * j, packed), "factor (dense pack)");
+            GLU_CUDA(panel(kj, kbj, kDenseNB * j, packed), "factor (dense panel)");
+            GLU_CUDA(pack(kj, kbj, kDenseNB * j, packed && !panel_packs(kj, kbj)), "factor (dense pack)");
             kk += kbj;
         }
         // the rest with the whole group (K = kk): the next group's first panel

@@ -31,11 +31,9 @@ namespace glu {
 // rows of L21 (x U11 = a), the rest 128 columns of U12 (L11 x = a), one per
 // thread, chunked (tri_rows_solve).  The rows or columns are copied to shared
 // memory asynchronously while the diagonal block is factored.  blockIdx.z
-// selects the value set.  With from_scratch set, block b of the launch is
-// block b + 1 of the step and takes the diagonal block already factored into
-// diag_scratch by a launch of block 0 alone (the same code, so the same
-// values) instead of factoring it again: for many value sets the redundant
-// factorizations would outweigh the row solves.
+// selects the value set.  Where the redundant factorizations would outweigh
+// the row solves (many value sets), block 0 is launched alone and
+// k_dense_panel_rows solves the rows and columns.
 constexpr int kPW = kPanelRows + 1;  // leading dimension of the panel work tile
 constexpr size_t kPanelSmem =
     sizeof(float) * (size_t(kDenseNB) * kPW + size_t(kDenseNB) * kTriML + size_t(kDenseNB) * kLuLD) +
@@ -47,8 +45,7 @@ static_assert(2 * kPanelRows == kTriThreads, "128 rows per panel block");
 __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, uint64_t stride,
                                                              const uint32_t *__restrict__ doff, uint32_t m,
                                                              uint32_t k0, uint32_t kb, const float *pert_z,
-                                                             float *diag_scratch, uint32_t last_has_l, uint32_t nL,
-                                                             uint32_t from_scratch) {
+                                                             float *diag_scratch, uint32_t last_has_l, uint32_t nL) {
     extern __shared__ float4 psm4[];
     float *sW = reinterpret_cast<float *>(psm4);  // [k][thread]: rows of L21 or columns of U12
     float *sM = sW + kDenseNB * kPW;               // U11 (row-major, pivot reciprocals in the padding) or L11^T
@@ -56,7 +53,7 @@ __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, ui
     uint32_t *sCol = reinterpret_cast<uint32_t *>(sS + kDenseNB * kLuLD);
     float *val = val_base + blockIdx.z * stride;
     const float pert = pert_z ? pert_z[blockIdx.z] : 0.0f;
-    const uint32_t tid = threadIdx.x, b = blockIdx.x + from_scratch;
+    const uint32_t tid = threadIdx.x, b = blockIdx.x;
     const uint32_t r0 = k0 + kb;
     if (tid < kb) sCol[tid] = doff[k0 + tid] + k0;
     // this block's rows (columns) of the panel, in flight during the LU
@@ -77,17 +74,16 @@ __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, ui
     tri_async_commit();
     __syncthreads();
     // the diagonal block (the identity past its end)
-    const float *ds = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
 #pragma unroll 16
     for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kTriThreads) {
         const uint32_t c = e / kDenseNB, r = e % kDenseNB;
         float v = r == c ? 1.0f : 0.0f;
-        if (r < kb && c < kb) v = from_scratch ? ld_cg(ds + e) : ld_cg(val + sCol[c] + r);
+        if (r < kb && c < kb) v = ld_cg(val + sCol[c] + r);
         sS[c * kLuLD + r] = v;
     }
     __syncthreads();
     // a pivot is perturbed only when its column has an L part
-    if (!from_scratch) tri_lu_smem(sS, kb, (r0 < m) || last_has_l, pert);
+    tri_lu_smem(sS, kb, (r0 < m) || last_has_l, pert);
     if (b == 0) {
         float *out = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
         for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kTriThreads)
@@ -129,6 +125,124 @@ __global__ void __launch_bounds__(kTriThreads) k_dense_panel(float *val_base, ui
         for (uint32_t e = tid; e < ncol * kb; e += kTriThreads) {
             const uint32_t cc = e / kb, rr = e - cc * kb;
             st_cg(val + doff[j0 + cc] + k0 + rr, sW[rr * kPW + cc]);
+        }
+    }
+}
+
+// Rows of L21 and columns of U12 of a full panel (kDenseNB columns at k0) from
+// the diagonal block factored into diag_scratch, and their BF16 parts for the
+// tensor-core update (packA, packB, as k_dense_pack writes them; null: none).
+// Blocks [0, nL) take 128 rows of L21 each, the rest 128 columns of U12;
+// blockIdx.z selects the value set.
+// What bounds it: the solves' reads of the 64 x 64 matrix from shared memory,
+// halved by two rows per thread; the packs come from the tile in shared
+// memory, so neither the panel is read again nor a launch spent on them.
+// Order 9,216, 12 value sets: 95 us; 101 (one row per thread) + 90 us for the
+// packs as launches of their own.  Blocks of 256 rows, two per SM instead of
+// four, leave a longer last wave (105 us).
+constexpr int kRowsBlock = 128;
+constexpr int kRowsLd = kRowsBlock + 1;
+constexpr size_t kRowsSmem = sizeof(float) * (size_t(kDenseNB) * kRowsLd + size_t(kDenseNB) * kTriML);
+static_assert((kDenseNB * kRowsLd) % 4 == 0, "16-byte aligned operand tiles");
+
+__global__ void __launch_bounds__(kRowsBlock, 4)
+    k_dense_panel_rows(float *val_base, uint64_t stride, const uint32_t *__restrict__ doff, uint32_t m, uint32_t k0,
+                       const float *__restrict__ diag_scratch, uint32_t nL, uint16_t *__restrict__ packA,
+                       uint16_t *__restrict__ packB, uint32_t slot0) {
+    extern __shared__ float4 psm4[];
+    float *sW = reinterpret_cast<float *>(psm4);  // [k][row of L21 or column of U12]
+    float *sM = sW + kDenseNB * kRowsLd;           // U11 (row-major, pivot reciprocals in the padding) or L11^T
+    float *val = val_base + blockIdx.z * stride;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool lrows = blockIdx.x < nL;
+    const uint32_t i0 = k0 + kDenseNB + (lrows ? blockIdx.x : blockIdx.x - nL) * kRowsBlock;
+    const uint32_t cnt = min(uint32_t(kRowsBlock), m - i0);
+    // warp w: L21's columns 16 w .. 16 w + 15, or the block's columns 32 w .. 32 w + 31
+    constexpr uint32_t kOwn = kDenseNB / (kRowsBlock / 32);
+    const uint32_t own = lrows ? (lane < kOwn ? doff[k0 + kOwn * warp + lane] + i0 : 0u)
+                               : (32 * warp + lane < cnt ? doff[i0 + 32 * warp + lane] + k0 : 0u);
+    if (lrows) {
+#pragma unroll
+        for (uint32_t c = 0; c < kOwn; ++c) {
+            const float *src = val + __shfl_sync(0xffffffffu, own, c);
+            float *dst = sW + (kOwn * warp + c) * kRowsLd;
+#pragma unroll
+            for (uint32_t t = lane; t < uint32_t(kRowsBlock); t += 32)
+                if (t < cnt) tri_async_copy(dst + t, src + t);
+        }
+    } else {
+#pragma unroll 8
+        for (uint32_t c = 0; c < 32; ++c) {
+            const float *src = val + __shfl_sync(0xffffffffu, own, c);
+            const uint32_t t = 32 * warp + c;
+            if (t < cnt) {
+                tri_async_copy(sW + lane * kRowsLd + t, src + lane);
+                tri_async_copy(sW + (lane + 32) * kRowsLd + t, src + lane + 32);
+            }
+        }
+    }
+    tri_async_commit();
+    const float *ds = diag_scratch + size_t(blockIdx.z) * kDenseNB * kDenseNB;
+#pragma unroll
+    for (uint32_t e = tid; e < uint32_t(kDenseNB * kDenseNB); e += kRowsBlock) {
+        const float v = ld_cg(ds + e);  // row e % 64 of column e / 64
+        sM[lrows ? (e % kDenseNB) * kTriML + e / kDenseNB : (e / kDenseNB) * kTriML + e % kDenseNB] = v;
+    }
+    if (lrows) {
+        __syncthreads();
+        if (tid < kDenseNB) sM[tid * kTriML + kTriMax] = 1.0f / sM[tid * kTriML + tid];
+    }
+    tri_async_wait();
+    __syncthreads();
+    // two of the four warps solve (entries past cnt are never stored): the
+    // first or the last two by turns, so that an SM's blocks use all its
+    // sub-partitions
+    const uint32_t turn = ((blockIdx.z * gridDim.x + blockIdx.x) / 148) & 1;
+    if (warp / 2 == turn) {
+        const uint32_t t = tid & 63;
+        if (lrows)
+            tri_two_rows_solve<true>(sW, kRowsLd, t, t + 64, sM);
+        else
+            tri_two_rows_solve<false>(sW, kRowsLd, t, t + 64, sM);
+    }
+    __syncthreads();
+    if (lrows) {
+#pragma unroll
+        for (uint32_t c = 0; c < kOwn; ++c) {
+            float *dst = val + __shfl_sync(0xffffffffu, own, c);
+            const float *src = sW + (kOwn * warp + c) * kRowsLd;
+#pragma unroll
+            for (uint32_t t = lane; t < uint32_t(kRowsBlock); t += 32)
+                if (t < cnt) st_cg(dst + t, src[t]);
+        }
+    } else {
+#pragma unroll 8
+        for (uint32_t c = 0; c < 32; ++c) {
+            float *dst = val + __shfl_sync(0xffffffffu, own, c);
+            const uint32_t t = 32 * warp + c;
+            if (t < cnt) {
+                st_cg(dst + lane, sW[lane * kRowsLd + t]);
+                st_cg(dst + lane + 32, sW[(lane + 32) * kRowsLd + t]);
+            }
+        }
+    }
+    if (packA == nullptr || tid >= cnt) return;
+    uint16_t *dst = (lrows ? packA : packB) + (size_t(blockIdx.z) * m + i0 + tid) * kDensePackRow + slot0;
+#pragma unroll 2
+    for (uint32_t k = 0; k < uint32_t(kDenseNB); k += 16) {
+        uint2 p[3][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = sW[(k + 4 * q + i) * kRowsLd + tid];
+            split_bf16x4(v, p[0][q], p[1][q], p[2][q]);
+        }
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+            uint4 *d = reinterpret_cast<uint4 *>(dst + part * (kDensePackRow / 3) + k);
+            d[0] = make_uint4(p[part][0].x, p[part][0].y, p[part][1].x, p[part][1].y);
+            d[1] = make_uint4(p[part][2].x, p[part][2].y, p[part][3].x, p[part][3].y);
         }
     }
 }
@@ -263,29 +377,35 @@ uint32_t dense_panel_launches(uint32_t count, uint32_t m, uint32_t k0, uint32_t 
 
 cudaError_t launch_dense_panel(float *val, uint64_t stride, uint32_t count, const uint32_t *doff,
                                uint32_t m, uint32_t k0, uint32_t kb, const float *pert_z,
-                               float *diag_scratch, uint32_t last_has_l, uint32_t num_sms, cudaStream_t st) {
+                               float *diag_scratch, uint32_t last_has_l, uint32_t num_sms, uint32_t slot0,
+                               uint16_t *packA, uint16_t *packB, cudaStream_t st) {
     static PerDeviceOnce attr;
     cudaError_t e = attr.run([] {
-        return cudaFuncSetAttribute(k_dense_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPanelSmem));
+        cudaError_t r = cudaFuncSetAttribute(k_dense_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPanelSmem));
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k_dense_panel_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRowsSmem));
+        return r;
     });
     if (e != cudaSuccess) return e;
     uint32_t rest = m - (k0 + kb);
     uint32_t nL = (rest + kPanelRows - 1) / kPanelRows;
     uint32_t nU = nL;
     // more blocks than a few waves: factor the diagonal blocks once, then the
-    // rows and columns from them (one launch more, the LU not repeated per block)
+    // rows and columns from them (the LU not repeated per block; rest > 0, so
+    // the panel is full)
     if (dense_panel_launches(count, m, k0, kb, num_sms) == 2) {
         k_dense_panel<<<dim3(1, 1, count), kTriThreads, kPanelSmem, st>>>(val, stride, doff, m, k0, kb, pert_z,
-                                                                           diag_scratch, last_has_l, nL, 0);
+                                                                           diag_scratch, last_has_l, nL);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        k_dense_panel<<<dim3(nL + nU, 1, count), kTriThreads, kPanelSmem, st>>>(val, stride, doff, m, k0, kb, pert_z,
-                                                                                 diag_scratch, last_has_l, nL, 1);
+        const uint32_t nR = (rest + kRowsBlock - 1) / kRowsBlock;
+        k_dense_panel_rows<<<dim3(2 * nR, 1, count), kRowsBlock, kRowsSmem, st>>>(val, stride, doff, m, k0,
+                                                                                  diag_scratch, nR, packA, packB, slot0);
         return cudaGetLastError();
     }
     dim3 grid(1 + nL + nU, 1, count);
     k_dense_panel<<<grid, kTriThreads, kPanelSmem, st>>>(val, stride, doff, m, k0, kb, pert_z, diag_scratch,
-                                                          last_has_l, nL, 0);
+                                                          last_has_l, nL);
     return cudaGetLastError();
 }
 

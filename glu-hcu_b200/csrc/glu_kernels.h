@@ -102,9 +102,11 @@ constexpr int kGemmTile = 128;      // trailing-update tile
 
 cudaError_t launch_dense_panel(float *val, uint64_t stride, uint32_t count, const uint32_t *doff,
                                uint32_t m, uint32_t k0, uint32_t kb, const float *pert_z,
-                               float *diag_scratch, uint32_t last_has_l, uint32_t num_sms, cudaStream_t st);
+                               float *diag_scratch, uint32_t last_has_l, uint32_t num_sms, uint32_t slot0,
+                               uint16_t *packA, uint16_t *packB, cudaStream_t st);
 // Launches one panel step makes: 2 when its blocks over all value sets fill
-// several waves (the diagonal blocks factored once in a launch of their own).
+// several waves (the diagonal blocks factored once in a launch of their own;
+// the second launch then writes the packs as well, unless packA is null).
 uint32_t dense_panel_launches(uint32_t count, uint32_t m, uint32_t k0, uint32_t kb, uint32_t num_sms);
 // Part of the trailing update after the panels [k0, k0 + kb) (kb <=
 // kDenseGroupMax x kDenseNB): rows [r_lo, r_hi) and columns [c_lo, c_hi) of the trailing block

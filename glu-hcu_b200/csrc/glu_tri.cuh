@@ -351,7 +351,68 @@ __device__ __forceinline__ void tri_rows_solve(float *sW, uint32_t ldw, uint32_t
     }
 }
 
-// The same with two threads per row (half 0 or 1; all 2 x rows threads of the
+// Two rows t0, t1 of one thread, w = 64: an entry of M read from shared memory
+// (four bytes to every lane, which is what bounds the solves of many rows)
+// serves both.
+template <bool kDiv>
+__device__ __forceinline__ void tri_two_rows_solve(float *sW, uint32_t ldw, uint32_t t0, uint32_t t1, const float *sM) {
+    constexpr uint32_t kCh = kTriMax / kTriChunk;
+#pragma unroll 1
+    for (uint32_t cb = 0; cb < kCh; ++cb) {
+        float x[2][kTriChunk];
+        const float *m = sM + cb * kTriChunk * kTriML;  // the chunk's rows of M
+        float *w = sW + cb * kTriChunk * ldw;
+#pragma unroll
+        for (int k = 0; k < kTriChunk; ++k) x[0][k] = w[k * ldw + t0], x[1][k] = w[k * ldw + t1];
+#pragma unroll
+        for (int k = 0; k < kTriChunk; ++k) {
+            const float4 *m4 = reinterpret_cast<const float4 *>(m + k * kTriML + cb * kTriChunk);
+            float mr[kTriChunk];
+#pragma unroll
+            for (int v = k / 4; v < kTriChunk / 4; ++v) {
+                const float4 t = m4[v];
+                mr[4 * v] = t.x, mr[4 * v + 1] = t.y, mr[4 * v + 2] = t.z, mr[4 * v + 3] = t.w;
+            }
+            if (kDiv) {
+                const float d = m[k * kTriML + kTriMax];
+                x[0][k] *= d, x[1][k] *= d;
+            }
+#pragma unroll
+            for (int p = k + 1; p < kTriChunk; ++p) {
+                x[0][p] = fmaf(-x[0][k], mr[p], x[0][p]);
+                x[1][p] = fmaf(-x[1][k], mr[p], x[1][p]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kTriChunk; ++k) w[k * ldw + t0] = x[0][k], w[k * ldw + t1] = x[1][k];
+#pragma unroll 1
+        for (uint32_t cj = cb + 1; cj < kCh; ++cj) {
+            float y[2][kTriChunk];
+            float *wj = sW + cj * kTriChunk * ldw;
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) y[0][k] = wj[k * ldw + t0], y[1][k] = wj[k * ldw + t1];
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) {
+                const float4 *m4 = reinterpret_cast<const float4 *>(m + k * kTriML + cj * kTriChunk);
+#pragma unroll
+                for (int v = 0; v < kTriChunk / 4; ++v) {
+                    const float4 t = m4[v];
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        y[r][4 * v] = fmaf(-x[r][k], t.x, y[r][4 * v]);
+                        y[r][4 * v + 1] = fmaf(-x[r][k], t.y, y[r][4 * v + 1]);
+                        y[r][4 * v + 2] = fmaf(-x[r][k], t.z, y[r][4 * v + 2]);
+                        y[r][4 * v + 3] = fmaf(-x[r][k], t.w, y[r][4 * v + 3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kTriChunk; ++k) wj[k * ldw + t0] = y[0][k], wj[k * ldw + t1] = y[1][k];
+        }
+    }
+}
+
+// The same as tri_rows_solve with two threads per row (half 0 or 1; all 2 x rows threads of the
 // block take part): chunk cj belongs to half cj % 2, which applies the earlier
 // chunks to it and solves it, so the two halves share the updates and only a
 // solved chunk is waited for (a block barrier each).  The caller has a barrier
