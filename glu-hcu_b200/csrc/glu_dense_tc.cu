@@ -187,16 +187,27 @@ __device__ __forceinline__ void tc_ld32x2(uint32_t ta, uint32_t tb, float (&va)[
 }
 
 struct Tile {
-    uint32_t z, rbase, cbase;
+    uint32_t z, rbase, cbase, r_hi, c_hi;  // value set, first row and column, limits of the tile's region
 };
-__device__ __forceinline__ Tile decode_tile(uint32_t t, uint32_t tiles_r, uint32_t tiles_c, const DenseRegion &reg) {
-    const uint32_t per = tiles_r * tiles_c;
+// The tiles of a launch: those of up to two regions (a look-ahead step's row
+// strip and column strip), value set after value set.
+struct TilePlan {
+    DenseRegion reg[2];
+    uint32_t tiles_c[2], tiles[2];  // tile columns and tiles of a region
+};
+__device__ __forceinline__ Tile decode_tile(uint32_t t, const TilePlan &T) {
+    const uint32_t per = T.tiles[0] + T.tiles[1];
     Tile o;
     o.z = t / per;
-    const uint32_t rem = t - o.z * per;
-    const uint32_t tr = rem / tiles_c;
+    uint32_t rem = t - o.z * per;
+    const uint32_t i = rem >= T.tiles[0] ? 1u : 0u;
+    if (i) rem -= T.tiles[0];
+    const DenseRegion &reg = T.reg[i];
+    const uint32_t tr = rem / T.tiles_c[i];
     o.rbase = reg.r_lo + tr * kTile;
-    o.cbase = reg.c_lo + (rem - tr * tiles_c) * kTile;
+    o.cbase = reg.c_lo + (rem - tr * T.tiles_c[i]) * kTile;
+    o.r_hi = reg.r_hi;
+    o.c_hi = reg.c_hi;
     return o;
 }
 
@@ -310,14 +321,15 @@ __global__ void __launch_bounds__(kCoupleThreads) k_couple_pack(const uint32_t *
 }
 
 // -------------------------------------------------------------- update --
-// Rows [r_lo, r_hi) x columns [c_lo, c_hi) of the trailing block after the
-// panels [k0, k0 + K) (relative to r0 = k0 + K), in 128 x 128 tiles; K =
+// Up to two regions, rows [r_lo, r_hi) x columns [c_lo, c_hi) of the trailing
+// block after the panels [k0, k0 + K) (relative to r0 = k0 + K), in 128 x 128
+// tiles; K =
 // 32 * nchunks (pack slots beyond the panels' width hold zeros).  Entries of
 // a tile outside the region are computed but neither read nor written.
 __global__ void __launch_bounds__(kThreads, 1)
     k_dense_update_tc(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       float *val_base, uint64_t stride, const uint32_t *__restrict__ doff, uint32_t m, uint32_t r0,
-                      uint32_t nchunks, DenseRegion reg, uint32_t tiles_r, uint32_t tiles_c, uint32_t count,
+                      uint32_t nchunks, const __grid_constant__ TilePlan plan, uint32_t count,
                       const float *__restrict__ diag_scratch, uint32_t *status, uint32_t spin_limit,
                       uint32_t *tile_counter) {
     extern __shared__ uint8_t tc_smem_raw[];
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t *tile_id = tmem_slot + 1;        // [kRing]
     uint32_t *epi_off = reinterpret_cast<uint32_t *>(smem + kStages * kStageBytes + kBarBytes);  // [warps][64]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t total = tiles_r * tiles_c * count;
+    const uint32_t total = (plan.tiles[0] + plan.tiles[1]) * count;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -383,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tile_id[slot] = t < total ? t : total;
                 mbar_arrive(&tile_full[slot]);
                 if (t >= total) break;
-                const Tile tl = decode_tile(t, tiles_r, tiles_c, reg);
+                const Tile tl = decode_tile(t, plan);
                 const int ya = int(r0 + tl.rbase), yb = int(r0 + tl.cbase), zz = int(tl.z);
                 for (uint32_t kc = 0; kc < nchunks; ++kc, ++g) {
                     const uint32_t s = g % kStages, ph = (g / kStages) & 1;
@@ -483,12 +495,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&tile_empty[slot]);
             if (t >= total) break;
-            const Tile tl = decode_tile(t, tiles_r, tiles_c, reg);
+            const Tile tl = decode_tile(t, plan);
             const float *val = val_base + tl.z * stride;
-            const uint32_t rows = min(uint32_t(kTile), reg.r_hi - tl.rbase);
+            const uint32_t rows = min(uint32_t(kTile), tl.r_hi - tl.rbase);
             for (uint32_t cc = lane; cc < uint32_t(kTile); cc += 32) {
                 const uint32_t col = tl.cbase + cc;
-                if (col >= reg.c_hi) break;
+                if (col >= tl.c_hi) break;
                 const float *p0 = val + __ldg(doff + r0 + col) + r0 + tl.rbase;
                 const uintptr_t a0 = reinterpret_cast<uintptr_t>(p0) & ~uintptr_t(127);
                 const uintptr_t a1 = reinterpret_cast<uintptr_t>(p0 + rows - 1);
@@ -508,6 +520,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t half = ew >> 2;
         const uint32_t row = q * 32 + lane;  // tile row of this thread
         uint32_t *soff = epi_off + ew * 64;
+        const DenseRegion &reg = plan.reg[0];
         if (reg.writeback) {
             // the factored diagonal block of the panel at wb_k0, kept in
             // scratch while that panel's blocks still read the original
@@ -532,11 +545,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&tile_empty[slot]);
             if (t >= total) break;
-            const Tile tl = decode_tile(t, tiles_r, tiles_c, reg);
+            const Tile tl = decode_tile(t, plan);
             float *val = val_base + tl.z * stride;
             const uint32_t c0 = tl.cbase + half * 64;  // first tile column of this warp
-            const uint32_t ncol = c0 < reg.c_hi ? min(64u, reg.c_hi - c0) : 0u;
-            const bool rok = tl.rbase + row < reg.r_hi;
+            const uint32_t ncol = c0 < tl.c_hi ? min(64u, tl.c_hi - c0) : 0u;
+            const bool rok = tl.rbase + row < tl.r_hi;
             const bool full_tile = __all_sync(0xffffffffu, rok) && ncol == 64;
             const uint32_t grow = r0 + tl.rbase + row;
             // column offsets of this warp's 64 columns (the previous tile's
@@ -645,40 +658,46 @@ cudaError_t launch_dense_pack(const float *val, uint64_t stride, uint32_t count,
 }
 
 namespace {
-// Rows [r_lo, r_hi) x columns [c_lo, c_hi) of the block from row and column
-// r0 on, K = 32 * nchunks.
+// The regions' rows x columns of the block from row and column r0 on, K = 32 *
+// nchunks; tile_counter is zero.
 cudaError_t launch_tc(const CUtensorMap &mapA, const CUtensorMap &mapB, float *val, uint64_t stride, uint32_t count,
                       const uint32_t *doff, uint32_t m, uint32_t r0, uint32_t nchunks, const float *diag_scratch,
-                      DenseRegion reg, uint32_t *status, uint32_t spin_limit, uint32_t num_sms,
-                      uint32_t *tile_counter, cudaStream_t st) {
+                      const DenseRegion *regs, uint32_t nregs, uint32_t *status, uint32_t spin_limit,
+                      uint32_t num_sms, uint32_t *tile_counter, cudaStream_t st) {
     static PerDeviceOnce attr;
     cudaError_t e = attr.run([] {
         return cudaFuncSetAttribute(k_dense_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
     });
     if (e != cudaSuccess) return e;
-    const uint32_t rows = reg.r_hi > reg.r_lo ? reg.r_hi - reg.r_lo : 0;
-    const uint32_t cols = reg.c_hi > reg.c_lo ? reg.c_hi - reg.c_lo : 0;
-    const uint32_t tiles_r = (rows + kTile - 1) / kTile, tiles_c = (cols + kTile - 1) / kTile;
-    const uint64_t total = uint64_t(tiles_r) * tiles_c * count;
-    if (total == 0 && !reg.writeback) return cudaSuccess;
+    TilePlan plan = {};
+    for (uint32_t i = 0; i < nregs; ++i) {
+        const DenseRegion &reg = regs[i];
+        const uint32_t rows = reg.r_hi > reg.r_lo ? reg.r_hi - reg.r_lo : 0;
+        const uint32_t cols = reg.c_hi > reg.c_lo ? reg.c_hi - reg.c_lo : 0;
+        const uint64_t tiles = uint64_t((rows + kTile - 1) / kTile) * ((cols + kTile - 1) / kTile);
+        if (tiles > 0x7FFFFFFFu) return cudaErrorInvalidValue;
+        plan.reg[i] = reg;
+        plan.tiles_c[i] = (cols + kTile - 1) / kTile;
+        plan.tiles[i] = uint32_t(tiles);
+    }
+    const bool writeback = plan.reg[0].writeback != 0;
+    const uint64_t total = (uint64_t(plan.tiles[0]) + plan.tiles[1]) * count;
+    if (total == 0 && !writeback) return cudaSuccess;
     if (r0 > m || total > 0xFFFFFFFFull || nchunks == 0 || nchunks * kChunk > kSlots) return cudaErrorInvalidValue;
     uint32_t grid = uint32_t(std::min<uint64_t>(std::max<uint64_t>(total, 1), num_sms));
-    if (reg.writeback) grid = std::max<uint32_t>(grid, std::min<uint32_t>(count, num_sms));
-    e = cudaMemsetAsync(tile_counter, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
-    k_dense_update_tc<<<grid, kThreads, kSmemBytes, st>>>(mapA, mapB, val, stride, doff, m, r0, nchunks, reg,
-                                                          tiles_r, tiles_c, count, diag_scratch, status, spin_limit,
-                                                          tile_counter);
+    if (writeback) grid = std::max<uint32_t>(grid, std::min<uint32_t>(count, num_sms));
+    k_dense_update_tc<<<grid, kThreads, kSmemBytes, st>>>(mapA, mapB, val, stride, doff, m, r0, nchunks, plan, count,
+                                                          diag_scratch, status, spin_limit, tile_counter);
     return cudaGetLastError();
 }
 }  // namespace
 
 cudaError_t launch_dense_update_tc(const CUtensorMap &mapA, const CUtensorMap &mapB, float *val, uint64_t stride,
                                    uint32_t count, const uint32_t *doff, uint32_t m, uint32_t k0, uint32_t kb,
-                                   const float *diag_scratch, DenseRegion reg, uint32_t *status,
+                                   const float *diag_scratch, const DenseRegion *regs, uint32_t nregs, uint32_t *status,
                                    uint32_t spin_limit, uint32_t num_sms, uint32_t *tile_counter, cudaStream_t st) {
-    return launch_tc(mapA, mapB, val, stride, count, doff, m, k0 + kb, (kb + kChunk - 1) / kChunk, diag_scratch, reg,
-                     status, spin_limit, num_sms, tile_counter, st);
+    return launch_tc(mapA, mapB, val, stride, count, doff, m, k0 + kb, (kb + kChunk - 1) / kChunk, diag_scratch, regs,
+                     nregs, status, spin_limit, num_sms, tile_counter, st);
 }
 
 cudaError_t launch_couple_pack(const DevPattern &P, const float *val, uint64_t stride, uint32_t count, uint32_t t,
@@ -703,7 +722,7 @@ cudaError_t launch_couple_update_tc(const CUtensorMap &mapA, const CUtensorMap &
                                     uint32_t *status, uint32_t spin_limit, uint32_t num_sms, uint32_t *tile_counter,
                                     cudaStream_t st) {
     const DenseRegion reg{0, m, 0, m, 0, 0};
-    return launch_tc(mapA, mapB, val, stride, count, doff, m, 0, (ncols + kChunk - 1) / kChunk, nullptr, reg, status,
+    return launch_tc(mapA, mapB, val, stride, count, doff, m, 0, (ncols + kChunk - 1) / kChunk, nullptr, &reg, 1, status,
                      spin_limit, num_sms, tile_counter, st);
 }
 

@@ -273,6 +273,7 @@ struct glu_handle_s {
     // tensor-core dense update: BF16 three-part operand packs and their TMA maps
     // (allocated on the first factorization that uses them)
     DevBuf d_packA, d_packB, d_tc_counter;
+    uint32_t tc_counters = 0;
     // dataflow factorization of the dense tail: finished tiles of every value
     // set, then ticket and ready flags (allocated on the first factorization
     // that uses them)
@@ -1805,13 +1806,19 @@ Status factor_buffers(glu_handle_s *h, uint32_t count, bool *use_flow) {
     // tensor-core updates for wide trailing blocks; their operand packs are
     // allocated once per handle
     const bool tc = h->m && h->tune.dense_tc_min && h->m >= h->tune.dense_tc_min;
+    // a tile counter per tensor-core launch of a factorization: at most two
+    // per panel and one per coupling group
+    const uint32_t counters = 2 * ((h->m + kDenseNB - 1) / kDenseNB) + uint32_t(h->couple_groups.size());
+    if (tc && (!flow || !h->couple_groups.empty()) && h->tc_counters < counters) {
+        GLU_CUDA(h->d_tc_counter.alloc(sizeof(uint32_t) * counters), "allocate tile counters");
+        h->tc_counters = counters;
+    }
     if (tc && (!flow || !h->couple_groups.empty()) && h->pack_m != h->m) {
         const size_t pack_bytes = sizeof(uint16_t) * kDensePackRow * size_t(h->m) * h->batch;
         GLU_CUDA(h->d_packA.alloc(pack_bytes), "allocate tensor-core operand packs");
         GLU_CUDA(h->d_packB.alloc(pack_bytes), "allocate tensor-core operand packs");
         GLU_CUDA(dense_tc_tensor_map(h->d_packA.as<uint16_t>(), h->m, h->batch, &h->map_packA), "tensor map");
         GLU_CUDA(dense_tc_tensor_map(h->d_packB.as<uint16_t>(), h->m, h->batch, &h->map_packB), "tensor map");
-        GLU_CUDA(h->d_tc_counter.alloc(sizeof(uint32_t) * 2), "allocate tile counters");
         h->pack_m = h->m;
     }
     if (h->m)
@@ -1909,6 +1916,9 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
     // only when the block updates on the tensor cores): per group of up to 128
     // columns, their tail rows of L and tail columns of U into the packs, then
     // A22 -= L U over the whole block.
+    uint32_t *tc_next = h->d_tc_counter.as<uint32_t>();
+    if (tc && (!flow || !h->couple_groups.empty()))
+        GLU_CUDA(cudaMemsetAsync(tc_next, 0, sizeof(uint32_t) * h->tc_counters, st), "factor (tile counters)");
     if (tc && !h->couple_groups.empty()) {
         const double mm = h->m;
         for (const CoupleGroup &gr : h->couple_groups) {
@@ -1920,7 +1930,7 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
                        "factor (coupling pack)");
             GLU_LAUNCH(KK_UPDATE_TC,
                        launch_couple_update_tc(h->map_packA, h->map_packB, dbase, dstride, count, doff, h->m, nc,
-                                               dstatus, h->spin_limit, h->num_sms, h->d_tc_counter.as<uint32_t>(), st),
+                                               dstatus, h->spin_limit, h->num_sms, tc_next++, st),
                        "factor (coupling update)");
             upd_bytes += double(count) * (8.0 * mm * mm + 8.0 * nc * mm);
             upd_flops += double(count) * 2.0 * nc * mm * mm;
@@ -1948,26 +1958,34 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
     const uint64_t tc_area = std::min<uint64_t>(uint64_t(2) * h->num_sms * kTcTile * kTcTile,
                                                 uint64_t(h->tune.dense_tc_min) * h->tune.dense_tc_min);
     auto tc_region = [&](uint32_t rows, uint32_t cols) { return tc && uint64_t(rows) * cols * count >= tc_area; };
-    auto update = [&](uint32_t k0, uint32_t kb, DenseRegion reg, cudaStream_t s) -> cudaError_t {
-        const uint32_t nr = reg.r_hi > reg.r_lo ? reg.r_hi - reg.r_lo : 0;
-        const uint32_t nc = reg.c_hi > reg.c_lo ? reg.c_hi - reg.c_lo : 0;
-        const double rows = nr, cols = nc;
-        upd_bytes += double(count) * (8.0 * rows * cols + 4.0 * kb * (rows + cols));
-        upd_flops += double(count) * 2.0 * kb * rows * cols;
-        cudaError_t e = pf.begin(s);
-        if (e != cudaSuccess) return e;
-        if (tc_region(nr, nc)) {
-            // a tile counter per stream (launches on one stream run in order)
-            uint32_t *ctr = h->d_tc_counter.as<uint32_t>() + (s == st ? 0 : 1);
-            e = launch_dense_update_tc(h->map_packA, h->map_packB, dbase, dstride, count, doff, h->m, k0, kb, dscr,
-                                       reg, dstatus, h->spin_limit, h->num_sms, ctr, s);
-            if (e == cudaSuccess) e = pf.end(KK_UPDATE_TC, s);
-        } else {
-            e = launch_dense_update(dbase, dstride, count, doff, h->m, k0, kb, dscr, reg, s);
-            if (e == cudaSuccess) e = pf.end(KK_UPDATE, s);
+    auto update = [&](uint32_t k0, uint32_t kb, std::initializer_list<DenseRegion> regs, cudaStream_t s) -> cudaError_t {
+        bool all_tc = true;
+        for (const DenseRegion &reg : regs) {
+            const uint32_t nr = reg.r_hi > reg.r_lo ? reg.r_hi - reg.r_lo : 0;
+            const uint32_t nc = reg.c_hi > reg.c_lo ? reg.c_hi - reg.c_lo : 0;
+            const double rows = nr, cols = nc;
+            upd_bytes += double(count) * (8.0 * rows * cols + 4.0 * kb * (rows + cols));
+            upd_flops += double(count) * 2.0 * kb * rows * cols;
+            all_tc = all_tc && tc_region(nr, nc);
         }
-        ++nlaunch;
-        return e;
+        if (all_tc) {  // one launch for both strips
+            cudaError_t e = pf.begin(s);
+            if (e == cudaSuccess)
+                e = launch_dense_update_tc(h->map_packA, h->map_packB, dbase, dstride, count, doff, h->m, k0, kb, dscr,
+                                           regs.begin(), uint32_t(regs.size()), dstatus, h->spin_limit, h->num_sms,
+                                           tc_next++, s);
+            if (e == cudaSuccess) e = pf.end(KK_UPDATE_TC, s);
+            ++nlaunch;
+            return e;
+        }
+        for (const DenseRegion &reg : regs) {
+            cudaError_t e = pf.begin(s);
+            if (e == cudaSuccess) e = launch_dense_update(dbase, dstride, count, doff, h->m, k0, kb, dscr, reg, s);
+            if (e == cudaSuccess) e = pf.end(KK_UPDATE, s);
+            if (e != cudaSuccess) return e;
+            ++nlaunch;
+        }
+        return cudaSuccess;
     };
     // BF16 three-part operands of panel k0 (slot0 = 64 j for panel j of a
     // look-ahead group), on the panel stream
@@ -2018,7 +2036,7 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
         else
             GLU_CUDA(pack(k0, kb0, 0, packed), "factor (dense pack)");
         if (g == 1) {  // small trailing blocks, last panels: plain steps
-            GLU_CUDA(update(k0, kb0, DenseRegion{0, rest0, 0, rest0, 1, k0}, ps), "factor (dense update)");
+            GLU_CUDA(update(k0, kb0, {DenseRegion{0, rest0, 0, rest0, 1, k0}}, ps), "factor (dense update)");
             k0 += kb0;
             continue;
         }
@@ -2029,8 +2047,8 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
         for (uint32_t j = 1; j < g; ++j) {
             const uint32_t kj = k0 + kk, kbj = std::min<uint32_t>(nb, h->m - kj), tj = h->m - kj;
             const uint32_t hj = std::min<uint32_t>(nb, tj);
-            GLU_CUDA(update(k0, kk, DenseRegion{0, hj, 0, tj, 1, kj - nb}, ps), "factor (dense update)");
-            if (tj > hj) GLU_CUDA(update(k0, kk, DenseRegion{hj, tj, 0, hj, 0, kj - nb}, ps), "factor (dense update)");
+            const DenseRegion rows{0, hj, 0, tj, 1, kj - nb}, cols{hj, tj, 0, hj, 0, kj - nb};
+            GLU_CUDA(tj > hj ? update(k0, kk, {rows, cols}, ps) : update(k0, kk, {rows}, ps), "factor (dense update)");
             GLU_CUDA(panel(kj, kbj, kDenseNB * j, packed), "factor (dense panel)");
             GLU_CUDA(pack(kj, kbj, kDenseNB * j, packed && !panel_packs(kj, kbj)), "factor (dense pack)");
             kk += kbj;
@@ -2041,13 +2059,13 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
         const uint32_t kl = k0 + kk - std::min<uint32_t>(nb, kk - (g - 1) * nb);  // last panel of the group
         const uint32_t rest1 = h->m - (k0 + kk);
         if (rest1 <= nb) {
-            GLU_CUDA(update(k0, kk, DenseRegion{0, rest1, 0, rest1, 1, kl}, ps), "factor (dense update)");
+            GLU_CUDA(update(k0, kk, {DenseRegion{0, rest1, 0, rest1, 1, kl}}, ps), "factor (dense update)");
         } else {
             GLU_CUDA(cudaEventRecord(h->ev_panel, ps), "event");
-            GLU_CUDA(update(k0, kk, DenseRegion{0, nb, 0, rest1, 1, kl}, ps), "factor (dense update)");
-            GLU_CUDA(update(k0, kk, DenseRegion{nb, rest1, 0, nb, 0, kl}, ps), "factor (dense update)");
+            GLU_CUDA(update(k0, kk, {DenseRegion{0, nb, 0, rest1, 1, kl}, DenseRegion{nb, rest1, 0, nb, 0, kl}}, ps),
+                     "factor (dense update)");
             GLU_CUDA(cudaStreamWaitEvent(st, h->ev_panel, 0), "stream wait");
-            GLU_CUDA(update(k0, kk, DenseRegion{nb, rest1, nb, rest1, 0, kl}, st), "factor (dense update)");
+            GLU_CUDA(update(k0, kk, {DenseRegion{nb, rest1, nb, rest1, 0, kl}}, st), "factor (dense update)");
             GLU_CUDA(cudaEventRecord(h->ev_rest, st), "event");
             rest_pending = true;
         }

@@ -131,9 +131,11 @@ cudaError_t dense_tc_tensor_map(uint16_t *pack, uint32_t m, uint32_t batch, CUte
 cudaError_t launch_dense_pack(const float *val, uint64_t stride, uint32_t count, const uint32_t *doff, uint32_t m,
                               uint32_t k0, uint32_t kb, uint32_t slot0, uint16_t *packA, uint16_t *packB,
                               cudaStream_t st);
+// One or two regions (disjoint; the first one's writeback counts), tile_counter:
+// a word that is zero.
 cudaError_t launch_dense_update_tc(const CUtensorMap &mapA, const CUtensorMap &mapB, float *val, uint64_t stride,
                                    uint32_t count, const uint32_t *doff, uint32_t m, uint32_t k0, uint32_t kb,
-                                   const float *diag_scratch, DenseRegion reg, uint32_t *status,
+                                   const float *diag_scratch, const DenseRegion *regs, uint32_t nregs, uint32_t *status,
                                    uint32_t spin_limit, uint32_t num_sms, uint32_t *tile_counter, cudaStream_t st);
 // The deferred coupling of the sparse part into the trailing block: sparse
 // columns whose update of the block is large skip it in the supernodal
