@@ -1,7 +1,7 @@
 // Trailing update of the dense tail on the 5th-generation tensor cores.
 //
 // The blocked dense LU of the trailing block (glu_factor_dense.cu) spends
-// almost all of its flops in A22 -= L21 U12 with K = 64 .. 256 (one panel or a
+// almost all of its flops in A22 -= L21 U12 with K = 64 .. 256 (one panel or 
 // group of up to four), and the deferred coupling of the sparse part adds products of the
 // same form.  Here that product runs as tcgen05.mma kind::f16 on BF16
 // operands with FP32 accuracy kept by splitting every operand into three BF16
@@ -264,17 +264,20 @@ __global__ void __launch_bounds__(256) k_dense_pack(const float *__restrict__ va
 // slot0 + ncols - 1): packA[z][i][256 p + s] = part p of L(t + i, k_s),
 // packB[z][j][256 p + s] = part p of U(k_s, t + j), zero where the pattern has
 // no entry and for slots past the group.  Block b < nblk takes tail rows
-// [128 b, 128 b + 128): four threads of slot s walk column k_s's CSC entries
-// [lstart[g][b], lstart[g][b + 1]) (g = slot0 + s), the ones in those rows.
-// Block nblk + b takes tail columns [128 b, 128 b + 128): four threads of slot
-// s walk row k_s's CSR entries [ustart[g][b], ustart[g][b + 1]), the ones in
-// those columns (their CSC positions from cpos).  The start tables (nblk + 1 entries
-// per slot) are computed with the plan.  A 128 x 128 tile in shared memory,
-// then coalesced writes of the three BF16 parts.
-constexpr uint32_t kCoupleLd = kTile + 1;
-constexpr size_t kCoupleSmem = sizeof(float) * kTile * kCoupleLd;
-constexpr uint32_t kCoupleWalkers = 4;  // threads walking one slot's entries
-constexpr uint32_t kCoupleThreads = kTile * kCoupleWalkers;
+// [128 b, 128 b + 128) of 64 slots (blockIdx.y): their entries are column k_s's
+// CSC entries [lstart[g][b], lstart[g][b + 1]) (g = slot0 + s).  Block nblk + b
+// takes tail columns [128 b, 128 b + 128): row k_s's CSR entries
+// [ustart[g][b], ustart[g][b + 1]) (their CSC positions from cpos).  The start
+// tables (nblk + 1 entries per slot) are computed with the plan.  A 128 x 64
+// tile in shared memory, then coalesced writes of the three BF16 parts.
+// What bounds it is the chain of loads from a slot's start to its values: 
+// warp takes eight slots, lanes along the entries, and has the loads of all
+// eight in flight at every step (four threads walking one slot each left 
+// chain of up to 32 of them: 41 us per group at order 3,968, now 12.6).
+constexpr uint32_t kCoupleSlots = 64;
+constexpr uint32_t kCoupleLd = kCoupleSlots + 1;
+constexpr uint32_t kCoupleThreads = 256;
+constexpr int kCoupleEach = kCoupleSlots / (kCoupleThreads / 32);  // slots of a warp
 
 __global__ void __launch_bounds__(kCoupleThreads) k_couple_pack(const uint32_t *__restrict__ ridx,
                                                        const uint32_t *__restrict__ cidx,
@@ -284,36 +287,58 @@ __global__ void __launch_bounds__(kCoupleThreads) k_couple_pack(const uint32_t *
                                                        const uint32_t *__restrict__ lstart,
                                                        const uint32_t *__restrict__ ustart, uint32_t nblk,
                                                        uint16_t *__restrict__ packA, uint16_t *__restrict__ packB) {
-    extern __shared__ float sT[];  // [128][kCoupleLd]: sT[r * kCoupleLd + s]
+    __shared__ __align__(16) float sT[kTile * kCoupleLd];  // sT[r * kCoupleLd + s]
     const float *val = val_base + blockIdx.z * stride;
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool aside = blockIdx.x < nblk;
-    const uint32_t b = aside ? blockIdx.x : blockIdx.x - nblk, b0 = b * kTile;
-    for (uint32_t e = tid; e < kTile * kCoupleLd; e += kCoupleThreads) sT[e] = 0.0f;
+    const uint32_t b = aside ? blockIdx.x : blockIdx.x - nblk, b0 = b * kTile, s0 = blockIdx.y * kCoupleSlots;
+    const uint32_t *idx = aside ? ridx : cidx;
+    // the warp's slots: lane u has the first entry of slot u, lane u + 8 its end
+    static_assert(kCoupleEach == 8, "slot starts in lanes 0..7, ends in 8..15");
+    uint32_t bound = 0;
+    {
+        const uint32_t sl = s0 + warp * kCoupleEach + (lane & 7);
+        if (lane < 16 && sl < ncols) bound = __ldg((aside ? lstart : ustart) + size_t(slot0 + sl) * (nblk + 1) + b + (lane >> 3));
+    }
+    for (uint32_t e = tid; e < kTile * kCoupleLd / 4; e += kCoupleThreads)
+        reinterpret_cast<float4 *>(sT)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    uint32_t p[kCoupleEach], end[kCoupleEach], longest = 0;
+#pragma unroll
+    for (int u = 0; u < kCoupleEach; ++u) {
+        p[u] = __shfl_sync(0xffffffffu, bound, u);
+        end[u] = __shfl_sync(0xffffffffu, bound, u + 8);
+        longest = max(longest, end[u] - p[u]);
+        p[u] += lane;
+    }
     __syncthreads();
-    // kCoupleWalkers threads per slot, each every kCoupleWalkers-th entry
-    const uint32_t sl = tid % kTile, wk = tid / kTile;
-    if (sl < ncols) {
-        const uint32_t *st = (aside ? lstart : ustart) + size_t(slot0 + sl) * (nblk + 1) + b;
-        const uint32_t p0 = __ldg(st) + wk, p1 = __ldg(st + 1);
-        if (aside) {
-            for (uint32_t p = p0; p < p1; p += kCoupleWalkers)
-                sT[(__ldg(ridx + p) - t - b0) * kCoupleLd + sl] = ld_cg(val + p);
-        } else {
-            for (uint32_t e = p0; e < p1; e += kCoupleWalkers)
-                sT[(__ldg(cidx + e) - t - b0) * kCoupleLd + sl] = ld_cg(val + __ldg(cpos + e));
+    for (uint32_t done = 0; done < longest; done += 32) {
+        uint32_t at[kCoupleEach], pos[kCoupleEach];
+        float v[kCoupleEach];
+#pragma unroll
+        for (int u = 0; u < kCoupleEach; ++u)
+            if (p[u] < end[u]) {
+                at[u] = __ldg(idx + p[u]);
+                pos[u] = aside ? p[u] : __ldg(cpos + p[u]);
+            }
+#pragma unroll
+        for (int u = 0; u < kCoupleEach; ++u)
+            if (p[u] < end[u]) v[u] = ld_cg(val + pos[u]);
+#pragma unroll
+        for (int u = 0; u < kCoupleEach; ++u) {
+            if (p[u] < end[u]) sT[(at[u] - t - b0) * kCoupleLd + warp * kCoupleEach + u] = v[u];
+            p[u] += 32;
         }
     }
     __syncthreads();
     uint16_t *pack = aside ? packA : packB;
     const uint32_t rows = min(uint32_t(kTile), m - b0);
-    for (uint32_t e = tid; e < rows * (kTile / 4); e += kCoupleThreads) {
-        const uint32_t r = e / (kTile / 4), q = e - r * (kTile / 4);
+    for (uint32_t e = tid; e < rows * (kCoupleSlots / 4); e += kCoupleThreads) {
+        const uint32_t r = e / (kCoupleSlots / 4), q = e % (kCoupleSlots / 4);
         const float *src = sT + r * kCoupleLd + 4 * q;
         const float v[4] = {src[0], src[1], src[2], src[3]};
         uint2 p0, p1, p2;
         split_bf16x4(v, p0, p1, p2);
-        uint16_t *dst = pack + (size_t(blockIdx.z) * m + b0 + r) * kPackRow + 4 * q;
+        uint16_t *dst = pack + (size_t(blockIdx.z) * m + b0 + r) * kPackRow + s0 + 4 * q;
         *reinterpret_cast<uint2 *>(dst) = p0;
         *reinterpret_cast<uint2 *>(dst + kSlots) = p1;
         *reinterpret_cast<uint2 *>(dst + 2 * kSlots) = p2;
@@ -705,15 +730,9 @@ cudaError_t launch_couple_pack(const DevPattern &P, const float *val, uint64_t s
                                const uint32_t *ustart, uint16_t *packA, uint16_t *packB, cudaStream_t st) {
     if (m == 0 || ncols == 0) return cudaSuccess;
     if (ncols > uint32_t(kTile)) return cudaErrorInvalidValue;
-    static PerDeviceOnce attr;
-    cudaError_t e = attr.run([] {
-        return cudaFuncSetAttribute(k_couple_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoupleSmem));
-    });
-    if (e != cudaSuccess) return e;
     const uint32_t nblk = (m + kTile - 1) / kTile;
-    k_couple_pack<<<dim3(2 * nblk, 1, count), kCoupleThreads, kCoupleSmem, st>>>(P.ridx, P.cidx, P.cpos, val, stride, t, m,
-                                                                      ncols, slot0, lstart, ustart, nblk, packA,
-                                                                      packB);
+    k_couple_pack<<<dim3(2 * nblk, (ncols + kCoupleSlots - 1) / kCoupleSlots, count), kCoupleThreads, 0, st>>>(
+        P.ridx, P.cidx, P.cpos, val, stride, t, m, ncols, slot0, lstart, ustart, nblk, packA, packB);
     return cudaGetLastError();
 }
 
