@@ -1130,10 +1130,13 @@ Status build_plan(glu_handle_s *h) {
     {
         // CSR position of the first column >= t in every tail row
         std::vector<uint32_t> trs(std::max<uint32_t>(m, 1), 0);
+        h->S.tail_longest = h->S.tail_row_longest = 0;
         for (uint32_t i = 0; i < m; ++i) {
             const uint32_t *b0 = s.csr_c_idx.data() + s.csr_r_ptr[t + i];
             const uint32_t *b1 = s.csr_c_idx.data() + s.csr_r_ptr[t + i + 1];
             trs[i] = uint32_t(std::lower_bound(b0, b1, t) - s.csr_c_idx.data());
+            h->S.tail_row_longest = std::max(h->S.tail_row_longest, trs[i] - s.csr_r_ptr[t + i]);
+            h->S.tail_longest = std::max(h->S.tail_longest, h->tail_start_h[i] - s.sym_c_ptr[t + i]);
         }
         GLU_CUDA(upload(h->d_tail_row_start, trs), "upload solve plan");
         h->S.tail_row_start = h->d_tail_row_start.as<uint32_t>();

@@ -309,6 +309,7 @@ struct SolvePlanDev {
     const uint32_t *doff;           // dense tail column offsets (into the dense view)
     const uint32_t *tail_start;     // CSC position of the first row >= t of each tail column
     const uint32_t *tail_row_start; // CSR position of the first column >= t of each tail row
+    uint32_t tail_longest, tail_row_longest;  // most entries a tail column (row) has before those
     SweepPlan sweep[4];             // L, U, U^T, L^T
     SnSweepPlan sn[2];              // supernodal L and U sweeps (nlev == 0: column sweeps)
     uint32_t cluster;               // CTAs of the thin-level cluster kernel

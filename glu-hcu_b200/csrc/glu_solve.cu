@@ -172,32 +172,96 @@ __global__ void __launch_bounds__(kSolveChainThreads) k_sweep_chain(DevPattern P
     }
 }
 
-// Coupling of the dense tail with the sparse unknowns, one warp per tail
-// column / row j (x_j final): y_i -= U(i,j) x_j for the U entries of tail
-// column j in rows i < t (kRow = false, before the sparse U sweep), or
-// y_c -= L(j,c) x_j for the L entries of tail row j in columns c < t
-// (kRow = true, before the sparse L^T sweep).
+// Coupling of the dense tail with the sparse unknowns, tail columns / rows j
+// (x_j final): y_i -= U(i,j) x_j for the U entries of tail column j in rows i <
+// t (kRow = false, before the sparse U sweep), or y_c -= L(j,c) x_j for the L
+// entries of tail row j in columns c < t (kRow = true, before the sparse L^T
+// sweep).  A warp takes the entries [64 blockIdx.x, 64 blockIdx.x + 64) of
+// kCoupleCols neighbouring columns.
+// What bounds it is the updates in L2, many on the same unknowns: neighbouring
+// tail columns mostly hold the same rows at the same places, so a lane sums up
+// their products as long as the row stays the same and issues one update.  The
+// entries are read while the dense sweep before still runs (a chained launch).
+// After its sweep: order 3,968 66 -> 55 us, order 1,100 20 -> 8 us (a warp per
+// column and an update per entry); order 9,216, 12 value sets of four
+// right-hand sides 1,141 -> 640 us.
+constexpr int kCoupleCols = 8;
+constexpr int kCoupleEach = 2;  // entries of a column per lane
+constexpr uint32_t kCoupleRhs = 4;
 template <bool kRow>
 __global__ void __launch_bounds__(256) k_tail_coupling(DevPattern P, uint32_t t, uint32_t m,
                                                        const uint32_t *__restrict__ tail_start,
                                                        const float *__restrict__ val, float *y, uint32_t nrhs,
                                                        uint64_t vstride, uint64_t ystride) {
-    val += blockIdx.z * vstride;  // value set blockIdx.z, its right-hand sides
-    y += blockIdx.z * ystride;
+    pdl_release();
+    // value set and kCoupleRhs right-hand sides of it
+    const uint32_t shares = (nrhs + kCoupleRhs - 1) / kCoupleRhs, z = blockIdx.z / shares;
+    const uint32_t v0 = (blockIdx.z - z * shares) * kCoupleRhs, v1 = min(v0 + kCoupleRhs, nrhs);
+    val += z * vstride;
+    y += z * ystride;
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t jj = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (jj >= m) return;
-    const uint32_t j = t + jj, n = P.n;
-    const uint32_t p0 = kRow ? P.rptr[j] : P.cptr[j], p1 = tail_start[jj];
-    for (uint32_t r = 0; r < nrhs; ++r) {
-        float *yr = y + size_t(r) * n;
-        const float xj = yr[j];
-        if (xj == 0.0f) continue;
-        for (uint32_t p = p0 + lane; p < p1; p += 32) {
-            const uint32_t tgt = kRow ? P.cidx[p] : P.ridx[p];
-            const float v = kRow ? val[P.cpos[p]] : val[p];
-            atomicAdd(yr + tgt, -__fmul_rn(v, xj));
+    const uint32_t j0 = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kCoupleCols;
+    const uint32_t n = P.n, off = blockIdx.x * (32 * kCoupleEach);
+    // lane g: column j0 + g, its entries from `off` on
+    const bool own = lane < uint32_t(kCoupleCols) && j0 + lane < m;
+    uint32_t b = 0, e = 0;
+    if (own) {
+        b = __ldg((kRow ? P.rptr : P.cptr) + t + j0 + lane) + off;
+        e = __ldg(tail_start + j0 + lane);
+    }
+    const bool any = __any_sync(0xffffffffu, b < e);
+    uint32_t tgt[kCoupleCols][kCoupleEach];
+    float v[kCoupleCols][kCoupleEach];
+    if (any) {
+        uint32_t pos[kCoupleCols][kCoupleEach];
+#pragma unroll
+        for (int g = 0; g < kCoupleCols; ++g) {
+            const uint32_t bg = __shfl_sync(0xffffffffu, b, g), eg = __shfl_sync(0xffffffffu, e, g);
+#pragma unroll
+            for (int u = 0; u < kCoupleEach; ++u) {
+                const uint32_t p = bg + 32 * u + lane;
+                tgt[g][u] = p < eg ? __ldg((kRow ? P.cidx : P.ridx) + p) : 0xffffffffu;
+                pos[g][u] = p < eg ? (kRow ? __ldg(P.cpos + p) : p) : 0u;
+            }
         }
+#pragma unroll
+        for (int g = 0; g < kCoupleCols; ++g)
+#pragma unroll
+            for (int u = 0; u < kCoupleEach; ++u) v[g][u] = tgt[g][u] != 0xffffffffu ? __ldg(val + pos[g][u]) : 0.0f;
+    }
+    pdl_wait();  // the tail's unknowns
+    if (!any) return;
+    float xs[kCoupleRhs];
+#pragma unroll
+    for (int q = 0; q < int(kCoupleRhs); ++q)
+        xs[q] = (own && v0 + q < v1) ? __ldcg(y + size_t(v0 + q) * n + t + j0 + lane) : 0.0f;
+#pragma unroll
+    for (int q = 0; q < int(kCoupleRhs); ++q) {
+        if (v0 + q >= v1) break;
+        float *yr = y + size_t(v0 + q) * n;
+        const float x = xs[q];
+        float sum[kCoupleEach];
+        uint32_t row[kCoupleEach];
+#pragma unroll
+        for (int u = 0; u < kCoupleEach; ++u) sum[u] = 0.0f, row[u] = 0xffffffffu;
+#pragma unroll
+        for (int g = 0; g < kCoupleCols; ++g) {
+            const float xj = __shfl_sync(0xffffffffu, x, g);
+            if (xj == 0.0f) continue;
+#pragma unroll
+            for (int u = 0; u < kCoupleEach; ++u) {
+                if (tgt[g][u] == 0xffffffffu) continue;
+                if (tgt[g][u] != row[u]) {
+                    if (row[u] != 0xffffffffu) atomicAdd(yr + row[u], -sum[u]);
+                    sum[u] = 0.0f;
+                    row[u] = tgt[g][u];
+                }
+                sum[u] = fmaf(v[g][u], xj, sum[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kCoupleEach; ++u)
+            if (row[u] != 0xffffffffu) atomicAdd(yr + row[u], -sum[u]);
     }
 }
 
@@ -364,6 +428,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 4 : 3)
     __shared__ uint32_t s_item;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nb = (m + kRB - 1) / kRB;
+    pdl_release();  // the coupling after an upper sweep reads its entries meanwhile
     if (tid == 0) s_item = atomicAdd(ticket, 1u) + ticket_base;
     __syncthreads();
     if (s_item >= nb * count * chunks) return;
@@ -529,6 +594,7 @@ __global__ void __launch_bounds__(256, R == 1 ? 3 : 2)
     __shared__ uint32_t s_item;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nb = (m + kRB - 1) / kRB;
+    pdl_release();  // the coupling after an upper sweep reads its entries meanwhile
     if (tid == 0) s_item = atomicAdd(ticket, 1u) + ticket_base;
     __syncthreads();
     if (s_item >= nb * count * chunks) return;
@@ -666,13 +732,14 @@ static cudaError_t dense_sweep(const SolvePlanDev &S, const float *dval, float *
 static cudaError_t tail_coupling(const DevPattern &P, const SolvePlanDev &S, const float *val, float *y,
                                  uint32_t nrhs, bool rows, const SolveBatch &B, cudaStream_t st) {
     if (S.m == 0 || S.t == 0) return cudaSuccess;
-    const dim3 grid((S.m + 7) / 8, 1, B.count);
+    const uint32_t longest = std::max<uint32_t>(1u, rows ? S.tail_row_longest : S.tail_longest), each = 32 * kCoupleEach;
+    const dim3 grid((longest + each - 1) / each, (S.m + 8 * kCoupleCols - 1) / (8 * kCoupleCols),
+                    B.count * ((nrhs + kCoupleRhs - 1) / kCoupleRhs));
     const uint64_t ystride = uint64_t(nrhs) * P.n;
-    if (rows)
-        k_tail_coupling<true><<<grid, 256, 0, st>>>(P, S.t, S.m, S.tail_row_start, val, y, nrhs, B.vstride, ystride);
-    else
-        k_tail_coupling<false><<<grid, 256, 0, st>>>(P, S.t, S.m, S.tail_start, val, y, nrhs, B.vstride, ystride);
-    return cudaGetLastError();
+    return rows ? launch_chained(k_tail_coupling<true>, grid, dim3(256), 0, st, P, S.t, S.m, S.tail_row_start, val, y,
+                                 nrhs, B.vstride, ystride)
+                : launch_chained(k_tail_coupling<false>, grid, dim3(256), 0, st, P, S.t, S.m, S.tail_start, val, y, nrhs,
+                                 B.vstride, ystride);
 }
 
 cudaError_t solve_lower_unit(const DevPattern &P, const SolvePlanDev &S, const float *val,
