@@ -437,47 +437,93 @@ cudaError_t launch_dense_update(float *val, uint64_t stride, uint32_t count, con
 }
 
 // ------------------------------------------------ dense buffer gather/scatter --
-// A block per tail column (a warp per column leaves a chain of one load per 32
-// entries: 36 us at order 1,920, now 9); the gather first clears its column.
-// blockIdx.z selects the value set.
+// A block per tail column and kSets value sets: what bounds a column is the chain
+// from its bounds over its rows to its values, walked once for all of them, with
+// kRows rows of each in flight per thread (a warp per column and one value set:
+// 36 us at order 1,920, now 8; a block per column and value set: 84 and 94 us at
+// order 577 with 96 value sets, with four of them 54 and 56).  One value set alone
+// takes more rows instead (order 3,968: 33 us, 47 with the other split).  The
+// gather first clears an incomplete column.
+
+template <uint32_t kSets, uint32_t kRows>
 __global__ void __launch_bounds__(128) k_dense_gather(DevPattern P, const float *__restrict__ val_base,
-                                                      uint64_t stride, uint32_t t, uint32_t m,
+                                                      uint64_t stride, uint32_t count, uint32_t t, uint32_t m,
                                                       const uint32_t *__restrict__ tail_start, float *dbuf) {
-    const float *val = val_base + blockIdx.z * stride;
-    const uint32_t j = blockIdx.x;
-    float *col = dbuf + size_t(blockIdx.z) * m * m + size_t(j) * m;
+    const uint32_t j = blockIdx.x, z0 = blockIdx.z * kSets, nz = min(kSets, count - z0);
+    const float *val = val_base + z0 * stride;
+    const size_t zs = size_t(m) * m;
+    float *col = dbuf + z0 * zs + size_t(j) * m;
     const uint32_t p0 = tail_start[j], p1 = P.cptr[t + j + 1];
     if (p1 - p0 < m) {
-        for (uint32_t i = threadIdx.x; i < m; i += 128) col[i] = 0.0f;
+        for (uint32_t z = 0; z < nz; ++z)
+            for (uint32_t i = threadIdx.x; i < m; i += 128) col[z * zs + i] = 0.0f;
         __syncthreads();
     }
-#pragma unroll 8
-    for (uint32_t p = p0 + threadIdx.x; p < p1; p += 128) col[__ldg(P.ridx + p) - t] = __ldg(val + p);
+    for (uint32_t p = p0 + threadIdx.x; p < p1; p += 128 * kRows) {
+        uint32_t at[kRows];
+        float v[kSets][kRows];
+#pragma unroll
+        for (uint32_t k = 0; k < kRows; ++k)
+            if (p + 128 * k < p1) at[k] = __ldg(P.ridx + p + 128 * k) - t;
+#pragma unroll
+        for (uint32_t z = 0; z < kSets; ++z)
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k)
+                if (z < nz && p + 128 * k < p1) v[z][k] = __ldg(val + z * stride + p + 128 * k);
+#pragma unroll
+        for (uint32_t z = 0; z < kSets; ++z)
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k)
+                if (z < nz && p + 128 * k < p1) col[z * zs + at[k]] = v[z][k];
+    }
 }
 
-__global__ void __launch_bounds__(128) k_dense_scatter(DevPattern P, float *val_base, uint64_t stride,
+template <uint32_t kSets, uint32_t kRows>
+__global__ void __launch_bounds__(128) k_dense_scatter(DevPattern P, float *val_base, uint64_t stride, uint32_t count,
                                                        uint32_t t, uint32_t m,
                                                        const uint32_t *__restrict__ tail_start,
                                                        const float *__restrict__ dbuf) {
-    float *val = val_base + blockIdx.z * stride;
-    const uint32_t j = blockIdx.x;
-    const float *col = dbuf + size_t(blockIdx.z) * m * m + size_t(j) * m;
+    const uint32_t j = blockIdx.x, z0 = blockIdx.z * kSets, nz = min(kSets, count - z0);
+    float *val = val_base + z0 * stride;
+    const size_t zs = size_t(m) * m;
+    const float *col = dbuf + z0 * zs + size_t(j) * m;
     const uint32_t p1 = P.cptr[t + j + 1];
-#pragma unroll 8
-    for (uint32_t p = tail_start[j] + threadIdx.x; p < p1; p += 128) val[p] = __ldg(col + (__ldg(P.ridx + p) - t));
+    for (uint32_t p = tail_start[j] + threadIdx.x; p < p1; p += 128 * kRows) {
+        uint32_t at[kRows];
+        float v[kSets][kRows];
+#pragma unroll
+        for (uint32_t k = 0; k < kRows; ++k)
+            if (p + 128 * k < p1) at[k] = __ldg(P.ridx + p + 128 * k) - t;
+#pragma unroll
+        for (uint32_t z = 0; z < kSets; ++z)
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k)
+                if (z < nz && p + 128 * k < p1) v[z][k] = __ldg(col + z * zs + at[k]);
+#pragma unroll
+        for (uint32_t z = 0; z < kSets; ++z)
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k)
+                if (z < nz && p + 128 * k < p1) val[z * stride + p + 128 * k] = v[z][k];
+    }
 }
 
 cudaError_t launch_dense_gather(const DevPattern &P, const float *val, uint64_t stride, uint32_t count,
                                 uint32_t t, uint32_t m, const uint32_t *tail_start, float *dbuf,
                                 cudaStream_t st) {
-    k_dense_gather<<<dim3(m, 1, count), 128, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
+    if (count == 1)
+        k_dense_gather<1, 8><<<m, 128, 0, st>>>(P, val, stride, count, t, m, tail_start, dbuf);
+    else
+        k_dense_gather<4, 4><<<dim3(m, 1, (count + 3) / 4), 128, 0, st>>>(P, val, stride, count, t, m, tail_start, dbuf);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dense_scatter(const DevPattern &P, float *val, uint64_t stride, uint32_t count,
                                  uint32_t t, uint32_t m, const uint32_t *tail_start, const float *dbuf,
                                  cudaStream_t st) {
-    k_dense_scatter<<<dim3(m, 1, count), 128, 0, st>>>(P, val, stride, t, m, tail_start, dbuf);
+    if (count == 1)
+        k_dense_scatter<1, 8><<<m, 128, 0, st>>>(P, val, stride, count, t, m, tail_start, dbuf);
+    else
+        k_dense_scatter<4, 4><<<dim3(m, 1, (count + 3) / 4), 128, 0, st>>>(P, val, stride, count, t, m, tail_start, dbuf);
     return cudaGetLastError();
 }
 
