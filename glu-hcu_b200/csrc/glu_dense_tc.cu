@@ -24,7 +24,8 @@
 // product), and the tile's C is read and written once.
 
 // Data flow per update:
-//   1. k_dense_pack, after each panel: the panel's L21 rows and U12 columns
+//   1. k_dense_pack, after each panel (for many value sets k_dense_panel_rows,
+//      with the panel): the panel's L21 rows and U12 columns
 //      split into their three BF16 parts, written K-major as rows of 768
 //      BF16 values (slots 0..255 part 0, 256..511 part 1, 512..767 part 2;
 //      panel j of a group fills slots 64 j .. 64 j + 63 of each part) -- the

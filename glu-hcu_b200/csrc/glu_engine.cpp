@@ -363,12 +363,16 @@ void find_full_tail(const SymbolicData &s, uint32_t min_m, uint32_t &t, uint32_t
 }
 
 // Cost model of the split point t: the columns [t, n) are factored as a dense
-// block, the columns in front of t level by level.  Dense: 2/3 m^3 flops at
-// kDenseRate plus kPanelLatency per panel step.  Sparse: the update work of
-// the columns < t at kSparseRate plus kLevelLatency per level that still has
-// an active column < t.  Returns the t of least estimated time with
-// m <= max_m (t = n: no dense tail).
-constexpr double kDenseRate = 30e12, kDenseRateTc = 120e12, kPanelLatency = 20e-6;
+// block, the columns in front of t level by level.  Dense: dense_seconds of the
+// handle's value sets (with tune.dense_rate set, one set's 2/3 m^3 flops at that
+// rate plus kPanelLatency per panel step).  Sparse: the update work of the columns <
+// t at kSparseRate plus kLevelLatency per level that still has an active
+// column < t.  Returns the t of least estimated time with m <= max_m (t = n: no
+// dense tail).  The constants are the best of a few, with the panels' rates and
+// one value set's work / these: n = 500 step 174 / 158 us, 96 value sets of n =
+// 1,500 1,645 / 1,576 us, n = 4,960 refactorization 586 / 575 us, grids of 63,001 and
+// 490,000 equal; with one value set's work alone the 96 sets take 1,730 us.
+constexpr double kPanelLatency = 20e-6;
 // Default width from which trailing blocks factor with panel look-ahead.
 constexpr uint32_t kLookaheadMin = 3072;
 // Default width from which trailing blocks update on the tensor cores.
@@ -377,7 +381,7 @@ constexpr uint32_t kDenseTcMin = 1024;
 // m x m dense block), in scattered supernode-update entries per entry of the
 // block.
 constexpr double kCoupleGroupCost = 0.25;
-constexpr double kSparseRate = 0.2e12, kLevelLatency = 8e-6;
+constexpr double kSparseRate = 0.1e12, kLevelLatency = 8e-6;
 
 // Runs a launch sequence on st: launched one by one the first time its key is
 // seen, captured into a graph the second, and from then on launched as that
@@ -436,10 +440,7 @@ Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStr
 }
 uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 
-// Whether the trailing blocks of order m of `count` value sets are factored by
-// the dataflow kernel (glu_dense_flow.cu) or by panels and updates.  With
-// widths set for look-ahead or tensor-core updates, the blocks below them.
-// With the default widths, whichever a model of both takes less time for:
+// Seconds of factoring the trailing blocks of order m of `count` value sets:
 //   dataflow  12.7 us per 64 columns (the diagonal chain) against the products
 //             at 36 TFLOP/s, the longer and three tenths of the shorter;
 //   panels    55 us per 64 columns plus the products at 130 TFLOP/s on the
@@ -447,18 +448,28 @@ uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 // Measured, dataflow / panels: order 1,920 0.40 / 1.51 ms, eight of them 1.18 /
 // 2.18, order 3,968 1.32 / 4.73, three of them 3.32 / 5.75, order 5,000 2.35 /
 // 6.27, 96 of order 576 0.60 / 0.99; twelve of order 9,360 take the panels
-// about 58 ms, the dataflow would take 180.
+// about 55 ms, the dataflow would take 180.
+struct DenseSeconds {
+    double flow, panels;
+};
+DenseSeconds dense_seconds(double m, uint32_t count) {
+    const double steps = std::ceil(m / kFlowTile), work = double(count) * (2.0 / 3.0) * m * m * m;
+    const double chain = steps * 12.7e-6, products = work / 36e12;
+    return {std::max(chain, products) + 0.3 * std::min(chain, products), steps * 55e-6 + work / 130e12};
+}
+// Whether they are factored by the dataflow kernel (glu_dense_flow.cu) or by
+// panels and updates: whichever takes less time; with widths set for look-ahead or
+// tensor-core updates, the blocks below them by the dataflow.
 bool dense_flow(const glu_tuning &tu, uint32_t m, uint32_t count) {
     if (m == 0) return false;
     if (tu.dense_lookahead != kLookaheadMin || tu.dense_tc_min != kDenseTcMin)
         return (tu.dense_lookahead == 0 || m < tu.dense_lookahead) && (tu.dense_tc_min == 0 || m < tu.dense_tc_min);
-    const double steps = std::ceil(double(m) / kFlowTile), work = double(count) * (2.0 / 3.0) * m * m * m;
-    const double chain = steps * 12.7e-6, products = work / 36e12;
-    return std::max(chain, products) + 0.3 * std::min(chain, products) <= steps * 55e-6 + work / 130e12;
+    const DenseSeconds d = dense_seconds(m, count);
+    return d.flow <= d.panels;
 }
 
 uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_ptr,
-                      const std::vector<int32_t> &level_idx, uint32_t max_m, const glu_tuning &tu) {
+                      const std::vector<int32_t> &level_idx, uint32_t max_m, const glu_tuning &tu, uint32_t batch) {
     const uint32_t n = s.n;
     // sparse work of column k and the first column of each level
     std::vector<double> pre(n + 1, 0.0);
@@ -486,11 +497,15 @@ uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_p
     for (int64_t tt = n; tt >= lo; tt -= 16) {
         const uint32_t t = uint32_t(tt);
         double m = double(n - t);
-        const double rate = tu.dense_rate ? 1e9 * tu.dense_rate
-                                          : (tu.dense_tc_min && m >= tu.dense_tc_min ? kDenseRateTc : kDenseRate);
-        double dense = m > 0 ? (2.0 / 3.0) * m * m * m / rate + std::ceil(m / kDenseNB) * kPanelLatency : 0;
+        double dense = 0;
+        if (tu.dense_rate && m > 0) {
+            dense = (2.0 / 3.0) * m * m * m / (1e9 * tu.dense_rate) + std::ceil(m / kDenseNB) * kPanelLatency;
+        } else if (m > 0) {
+            const DenseSeconds d = dense_seconds(m, batch);
+            dense = std::min(d.flow, d.panels);
+        }
         double nlev = double(std::lower_bound(lev_first.begin(), lev_first.end(), t) - lev_first.begin());
-        double sparse = pre[t] / kSparseRate + nlev * kLevelLatency;
+        double sparse = (tu.dense_rate ? 1u : batch) * pre[t] / kSparseRate + nlev * kLevelLatency;
         if (dense + sparse < best) {
             best = dense + sparse;
             best_t = t;
@@ -1017,7 +1032,7 @@ Status build_plan(glu_handle_s *h) {
             if (cap < max_m) max_m = uint32_t(cap);
         }
     }
-    uint32_t t_opt = choose_split(s, h->level_ptr, h->level_idx, std::max(max_m, m_full), h->tune);
+    uint32_t t_opt = choose_split(s, h->level_ptr, h->level_idx, std::max(max_m, m_full), h->tune, h->batch);
     h->dense_buffer = false;
     if (t_opt >= t_full) {
         h->t = t_opt;  // any trailing block of a fully dense block is fully dense
