@@ -364,15 +364,19 @@ void find_full_tail(const SymbolicData &s, uint32_t min_m, uint32_t &t, uint32_t
 
 // Cost model of the split point t: the columns [t, n) are factored as a dense
 // block, the columns in front of t level by level.  Dense: dense_seconds of the
-// handle's value sets (with tune.dense_rate set, one set's 2/3 m^3 flops at that
-// rate plus kPanelLatency per panel step).  Sparse: the update work of the columns <
-// t at kSparseRate plus kLevelLatency per level that still has an active
-// column < t.  Returns the t of least estimated time with m <= max_m (t = n: no
-// dense tail).  The constants are the best of a few, with the panels' rates and
-// one value set's work / these: n = 500 step 174 / 158 us, 96 value sets of n =
-// 1,500 1,645 / 1,576 us, n = 4,960 refactorization 586 / 575 us, grids of 63,001 and
-// 490,000 equal; with one value set's work alone the 96 sets take 1,730 us.
-constexpr double kPanelLatency = 20e-6;
+// handle's value sets.  Sparse: their update work of the columns < t at
+// kSparseRate plus kLevelLatency per level that still has an active column < t.
+// Returns the t of least estimated time with m <= max_m (t = n: no dense tail).
+// The constants are the best of a few, against one set's work at the rates below:
+// n = 300 step 158 / 174 us, 96 value sets of n = 1,500 1,576 / 1,645 us, n = 4,960
+// refactorization 575 / 586 us, grids of 90,000 and 490,000 equal; with the
+// panels' time but one set's work the 96 sets take 1,730 us.
+// With a rate (tune.dense_rate) or widths of the dense paths set: one set's 2/3 m^3
+// flops at that rate, or by whether the block updates on the tensor cores at
+// kDenseRate or kDenseRateTc, plus kPanelLatency per panel step, and its
+// sparse work at kTunedSparseRate.
+constexpr double kSparseRate = 0.1e12, kLevelLatency = 8e-6;
+constexpr double kDenseRate = 30e12, kDenseRateTc = 120e12, kPanelLatency = 20e-6, kTunedSparseRate = 0.2e12;
 // Default width from which trailing blocks factor with panel look-ahead.
 constexpr uint32_t kLookaheadMin = 3072;
 // Default width from which trailing blocks update on the tensor cores.
@@ -381,7 +385,6 @@ constexpr uint32_t kDenseTcMin = 1024;
 // m x m dense block), in scattered supernode-update entries per entry of the
 // block.
 constexpr double kCoupleGroupCost = 0.25;
-constexpr double kSparseRate = 0.1e12, kLevelLatency = 8e-6;
 
 // Runs a launch sequence on st: launched one by one the first time its key is
 // seen, captured into a graph the second, and from then on launched as that
@@ -457,12 +460,16 @@ DenseSeconds dense_seconds(double m, uint32_t count) {
     const double chain = steps * 12.7e-6, products = work / 36e12;
     return {std::max(chain, products) + 0.3 * std::min(chain, products), steps * 55e-6 + work / 130e12};
 }
+bool default_widths(const glu_tuning &tu) {
+    return tu.dense_lookahead == kLookaheadMin && tu.dense_tc_min == kDenseTcMin;
+}
+
 // Whether they are factored by the dataflow kernel (glu_dense_flow.cu) or by
 // panels and updates: whichever takes less time; with widths set for look-ahead or
 // tensor-core updates, the blocks below them by the dataflow.
 bool dense_flow(const glu_tuning &tu, uint32_t m, uint32_t count) {
     if (m == 0) return false;
-    if (tu.dense_lookahead != kLookaheadMin || tu.dense_tc_min != kDenseTcMin)
+    if (!default_widths(tu))
         return (tu.dense_lookahead == 0 || m < tu.dense_lookahead) && (tu.dense_tc_min == 0 || m < tu.dense_tc_min);
     const DenseSeconds d = dense_seconds(m, count);
     return d.flow <= d.panels;
@@ -493,19 +500,23 @@ uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_p
     std::sort(lev_first.begin(), lev_first.end());
     double best = 1e300;
     uint32_t best_t = n;
+    const bool modelled = default_widths(tu) && tu.dense_rate == 0;
     const int64_t lo = max_m >= n ? 0 : int64_t(n) - max_m;
     for (int64_t tt = n; tt >= lo; tt -= 16) {
         const uint32_t t = uint32_t(tt);
         double m = double(n - t);
-        double dense = 0;
-        if (tu.dense_rate && m > 0) {
-            dense = (2.0 / 3.0) * m * m * m / (1e9 * tu.dense_rate) + std::ceil(m / kDenseNB) * kPanelLatency;
-        } else if (m > 0) {
+        const double nlev = double(std::lower_bound(lev_first.begin(), lev_first.end(), t) - lev_first.begin());
+        double dense = 0, sparse = nlev * kLevelLatency;
+        if (modelled) {
             const DenseSeconds d = dense_seconds(m, batch);
             dense = std::min(d.flow, d.panels);
+            sparse += batch * pre[t] / kSparseRate;
+        } else {
+            const double rate = tu.dense_rate ? 1e9 * tu.dense_rate
+                                              : (tu.dense_tc_min && m >= tu.dense_tc_min ? kDenseRateTc : kDenseRate);
+            dense = (2.0 / 3.0) * m * m * m / rate + std::ceil(m / kDenseNB) * kPanelLatency;
+            sparse += pre[t] / kTunedSparseRate;
         }
-        double nlev = double(std::lower_bound(lev_first.begin(), lev_first.end(), t) - lev_first.begin());
-        double sparse = (tu.dense_rate ? 1u : batch) * pre[t] / kSparseRate + nlev * kLevelLatency;
         if (dense + sparse < best) {
             best = dense + sparse;
             best_t = t;
