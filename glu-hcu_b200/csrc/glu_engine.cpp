@@ -1852,9 +1852,13 @@ Status factor_buffers(glu_handle_s *h, uint32_t count, bool *use_flow) {
     }
     if (h->m)
         GLU_CUDA(h->d_dinv.ensure(sizeof(float) * dinv_per_set(h) * h->batch), "allocate diagonal-block inverses");
+    // One buffer for all value sets, or none until the plan changes: a set
+    // factored without it has no inverses, so it must not appear later.
     if (h->use_sn && h->nwide &&
-        h->d_sn_inv.ensure(sizeof(float) * uint64_t(h->nwide) * kSnInvFloats * h->batch) != cudaSuccess)
-        cudaGetLastError();  // (the sweeps then solve those blocks column by column)
+        h->d_sn_inv.ensure(sizeof(float) * uint64_t(h->nwide) * kSnInvFloats * h->batch) != cudaSuccess) {
+        cudaGetLastError();
+        h->nwide = 0;  // the sweeps solve those blocks column by column
+    }
     return GLU_OK;
 }
 
