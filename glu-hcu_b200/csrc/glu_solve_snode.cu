@@ -193,20 +193,35 @@ __device__ __forceinline__ void sn_sweep_u_small(const DevPattern &P, const SnSw
     }
     const float piv = lane < w ? __ldg(val + dl) : 1.0f;
     // reciprocals before the chain, unless a pivot is too large or too small
+    // (or, below, an unknown turns out not to be finite)
     const float mag = fabsf(piv), rec = lu_reciprocal(piv);
     const bool quick = __all_sync(kFull, mag > 1e-30f && mag < 1e30f);
     pdl_wait();  // the previous level's x
     for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
-        float v = lane < w ? __ldcg(yq + s + lane) : 0.0f;
+        const float v0 = lane < w ? __ldcg(yq + s + lane) : 0.0f;
+        float v = v0;
+        bool solved = false;
+        if (quick) {
 #pragma unroll
-        for (int cc = SW - 1; cc >= 0; --cc) {
-            if (uint32_t(cc) >= w) continue;
-            // every lane divides its own value, so that the step is one shuffle long
-            const float d = quick ? lu_quotient(v, piv, rec) : v / piv;
-            const float xc = __shfl_sync(kFull, d, cc);
-            if (lane == uint32_t(cc)) v = xc;
-            if (lane < uint32_t(cc)) v = __fsub_rn(v, __fmul_rn(urow[cc], xc));
+            for (int cc = SW - 1; cc >= 0; --cc) {
+                if (uint32_t(cc) >= w) continue;
+                // every lane divides its own value, so that the step is one shuffle long
+                const float xc = __shfl_sync(kFull, lu_quotient(v, piv, rec), cc);
+                if (lane == uint32_t(cc)) v = xc;
+                if (lane < uint32_t(cc)) v = __fsub_rn(v, __fmul_rn(urow[cc], xc));
+            }
+            solved = __all_sync(kFull, isfinite(v));
+        }
+        if (!solved) {
+            v = v0;
+#pragma unroll
+            for (int cc = SW - 1; cc >= 0; --cc) {
+                if (uint32_t(cc) >= w) continue;
+                const float xc = __shfl_sync(kFull, v / piv, cc);
+                if (lane == uint32_t(cc)) v = xc;
+                if (lane < uint32_t(cc)) v = __fsub_rn(v, __fmul_rn(urow[cc], xc));
+            }
         }
         if (lane < w) xo[size_t(q) * n + s + lane] = v;
         const float xe = __shfl_sync(kFull, v, col);
@@ -595,16 +610,25 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
         } else {
             if (tid < 32) {
                 const uint32_t k0 = tid, k1 = tid + 32;
-                float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
-                float v1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
-                for (uint32_t cc = w; cc-- > 0;) {
-                    // every lane divides its own value, so that the step is one shuffle long
-                    const float v = cc < 32 ? v0 : v1, p = cc < 32 ? pv0 : pv1, rc = cc < 32 ? rc0 : rc1;
-                    const float xc = __shfl_sync(0xffffffffu, quick ? lu_quotient(v, p, rc) : v / p, cc & 31);
+                const float b0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f, b1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
+                float v0 = b0, v1 = b1;
+                auto step = [&](uint32_t cc, float quotient) {
+                    const float xc = __shfl_sync(kFull, quotient, cc & 31);
                     if (k0 == cc) v0 = xc;
                     if (k1 == cc) v1 = xc;
                     if (k0 < cc) v0 = __fsub_rn(v0, __fmul_rn(sT[cc * kLD + k0], xc));
                     if (k1 < cc) v1 = __fsub_rn(v1, __fmul_rn(sT[cc * kLD + k1], xc));
+                };
+                bool solved = false;
+                if (quick) {
+                    // every lane divides its own value, so that the step is one shuffle long
+                    for (uint32_t cc = w; cc-- > 0;)
+                        step(cc, cc < 32 ? lu_quotient(v0, pv0, rc0) : lu_quotient(v1, pv1, rc1));
+                    solved = __all_sync(kFull, isfinite(v0) && isfinite(v1));
+                }
+                if (!solved) {
+                    v0 = b0, v1 = b1;
+                    for (uint32_t cc = w; cc-- > 0;) step(cc, (cc < 32 ? v0 : v1) / sT[cc * kLD + cc]);
                 }
                 if (k0 < w) xs[k0] = v0;
                 if (k1 < w) xs[k1] = v1;

@@ -35,10 +35,17 @@ constexpr int kLuChunk = 8;         // columns per step of the block LU
 
 // a / p from r, p's reciprocal to about one unit in the last place: the
 // quotient's estimate corrected by its remainder (Markstein, IBM J. Res. Dev.
-// 34, 1990).
+// 34, 1990).  For finite quotients: an infinite one, which the division gives
+// as such, comes out as NaN here (its remainder is infinite too), so whoever
+// uses it looks for values that are not finite and divides instead, or takes
+// lu_quotient_wide, which is infinite where the estimate is.
 __device__ __forceinline__ float lu_quotient(float a, float p, float r) {
     const float q = a * r;
     return fmaf(fmaf(-q, p, a), r, q);
+}
+__device__ __forceinline__ float lu_quotient_wide(float a, float p, float r) {
+    const float q = a * r;
+    return isfinite(q) ? fmaf(fmaf(-q, p, a), r, q) : q;
 }
 __device__ __forceinline__ float lu_reciprocal(float p) {
     float r;
@@ -53,6 +60,9 @@ __device__ __forceinline__ float lu_reciprocal(float p) {
 // multiply-add; each lane carries two of the rows below along.
 // kDivide: quotients by division; otherwise by lu_quotient, and nothing is
 // stored and false returned when a pivot is too large or too small for it.
+// (Entries of the diagonal block that are not finite make a pivot of it so; the
+// rows below have none and take lu_quotient_wide, off the chain of pivots. A
+// vote on them in front of the stores took a level of the grids 0.7 us longer.)
 template <bool kDivide>
 __device__ __forceinline__ bool lu_panel_try(float *S, uint32_t base, uint32_t w, bool last_l, float pert,
                                              uint32_t lane) {
@@ -83,8 +93,8 @@ __device__ __forceinline__ bool lu_panel_try(float *S, uint32_t base, uint32_t w
 #pragma unroll
         for (int i = 0; i < N; ++i)
             if (i > c) d[i][c] = kDivide ? d[i][c] / p : lu_quotient(d[i][c], p, r);
-        a0[c] = kDivide ? a0[c] / p : lu_quotient(a0[c], p, r);
-        a1[c] = kDivide ? a1[c] / p : lu_quotient(a1[c], p, r);
+        a0[c] = kDivide ? a0[c] / p : lu_quotient_wide(a0[c], p, r);
+        a1[c] = kDivide ? a1[c] / p : lu_quotient_wide(a1[c], p, r);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             if (j <= c) continue;
