@@ -307,6 +307,14 @@ __device__ __forceinline__ void wide_solve(const float (&iv)[16], const float *v
     if (tid < kSnMaxWidth) xs[tid] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
     __syncthreads();
 }
+// Whether that x is finite, the same to all warps; else it is solved for by
+// substitution: an inverse can overflow where that does not (a block graded by
+// its rows' and columns' scales), and an infinite v makes every unknown NaN.
+// (Asked beside the products with x, not in front of them: a vote in the barrier
+// took a solve of a 251 x 251 grid from 291 to 297 us.)
+__device__ __forceinline__ bool wide_finite(const float *xs, uint32_t tid) {
+    return __all_sync(kFull, isfinite(xs[tid & 31]) && isfinite(xs[(tid & 31) + 32]));
+}
 __device__ __forceinline__ void load_inverse(float (&iv)[16], const float *__restrict__ inv, uint32_t tid) {
     inv += (tid >> 6) * 16 * kSnMaxWidth + (tid & 63);
 #pragma unroll
@@ -377,12 +385,8 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     pdl_wait();  // the previous level's x
     for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
-        if (wide != UINT32_MAX) {
-            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
-            __syncthreads();
-            wide_solve(iv, vs, part, xs, tid);
-            if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
-        } else {
+        // the chain over the columns, by one warp, from the block in sT
+        auto substitute = [&] {
             if (tid < 32) {
                 const uint32_t k0 = tid, k1 = tid + 32;
                 float v0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f;
@@ -394,26 +398,45 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
                 }
                 if (k0 < w) xs[k0] = v0;
                 if (k1 < w) xs[k1] = v1;
-                if (t == 0) {
-                    if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
-                    if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
-                }
             }
             __syncthreads();
+        };
+        if (wide != UINT32_MAX) {
+            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
+            __syncthreads();
+            wide_solve(iv, vs, part, xs, tid);
+        } else {
+            substitute();
         }
         // four sums: one chain of 64 multiply-adds would take as long as the solve
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        const float4 *x4 = reinterpret_cast<const float4 *>(xs);
+        auto product = [&] {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            const float4 *x4 = reinterpret_cast<const float4 *>(xs);
 #pragma unroll
-        for (int c = 0; c < int(kSnMaxWidth); c += 4) {
-            if (uint32_t(c) >= w) break;
-            const float4 x = x4[c / 4];
-            acc[0] = fmaf(lr[c], x.x, acc[0]);
-            acc[1] = fmaf(lr[c + 1], x.y, acc[1]);
-            acc[2] = fmaf(lr[c + 2], x.z, acc[2]);
-            acc[3] = fmaf(lr[c + 3], x.w, acc[3]);
+            for (int c = 0; c < int(kSnMaxWidth); c += 4) {
+                if (uint32_t(c) >= w) break;
+                const float4 x = x4[c / 4];
+                acc[0] = fmaf(lr[c], x.x, acc[0]);
+                acc[1] = fmaf(lr[c + 1], x.y, acc[1]);
+                acc[2] = fmaf(lr[c + 2], x.z, acc[2]);
+                acc[3] = fmaf(lr[c + 3], x.w, acc[3]);
+            }
+            return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        };
+        float sum = product();
+        if (wide != UINT32_MAX && !wide_finite(xs, tid)) {
+            __syncthreads();  // all warps have read xs
+#pragma unroll 1
+            for (uint32_t e = tid; e < w * kSnMaxWidth; e += 256) {
+                const uint32_t c = e >> 6, k = e & 63;
+                if (k < w && k > c) sT[c * kLD + k] = __ldg(val + sB[c] + (k - c));
+            }
+            if (tid < kSnMaxWidth) xs[tid] = 0.0f;
+            __syncthreads();
+            substitute();
+            sum = product();
         }
-        const float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
         if (r < m && sum != 0.0f) atomicAdd(yq + target, -sum);
         if (q + 1 < Q.q1) __syncthreads();
     }
@@ -598,16 +621,13 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
     }
     const float rc0 = lu_reciprocal(pv0), rc1 = lu_reciprocal(pv1);
     const float g0 = fabsf(pv0), g1 = fabsf(pv1);
-    const bool quick = __all_sync(kFull, g0 > 1e-30f && g0 < 1e30f && g1 > 1e-30f && g1 < 1e30f);
+    const bool quick =
+        __all_sync(kFull, wide == UINT32_MAX && g0 > 1e-30f && g0 < 1e30f && g1 > 1e-30f && g1 < 1e30f);
     pdl_wait();  // the previous level's x
     for (uint32_t q = Q.q0; q < Q.q1; ++q) {
         float *yq = y + size_t(q) * n;
-        if (wide != UINT32_MAX) {
-            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
-            __syncthreads();
-            wide_solve(iv, vs, part, xs, tid);
-            if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
-        } else {
+        // the chain over the columns, by one warp, from the block in sT
+        auto substitute = [&] {
             if (tid < 32) {
                 const uint32_t k0 = tid, k1 = tid + 32;
                 const float b0 = k0 < w ? __ldcg(yq + s + k0) : 0.0f, b1 = k1 < w ? __ldcg(yq + s + k1) : 0.0f;
@@ -632,13 +652,27 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
                 }
                 if (k0 < w) xs[k0] = v0;
                 if (k1 < w) xs[k1] = v1;
-                if (t == 0) {
-                    if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
-                    if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
-                }
             }
             __syncthreads();
+        };
+        if (wide != UINT32_MAX) {
+            if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
+            __syncthreads();
+            wide_solve(iv, vs, part, xs, tid);
+            if (!wide_finite(xs, tid)) {
+                __syncthreads();  // all warps have read xs
+#pragma unroll 1
+                for (uint32_t e = tid; e < w * kSnMaxWidth; e += 256) {
+                    const uint32_t c = e >> 6, k = e & 63;
+                    if (k <= c) sT[c * kLD + k] = __ldg(val + sB[c] - (c - k));
+                }
+                __syncthreads();
+                substitute();
+            }
+        } else {
+            substitute();
         }
+        if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
             if (ecol[u] >= kSnMaxWidth) continue;
