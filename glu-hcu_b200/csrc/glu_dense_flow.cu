@@ -24,10 +24,17 @@
 // left), 16 columns of a solved tile while it solves the next; the solve and
 // the last product in front of a diagonal tile start on them.  A publisher warp
 // releases the pieces (their count is the tile's flag), so no computing warp
-// waits for its stores; a producer warp waits (bounded) for the flags and
-// brings the operands in by bulk copies, two stages ahead of the products.  The
+// waits for its stores; a producer warp waits for the flags and brings the
+// operands in by bulk copies, two stages ahead of the products.  The
 // workspace is the block's size again; the rule that chooses this kernel is
 // in glu_engine.cpp (dense_flow).
+//
+// The waits for the flags are the only ones on another block.  They are bounded
+// (the handle's wait limit, at least kFlowPolls polls); one that runs out sets
+// DEV_TIMEOUT, and from then on its block's stages pass through without a
+// copy: every barrier of the block still gets the arrivals that it expects, the
+// computing warps run to their end with whatever the stages hold, the block's
+// pieces are released, and so the launch drains.
 //
 // A column step of the chain takes 12.5 us (order 1,920, one block per SM), 7 of
 // them the LU; 16.5 us with whole tiles handed on (LU 7.0, publishing it 1.5,
@@ -42,6 +49,8 @@
 //
 // The reference's counterpart is the per-column work of RL_onecol_factorizeCurrentCol
 // and RL_onecol_updateSubmat (src/numeric.cu:205-319).
+#include <algorithm>
+
 #include "glu_common.cuh"
 #include "glu_kernels.h"
 #include "glu_tri.cuh"
@@ -77,8 +86,11 @@ __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; ++i) {
+// For another warp of the block or a copy of the block's own: both end by
+// themselves, so the bound is a fixed one that a sound block never meets.
+__device__ __forceinline__ void bar_wait(uint64_t *bar, uint32_t parity, uint32_t *status) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpinLimit; ++i) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -87,9 +99,9 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, uint32_
             : "=r"(ok)
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
-        if (ok) return true;
+        if (ok) return;
     }
-    return false;
+    atomicOr(status, DEV_TIMEOUT);
 }
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -101,15 +113,24 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
 // by ordinary stores, the copy reads through the asynchronous proxy.
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-// Bounded wait until `pieces` pieces of a tile are ready (one thread).
-__device__ __forceinline__ void wait_tile(const uint32_t *flag, uint32_t pieces, uint32_t *status, uint32_t limit) {
+// A tile waits here while blocks in front of it still factor: about a step of
+// the chain (12.5 us), a few milliseconds in the largest blocks.  A wait limit
+// that suits the solves' waits (a link of theirs takes a microsecond) must not
+// end that, so the limit counts from this many polls (about 0.1 s) on.
+constexpr uint32_t kFlowPolls = 1u << 17;
+
+// Bounded wait until `pieces` pieces of a tile are ready (one thread); false if
+// it ran out, or another wait did.
+__device__ __forceinline__ bool wait_tile(const uint32_t *flag, uint32_t pieces, uint32_t *status, uint32_t limit) {
+#pragma unroll 1
     for (uint32_t spins = 0; ld_acquire_gpu(flag) < pieces; ++spins) {
         if (spins >= limit) {
             atomicOr(status, DEV_TIMEOUT);
-            return;
+            return false;
         }
-        if ((spins & 255u) == 255u && (ld_acquire_gpu(status) & DEV_TIMEOUT)) return;
+        if ((spins & 255u) == 255u && (ld_acquire_gpu(status) & DEV_TIMEOUT)) return false;
     }
+    return true;
 }
 
 // x M = a for the 64 vectors of W ([k][vector], leading dimension kLdW) by 256
@@ -179,14 +200,14 @@ __device__ __forceinline__ FlowTile flow_tile(uint32_t idx, uint32_t nt) {
 __global__ void __launch_bounds__(kThreads, 2)
     k_dense_flow(float *val_base, uint64_t stride, const uint32_t *__restrict__ doff, uint32_t m, uint32_t nt,
                  uint32_t count, const float *pert_z, float *work, uint64_t work_stride, uint32_t *ctl,
-                 uint32_t *status, uint32_t spin_limit) {
+                 uint32_t *status, uint32_t spin_limit, uint32_t ticket_base) {
     extern __shared__ __align__(128) unsigned char flow_smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], last_full[kPieces], diag_full[kPieces];
     __shared__ __align__(8) uint64_t written[kPieces];  // one phase each: a piece may be written before the last is released
     __shared__ uint32_t s_item;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        s_item = atomicAdd(ctl, 1u);
+        s_item = atomicAdd(ctl, 1u) + ticket_base;
         const uint32_t item = s_item;
         const FlowTile t0 = item < nt * nt * count ? flow_tile(item / count, nt) : FlowTile{0, 0, 0};
         for (int s = 0; s < kStages; ++s) {
@@ -210,51 +231,60 @@ __global__ void __launch_bounds__(kThreads, 2)
     float *diags = tiles + size_t(nt) * nt * kT * kT;            // [k][0: U rows, 1: L columns]
     if (warp == kTriThreads / 32) {  // producer: operands as they become ready
         if (lane == 0) {
+            bool ok = true;  // until a wait for a tile gives up: then arrivals without copies
             for (uint32_t s = 0; s < t.k; ++s) {
                 const uint32_t st = s % kStages;
                 unsigned char *dst = flow_smem + st * kStageBytes;
                 const float *srcL = tiles + (size_t(t.i) * nt + s) * kT * kT, *srcU = tiles + (size_t(s) * nt + t.j) * kT * kT;
                 const uint32_t *fL = ready + size_t(t.i) * nt + s, *fU = ready + size_t(s) * nt + t.j;
-                if (s >= uint32_t(kStages) && !bar_wait(&empty[st], (s / kStages - 1) & 1, spin_limit))
-                    atomicOr(status, DEV_TIMEOUT);
+                if (s >= uint32_t(kStages)) bar_wait(&empty[st], (s / kStages - 1) & 1, status);
                 if (s + 1 < t.k) {
-                    wait_tile(fL, kPieces, status, spin_limit);
-                    wait_tile(fU, kPieces, status, spin_limit);
-                    proxy_fence();
-                    bar_expect(&full[st], 2 * kTileBytes);
-                    bulk_load(dst, srcL, kTileBytes, &full[st]);
-                    bulk_load(dst + kTileBytes, srcU, kTileBytes, &full[st]);
+                    ok = ok && wait_tile(fL, kPieces, status, spin_limit) && wait_tile(fU, kPieces, status, spin_limit);
+                    if (ok) {
+                        proxy_fence();
+                        bar_expect(&full[st], 2 * kTileBytes);
+                        bulk_load(dst, srcL, kTileBytes, &full[st]);
+                        bulk_load(dst + kTileBytes, srcU, kTileBytes, &full[st]);
+                    } else {
+                        bar_arrive(&full[st]);
+                    }
                 } else {  // the last step's operands may be in the making: piece by piece
                     for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
-                        wait_tile(fL, p + 1, status, spin_limit);
-                        wait_tile(fU, p + 1, status, spin_limit);
-                        proxy_fence();
-                        bar_expect(&last_full[p], 2 * kPieceBytes);
-                        bulk_load(dst + p * kPieceBytes, srcL + p * (kPieceBytes / 4), kPieceBytes, &last_full[p]);
-                        bulk_load(dst + kTileBytes + p * kPieceBytes, srcU + p * (kPieceBytes / 4), kPieceBytes,
-                                  &last_full[p]);
+                        ok = ok && wait_tile(fL, p + 1, status, spin_limit) && wait_tile(fU, p + 1, status, spin_limit);
+                        if (ok) {
+                            proxy_fence();
+                            bar_expect(&last_full[p], 2 * kPieceBytes);
+                            bulk_load(dst + p * kPieceBytes, srcL + p * (kPieceBytes / 4), kPieceBytes, &last_full[p]);
+                            bulk_load(dst + kTileBytes + p * kPieceBytes, srcU + p * (kPieceBytes / 4), kPieceBytes,
+                                      &last_full[p]);
+                        } else {
+                            bar_arrive(&last_full[p]);
+                        }
                     }
                 }
             }
             if (t.i != t.j) {
                 const uint32_t st = t.k % kStages;
-                if (t.k >= uint32_t(kStages) && !bar_wait(&empty[st], (t.k / kStages - 1) & 1, spin_limit))
-                    atomicOr(status, DEV_TIMEOUT);
+                if (t.k >= uint32_t(kStages)) bar_wait(&empty[st], (t.k / kStages - 1) & 1, status);
                 const float *src = diags + (size_t(t.k) * 2 + (t.i > t.j ? 0 : 1)) * kFlowDiagFloats;
                 for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
-                    wait_tile(ready + size_t(t.k) * nt + t.k, p + 1, status, spin_limit);
-                    proxy_fence();
-                    bar_expect(&diag_full[p], kDiagPieceBytes);
-                    bulk_load(flow_smem + st * kStageBytes + p * kDiagPieceBytes, src + p * (kDiagPieceBytes / 4),
-                              kDiagPieceBytes, &diag_full[p]);
+                    ok = ok && wait_tile(ready + size_t(t.k) * nt + t.k, p + 1, status, spin_limit);
+                    if (ok) {
+                        proxy_fence();
+                        bar_expect(&diag_full[p], kDiagPieceBytes);
+                        bulk_load(flow_smem + st * kStageBytes + p * kDiagPieceBytes, src + p * (kDiagPieceBytes / 4),
+                                  kDiagPieceBytes, &diag_full[p]);
+                    } else {
+                        bar_arrive(&diag_full[p]);
+                    }
                 }
             }
             // the block must not end with copies in flight
             for (uint32_t s = t.k > uint32_t(kStages) + 1 ? t.k - 1 - kStages : 0; s + 1 < t.k; ++s)
-                bar_wait(&full[s % kStages], (s / kStages) & 1, spin_limit);
+                bar_wait(&full[s % kStages], (s / kStages) & 1, status);
             for (int p = 0; p < kPieces; ++p) {
-                if (t.k) bar_wait(&last_full[p], 0, spin_limit);
-                if (t.i != t.j) bar_wait(&diag_full[p], 0, spin_limit);
+                if (t.k) bar_wait(&last_full[p], 0, status);
+                if (t.i != t.j) bar_wait(&diag_full[p], 0, status);
             }
         }
         return;
@@ -262,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (warp == kTriThreads / 32 + 1) {  // publisher: releases each piece once it is written
         if (lane == 0 && (t.i != t.j || t.k + 1 < nt))
             for (uint32_t p = 0; p < uint32_t(kPieces); ++p) {
-                if (!bar_wait(&written[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+                bar_wait(&written[p], 0, status);
                 st_release_gpu(ready + size_t(t.i) * nt + t.j, p + 1);
             }
         return;
@@ -286,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (uint32_t s = 0; s < t.k; ++s) {
         const uint32_t st = s % kStages;
         const bool last = s + 1 == t.k;
-        if (!last && !bar_wait(&full[st], (s / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+        if (!last) bar_wait(&full[st], (s / kStages) & 1, status);
         const float *sL = reinterpret_cast<const float *>(flow_smem + st * kStageBytes) + tr * 4;
         const float *sU = reinterpret_cast<const float *>(flow_smem + st * kStageBytes + kTileBytes) + tc * 4;
         // the 64 products in a sum of their own, subtracted once: its roundings
@@ -298,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             for (int b = 0; b < 4; ++b) sum[a][b] = 0.0f;
 #pragma unroll 1
         for (int p = 0; p < kPieces; ++p) {
-            if (last && !bar_wait(&last_full[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+            if (last) bar_wait(&last_full[p], 0, status);
 #pragma unroll
             for (int kk = 0; kk < kT / kPieces; ++kk) {
                 const int k = p * (kT / kPieces) + kk;
@@ -361,9 +391,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     tri_sync();
     const float *M = reinterpret_cast<const float *>(flow_smem + (t.k % kStages) * kStageBytes);
     float *out = tiles + (size_t(t.i) * nt + t.j) * kT * kT;
-    auto before = [&](uint32_t p) {
-        if (!bar_wait(&diag_full[p], 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
-    };
+    auto before = [&](uint32_t p) { bar_wait(&diag_full[p], 0, status); };
     auto after = [&](uint32_t p) {  // piece p of the tile
         const uint32_t k = 16 * p + (tid >> 4), v = (tid & 15) * 4;
         const float *w = W + k * kLdW + v;
@@ -394,7 +422,7 @@ size_t dense_flow_ctl_words(uint32_t m, uint32_t count) {
 
 cudaError_t launch_dense_flow(float *val, uint64_t stride, uint32_t count, const uint32_t *doff, uint32_t m,
                               const float *pert_z, float *work, uint32_t *ctl, uint32_t *status, uint32_t spin_limit,
-                              cudaStream_t st) {
+                              uint32_t ticket_base, cudaStream_t st) {
     static PerDeviceOnce attr;
     cudaError_t e = attr.run([] {
         return cudaFuncSetAttribute(k_dense_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlone));
@@ -410,7 +438,8 @@ cudaError_t launch_dense_flow(float *val, uint64_t stride, uint32_t count, const
     // order 576 0.73 / 0.59; equal at order 3,968 and sixteen of 641.
     const size_t smem = uint64_t(nt) * nt * count <= 3000 ? kSmemAlone : kSmem;
     k_dense_flow<<<nt * nt * count, kThreads, smem, st>>>(val, stride, doff, m, nt, count, pert_z, work,
-                                                           dense_flow_floats(m), ctl, status, spin_limit);
+                                                           dense_flow_floats(m), ctl, status,
+                                                           std::max(spin_limit, kFlowPolls), ticket_base);
     return cudaGetLastError();
 }
 

@@ -18,6 +18,7 @@
 #include <numeric>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -286,6 +287,7 @@ struct glu_handle_s {
     uint32_t num_sms = 148;
     uint32_t spin_limit = kSpinLimit;
     bool inject_unset_flag = false;  // GLU_INJECT_UNSET_SOLVE_FLAG, for the next solve
+    bool inject_unset_tile = false;  // GLU_INJECT_UNSET_FACTOR_FLAG, for the next factorization
     // statistics of a factorization enqueued and not yet finished
     uint64_t pending_launches = 0;
     double pending_upd_bytes = 0, pending_upd_flops = 0;
@@ -1863,9 +1865,10 @@ Status factor_buffers(glu_handle_s *h, uint32_t count, bool *use_flow) {
 }
 
 // The kernels of a factorization, on st; their number and the dense update's
-// statistics go to `note`.
-Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, bool flow, cudaStream_t st,
-                       LaunchGraph &note) {
+// statistics go to `note`.  ticket_base: of the dataflow launch (1: an injected
+// failure).
+Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, bool flow, uint32_t ticket_base,
+                       cudaStream_t st, LaunchGraph &note) {
     Status s = GLU_OK;
     float *val = h->d_val.as<float>() + size_t(first) * h->nnz;
     const uint64_t stride = h->nnz;
@@ -1973,7 +1976,7 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
         GLU_LAUNCH(KK_UPDATE,
                    launch_dense_flow(dbase, dstride, count, doff, h->m, pert, h->d_flow_work.as<float>(),
                                      reinterpret_cast<uint32_t *>(h->d_flow_work.as<float>() + flow_floats), dstatus,
-                                     h->spin_limit, st),
+                                     h->spin_limit, ticket_base, st),
                    "factor (dense block)");
         const double mm = h->m;
         upd_bytes += double(count) * 8.0 * mm * mm;
@@ -2145,11 +2148,14 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
     GLU_CUDA(cudaEventRecord(h->ev0, st), "event");
     h->prof.used = 0;
     LaunchGraph note;
-    auto enqueue = [&](cudaStream_t to, LaunchGraph &n) { return factor_launches(h, first, count, perturb, flow, to, n); };
+    const bool inject = std::exchange(h->inject_unset_tile, false);  // (for this factorization only)
+    auto enqueue = [&](cudaStream_t to, LaunchGraph &n) {
+        return factor_launches(h, first, count, perturb, flow, inject ? 1u : 0u, to, n);
+    };
     // (the profiler's events are per launch; with look-ahead the launches of
     // two streams are long enough to hide their cost)
     const bool lookahead = !flow && h->tune.dense_lookahead && h->m >= h->tune.dense_lookahead;
-    if (h->prof.on || lookahead)
+    if (h->prof.on || lookahead || inject)
         s = enqueue(st, note);
     else
         s = run_graphed(h, {3u, first, count, perturb != 0, flow, key_of(h->d_flow_work.p), key_of(h->d_dinv.p),
@@ -2537,6 +2543,12 @@ glu_status glu_debug_inject(glu_handle_t h, int what, uint32_t value) {
             if (!h) return set_error(GLU_ERR_ARG, "null handle");
             if (h->m == 0) return set_error(GLU_ERR_UNSUPPORTED, "the factorization has no dense trailing block");
             h->inject_unset_flag = true;
+            return GLU_OK;
+        case GLU_INJECT_UNSET_FACTOR_FLAG:
+            if (!h) return set_error(GLU_ERR_ARG, "null handle");
+            if (!dense_flow(h->tune, h->m, h->batch))
+                return set_error(GLU_ERR_UNSUPPORTED, "no dense trailing block that is factored tile by tile");
+            h->inject_unset_tile = true;
             return GLU_OK;
         default:
             return set_error(GLU_ERR_ARG, "unknown injection %d", what);

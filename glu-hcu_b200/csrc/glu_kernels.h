@@ -159,14 +159,15 @@ cudaError_t launch_couple_update_tc(const CUtensorMap &mapA, const CUtensorMap &
 // The whole trailing block by one launch, a dataflow of 64 x 64 tiles
 // (glu_dense_flow.cu).  work: dense_flow_floats(m) floats per value set
 // (16-byte aligned), ctl: dense_flow_ctl_words(m, count) words, zeroed by the
-// launch.
+// launch.  ticket_base: first tile ticket (0; 1 leaves the first tile of the
+// first value set unclaimed, an injected failure).
 constexpr int kFlowTile = 64;
 constexpr int kFlowDiagFloats = 64 * 68;
 size_t dense_flow_floats(uint32_t m);
 size_t dense_flow_ctl_words(uint32_t m, uint32_t count);
 cudaError_t launch_dense_flow(float *val, uint64_t stride, uint32_t count, const uint32_t *doff, uint32_t m,
                               const float *pert_z, float *work, uint32_t *ctl, uint32_t *status, uint32_t spin_limit,
-                              cudaStream_t st);
+                              uint32_t ticket_base, cudaStream_t st);
 // A trailing block that is dense but not completely filled is factored in a
 // separate m x m column-major buffer: gather copies the block's pattern
 // entries of the CSC values into the (zeroed) buffer, scatter copies the

@@ -29,6 +29,7 @@ GLU_HOST = 0
 GLU_DEVICE = 1
 GLU_INJECT_ALLOC_FAILURES = 1
 GLU_INJECT_UNSET_SOLVE_FLAG = 2
+GLU_INJECT_UNSET_FACTOR_FLAG = 3
 
 # Every symbol the engine exports (checked by the tests against the header).
 ENGINE_SYMBOLS = [
