@@ -191,11 +191,38 @@ struct LaunchGraph {
     std::array<uint64_t, 12> key{};
     cudaGraphExec_t exec = nullptr;
     bool failed = false;  // could not be captured: launched one by one
+    uint64_t calls = 0, last = 0;  // API calls that made the sequence, the number of the last one
     // what the sequence's launches add to a factorization's statistics
     uint64_t launches = 0;
     double upd_bytes = 0, upd_flops = 0;
 };
-constexpr size_t kMaxGraphs = 8;  // per handle
+// The sequences that a handle made last.
+struct GraphCache {
+    static constexpr size_t kMax = 8;
+    std::vector<LaunchGraph> slots;
+    void clear() {
+        for (LaunchGraph &g : slots)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+        slots.clear();
+    }
+    ~GraphCache() { clear(); }
+    // The key's slot; a new one in place of the one that was not made for longest.
+    LaunchGraph &find(const std::array<uint64_t, 12> &key) {
+        LaunchGraph *old = nullptr;
+        for (LaunchGraph &g : slots) {
+            if (g.key == key) return g;
+            if (!old || g.last < old->last) old = &g;
+        }
+        if (slots.size() < kMax) {
+            old = &slots.emplace_back();
+        } else {
+            if (old->exec) cudaGraphExecDestroy(old->exec);
+            *old = LaunchGraph{};
+        }
+        old->key = key;
+        return *old;
+    }
+};
 
 struct glu_handle_s {
     int device = 0;
@@ -260,9 +287,9 @@ struct glu_handle_s {
     // work buffers
     DevBuf d_status, d_pert, d_colmax, d_diag_scratch, d_ticket, d_y, d_io32, d_b64,
         d_x64, d_r64, d_norms;
-    std::vector<LaunchGraph> graphs;
-    size_t next_graph = 0;            // slot replaced next, when all are taken
+    GraphCache factor_graphs, solve_graphs;
     cudaStream_t capture = nullptr;   // for capturing them
+    uint64_t api_calls = 0;           // factorizations and solves of the caller
     uint32_t *h_status = nullptr;  // pinned
     double *h_norms = nullptr;     // pinned
     size_t h_norms_cap = 0;
@@ -296,13 +323,10 @@ struct glu_handle_s {
     glu_stats stats{};
 
     void clear_graphs() {
-        for (LaunchGraph &g : graphs)
-            if (g.exec) cudaGraphExecDestroy(g.exec);
-        graphs.clear();
-        next_graph = 0;
+        factor_graphs.clear();
+        solve_graphs.clear();
     }
     ~glu_handle_s() {
-        clear_graphs();
         if (capture) cudaStreamDestroy(capture);
         if (pos_bytes && device >= 0 && device < kMaxDevices) g_pos_bytes[device] -= pos_bytes;
         if (h_status) cudaFreeHost(h_status);
@@ -388,59 +412,50 @@ constexpr uint32_t kDenseTcMin = 1024;
 // block.
 constexpr double kCoupleGroupCost = 0.25;
 
-// Runs a launch sequence on st: launched one by one the first time its key is
-// seen, captured into a graph the second, and from then on launched as that
-// graph.  The sequences are dozens of launches of a few microseconds each, and
-// a launch costs the host 3-4 us, a graph about as much as two launches
-// (measured: FP32 solve of a 251 x 251 grid, 77 launches, 399 -> 369 us;
-// transposed refined solve at n = 9,973 1,035 -> 931 us).  Waiting for the
-// second call keeps a handle's first solve as quick as it was.
+// Runs a launch sequence on st: launched one by one by the first kGraphCalls
+// API calls that make it, captured into a graph by the next one, and from then on
+// launched as that graph.  The sequences are dozens of launches of a few
+// microseconds each, and a launch costs the host 3-4 us, a graph about as much
+// as two launches (FP32 solve of a 251 x 251 grid, 77 launches: 293 -> 256 us;
+// n = 300 step 202 -> 170; transposed refined solve at n = 9,973 612 -> 590).
+// Capturing and instantiating takes 100 to 400 us, what the graph then saves in
+// about kGraphCalls calls (those three: 11, 8, 8; 2 to 57 over the benchmark's
+// kinds of calls).  So a handle that is called a few times (and a one-shot
+// refined solve, which makes the same sweeps twice and more) pays nothing for it,
+// and no pattern of calls pays more than about twice what the launches cost.
 // enqueue(stream, slot) makes the launches and notes their statistics in the
 // slot, which `slot` (nullable) returns.
+constexpr uint64_t kGraphCalls = 8;
 template <class Enqueue>
-Status run_graphed(glu_handle_s *h, const std::array<uint64_t, 12> &key, cudaStream_t st, Enqueue &&enqueue,
-                   LaunchGraph *slot = nullptr) {
-    LaunchGraph *g = nullptr;
+Status run_graphed(glu_handle_s *h, GraphCache &cache, const std::array<uint64_t, 12> &key, cudaStream_t st,
+                   Enqueue &&enqueue, LaunchGraph *slot = nullptr) {
+    LaunchGraph &g = cache.find(key);
+    if (g.last != h->api_calls) ++g.calls;
+    g.last = h->api_calls;
     Status s = GLU_OK;
-    for (LaunchGraph &c : h->graphs)
-        if (c.key == key) g = &c;
-    if (!g) {
-        if (h->graphs.size() < kMaxGraphs) {
-            h->graphs.emplace_back();
-            g = &h->graphs.back();
-        } else {
-            g = &h->graphs[h->next_graph++ % kMaxGraphs];
-            if (g->exec) cudaGraphExecDestroy(g->exec);
-            *g = LaunchGraph{};
-        }
-        g->key = key;
-        s = enqueue(st, *g);
-        if (slot) *slot = *g;
-        return s;
-    }
-    if (!g->exec && !g->failed) {
-        g->failed = true;
+    if (!g.exec && !g.failed && g.calls > kGraphCalls) {
+        g.failed = true;
         if (!h->capture && cudaStreamCreateWithFlags(&h->capture, cudaStreamNonBlocking) != cudaSuccess)
             h->capture = nullptr;
         if (h->capture && cudaStreamBeginCapture(h->capture, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            s = enqueue(h->capture, *g);
+            s = enqueue(h->capture, g);
             cudaGraph_t graph = nullptr;
             const cudaError_t e = cudaStreamEndCapture(h->capture, &graph);
             if (s == GLU_OK && e == cudaSuccess && graph &&
-                cudaGraphInstantiate(&g->exec, graph, 0) == cudaSuccess)
-                g->failed = false;
+                cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess)
+                g.failed = false;
             else
-                g->exec = nullptr;
+                g.exec = nullptr;
             if (graph) cudaGraphDestroy(graph);
         }
         cudaGetLastError();
     }
     s = GLU_OK;
-    if (!g->exec)
-        s = enqueue(st, *g);
+    if (!g.exec)
+        s = enqueue(st, g);
     else
-        GLU_CUDA(cudaGraphLaunch(g->exec, st), "launch graph");
-    if (slot) *slot = *g;
+        GLU_CUDA(cudaGraphLaunch(g.exec, st), "launch graph");
+    if (slot) *slot = g;
     return s;
 }
 uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
@@ -1437,8 +1452,9 @@ Status solve_inplace(glu_handle_s *h, uint32_t z, uint32_t count, float *y, uint
         return GLU_OK;
     };
     if (S.ticket_base) return enqueue(st, none);  // an injected failure, for this solve only
-    return run_graphed(h, {trans ? 2u : 1u, z, count, nrhs, key_of(val), key_of(dval), key_of(y), key_of(xo),
-                           key_of(B.dinv), key_of(B.sn_inv), key_of(B.sweep_done) ^ key_of(tk), S.spin_limit},
+    return run_graphed(h, h->solve_graphs,
+                       {trans ? 2u : 1u, z, count, nrhs, key_of(val), key_of(dval), key_of(y), key_of(xo),
+                        key_of(B.dinv), key_of(B.sn_inv), key_of(B.sweep_done) ^ key_of(tk), S.spin_limit},
                        st, enqueue);
 }
 
@@ -1461,6 +1477,7 @@ Status solve_f32(glu_handle_s *h, uint32_t inst, uint32_t nrhs, const float *b, 
     }
     GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
     const TransformDev &T = h->T;
+    ++h->api_calls;
     h->stats.solve_launches = 2;  // the two transforms; solve_inplace adds the sweeps
     SolveInit init;
     Status s = solve_buffers(h, nrhs, &init);
@@ -2142,6 +2159,7 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
 // asynchronously.  factor_finish reads them once st has completed.
 Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int perturb, cudaStream_t st) {
     bool flow = false;
+    ++h->api_calls;
     Status s = factor_buffers(h, count, &flow);
     if (s != GLU_OK) return s;
     GLU_CUDA(cudaMemsetAsync(h->d_status.p, 0, sizeof(uint32_t), st), "reset status");
@@ -2158,8 +2176,9 @@ Status factor_enqueue(glu_handle_s *h, uint32_t first, uint32_t count, int pertu
     if (h->prof.on || lookahead || inject)
         s = enqueue(st, note);
     else
-        s = run_graphed(h, {3u, first, count, perturb != 0, flow, key_of(h->d_flow_work.p), key_of(h->d_dinv.p),
-                            key_of(h->d_sn_inv.p), key_of(h->d_packA.p), key_of(h->d_dense.p), h->spin_limit, 0u},
+        s = run_graphed(h, h->factor_graphs,
+                        {3u, first, count, perturb != 0, flow, key_of(h->d_flow_work.p), key_of(h->d_dinv.p),
+                         key_of(h->d_sn_inv.p), key_of(h->d_packA.p), key_of(h->d_dense.p), h->spin_limit, 0u},
                         st, enqueue, &note);
     if (s != GLU_OK) return s;
     GLU_CUDA(cudaEventRecord(h->ev1, st), "event");
@@ -2290,6 +2309,7 @@ Status refine_prepare(RefineJob &j) {
     if (uint64_t(j.nrhs) * j.count > 65535)
         return set_error(GLU_ERR_UNSUPPORTED, "count * nrhs = %llu right-hand sides exceed 65,535 per call",
                          (unsigned long long)j.nrhs * j.count);
+    ++h->api_calls;
     j.nvec = j.nrhs * j.count;
     j.len = size_t(h->n) * j.nvec;
     GLU_CUDA(h->d_y.ensure(sizeof(float) * j.len), "allocate");

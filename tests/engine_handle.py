@@ -21,9 +21,9 @@ class Handle:
 
         self.capi, self.eng, self.ptr = _capi, _capi.engine(), _capi.ptr
         self.n = A.shape[0]
-        ap, self.rows, self.cols = pattern(A)
+        self.ap, self.rows, self.cols = pattern(A)
         self.sym, self.h = C.c_void_p(), C.c_void_p()
-        _capi.check(self.eng.glu_symbolic_analyze(self.n, self.rows.size, self.ptr(ap), self.ptr(self.rows),
+        _capi.check(self.eng.glu_symbolic_analyze(self.n, self.rows.size, self.ptr(self.ap), self.ptr(self.rows),
                                                   C.byref(self.sym)))
         _capi.check(self.eng.glu_create(self.sym, 0, sets, C.byref(self.h)))
         if not dense:
@@ -49,6 +49,15 @@ class Handle:
                                 self.ptr(val))
         self.capi.check(self.eng.glu_load_lu_values(self.h, z, 1, self.ptr(val), self.capi.GLU_HOST, None))
 
+    def source(self, mats):
+        """The matrices as sources of all value sets: for refined solves."""
+        slots = np.empty(self.rows.size, np.uint32)
+        self.eng.glu_symbolic_slots(self.sym, self.ptr(slots))
+        self.capi.check(self.eng.glu_set_source(self.h, self.rows.size, self.ptr(self.ap), self.ptr(self.rows),
+                                                self.ptr(slots), None))
+        ax = np.stack([np.ascontiguousarray(A.T[self.cols, self.rows], np.float64) for A in mats])
+        self.capi.check(self.eng.glu_load_source_values(self.h, 0, len(mats), self.ptr(ax), self.capi.GLU_HOST, None))
+
     def factor(self, first=0, count=1, perturb=0):
         return self.eng.glu_factor(self.h, first, count, perturb, None)
 
@@ -69,6 +78,15 @@ class Handle:
         call = self.eng.glu_solve_transposed if transposed else self.eng.glu_solve
         self.capi.check(call(self.h, z, b.size // self.n, self.ptr(b), self.ptr(x), self.capi.GLU_HOST, None))
         return x
+
+    def solve_refined(self, z, b, tol, steps):
+        """FP64 solution of value set z, at most ``steps`` refinements."""
+        b = np.ascontiguousarray(b, np.float64)
+        x, st = np.empty_like(b), self.capi.RefineStats()
+        r = self.eng.glu_solve_refined(self.h, z, 1, b.size // self.n, self.ptr(b), self.ptr(x), tol, steps, 0,
+                                       self.capi.GLU_HOST, C.byref(st), None)
+        assert r in (self.capi.GLU_OK, self.capi.GLU_ERR_NOT_CONVERGED)
+        return x, st
 
 
 @contextlib.contextmanager

@@ -38,7 +38,7 @@ def test_wait_for_a_tile_runs_out_and_handle_stays_usable(n, sets):
     with handle(mats[0], sets) as H:
         capi, eng = H.capi, H.eng
         assert H.stats().dense_tail > 64
-        for again in range(3):  # with the later ones' launches as a graph
+        for _ in range(3):
             for z, A in enumerate(mats):
                 H.load(z, A)
             capi.check(eng.glu_set_wait_limit(H.h, 1000))
