@@ -294,9 +294,11 @@ __device__ __forceinline__ void tri_lu_smem(float *S, uint32_t w, bool last_l, f
 // row's padding holds the pivot's reciprocal, M[c * kTriML + kTriMax] = 1 /
 // M(c, c) (correctly rounded), so that the solve's dependency chain is a
 // multiply and a fused multiply-add per column instead of a division (one
-// extra rounding of each L entry).
+// extra rounding of each L entry).  The row's entries before `first` are
+// structural zeros: they are not multiplied, as M may not be finite there.
 template <bool kDiv, int N>
-__device__ __forceinline__ void tri_chunk_solve(float (&x)[N], const float *sM, uint32_t cb, uint32_t w) {
+__device__ __forceinline__ void tri_chunk_solve(float (&x)[N], const float *sM, uint32_t cb, uint32_t w,
+                                                uint32_t first = 0) {
     static_assert(N <= kTriChunk, "one chunk");
     constexpr int NV = (N + 3) / 4;
 #pragma unroll
@@ -312,14 +314,15 @@ __device__ __forceinline__ void tri_chunk_solve(float (&x)[N], const float *sM, 
         }
         if (kDiv) x[k] = x[k] * sM[c * kTriML + kTriMax];
 #pragma unroll
-        for (int p = k + 1; p < N; ++p) x[p] = fmaf(-x[k], mr[p], x[p]);
+        for (int p = k + 1; p < N; ++p)
+            if (c >= first) x[p] = fmaf(-x[k], mr[p], x[p]);
     }
 }
 
 // y (chunk cj) -= x (solved chunk cb) times M(chunk cb rows, chunk cj columns),
-// rows of M in increasing order.
+// rows of M in increasing order, from `first` on.
 __device__ __forceinline__ void tri_chunk_update(float (&y)[kTriChunk], const float (&x)[kTriChunk], const float *sM,
-                                                 uint32_t cb, uint32_t cj, uint32_t w) {
+                                                 uint32_t cb, uint32_t cj, uint32_t w, uint32_t first = 0) {
 #pragma unroll
     for (int k = 0; k < kTriChunk; ++k) {
         const uint32_t c = cb * kTriChunk + k;
@@ -328,6 +331,7 @@ __device__ __forceinline__ void tri_chunk_update(float (&y)[kTriChunk], const fl
 #pragma unroll
         for (int v = 0; v < kTriChunk / 4; ++v) {
             const float4 t = m4[v];
+            if (c < first) continue;
             y[4 * v] = fmaf(-x[k], t.x, y[4 * v]);
             y[4 * v + 1] = fmaf(-x[k], t.y, y[4 * v + 1]);
             y[4 * v + 2] = fmaf(-x[k], t.z, y[4 * v + 2]);
@@ -429,14 +433,14 @@ __device__ __forceinline__ void tri_two_rows_solve(float *sW, uint32_t ldw, uint
 // between its writes and the call and before it reads the result.
 template <bool kDiv>
 __device__ __forceinline__ void tri_rows_solve_halves(float *sW, uint32_t ldw, uint32_t t, uint32_t half, const float *sM,
-                                                      uint32_t w) {
+                                                      uint32_t w, uint32_t first = 0) {
     const uint32_t nch = (w + kTriChunk - 1) / kTriChunk;
     for (uint32_t cb = 0; cb < nch; ++cb) {
         if (half == (cb & 1)) {
             float x[kTriChunk];
 #pragma unroll
             for (int k = 0; k < kTriChunk; ++k) x[k] = sW[(cb * kTriChunk + k) * ldw + t];
-            tri_chunk_solve<kDiv>(x, sM, cb, w);
+            tri_chunk_solve<kDiv>(x, sM, cb, w, first);
 #pragma unroll
             for (int k = 0; k < kTriChunk; ++k) sW[(cb * kTriChunk + k) * ldw + t] = x[k];
         }
@@ -449,7 +453,7 @@ __device__ __forceinline__ void tri_rows_solve_halves(float *sW, uint32_t ldw, u
             float y[kTriChunk];
 #pragma unroll
             for (int k = 0; k < kTriChunk; ++k) y[k] = sW[(cj * kTriChunk + k) * ldw + t];
-            tri_chunk_update(y, x, sM, cb, cj, w);
+            tri_chunk_update(y, x, sM, cb, cj, w, first);
 #pragma unroll
             for (int k = 0; k < kTriChunk; ++k) sW[(cj * kTriChunk + k) * ldw + t] = y[k];
         }
