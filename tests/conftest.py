@@ -26,6 +26,31 @@ def _has_gpu():
 HAS_GPU = _has_gpu()
 
 
+# What needs third-party code that is built only where its sources are: the
+# preprocessing library behind pyglu's analysis, the command line tool linked to it.
+def _without_preprocessing():
+    from pyglu import _capi
+
+    if os.path.exists(_capi.NICSLU_PATH):
+        return
+
+    def load_preprocess():
+        pytest.skip(f"{os.path.basename(_capi.NICSLU_PATH)} not built (its sources are not here)")
+
+    _capi.load_preprocess = load_preprocess
+
+
+_without_preprocessing()
+LU_CMD = os.path.join(ROOT, "glu-hcu_b200", "bin", "lu_cmd")
+NEEDS_FILE = {
+    "test_cli.py::test_usage_and_bad_arguments": LU_CMD,
+    "test_cli.py::test_lu_cmd_solves_and_writes_x": LU_CMD,
+    "test_zz_no_alloc.py::test_noalloc_rejects_dense_tail_beyond_its_array": os.path.join(
+        ROOT, "glu-hcu_b200", "lib", "libglu_nicslu.so"),
+    "test_cpu_dist.py::test_reference_arm_runs_on_rank_zero_only": os.path.join(ROOT, "oracle", "_ref", "libglu_ref.so"),
+}
+
+
 def pytest_collection_modifyitems(config, items):
     import oracle
 
@@ -36,3 +61,6 @@ def pytest_collection_modifyitems(config, items):
             it.add_marker(skip_gpu)
         if "ref" in it.keywords and not oracle.ref_available():
             it.add_marker(skip_ref)
+        path = NEEDS_FILE.get(f"{it.path.name}::{it.name}")
+        if path and not os.path.exists(path):
+            it.add_marker(pytest.mark.skip(reason=f"{os.path.basename(path)} not built"))
