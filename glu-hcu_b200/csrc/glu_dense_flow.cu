@@ -36,7 +36,7 @@
 // computing warps run to their end with whatever the stages hold, the block's
 // pieces are released, and so the launch drains.
 //
-// A column step of the chain takes 12.5 us (order 1,920, one block per SM), 7 of
+// A column step of the chain takes 13 us (order 1,920, one block per SM), 7 of
 // them the LU; 16.5 us with whole tiles handed on (LU 7.0, publishing it 1.5,
 // flag and copy 1.1, triangular solve 2.6, publishing 0.8, flag and copy 1.2,
 // product 1.9), 50 us in panel, pack and update kernels.  The whole block: 0.40

@@ -1,7 +1,7 @@
 // Trailing update of the dense tail on the 5th-generation tensor cores.
 //
 // The blocked dense LU of the trailing block (glu_factor_dense.cu) spends
-// almost all of its flops in A22 -= L21 U12 with K = 64 .. 256 (one panel or 
+// almost all of its flops in A22 -= L21 U12 with K = 64 .. 256 (one panel or a
 // group of up to four), and the deferred coupling of the sparse part adds products of the
 // same form.  Here that product runs as tcgen05.mma kind::f16 on BF16
 // operands with FP32 accuracy kept by splitting every operand into three BF16
@@ -271,9 +271,9 @@ __global__ void __launch_bounds__(256) k_dense_pack(const float *__restrict__ va
 // [ustart[g][b], ustart[g][b + 1]) (their CSC positions from cpos).  The start
 // tables (nblk + 1 entries per slot) are computed with the plan.  A 128 x 64
 // tile in shared memory, then coalesced writes of the three BF16 parts.
-// What bounds it is the chain of loads from a slot's start to its values: 
+// What bounds it is the chain of loads from a slot's start to its values: a
 // warp takes eight slots, lanes along the entries, and has the loads of all
-// eight in flight at every step (four threads walking one slot each left 
+// eight in flight at every step (four threads walking one slot each left a
 // chain of up to 32 of them: 41 us per group at order 3,968, now 12.6).
 constexpr uint32_t kCoupleSlots = 64;
 constexpr uint32_t kCoupleLd = kCoupleSlots + 1;

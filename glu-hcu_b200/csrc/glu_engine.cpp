@@ -464,7 +464,10 @@ uint64_t key_of(const void *p) { return reinterpret_cast<uintptr_t>(p); }
 //   dataflow  12.7 us per 64 columns (the diagonal chain) against the products
 //             at 36 TFLOP/s, the longer and three tenths of the shorter;
 //   panels    55 us per 64 columns plus the products at 130 TFLOP/s on the
-//             tensor cores.
+//             tensor cores.  (Blocks below tune.dense_tc_min update at the FP32
+//             rate, which this leaves out: from 57 value sets on, orders from
+//             about 820 up to 1,023 take the panels though the dataflow would be
+//             quicker: 96 of order 960 4.0 ms, 64 by the dataflow 1.4.)
 // Measured, dataflow / panels: order 1,920 0.40 / 1.51 ms, eight of them 1.18 /
 // 2.18, order 3,968 1.32 / 4.73, three of them 3.32 / 5.75, order 5,000 2.35 /
 // 6.27, 96 of order 576 0.60 / 0.99; twelve of order 9,360 take the panels

@@ -7,17 +7,19 @@
 //
 //  * sparse columns (in front of the dense trailing block) are processed level
 //    by level, with level sets of each sweep's own dependency graph computed
-//    once per pattern: a level with many columns gets its own launch (one warp
-//    per column); a run of thin levels executes inside one thread-block
-//    cluster that steps from level to level with hardware cluster barriers.
-//    L and U sweeps scatter (x_i -= L(i,j) x_j with atomics), the transposed
-//    sweeps gather (dot products, no atomics);
+//    once per pattern (the L and U sweeps by supernodes, glu_solve_snode.cu,
+//    unless those are off): a level with many items, chunks of a column's or
+//    row's entries, gets its own launch (a warp per item); a run of thin levels
+//    executes inside one thread-block cluster that steps from level to level
+//    with hardware cluster barriers.  All four sweeps scatter (x_i -= L(i,j)
+//    x_j with atomics; the transposed ones along the rows);
 //  * the dense trailing block is solved by row blocks of 64: a block adds the
 //    contribution of every finished earlier block (one 64 x 64 tile each, in
-//    registers) and then solves its diagonal tile; blocks are claimed in order
-//    through a ticket and wait (bounded) for the entries they read;
+//    registers) and then multiplies by the inverse of its diagonal tile; blocks
+//    are claimed in order through a ticket and wait (bounded) for the entries
+//    they read;
 //  * the coupling between the two (U entries of tail columns in sparse rows)
-//    is one parallel scatter or gather over the tail columns.
+//    is one parallel scatter over the tail columns.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -5,8 +5,8 @@
 // [s, s+w) with a dense diagonal block and a common lower pattern) a sweep
 // step is a whole supernode: its w unknowns are solved against the dense
 // diagonal block (wide ones: a product with the block's inverse, computed once
-// per factorization by k_sn_diag_inv; else a chain over the columns by one
-// warp) and their off-diagonal entries are then scattered into the unknowns
+// per factorization by k_sn_diag_inv; else, or where that product is not finite,
+// a chain over the columns by one warp) and their off-diagonal entries are then scattered into the unknowns
 // they feed:
 //   L (forward, unit):  x_S = L11^-1 y_S;  y_r -= L21(r,:) x_S for the m rows
 //                       below the block (one thread per row, dot over w);
@@ -758,11 +758,11 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
             k_sn_sweep_l<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv,
                                                B.sn_inv_stride, done, ticket, status, spin_limit);
     } else {
-        // one launch per level (two where its small-supernode groups get
-        // their own), each chained to the one before (its blocks start while
-        // the previous launch drains, and wait for its x); the supernodes of
-        // one level do not feed each other, so its two launches may run in
-        // either order
+        // one launch per level (up to three where its narrow parts or its
+        // small-supernode groups get their own), each chained to the one
+        // before (its blocks start while the previous launch drains, and wait
+        // for its x); the supernodes of one level do not feed each other, so
+        // its launches may run in any order
         for (uint32_t l = 0; l < W.nlev; ++l) {
             const SnSweepLevel &lv = W.levels[l];
             const uint3 k3 = sn_sweep_level_launches(lv, upper);

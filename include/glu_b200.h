@@ -140,9 +140,10 @@ glu_status glu_factor(glu_handle_t h, uint32_t first, uint32_t count, int pertur
 
 /* ------------------------------------------------------------------- solve --
  * FP32 solve of A x = b with value set `inst` for nrhs right-hand sides
- * (b and x: nrhs x n, one right-hand side after another).  Same arithmetic
- * sequence as Symbolic_Matrix::solve (src/symbolic.cc:200-251): permute and
- * scale b, unit-L sweep, U sweep, permute and scale back.  x may alias b. */
+ * (b and x: nrhs x n, one right-hand side after another).  The steps of
+ * Symbolic_Matrix::solve (src/symbolic.cc:200-251): permute and scale b, unit-L
+ * sweep, U sweep, permute and scale back; sums in another order, and wide
+ * diagonal blocks by their inverses.  x may alias b. */
 glu_status glu_solve(glu_handle_t h, uint32_t inst, uint32_t nrhs, const float *b, float *x,
                      glu_memory where, glu_stream stream);
 /* glu_solve for callers that cannot allocate device memory.  No counterpart in
@@ -259,9 +260,9 @@ glu_status glu_measure_fp32_peak(int device, double *tflops);
  * flag, finishes without further waiting, and the call returns
  * GLU_ERR_TIMEOUT with the handle still usable.  The waits for tiles, which
  * last as long as the tiles in front take, never give up before 2^17 polls
- * (about 0.1 s).  0 restores the default (2^24 polls, a few seconds).  The reference has no bounded
- * waits: a stuck kernel blocks its per-level cudaDeviceSynchronize
- * (src/numeric.cu:615-616) forever. */
+ * (about 0.1 s).  0 restores the default (2^24 polls, a few seconds).  The
+ * reference has no bounded waits: a stuck kernel blocks its per-level
+ * cudaDeviceSynchronize (src/numeric.cu:615-616) forever. */
 glu_status glu_set_wait_limit(glu_handle_t h, uint32_t polls);
 
 /* Failure injection for tests of the error paths; no counterpart in the
@@ -314,9 +315,10 @@ typedef struct {
                                   model assumes; 0: built in (the time of the
                                   path that factors the block)                   */
     uint32_t sn_sweep_fused;   /* 0 (default): one launch per supernodal solve
-                                  sweep level (a second one for the groups of
-                                  small supernodes of a wide level, or only
-                                  that one where the level has nothing else);
+                                  sweep level (up to two more for its narrow
+                                  supernodes and for the groups of small ones of
+                                  a wide level, or only those where the level
+                                  has nothing else);
                                   1: each sweep is one launch in
                                   which a supernode waits (bounded) for the ones
                                   that update it (slower on the patterns
