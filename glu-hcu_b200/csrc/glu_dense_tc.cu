@@ -49,6 +49,8 @@
 // All waits on mbarriers are bounded (spin_limit polls); a wait that runs out
 // sets DEV_TIMEOUT, every role leaves its loop, the CTA waits for its own
 // copies and MMAs in flight and frees its tensor memory before returning.
+// Those last waits end by themselves, so they keep kSpinLimit: with a short
+// limit of the handle's the CTA could end before them.
 //
 // The reference's counterpart is the per-column Schur update
 // RL_onecol_updateSubmat (src/numeric.cu:270-319).
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const uint32_t drain_limit = max(spin_limit, kSpinLimit);
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // the last load into every stage lands before the CTA may exit
             for (uint32_t s = 0; s < uint32_t(kStages) && s < g; ++s) {
                 const uint32_t f = s + ((g - 1 - s) / kStages) * kStages;
-                if (!mbar_wait(&full[s], (f / kStages) & 1, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+                if (!mbar_wait(&full[s], (f / kStages) & 1, drain_limit)) atomicOr(status, DEV_TIMEOUT);
             }
         }
     } else if (warp == 1) {
@@ -504,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             if (!ok) atomicOr(status, DEV_TIMEOUT);
             tc_commit(done);
-            if (!mbar_wait(done, 0, spin_limit)) atomicOr(status, DEV_TIMEOUT);
+            if (!mbar_wait(done, 0, drain_limit)) atomicOr(status, DEV_TIMEOUT);
         }
     } else if (warp == kPrefetchWarp) {
         // ------------------------------------------------ C prefetch
