@@ -389,20 +389,18 @@ void find_full_tail(const SymbolicData &s, uint32_t min_m, uint32_t &t, uint32_t
 }
 
 // Cost model of the split point t: the columns [t, n) are factored as a dense
-// block, the columns in front of t level by level.  Dense: dense_seconds of the
-// handle's value sets.  Sparse: their update work of the columns < t at
-// kSparseRate plus kLevelLatency per level that still has an active column < t.
-// Returns the t of least estimated time with m <= max_m (t = n: no dense tail).
-// The constants are the best of a few, against one set's work at the rates below:
-// n = 300 step 158 / 174 us, 96 value sets of n = 1,500 1,576 / 1,645 us, n = 4,960
-// refactorization 575 / 586 us, grids of 90,000 and 490,000 equal; with the
-// panels' time but one set's work the 96 sets take 1,730 us.
-// With a rate (tune.dense_rate) or widths of the dense paths set: one set's 2/3 m^3
-// flops at that rate, or by whether the block updates on the tensor cores at
-// kDenseRate or kDenseRateTc, plus kPanelLatency per panel step, and its
-// sparse work at kTunedSparseRate.
-constexpr double kSparseRate = 0.1e12, kLevelLatency = 8e-6;
-constexpr double kDenseRate = 30e12, kDenseRateTc = 120e12, kPanelLatency = 20e-6, kTunedSparseRate = 0.2e12;
+// block, the columns in front of t level by level.  Dense: 2/3 m^3 flops at
+// kDenseRate plus kPanelLatency per panel step.  Sparse: the update work of
+// the columns < t at kSparseRate plus kLevelLatency per level that still has
+// an active column < t.  Returns the t of least estimated time with
+// m <= max_m (t = n: no dense tail).
+// The rates are those of one value set's panels and updates.  With the dataflow's
+// time for all value sets (dense_seconds) in their place the dense blocks of
+// circuits come out a little better (n = 300 step 175 -> 164 us, 96 value sets of n
+// = 1,500 1,637 -> 1,588), but a sparse rate that holds there is tens of times too
+// low for wide supernodes: 16 value sets of twenty filled 300 x 300 blocks 0.9 -> 9.5
+// ms, of 4,000 columns in 32-wide blocks with a border of 100 1.2 -> 7.7 ms.
+constexpr double kDenseRate = 30e12, kDenseRateTc = 120e12, kPanelLatency = 20e-6;
 // Default width from which trailing blocks factor with panel look-ahead.
 constexpr uint32_t kLookaheadMin = 3072;
 // Default width from which trailing blocks update on the tensor cores.
@@ -411,6 +409,7 @@ constexpr uint32_t kDenseTcMin = 1024;
 // m x m dense block), in scattered supernode-update entries per entry of the
 // block.
 constexpr double kCoupleGroupCost = 0.25;
+constexpr double kSparseRate = 0.2e12, kLevelLatency = 8e-6;
 
 // Runs a launch sequence on st: launched one by one by the first kGraphCalls
 // API calls that make it, captured into a graph by the next one, and from then on
@@ -496,7 +495,7 @@ bool dense_flow(const glu_tuning &tu, uint32_t m, uint32_t count) {
 }
 
 uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_ptr,
-                      const std::vector<int32_t> &level_idx, uint32_t max_m, const glu_tuning &tu, uint32_t batch) {
+                      const std::vector<int32_t> &level_idx, uint32_t max_m, const glu_tuning &tu) {
     const uint32_t n = s.n;
     // sparse work of column k and the first column of each level
     std::vector<double> pre(n + 1, 0.0);
@@ -520,23 +519,15 @@ uint32_t choose_split(const SymbolicData &s, const std::vector<int32_t> &level_p
     std::sort(lev_first.begin(), lev_first.end());
     double best = 1e300;
     uint32_t best_t = n;
-    const bool modelled = default_widths(tu) && tu.dense_rate == 0;
     const int64_t lo = max_m >= n ? 0 : int64_t(n) - max_m;
     for (int64_t tt = n; tt >= lo; tt -= 16) {
         const uint32_t t = uint32_t(tt);
         double m = double(n - t);
-        const double nlev = double(std::lower_bound(lev_first.begin(), lev_first.end(), t) - lev_first.begin());
-        double dense = 0, sparse = nlev * kLevelLatency;
-        if (modelled) {
-            const DenseSeconds d = dense_seconds(m, batch);
-            dense = std::min(d.flow, d.panels);
-            sparse += batch * pre[t] / kSparseRate;
-        } else {
-            const double rate = tu.dense_rate ? 1e9 * tu.dense_rate
-                                              : (tu.dense_tc_min && m >= tu.dense_tc_min ? kDenseRateTc : kDenseRate);
-            dense = (2.0 / 3.0) * m * m * m / rate + std::ceil(m / kDenseNB) * kPanelLatency;
-            sparse += pre[t] / kTunedSparseRate;
-        }
+        const double rate = tu.dense_rate ? 1e9 * tu.dense_rate
+                                          : (tu.dense_tc_min && m >= tu.dense_tc_min ? kDenseRateTc : kDenseRate);
+        double dense = m > 0 ? (2.0 / 3.0) * m * m * m / rate + std::ceil(m / kDenseNB) * kPanelLatency : 0;
+        double nlev = double(std::lower_bound(lev_first.begin(), lev_first.end(), t) - lev_first.begin());
+        double sparse = pre[t] / kSparseRate + nlev * kLevelLatency;
         if (dense + sparse < best) {
             best = dense + sparse;
             best_t = t;
@@ -1063,7 +1054,7 @@ Status build_plan(glu_handle_s *h) {
             if (cap < max_m) max_m = uint32_t(cap);
         }
     }
-    uint32_t t_opt = choose_split(s, h->level_ptr, h->level_idx, std::max(max_m, m_full), h->tune, h->batch);
+    uint32_t t_opt = choose_split(s, h->level_ptr, h->level_idx, std::max(max_m, m_full), h->tune);
     h->dense_buffer = false;
     if (t_opt >= t_full) {
         h->t = t_opt;  // any trailing block of a fully dense block is fully dense

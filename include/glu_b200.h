@@ -312,8 +312,8 @@ typedef struct {
                                   min(dense_tc_min^2, two 128 x 128 tiles per
                                   SM); 0: FP32 FMA always                      */
     uint32_t dense_rate;       /* dense-block throughput (GFLOP/s) the split cost
-                                  model assumes; 0: built in (the time of the
-                                  path that factors the block)                   */
+                                  model assumes; 0: built in (FMA or tensor-core
+                                  rate, whichever the block would use)           */
     uint32_t sn_sweep_fused;   /* 0 (default): one launch per supernodal solve
                                   sweep level (up to two more for its narrow
                                   supernodes and for the groups of small ones of
