@@ -321,7 +321,13 @@ __device__ __forceinline__ void load_inverse(float (&iv)[16], const float *__res
     for (int k = 0; k < 16; ++k) iv[k] = __ldg(inv + k * kSnMaxWidth);
 }
 
-__global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
+// kInv: the wide supernodes' inverses are there (invs).  Without them the kernels need
+// fewer registers, and more blocks fit on an SM, which is what bounds the sweeps
+// of many value sets (64 of a hundred filled 40 x 40 blocks, where the inverses are
+// over their budget: L 150 -> 87 us, U 93 -> 77 us a launch with kernels of
+// their own and the rows of L21 behind a branch).
+template <bool kInv>
+__global__ void __launch_bounds__(256, kInv ? 2 : 3) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                     uint64_t vstride, uint64_t ystride,
                                                     const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
@@ -348,21 +354,24 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
     const uint32_t s = md.x, w = md.y, lbase = md.z, m = md.w, t = bi.y;
     const uint32_t l = s + w - 1;
     const uint32_t tid = threadIdx.x, n = P.n;
-    const uint32_t wide = (invs && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
+    const uint32_t wide = (kInv && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
     __shared__ uint32_t sB[kSnMaxWidth];
     if (tid < w) sB[tid] = P.diag[s + tid];
     __syncthreads();
     // This thread's L21 row and its target: they do not depend on x, so they
     // are loaded before the dependency chain (and serve every right-hand side).
+    // (Behind a branch: warps without rows, all of a block diagonal matrix, skip it and the products.)
     const uint32_t r = t * blockDim.x + tid;  // L21 row of this thread
     float lr[kSnMaxWidth];
     uint32_t target = 0;
+    if (r < m) {
+        target = __ldg(P.ridx + lbase + r);
 #pragma unroll
-    for (int c = 0; c < int(kSnMaxWidth); ++c)
-        lr[c] = (r < m && uint32_t(c) < w) ? __ldg(val + sB[c] + (l + 1 - (s + c)) + r) : 0.0f;
-    if (r < m) target = __ldg(P.ridx + lbase + r);
+        for (int c = 0; c < int(kSnMaxWidth); ++c)
+            lr[c] = uint32_t(c) < w ? __ldg(val + sB[c] + (l + 1 - (s + c)) + r) : 0.0f;
+    }
     float iv[16];
-    if (wide != UINT32_MAX) {
+    if (kInv && wide != UINT32_MAX) {
         load_inverse(iv, invs + bz.y * inv_stride + (size_t(wide) * 2) * kSnMaxWidth * kSnMaxWidth, tid);
     } else {
         // L11, strictly lower: L(s+k, s+c) at diag[s+c] + (k - c); eight loads in flight per thread
@@ -398,10 +407,14 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
                 }
                 if (k0 < w) xs[k0] = v0;
                 if (k1 < w) xs[k1] = v1;
+                if (t == 0) {
+                    if (k0 < w) xo[size_t(q) * n + s + k0] = v0;
+                    if (k1 < w) xo[size_t(q) * n + s + k1] = v1;
+                }
             }
             __syncthreads();
         };
-        if (wide != UINT32_MAX) {
+        if (kInv && wide != UINT32_MAX) {
             if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
             __syncthreads();
             wide_solve(iv, vs, part, xs, tid);
@@ -423,8 +436,9 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
             }
             return (acc[0] + acc[1]) + (acc[2] + acc[3]);
         };
-        float sum = product();
-        if (wide != UINT32_MAX && !wide_finite(xs, tid)) {
+        float sum = 0.0f;
+        if (r < m) sum = product();
+        if (kInv && wide != UINT32_MAX && !wide_finite(xs, tid)) {
             __syncthreads();  // all warps have read xs
 #pragma unroll 1
             for (uint32_t e = tid; e < w * kSnMaxWidth; e += 256) {
@@ -434,10 +448,10 @@ __global__ void __launch_bounds__(256, 2) k_sn_sweep_l(DevPattern P, SnSweepPlan
             if (tid < kSnMaxWidth) xs[tid] = 0.0f;
             __syncthreads();
             substitute();
-            sum = product();
+            if (r < m) sum = product();
         }
-        if (t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
-        if (r < m && sum != 0.0f) atomicAdd(yq + target, -sum);
+        if (kInv && wide != UINT32_MAX && t == 0 && tid < w) xo[size_t(q) * n + s + tid] = xs[tid];
+        if (sum != 0.0f) atomicAdd(yq + target, -sum);
         if (q + 1 < Q.q1) __syncthreads();
     }
     sweep_release(W, blk, done);
@@ -508,7 +522,8 @@ __global__ void __launch_bounds__(256, 4) k_sn_sweep_l_narrow(DevPattern P, SnSw
     }
 }
 
-__global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
+template <bool kInv>
+__global__ void __launch_bounds__(256, kInv ? 3 : 4) k_sn_sweep_u(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                     uint64_t vstride, uint64_t ystride,
                                                     const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
@@ -534,7 +549,7 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
     }
     const uint32_t s = W.meta[bi.x].x, w = W.meta[bi.x].y, t = bi.y;
     const uint32_t tid = threadIdx.x, n = P.n;
-    const uint32_t wide = (invs && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
+    const uint32_t wide = (kInv && w > kSnSmallWidth) ? __ldg(W.wide + bi.x) : UINT32_MAX;
     __shared__ uint32_t sB[kSnMaxWidth], sC[kSnMaxWidth];
     if (tid < 32) {
         // entries of column s+c above the block: positions cptr[s+c] .. diag[s+c]-c-1
@@ -567,7 +582,7 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
     }
     __syncthreads();
     float iv[16];
-    if (wide != UINT32_MAX) {
+    if (kInv && wide != UINT32_MAX) {
         load_inverse(iv, invs + bz.y * inv_stride + (size_t(wide) * 2 + 1) * kSnMaxWidth * kSnMaxWidth, tid);
     } else {
         // U11 with its diagonal: U(s+k, s+c), k <= c, at diag[s+c] - (c - k); eight loads in flight
@@ -655,7 +670,7 @@ __global__ void __launch_bounds__(256, 3) k_sn_sweep_u(DevPattern P, SnSweepPlan
             }
             __syncthreads();
         };
-        if (wide != UINT32_MAX) {
+        if (kInv && wide != UINT32_MAX) {
             if (tid < kSnMaxWidth) vs[tid] = tid < w ? __ldcg(yq + s + tid) : 0.0f;
             __syncthreads();
             wide_solve(iv, vs, part, xs, tid);
@@ -745,18 +760,16 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
         const uint64_t have = std::max<uint64_t>(uint64_t(blocks) * B.count, 1);
         return uint32_t(std::min<uint64_t>(nrhs, std::max<uint64_t>(1, 4 * 148 / have)));
     };
+    const auto full = upper ? (B.sn_inv ? k_sn_sweep_u<true> : k_sn_sweep_u<false>)
+                            : (B.sn_inv ? k_sn_sweep_l<true> : k_sn_sweep_l<false>);
     if (W.fused && done && W.nblocks) {
         // one launch: blocks in map order by ticket, supernodes wait for their releases
         cudaError_t e = cudaMemsetAsync(done, 0, sizeof(uint32_t) * size_t(W.ns) * B.count, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t) * B.count, st);
         if (e != cudaSuccess) return e;
         const dim3 grid(W.nblocks, 1, B.count);
-        if (upper)
-            k_sn_sweep_u<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv,
-                                               B.sn_inv_stride, done, ticket, status, spin_limit);
-        else
-            k_sn_sweep_l<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv,
-                                               B.sn_inv_stride, done, ticket, status, spin_limit);
+        full<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv, B.sn_inv_stride, done,
+                                   ticket, status, spin_limit);
     } else {
         // one launch per level (up to three where its narrow parts or its
         // small-supernode groups get their own), each chained to the one
@@ -771,14 +784,9 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
             if (k3.x) {  // the full kernel: every block that no other launch takes
                 const uint32_t nblk = k3.y ? lv.wide : rest;
                 const dim3 grid(nblk, shares(nblk), B.count);
-                if (upper)
-                    e = launch_chained(k_sn_sweep_u, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride,
-                                       ystride, B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr,
-                                       status, spin_limit);
-                else
-                    e = launch_chained(k_sn_sweep_l, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride,
-                                       ystride, B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr,
-                                       status, spin_limit);
+                e = launch_chained(full, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride, ystride,
+                                   B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr, status,
+                                   spin_limit);
                 if (e != cudaSuccess) return e;
             }
             if (k3.y) {  // L: the narrow parts (and the groups, unless they launch apart)
