@@ -166,6 +166,7 @@ struct SnLevel {
     uint32_t pb0, pblocks;  // blocks in the panel map
     uint32_t ub0, ublocks;  // tiles in the update map
     uint32_t db0, dblocks;  // blocks in the diagonal-block map (supernodes of width >= 2)
+    uint32_t dwide;         // of them one wide supernode each, the first ones
     uint32_t atomic;
     uint32_t panel_w;       // widest supernode with a block of its own in the panel map
 };
@@ -808,12 +809,13 @@ Status build_sn_plan(glu_handle_s *h) {
                                                                                              psmall.size() - g))));
         for (size_t g = us0; g < usmall.size(); g += 8)
             umap.push_back(make_uint2(uint32_t(g), kSnSmallFlag | uint32_t(std::min<size_t>(8, usmall.size() - g))));
+        const uint32_t dwide = uint32_t(dmap.size()) - db0;
         for (size_t g = ds0; g < dsmall.size(); g += kSnDiagSmallPerBlock)
             dmap.push_back(make_uint2(uint32_t(g), kSnSmallFlag | uint32_t(std::min<size_t>(kSnDiagSmallPerBlock,
                                                                                              dsmall.size() - g))));
         const uint32_t i0 = lcount[l], i1 = lcount[l + 1];
         h->sn_levels.push_back(SnLevel{i0, i1, pb0, uint32_t(pmap.size()) - pb0, ub0, uint32_t(umap.size()) - ub0,
-                                       db0, uint32_t(dmap.size()) - db0, updating > 1 ? 1u : 0u, panel_w});
+                                       db0, uint32_t(dmap.size()) - db0, dwide, updating > 1 ? 1u : 0u, panel_w});
     }
     h->nsn = ns;
     GLU_CUDA(upload(h->d_sn_meta, meta), "upload supernodes");
@@ -1901,9 +1903,13 @@ Status factor_launches(glu_handle_s *h, uint32_t first, uint32_t count, int pert
     const uint32_t NL = h->use_sn ? 0u : uint32_t(h->levels_h.size());
     if (h->use_sn) {
         for (const SnLevel &lv : h->sn_levels) {
-            if (lv.dblocks)
-                GLU_LAUNCH(KK_SN_DIAG, launch_sn_diag(h->P, h->SN, val, stride, count, pert, lv.db0, lv.dblocks, st),
+            const uint2 db = sn_diag_blocks(lv.dblocks, lv.dwide, count, h->num_sms);
+            if (db.x)
+                GLU_LAUNCH(KK_SN_DIAG, launch_sn_diag(h->P, h->SN, val, stride, count, pert, lv.db0, db.x, false, st),
                            "factor (supernode diagonal blocks)");
+            if (db.y)
+                GLU_LAUNCH(KK_SN_DIAG, launch_sn_diag(h->P, h->SN, val, stride, count, pert, lv.db0 + db.x, db.y, true, st),
+                           "factor (narrow diagonal blocks)");
             if (lv.pblocks)
                 GLU_LAUNCH(KK_SN_PANEL,
                            launch_sn_panel(h->P, h->SN, val, stride, count, pert, lv.pb0, lv.pblocks, lv.panel_w, st),

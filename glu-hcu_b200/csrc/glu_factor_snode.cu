@@ -273,6 +273,8 @@ __device__ __forceinline__ void sn_update_small(const DevPattern &P, const SnPla
 // an L part (c < w - 1, or m > 0); step c: L(i,c) = A(i,c) / U(c,c), then
 // A(i,j) -= L(i,c) U(c,j) for j > c, as in the column algorithm.  blockIdx.z
 // selects the value set.
+// (127 registers for the wide blocks' LU: two blocks per SM.  Where the narrow ones' groups are
+// more than a few waves of those they go to k_sn_diag_small instead.)
 __global__ void __launch_bounds__(kTriThreads, 2) k_sn_diag(DevPattern P, SnPlanDev S, float *val_base, uint64_t stride,
                                                             const float *pert_z, uint32_t b0) {
     __shared__ __align__(16) float sS[kSnMaxWidth * kLuLD];
@@ -311,6 +313,19 @@ __global__ void __launch_bounds__(kTriThreads, 2) k_sn_diag(DevPattern P, SnPlan
         const uint32_t c = e / kSnMaxWidth, r = e % kSnMaxWidth;
         if (r < w) st_cg(val + sBase[c] + r, sS[c * kLuLD + r]);
     }
+}
+
+// The groups of narrow supernodes alone, blocks [b0, b0 + gridDim.x) of the
+// diagonal map.  Each warp's chain is latency-bound, so resident warps set the rate
+// (factorization of 64 value sets of 5,000 filled 4 x 4 blocks: 471 us in k_sn_diag,
+// two blocks per SM, 335 here; of 2,000 10 x 10 blocks 395 and 309).
+__global__ void __launch_bounds__(kTriThreads, 5) k_sn_diag_small(DevPattern P, SnPlanDev S, float *val_base,
+                                                                  uint64_t stride, const float *pert_z, uint32_t b0) {
+    pdl_release();
+    const uint2 bi = S.dmap[b0 + blockIdx.x];
+    const uint32_t wi = threadIdx.x >> 5;
+    if (wi < (bi.y & ~kSnSmallFlag))
+        sn_diag_small(P, S, val_base + blockIdx.z * stride, S.dsmall[bi.x + wi], pert_z, threadIdx.x & 31);
 }
 
 // Panel launch of one level (after its diagonal blocks): blocks [b0, b0 +
@@ -701,10 +716,18 @@ __global__ void __launch_bounds__(256) k_sn_positions(DevPattern P, SnPlanDev S,
     }
 }
 
+uint2 sn_diag_blocks(uint32_t blocks, uint32_t wide, uint32_t count, uint32_t num_sms) {
+    const uint32_t groups = blocks - wide;
+    // groups next to wide blocks run with them unless they are eight times as
+    // many as there are SMs: the two launches wait for each other, which costs
+    // about what four waves of groups do
+    const bool apart = groups && (wide == 0 || uint64_t(groups) * count > 8ull * num_sms);
+    return apart ? make_uint2(wide, groups) : make_uint2(blocks, 0u);
+}
 cudaError_t launch_sn_diag(const DevPattern &P, const SnPlanDev &S, float *val, uint64_t stride, uint32_t count,
-                           const float *pert_z, uint32_t b0, uint32_t blocks, cudaStream_t st) {
+                           const float *pert_z, uint32_t b0, uint32_t blocks, bool small, cudaStream_t st) {
     if (blocks == 0) return cudaSuccess;
-    return launch_chained(k_sn_diag, dim3(blocks, 1, count), dim3(kTriThreads), 0, st, P, S, val, stride, pert_z, b0);
+    return launch_chained(small ? k_sn_diag_small : k_sn_diag, dim3(blocks, 1, count), dim3(kTriThreads), 0, st, P, S, val, stride, pert_z, b0);
 }
 
 cudaError_t launch_sn_panel(const DevPattern &P, const SnPlanDev &S, float *val, uint64_t stride, uint32_t count,

@@ -81,8 +81,12 @@ struct SnPlanDev {
 
 // Blocks [b0, b0 + blocks) of one level's diagonal-block, panel or update
 // map.  diag runs before panel, panel before update.
+// The diagonal blocks' launches: blocks of the full kernel's (0: none), then of the
+// narrow groups' own (0: none), of a level with `blocks`, the first `wide` of
+// them one wide supernode each.
+uint2 sn_diag_blocks(uint32_t blocks, uint32_t wide, uint32_t count, uint32_t num_sms);
 cudaError_t launch_sn_diag(const DevPattern &P, const SnPlanDev &S, float *val, uint64_t stride, uint32_t count,
-                           const float *pert_z, uint32_t b0, uint32_t blocks, cudaStream_t st);
+                           const float *pert_z, uint32_t b0, uint32_t blocks, bool small, cudaStream_t st);
 cudaError_t launch_sn_panel(const DevPattern &P, const SnPlanDev &S, float *val, uint64_t stride, uint32_t count,
                             const float *pert_z, uint32_t b0, uint32_t blocks, uint32_t max_width, cudaStream_t st);
 cudaError_t launch_sn_update(const DevPattern &P, const SnPlanDev &S, float *val, uint64_t stride, uint32_t count,
