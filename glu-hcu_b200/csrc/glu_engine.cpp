@@ -862,7 +862,12 @@ Status build_sn_plan(glu_handle_s *h) {
     cudaGetLastError();
     // Wide supernodes, whose diagonal blocks the sweeps multiply by their
     // inverses.  Those take 32 KB each and value set: kept while they are at
-    // most half of the values themselves, or 64 MB.
+    // most half of the values themselves, or 64 MB.  And they take time: 10 us a
+    // factorization and 0.05 us per block, which the solves earn level by level (about
+    // 5 us each of a plain solve: 251 x 251 grid 399 -> 290 with all of its
+    // steps).  Where all the wide supernodes stand in one level there is next to
+    // nothing to earn (16 value sets of a hundred filled 40 x 40 blocks: factorization
+    // 97 us without inverses and 175 with, refined solve 190 either way).
     std::vector<uint2> wide;
     std::vector<uint32_t> wide_no(ns, UINT32_MAX);
     for (uint32_t q = 0; q < ns; ++q)
@@ -873,6 +878,9 @@ Status build_sn_plan(glu_handle_s *h) {
     if (sizeof(float) * kSnInvFloats * double(wide.size()) * h->batch >
         std::max(0.5 * sizeof(float) * double(h->nnz) * h->batch, 64e6))
         wide.clear();
+    uint32_t wide_levels = 0;
+    for (const SnLevel &lv : h->sn_levels) wide_levels += lv.dwide ? 1u : 0u;
+    if (wide_levels < 2) wide.clear();
     h->nwide = uint32_t(wide.size());
     h->d_sn_inv.release();
     GLU_CUDA(upload(h->d_wide, wide), "upload solve plan");

@@ -23,7 +23,8 @@ def _lu(A):
 
 
 @pytest.mark.parametrize("sets", [1, 5, 160])
-@pytest.mark.parametrize("widths", [[2] * 60, [10] * 30, [16, 17] * 6, [40] * 8, [64, 3, 33, 5, 7] * 4, [9] * 80])
+@pytest.mark.parametrize("widths", [[2] * 60, [10] * 30, [16, 17] * 6, [40] * 8, [64, 3, 33, 5, 7] * 4, [9] * 80,
+                                    [40] + [9] * 79 + [17]])
 def test_factors_and_solutions(widths, sets):
     n = sum(widths)
     ends = np.cumsum(widths)
