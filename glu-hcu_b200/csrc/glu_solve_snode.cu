@@ -79,7 +79,7 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
     for (int c = 0; c < SW; ++c) {
         const uint32_t dc = __shfl_sync(kFull, dl, c);
         lrow[c] = (uint32_t(c) < lane && lane < w) ? __ldg(val + dc + (lane - c)) : 0.0f;
-        l21[c] = (lane < m && uint32_t(c) < w) ? __ldg(val + dc + (l + 1 - (s + c)) + lane) : 0.0f;
+        if (m) l21[c] = (lane < m && uint32_t(c) < w) ? __ldg(val + dc + (l + 1 - (s + c)) + lane) : 0.0f;
     }
     const uint32_t target = lane < m ? __ldg(P.ridx + lbase + lane) : 0u;
     pdl_wait();  // the previous level's x
@@ -93,6 +93,7 @@ __device__ __forceinline__ void sn_sweep_l_small(const DevPattern &P, const SnSw
             if (lane > uint32_t(c) && lane < w) v = __fsub_rn(v, __fmul_rn(lrow[c], xc));
         }
         if (lane < w) xo[size_t(q) * n + s + lane] = v;
+        if (m == 0) continue;
         float acc = 0.0f;
 #pragma unroll
         for (int c = 0; c < SW; ++c) {
@@ -326,8 +327,13 @@ __device__ __forceinline__ void load_inverse(float (&iv)[16], const float *__res
 // of many value sets (64 of a hundred filled 40 x 40 blocks, where the inverses are
 // over their budget: L 150 -> 87 us, U 93 -> 77 us a launch with kernels of
 // their own and the rows of L21 behind a branch).
-template <bool kInv>
-__global__ void __launch_bounds__(256, kInv ? 2 : 3) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
+// kBlocks of them per SM: three (85 registers, a few spilled) once there are
+// kManyBlocks of the launch, for which the rate counts; with fewer the time of one does (64 x 64
+// blocks, per launch: 63 of them 7.3 us at three and 5.9 at two, 1,008 20.5 and 19.5,
+// 4,032 70 and 83).
+constexpr uint64_t kManyBlocks = 12 * 148;
+template <bool kInv, int kBlocks>
+__global__ void __launch_bounds__(256, kBlocks) k_sn_sweep_l(DevPattern P, SnSweepPlan W, const float *__restrict__ val,
                                                     float *y, float *xo, uint32_t nrhs, uint32_t b0,
                                                     uint64_t vstride, uint64_t ystride,
                                                     const float *__restrict__ invs, uint64_t inv_stride, uint32_t *done,
@@ -760,15 +766,18 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
         const uint64_t have = std::max<uint64_t>(uint64_t(blocks) * B.count, 1);
         return uint32_t(std::min<uint64_t>(nrhs, std::max<uint64_t>(1, 4 * 148 / have)));
     };
-    const auto full = upper ? (B.sn_inv ? k_sn_sweep_u<true> : k_sn_sweep_u<false>)
-                            : (B.sn_inv ? k_sn_sweep_l<true> : k_sn_sweep_l<false>);
+    auto full = [&](uint32_t blocks) {
+        if (upper) return B.sn_inv ? k_sn_sweep_u<true> : k_sn_sweep_u<false>;
+        if (B.sn_inv) return k_sn_sweep_l<true, 2>;
+        return uint64_t(blocks) * B.count > kManyBlocks ? k_sn_sweep_l<false, 3> : k_sn_sweep_l<false, 2>;
+    };
     if (W.fused && done && W.nblocks) {
         // one launch: blocks in map order by ticket, supernodes wait for their releases
         cudaError_t e = cudaMemsetAsync(done, 0, sizeof(uint32_t) * size_t(W.ns) * B.count, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t) * B.count, st);
         if (e != cudaSuccess) return e;
         const dim3 grid(W.nblocks, 1, B.count);
-        full<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv, B.sn_inv_stride, done,
+        full(W.nblocks)<<<grid, 256, 0, st>>>(P, W, val, y, xo, nrhs, 0, B.vstride, ystride, B.sn_inv, B.sn_inv_stride, done,
                                    ticket, status, spin_limit);
     } else {
         // one launch per level (up to three where its narrow parts or its
@@ -784,7 +793,7 @@ cudaError_t run_sn_sweep(const DevPattern &P, const SnSweepPlan &W, bool upper, 
             if (k3.x) {  // the full kernel: every block that no other launch takes
                 const uint32_t nblk = k3.y ? lv.wide : rest;
                 const dim3 grid(nblk, shares(nblk), B.count);
-                e = launch_chained(full, grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride, ystride,
+                e = launch_chained(full(nblk), grid, dim3(256), 0, st, P, W, val, y, xo, nrhs, lv.b0, B.vstride, ystride,
                                    B.sn_inv, B.sn_inv_stride, (uint32_t *)nullptr, (uint32_t *)nullptr, status,
                                    spin_limit);
                 if (e != cudaSuccess) return e;
