@@ -416,11 +416,11 @@ constexpr double kSparseRate = 0.2e12, kLevelLatency = 8e-6;
 // API calls that make it, captured into a graph by the next one, and from then on
 // launched as that graph.  The sequences are dozens of launches of a few
 // microseconds each, and a launch costs the host 3-4 us, a graph about as much
-// as two launches (FP32 solve of a 251 x 251 grid, 77 launches: 293 -> 256 us;
-// n = 300 step 202 -> 170; transposed refined solve at n = 9,973 612 -> 590).
+// as two launches (FP32 solve of a 251 x 251 grid, 77 launches: 291 -> 245 us;
+// n = 300 step 225 -> 187; transposed refined solve at n = 9,973 630 -> 578).
 // Capturing and instantiating takes 100 to 400 us, what the graph then saves in
-// about kGraphCalls calls (those three: 11, 8, 8; 2 to 57 over the benchmark's
-// kinds of calls).  So a handle that is called a few times (and a one-shot
+// about kGraphCalls calls (those three: 9, 8, 4; 1 to 22 over steps, solves and
+// refactorizations of circuits and grids).  So a handle that is called a few times (and a one-shot
 // refined solve, which makes the same sweeps twice and more) pays nothing for it,
 // and no pattern of calls pays more than about twice what the launches cost.
 // enqueue(stream, slot) makes the launches and notes their statistics in the
@@ -864,8 +864,8 @@ Status build_sn_plan(glu_handle_s *h) {
     // inverses.  Those take 32 KB each and value set: kept while they are at
     // most half of the values themselves, or 64 MB.  And they take time: 10 us a
     // factorization and 0.05 us per block, which the solves earn level by level (about
-    // 5 us each of a plain solve: 251 x 251 grid 399 -> 290 with all of its
-    // steps).  Where all the wide supernodes stand in one level there is next to
+    // 2 us each of a solve: refined solve of twenty filled 300 x 300 blocks, five
+    // levels, 217 -> 171; Newton step on the 300 x 300 grid 2,993 -> 2,833).  Where all the wide supernodes stand in one level there is next to
     // nothing to earn (16 value sets of a hundred filled 40 x 40 blocks: factorization
     // 97 us without inverses and 175 with, refined solve 190 either way).
     std::vector<uint2> wide;
